@@ -266,6 +266,15 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
                      d->K, (uint32_t)log2_exact(d->group), d->out_f32 != 0, ctx->err_counter + 1, st));
     return ZTVM_OK;
   }
+  // Rows whose weights may not be rounded to f16 -- 8-bit codes, and router logits at any width -- in one launch of the
+  // exact-code batched kernel instead of one GEMV per eight rows: on 2048 x 257, 2048 rows, 3.3 ms became 13 us.
+  if (d->M > 8 && (d->bits == 8 || ctx->no_gemm)) {
+    const ztvm::GemvParams p = gemv_params(d, y, x, scales, packed_w, biases);
+    if (ztvm::batch_mma_supported(p, (int)d->bits)) {
+      ZTVM_CUDA(ztvm::launch_batch_mma(p, (int)d->bits, ctx->sm_count, st));
+      return ZTVM_OK;
+    }
+  }
   // Otherwise rows are processed in slabs of at most 8 by the GEMV.
   for (uint32_t m0 = 0; m0 < d->M; m0 += 8) {
     ztvm_mm_desc dd = *d;
@@ -515,7 +524,7 @@ ztvm_status ztvm_host_wait(ztvm_ctx* ctx) {
 
 // Which grouped kernel serves a MoE launch: 0 none (per-pair GEMV), 1 tensor-core tiles with the weights in tensor
 // memory, 2 streaming kernel, 3 tensor-core tiles with both operands in shared memory (ZTVM_MOE_TILES=sm, or shapes
-// only it takes). `forced` is the context's ZTVM_MOE_GROUPED knob (-1 = by size).
+// only it takes), 4 the exact-code batched kernel (3-bit experts). `forced` is the context's ZTVM_MOE_GROUPED knob (-1 = by size).
 static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::GemvParams& p, const void* y) {
   const int forced = ctx->moe_grouped;
   const ztvm_mm_desc* d = &md->mm;
@@ -531,6 +540,7 @@ static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::Ge
   // pair). They meet near 12.6 pairs per expert for the long-K projections and 6.6 for the short-K one; one threshold
   // for both keeps the three projections of a block on one kernel, whose plan they can then share.
   const bool few_per_expert = pairs < 10ull * md->experts;
+  if (d->bits == 3) return ztvm::batch_moe_supported(p, 3) ? 4 : 0;    // exact codes at every pair count
   if (forced == 1) return tiles ? tiles : stream_ok ? 2 : 0;
   if (forced == 2) return stream_ok ? 2 : tiles;
   return (stream_ok && (few_per_expert || !tiles)) ? 2 : tiles;
@@ -576,7 +586,7 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
   // expert's weights once (streaming kernel); with many pairs per expert it is a real contraction (tensor-core tiles,
   // each expert's weights dequantised once per 128 pairs).
   const uint64_t pairs = (uint64_t)md->tokens * md->slots;
-  const bool want_grouped = ctx->moe_grouped < 0 ? pairs >= 128 : ctx->moe_grouped >= 1;
+  const bool want_grouped = ctx->moe_grouped < 0 ? pairs >= (d->bits == 3 ? 32u : 128u) : ctx->moe_grouped >= 1;
   if (want_grouped && pairs < (1ull << 31)) {
     const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
     const int pick = moe_pick(ctx, md, p, y);
@@ -588,12 +598,13 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
         ctx->plan_ids = nullptr;
       }
       uint32_t* ws = static_cast<uint32_t*>(ctx->d_ws);
-      const uint32_t tile_rows = pick == 2 ? ztvm::kMoeTcTileRows : ztvm::kMoeTaTileRows;
+      const uint32_t tile_rows = pick == 4 ? ztvm::batch_moe_tile_rows(md->experts, pairs) : pick == 2 ? ztvm::kMoeTcTileRows : ztvm::kMoeTaTileRows;
       // gate, up and down of one step walk the same id list: with ztvm_moe_plan_reuse on, its plan is built once
       const bool reuse = ctx->plan_reuse && pick != 3 && ctx->plan_ids == ids && ctx->plan_segs == nullptr &&
                          ctx->plan_tokens == md->tokens && ctx->plan_slots == md->slots && ctx->plan_stride == md->ids_stride &&
                          ctx->plan_tile_rows == tile_rows && ctx->plan_experts == md->experts;
-      if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
+      if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe(p, md->tokens, md->slots, ws, st, reuse));
+      else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
       else if (pick == 1) ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, md->slots, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
       else ZTVM_CUDA(ztvm::launch_moe_grouped(p, md->tokens, md->slots, ws, ctx->err_counter + 1, st));
       ctx->plan_ids = pick != 3 ? ids : nullptr; ctx->plan_segs = nullptr; ctx->plan_tokens = md->tokens; ctx->plan_slots = md->slots;
@@ -647,7 +658,7 @@ ztvm_status ztvm_int4_matmul_moe_noalloc(ztvm_ctx* ctx, const ztvm_moe_desc* md,
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
   const int pick = moe_pick(ctx, md, p, y);   // the same choice ztvm_int4_matmul_moe makes
-  if (!pick)
+  if (!pick || pick == 4)
     return fail(ZTVM_ERR_UNSUPPORTED,
                 "this entry point runs the grouped kernels only: bits=4, group=64, K %% 64 == 0, N %% 8 == 0 "
                 "(got bits=%u group=%u K=%u N=%u)", d->bits, d->group, d->K, d->N);

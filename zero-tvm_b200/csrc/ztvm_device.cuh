@@ -47,6 +47,7 @@ __device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t mask, uint3
   return r;
 }
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t h2_as_u32(const __half2& h) { return *reinterpret_cast<const uint32_t*>(&h); }
 
 __device__ __forceinline__ Codes8 unpack4(uint32_t w) {
   const __half2 k1024 = u32_as_h2(0x64006400u), k64 = u32_as_h2(0x54005400u);
@@ -97,6 +98,10 @@ __device__ __forceinline__ void codes8_f32(uint32_t w0, uint32_t w1, float q[8])
   }
 }
 
+// In place for the matrix unit: bytes 0, 2 and bytes 1, 3 of a word as pairs of f16 subnormals q * 2^-24.
+__device__ __forceinline__ uint32_t codes8_inplace_even(uint32_t w) { return w & 0x00FF00FFu; }
+__device__ __forceinline__ uint32_t codes8_inplace_odd(uint32_t w) { return (w >> 8) & 0x00FF00FFu; }
+
 // ---- 3-bit codes ---------------------------------------------------------------------------
 // A row is one LSB-first bitstream; 32 codes occupy exactly three words. Codes 8b..8b+7 of such a
 // triple are the 24-bit window starting at bit 24b.
@@ -133,6 +138,19 @@ __device__ __forceinline__ void codes3_inplace(const uint32_t (&w)[6], int k, ui
   else v = __funnelshift_r(w[j], w[j + 1 < 6 ? j + 1 : 5], sh);
   r0 = v & (k < 15 ? kM0 : (kM0 & 0xFFFFu));
   r1 = v & (k < 15 ? kM1 : (kM1 & 0xFFFFu));
+}
+
+// Sixteen consecutive codes (48 bits: f0 = the first 32, the low half of f1 = the rest) as eight registers of code pairs
+// (i | i + 8): r[i / 2] for even i holds fields at bits 0..2 of each half (q * 2^-24), r[4 + i / 2] holds codes
+// (i + 1 | i + 9) at bits 3..5 (q * 2^-21). Both halves of a register carry the same power of two, so the activations
+// go in unscaled. Bits of a neighbouring half that a shift drags along land above bit 5 and are masked off.
+__device__ __forceinline__ void codes3_inplace16(uint32_t f0, uint32_t f1, uint32_t (&r)[8]) {
+  const uint32_t fh = __funnelshift_r(f0, f1, 24);            // codes 8..15 from bit 0
+  const uint32_t p0 = __byte_perm(f0, fh, 0x5410);            // bits 0..15 of both runs of eight codes
+  const uint32_t p1 = __byte_perm(f0, fh, 0x6521);            // bits 8..23
+  const uint32_t v[4] = {p0, p0 >> 6, p1 >> 4, p1 >> 10};     // codes 0,1 | 2,3 | 4,5 | 6,7 (and + 8) at bits 0, 3
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { r[i] = v[i] & 0x00070007u; r[4 + i] = v[i] & 0x00380038u; }
 }
 
 // ---- canonical dequantisers ----------------------------------------------------------------

@@ -56,6 +56,15 @@ cudaError_t launch_gemv_tc(const GemvParams& p, int sm_count, cudaStream_t st);
 bool gemv_tc3_supported(const GemvParams& p, int bits, int sm_count);
 cudaError_t launch_gemv_tc3(const GemvParams& p, int sm_count, cudaStream_t st);
 
+// 8-bit / 4-bit affine group-64 weights, any number of rows, exact codes and f32 weights on the warp matrix unit
+// (ztvm_batch_mma.cu).
+bool batch_mma_supported(const GemvParams& p, int bits);
+cudaError_t launch_batch_mma(const GemvParams& p, int bits, int sm_count, cudaStream_t st);
+// The grouped form for 3-bit experts: pairs sorted by expert, tiles of batch_moe_tile_rows pairs.
+bool batch_moe_supported(const GemvParams& g, int bits);
+uint32_t batch_moe_tile_rows(uint32_t experts, uint64_t pairs);
+cudaError_t launch_batch_moe(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan);
+
 // 4-bit weights, M > 8: tcgen05 GEMM with TMEM accumulators (ztvm_gemm.cu). status[0] receives a non-zero code
 // if a pipeline wait inside the kernel ran out.
 bool gemm_w4_supported(int bits, uint32_t group, uint32_t K);

@@ -183,8 +183,6 @@ __device__ __forceinline__ DqGroup dq_group(unsigned short s16, unsigned short b
   return g;
 }
 
-__device__ __forceinline__ uint32_t h2_as_u32(const __half2& h) { return *reinterpret_cast<const uint32_t*>(&h); }
-
 // Dequantise one 8-code word into 8 f16 weights in natural order (as one uint4).
 template <bool AFFINE>
 __device__ __forceinline__ uint4 dequant_word_w16(uint32_t w, const DqGroup& g) {
