@@ -112,7 +112,7 @@ bool use_mma(const ztvm_ctx* ctx, const ztvm_mm_desc* d, uint32_t m) {
   return ctx->gemv_path == 2 || ((ctx->gemv_path == 0 || ctx->gemv_path == 3) && m > 1);
 }
 
-ztvm::GemvParams gemv_params(const ztvm_mm_desc* d, void* y, const void* x, const void* s, const void* w,
+ztvm::GemvParams gemv_params(const ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, const void* x, const void* s, const void* w,
                              const void* b) {
   ztvm::GemvParams p;
   memset(&p, 0, sizeof(p));
@@ -128,6 +128,7 @@ ztvm::GemvParams gemv_params(const ztvm_mm_desc* d, void* y, const void* x, cons
   p.out_f32 = d->out_f32 ? 1u : 0u;
   p.x_row_stride = d->K;
   p.y_row_stride = d->N;
+  p.err_counter = ctx->err_counter;
   return p;
 }
 
@@ -269,7 +270,7 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
   // Rows whose weights may not be rounded to f16 -- 8-bit codes, and router logits at any width -- in one launch of the
   // exact-code batched kernel instead of one GEMV per eight rows: on 2048 x 257, 2048 rows, 3.3 ms became 13 us.
   if (d->M > 8 && (d->bits == 8 || ctx->no_gemm)) {
-    const ztvm::GemvParams p = gemv_params(d, y, x, scales, packed_w, biases);
+    const ztvm::GemvParams p = gemv_params(ctx, d, y, x, scales, packed_w, biases);
     if (ztvm::batch_mma_supported(p, (int)d->bits)) {
       ZTVM_CUDA(ztvm::launch_batch_mma(p, (int)d->bits, ctx->sm_count, st));
       return ZTVM_OK;
@@ -279,12 +280,12 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
   for (uint32_t m0 = 0; m0 < d->M; m0 += 8) {
     ztvm_mm_desc dd = *d;
     dd.M = d->M - m0 < 8 ? d->M - m0 : 8;
-    ztvm::GemvParams p = gemv_params(&dd, y, x, scales, packed_w, biases);
+    ztvm::GemvParams p = gemv_params(ctx, &dd, y, x, scales, packed_w, biases);
     p.X = static_cast<const __half*>(x) + (size_t)m0 * d->K;
     p.Y = d->out_f32 ? static_cast<void*>(static_cast<float*>(y) + (size_t)m0 * d->N)
                      : static_cast<void*>(static_cast<__half*>(y) + (size_t)m0 * d->N);
     const bool want_tc = ctx->gemv_path == 0 || (ctx->gemv_path == 3 && dd.M > 1);
-    if (want_tc && ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc(p, ctx->sm_count, st));
+    if (want_tc && ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st));
     else if (want_tc && ztvm::gemv_tc3_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc3(p, ctx->sm_count, st));
     else if (use_mma(ctx, d, dd.M)) ZTVM_CUDA(ztvm::launch_gemv_mma(p, false, 1, 1, st));
     else ZTVM_CUDA(ztvm::launch_gemv(p, (int)d->bits, false, 1, 1, ctx->sm_count, st));
@@ -373,11 +374,11 @@ ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* h, const 
   if ((s = check_buffers(&gu, h, x, scales, packed_w, biases))) return s;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   if (d->M <= 8 && ctx->gemv_path == 0) {
-    ztvm::GemvParams p = gemv_params(&gu, h, x, scales, packed_w, biases);
+    ztvm::GemvParams p = gemv_params(ctx, &gu, h, x, scales, packed_w, biases);
     p.pair_rows = d->N;
     p.y_row_stride = d->N;
     if (ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) {
-      ZTVM_CUDA(ztvm::launch_gemv_tc(p, ctx->sm_count, st));
+      ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st));
       return ZTVM_OK;
     }
   }
@@ -450,15 +451,15 @@ ztvm_status ztvm_int4_matmul_multi(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* c
   if (d->M > 8) return fail(ZTVM_ERR_UNSUPPORTED, "the multi-destination form is the decode GEMV: M=%u exceeds 8", d->M);
   if (y_row_stride < d->N) return fail(ZTVM_ERR_BAD_DIMS, "y_row_stride=%u < N=%u", y_row_stride, d->N);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  ztvm::GemvParams p = gemv_params(d, y_dsts[0], x, scales, packed_w, biases);
+  ztvm::GemvParams p = gemv_params(ctx, d, y_dsts[0], x, scales, packed_w, biases);
   p.y_row_stride = y_row_stride;
   p.n_more = n_dst - 1;
   for (uint32_t i = 1; i < n_dst; ++i) p.y_more[i - 1] = y_dsts[i];
-  if (!ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count))
+  if (d->bits != 4 || d->group != 64 || d->K % 256 || !ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count))
     return fail(ZTVM_ERR_UNSUPPORTED,
                 "the multi-destination form runs the persistent GEMV only: bits=4, group=64, K %% 256 == 0, 16-byte aligned "
                 "x and weights (got bits=%u group=%u K=%u)", d->bits, d->group, d->K);
-  ZTVM_CUDA(ztvm::launch_gemv_tc(p, ctx->sm_count, st));
+  ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st));
   return ZTVM_OK;
 }
 
@@ -550,7 +551,7 @@ static ztvm::GemvParams moe_params(ztvm_ctx* ctx, const ztvm_moe_desc* md, void*
                                    const void* packed_w, const void* biases, const uint32_t* ids) {
   ztvm_mm_desc dd = md->mm;
   dd.M = 1;
-  ztvm::GemvParams p = gemv_params(&dd, y, x, scales, packed_w, biases);
+  ztvm::GemvParams p = gemv_params(ctx, &dd, y, x, scales, packed_w, biases);
   p.ids = ids;
   p.experts = md->experts;
   p.in_slot_stride = md->in_slot_stride; p.out_slot_stride = md->out_slot_stride;
@@ -615,7 +616,7 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
   // grid.y carries the token: split very long token lists into slabs of 65535
   for (uint32_t t0 = 0; t0 < md->tokens; t0 += 65535) {
     const uint32_t nt = md->tokens - t0 < 65535 ? md->tokens - t0 : 65535;
-    ztvm::GemvParams p = gemv_params(&dd, y, x, scales, packed_w, biases);
+    ztvm::GemvParams p = gemv_params(ctx, &dd, y, x, scales, packed_w, biases);
     p.X = static_cast<const __half*>(x) + (size_t)t0 * md->in_tok_stride;
     p.Y = static_cast<__half*>(y) + (size_t)t0 * md->out_tok_stride;
     p.ids = ids + (size_t)t0 * md->ids_stride;

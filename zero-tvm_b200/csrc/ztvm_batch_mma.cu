@@ -224,7 +224,7 @@ batch_mma_kernel(const BatchParams p) {
           uint32_t pos = run;
           if constexpr (BITS == 4) pos = run ^ (RUNS == 2 ? (row >> 1) & 1u : row & 3u);
           if constexpr (BITS == 8) pos = run ^ (row & 1u);
-          F::a(F::load(wbase + row * C::kRowBytes + pos * F::kRunBytes, c), a[t][h]);
+          F::a(F::load(bm_smem + (wbase - sm) + row * C::kRowBytes + pos * F::kRunBytes + F::lane_byte(c), c), a[t][h]);
         }
 #pragma unroll
       for (int j = 0; j < NBW; ++j) {

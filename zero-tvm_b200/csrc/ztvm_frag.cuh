@@ -24,11 +24,9 @@ struct Frag<4> {
   static constexpr bool kTwoClasses = true;
   static constexpr float kUnit = 1048576.f, kRatio = 16.f;
   struct Raw { uint2 w; };
-  __device__ __forceinline__ static Raw load(uint32_t run_addr, int c) {
-    Raw r;
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(r.w.x), "=r"(r.w.y) : "r"(run_addr + 8u * (uint32_t)c));
-    return r;
-  }
+  // `p`: the lane's first byte of the run in shared memory
+  __device__ __forceinline__ static Raw load(const uint8_t* p, int) { return Raw{*reinterpret_cast<const uint2*>(p)}; }
+  __host__ __device__ static constexpr uint32_t lane_byte(int c) { return 8u * (uint32_t)c; }
   __device__ __forceinline__ static void a(const Raw& v, uint32_t (&r)[8]) {
     const Inplace4 p = codes4_inplace(v.w.x), q = codes4_inplace(v.w.y);
     r[0] = p.lo04; r[1] = p.lo26; r[2] = q.lo04; r[3] = q.lo26;
@@ -48,12 +46,8 @@ struct Frag<8> {
   static constexpr bool kTwoClasses = false;
   static constexpr float kUnit = 16777216.f, kRatio = 0.f;
   struct Raw { uint4 w; };
-  __device__ __forceinline__ static Raw load(uint32_t run_addr, int c) {
-    Raw r;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.w.x), "=r"(r.w.y), "=r"(r.w.z), "=r"(r.w.w)
-                 : "r"(run_addr + 16u * (uint32_t)c));
-    return r;
-  }
+  __device__ __forceinline__ static Raw load(const uint8_t* p, int) { return Raw{*reinterpret_cast<const uint4*>(p)}; }
+  __host__ __device__ static constexpr uint32_t lane_byte(int c) { return 16u * (uint32_t)c; }
   __device__ __forceinline__ static void a(const Raw& v, uint32_t (&r)[8]) {
     const uint32_t w[4] = {v.w.x, v.w.y, v.w.z, v.w.w};
 #pragma unroll
@@ -73,16 +67,11 @@ struct Frag<3> {
   static constexpr bool kTwoClasses = true;
   static constexpr float kUnit = 2097152.f, kRatio = 8.f;
   struct Raw { uint32_t f0, f1; };   // the lane's 48 bits (f1: 16 valid bits, rubbish above)
-  __device__ __forceinline__ static Raw load(uint32_t run_addr, int c) {
-    // byte 6c of the run: words 0,1 | 1,2 | 3,4 | 4,5; odd lanes start in the middle of their first word
-    const uint32_t a = run_addr + ((6u * (uint32_t)c) & ~3u), sh = ((uint32_t)c & 1u) << 4;
-    uint32_t w0, w1;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(a));
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w1) : "r"(a + 4u));
-    Raw r;
-    r.f0 = __funnelshift_r(w0, w1, sh);
-    r.f1 = w1 >> sh;
-    return r;
+  // byte 6c of the run: words 0,1 | 1,2 | 3,4 | 4,5; odd lanes start in the middle of their first word
+  __host__ __device__ static constexpr uint32_t lane_byte(int c) { return (6u * (uint32_t)c) & ~3u; }
+  __device__ __forceinline__ static Raw load(const uint8_t* p, int c) {
+    const uint32_t w0 = *reinterpret_cast<const uint32_t*>(p), w1 = *reinterpret_cast<const uint32_t*>(p + 4), sh = ((uint32_t)c & 1u) << 4;
+    return Raw{__funnelshift_r(w0, w1, sh), w1 >> sh};
   }
   __device__ __forceinline__ static void a(const Raw& v, uint32_t (&r)[8]) { codes3_inplace16(v.f0, v.f1, r); }
   __device__ __forceinline__ static void b(const uint4& x0, const uint4& x1, uint32_t (&r)[8]) {

@@ -82,9 +82,9 @@ __global__ void dequant_kernel(const uint32_t* W, const __half* S, const __half*
   }
 }
 
-// The codes as the streaming kernels see them: in-place masks that are f16 subnormals (codes4_inplace / codes3_inplace,
+// The codes as the streaming kernels see them: in-place masks that are f16 subnormals (codes4_inplace / codes3_inplace / codes3_inplace16,
 // the functions those kernels call), scaled back to integers. 4-bit: one thread per word. 3-bit: one thread per
-// (row, scale group of 64 codes = six words), the unit a lane of the 3-bit GEMV owns.
+// (row, scale group of 64 codes = six words), the run a quad of the 3-bit kernels owns.
 __device__ __forceinline__ uint32_t sub_to_code(uint32_t halfbits, float scale) {
   return (uint32_t)(__half2float(__ushort_as_half((unsigned short)halfbits)) * scale);
 }
@@ -114,6 +114,8 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
 #pragma unroll
       for (int j = 0; j < 6; ++j) w[j] = W[(size_t)n * KP + g * 6 + j];
       uint8_t* dst = codes + (size_t)n * K + (size_t)g * 64;
+      // Both in-place views of the stream: the single-row GEMV's 17 windows, and the quad fragments of the batched kernel
+      // (lane q: codes 16 q .. 16 q + 15, the 48 bits from byte 6 q). A code they disagree on comes out as 255.
 #pragma unroll
       for (int k = 0; k < kCodes3Views; ++k) {
         uint32_t r0, r1;
@@ -125,6 +127,22 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
           dst[c0 + 6] = (uint8_t)sub_to_code(r0 >> 16, 4194304.f);           // offset 2: q * 2^-22
           dst[c0 + 7] = (uint8_t)sub_to_code(r1 >> 16, 524288.f);            // offset 5: q * 2^-19
         }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = 3 * q / 2, sh = (q & 1) * 16;
+        uint32_t r[8];
+        codes3_inplace16(__funnelshift_r(w[j], w[j + 1], sh), w[j + 1] >> sh, r);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c0 = 16 * q + 2 * i + 8 * h;
+            const uint32_t even = sub_to_code(h ? r[i] >> 16 : r[i] & 0xFFFFu, 16777216.f);          // offset 0: q * 2^-24
+            const uint32_t odd = sub_to_code(h ? r[4 + i] >> 16 : r[4 + i] & 0xFFFFu, 2097152.f);    // offset 3: q * 2^-21
+            if (dst[c0] != even) dst[c0] = 255;
+            if (dst[c0 + 1] != odd) dst[c0 + 1] = 255;
+          }
       }
     }
   }

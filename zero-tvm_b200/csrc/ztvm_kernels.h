@@ -18,7 +18,7 @@ struct GemvParams {
   uint32_t group_shift;  // log2(group)
   uint32_t out_f32;
   uint32_t x_row_stride, y_row_stride;  // elements between batch rows
-  uint32_t tile_units;                  // set by the launcher
+  uint32_t tile_units;                  // set by the launcher: K extent staged at a time, in the kernel's unit
   // MoE indirection (int4_matmul.gen.ts:216-225)
   const uint32_t* ids;
   uint32_t experts, in_slot_stride, out_slot_stride, in_tok_stride, out_tok_stride, ids_stride;
@@ -47,10 +47,10 @@ cudaError_t launch_gemv(GemvParams p, int bits, bool moe, uint32_t tokens, uint3
 bool gemv_mma_supported(int bits, uint32_t group);
 cudaError_t launch_gemv_mma(GemvParams p, bool moe, uint32_t tokens, uint32_t slots, cudaStream_t st);
 
-// 4-bit / group-64 weights, M <= 8, persistent matrix-unit GEMV (ztvm_gemv_tc.cu). `gemv_tc_supported` checks shape
-// and alignment; anything it refuses goes to the kernels above.
+// Persistent matrix-unit GEMV, M <= 8: 4-bit groups of 64 / 32 and 8-bit groups of 64 (ztvm_gemv_tc.cuh).
+// `gemv_tc_supported` checks shape and alignment; anything it refuses goes to the kernels above.
 bool gemv_tc_supported(const GemvParams& p, int bits, int sm_count);
-cudaError_t launch_gemv_tc(const GemvParams& p, int sm_count, cudaStream_t st);
+cudaError_t launch_gemv_tc(const GemvParams& p, int bits, int sm_count, cudaStream_t st);
 
 // 3-bit / group-64 weights, M = 1, persistent matrix-unit GEMV (ztvm_gemv_tc3.cu).
 bool gemv_tc3_supported(const GemvParams& p, int bits, int sm_count);

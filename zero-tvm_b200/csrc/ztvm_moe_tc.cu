@@ -2,7 +2,7 @@
 //   y[token, slot, :] = x[token, slot, :] * W[ids[token, slot]]^T        (int4_matmul.gen.ts:229-254)
 // for token counts where an expert sees a handful of pairs (a few hundred tokens over 256 experts). There the job
 // is bound by reading every active expert's weights once, not by the multiplies, so it is built like the
-// persistent decode GEMV (ztvm_gemv_tc.cu) rather than like the tensor-core tiles of ztvm_moe_gemm.cu:
+// persistent decode GEMV (ztvm_gemv_tc.cuh) rather than like the tensor-core tiles of ztvm_moe_gemm.cu:
 //   * the plan (ztvm_moe_plan.cuh) sorts the pairs by expert and cuts each expert's list into chunks of <= 8 pairs:
 //     a chunk is the 8 columns of an mma.sync.m16n8k16;
 //   * work unit = (chunk, 16 weight rows). The units, in chunk-major order, are split evenly over one CTA per SM;

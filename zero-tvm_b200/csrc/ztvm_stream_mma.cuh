@@ -1,4 +1,4 @@
-// Pieces shared by the streaming matrix-unit kernels (ztvm_gemv_tc.cu, ztvm_moe_tc.cu): the per-warp cp.async ring
+// Pieces shared by the streaming matrix-unit kernels (ztvm_gemv_tc.cuh, ztvm_moe_tc.cu, ztvm_batch_mma.cu): the per-warp cp.async ring
 // geometry and the inline-PTX wrappers (mma.sync, cp.async, shared loads, two-wide f32 FMA).
 #pragma once
 #include "ztvm_device.cuh"
