@@ -14,6 +14,7 @@ only matters for the MoE kernels, where y is the token count and z the slot coun
 """
 from __future__ import annotations
 
+import functools
 import re
 from dataclasses import dataclass
 from typing import Optional, Sequence
@@ -102,6 +103,7 @@ class EntryInfo:
     fixed_m: Optional[int]  # batched_m4
 
 
+@functools.lru_cache(maxsize=256)
 def parse_entry(entry: str) -> EntryInfo:
     """Decodes what an entry name fixes. Unknown names raise KeyError, as a missing pipeline does."""
     if entry == "int4_matmul_batched_m4":
@@ -234,6 +236,31 @@ def pick_chunk_gemm(requested: Optional[str], *, affine: bool, K: int, cap: int 
 
 
 # ---- the dispatch surface ---------------------------------------------------------------------------
+@functools.lru_cache(maxsize=4096)
+def _decode_matmul(entry: str, pod: Sequence):
+    """(affine, moe, descriptor) of an entry name and its PODArgs; MoE: (mm, strides, K_PACKED), the rest is per call.
+    Decoding costs more than the launch (a dispatch took 8 us without the cache), and a call site passes the same name and
+    PODArgs for ever."""
+    info = parse_entry(entry)
+    k_packed, spr, n = int(pod[0]), int(pod[1]), int(pod[2])
+    if k_packed <= 0 or spr <= 0 or (k_packed * 32) % info.bits:
+        raise ValueError(f"{entry}: bad PODArgs {list(pod)}")
+    K = k_packed * 32 // info.bits
+    group = K // spr
+    if info.moe:
+        desc = None if len(pod) < 8 else (MmDesc(K, n, 1, group, info.bits, 1, 0), tuple(int(v) for v in pod[3:8]), k_packed)
+        return info.affine, True, desc
+    if info.fixed_m is not None:
+        M = info.fixed_m
+    elif info.has_m_rows:
+        if len(pod) < 4:
+            raise ValueError(f"{entry}: runtime-M kernels read M_ROWS from PODArgs[3]")
+        M = int(pod[3])
+    else:
+        M = 1
+    return info.affine, False, None if M == 0 else MmDesc(K, n, M, group, info.bits, int(info.affine), int(info.out_f32))
+
+
 class CudaMatmulBackend:
     """Drop-in for the matmul entries of compile() + dispatch(): one object per GPU."""
 
@@ -250,40 +277,29 @@ class CudaMatmulBackend:
         stream=None launches on the context's own stream, which is non-blocking: work queued on another stream (a
         tensor library's fills and copies, say) is NOT ordered against it. Pass that library's stream (a handle, a
         torch.cuda.Stream, or 1 for the legacy default stream), or synchronise both sides around the call."""
-        info = parse_entry(entry)
         if len(bindings) < 5:
+            parse_entry(entry)
             raise ValueError("bind group needs [out, in, scales, weights, PODArgs, ...]")
         out, x, scales, weights, pod = bindings[:5]
+        try:
+            known = _decode_matmul(entry, tuple(pod))
+        except TypeError:                        # PODArgs that do not hash
+            known = _decode_matmul.__wrapped__(entry, pod)
+        affine, moe, desc = known
         biases = bindings[5] if len(bindings) > 5 else None
-        ids = bindings[6] if len(bindings) > 6 else None
-        if info.affine and biases is None:
+        if affine and biases is None:
             raise ValueError(f"{entry}: affine variants bind biases at slot 5")
-        k_packed, spr, n = int(pod[0]), int(pod[1]), int(pod[2])
-        if k_packed <= 0 or spr <= 0 or (k_packed * 32) % info.bits:
-            raise ValueError(f"{entry}: bad PODArgs {list(pod)}")
-        K = k_packed * 32 // info.bits
-        group = K // spr
-        if info.moe:
-            if len(pod) < 8 or ids is None:
-                raise ValueError(f"{entry}: MoE variants need 8 PODArgs fields and ids at slot 6")
-            gx, gy, gz = (list(grid) + [1, 1, 1])[:3]
-            desc = MoeDesc(MmDesc(K, n, 1, group, info.bits, 1, 0), 0, gz, gy, int(pod[3]), int(pod[4]),
-                           int(pod[5]), int(pod[6]), int(pod[7]))
-            desc.experts = self._experts_of(weights, n, k_packed)
-            self.ctx.int4_matmul_moe(desc, out, x, scales, weights, biases, ids, stream)
+        if not moe:
+            if desc is not None:                 # None: M_ROWS = 0
+                self.ctx.int4_matmul(desc, out, x, scales, weights, biases if affine else None, stream)
             return
-        if info.fixed_m is not None:
-            M = info.fixed_m
-        elif info.has_m_rows:
-            if len(pod) < 4:
-                raise ValueError(f"{entry}: runtime-M kernels read M_ROWS from PODArgs[3]")
-            M = int(pod[3])
-            if M == 0:
-                return
-        else:
-            M = 1
-        desc = MmDesc(K, n, M, group, info.bits, int(info.affine), int(info.out_f32))
-        self.ctx.int4_matmul(desc, out, x, scales, weights, biases if info.affine else None, stream)
+        ids = bindings[6] if len(bindings) > 6 else None
+        if desc is None or ids is None:
+            raise ValueError(f"{entry}: MoE variants need 8 PODArgs fields and ids at slot 6")
+        mm, strides, k_packed = desc
+        _gx, gy, gz = (list(grid) + [1, 1, 1])[:3]
+        self.ctx.int4_matmul_moe(MoeDesc(mm, self._experts_of(weights, mm.N, k_packed), gz, gy, *strides), out, x, scales, weights,
+                                 biases, ids, stream)
 
     @staticmethod
     def _experts_of(weights, n: int, k_packed: int) -> int:

@@ -131,6 +131,15 @@ def ptr(buf):
     raise TypeError(f"cannot take the address of {type(buf)!r}")
 
 
+def addr(buf):
+    """`ptr` as a plain int (what ctypes converts fastest): the call path of the launching entry points."""
+    try:
+        return buf.data_ptr()
+    except AttributeError:
+        p = ptr(buf)
+        return None if p is None else p.value
+
+
 def stream_ptr(stream):
     if stream is None:
         return None
@@ -152,6 +161,7 @@ class Context:
         h = C.c_void_p()
         check(self._lib.ztvm_init(device, C.byref(h)))
         self.handle = h
+        self._matmul = self._lib.ztvm_int4_matmul
         self.device = device
 
     def close(self):
@@ -170,65 +180,67 @@ class Context:
 
     # -- entry points, thin and literal --------------------------------------------------------
     def int4_matmul(self, desc: MmDesc, y, x, scales, packed_w, biases=None, stream=None):
-        check(self._lib.ztvm_int4_matmul(self.handle, C.byref(desc), ptr(y), ptr(x), ptr(scales), ptr(packed_w),
-                                         ptr(biases), stream_ptr(stream)))
+        st = self._matmul(self.handle, C.byref(desc), addr(y), addr(x), addr(scales), addr(packed_w),
+                          None if biases is None else addr(biases), None if stream is None else stream_ptr(stream))
+        if st:
+            check(st)
 
     def int4_matmul_host_async(self, desc: MmDesc, y_host, x_host, scales, packed_w, biases=None):
         """Queued form of int4_matmul_host (page-locked buffers, three lanes round robin); host_wait() completes them."""
-        check(self._lib.ztvm_int4_matmul_host_async(self.handle, C.byref(desc), ptr(y_host), ptr(x_host), ptr(scales),
-                                                    ptr(packed_w), ptr(biases)))
+        check(self._lib.ztvm_int4_matmul_host_async(self.handle, C.byref(desc), addr(y_host), addr(x_host), addr(scales),
+                                                    addr(packed_w), addr(biases)))
 
     def host_wait(self):
         check(self._lib.ztvm_host_wait(self.handle))
 
     def int4_matmul_host(self, desc: MmDesc, y_host, x_host, scales, packed_w, biases=None):
-        check(self._lib.ztvm_int4_matmul_host(self.handle, C.byref(desc), ptr(y_host), ptr(x_host), ptr(scales),
-                                              ptr(packed_w), ptr(biases)))
+        check(self._lib.ztvm_int4_matmul_host(self.handle, C.byref(desc), addr(y_host), addr(x_host), addr(scales),
+                                              addr(packed_w), addr(biases)))
 
     def int4_matmul_multi(self, desc: MmDesc, y_dsts, y_row_stride, x, scales, packed_w, biases=None, stream=None):
         """Decode matmul whose result goes to every address in `y_dsts` (ints or tensors; peers' buffers included)."""
         addrs = [d if isinstance(d, int) else d.data_ptr() for d in y_dsts]
         arr = (C.c_void_p * len(addrs))(*addrs)
-        check(self._lib.ztvm_int4_matmul_multi(self.handle, C.byref(desc), arr, len(addrs), y_row_stride, ptr(x),
-                                               ptr(scales), ptr(packed_w), ptr(biases), stream_ptr(stream)))
+        check(self._lib.ztvm_int4_matmul_multi(self.handle, C.byref(desc), arr, len(addrs), y_row_stride, addr(x),
+                                               addr(scales), addr(packed_w), addr(biases), stream_ptr(stream)))
 
     def int4_matmul_moe(self, desc: MoeDesc, y, x, scales, packed_w, biases, ids, stream=None):
-        check(self._lib.ztvm_int4_matmul_moe(self.handle, C.byref(desc), ptr(y), ptr(x), ptr(scales),
-                                             ptr(packed_w), ptr(biases), ptr(ids), stream_ptr(stream)))
+        check(self._lib.ztvm_int4_matmul_moe(self.handle, C.byref(desc), addr(y), addr(x), addr(scales),
+                                             addr(packed_w), addr(biases), addr(ids), stream_ptr(stream)))
 
     def int4_matmul_moe_noalloc(self, desc: MoeDesc, y, x, scales, packed_w, biases, ids, stream=None):
         """The grouped MoE matmul with its plan in a fixed device array (no allocation; limits in the header)."""
-        check(self._lib.ztvm_int4_matmul_moe_noalloc(self.handle, C.byref(desc), ptr(y), ptr(x), ptr(scales),
-                                                     ptr(packed_w), ptr(biases), ptr(ids), stream_ptr(stream)))
+        check(self._lib.ztvm_int4_matmul_moe_noalloc(self.handle, C.byref(desc), addr(y), addr(x), addr(scales),
+                                                     addr(packed_w), addr(biases), addr(ids), stream_ptr(stream)))
 
     def moe_router_logits(self, D, rows, tokens, bits, logits, x, w, scales=None, biases=None, stream=None):
-        check(self._lib.ztvm_moe_router_logits(self.handle, D, rows, tokens, bits, ptr(logits), ptr(x), ptr(w), ptr(scales),
-                                               ptr(biases), stream_ptr(stream)))
+        check(self._lib.ztvm_moe_router_logits(self.handle, D, rows, tokens, bits, addr(logits), addr(x), addr(w), addr(scales),
+                                               addr(biases), stream_ptr(stream)))
 
     def embedding_affine(self, D, bits, vocab, seq_len, out, input_ids, scales, weights, biases, stream=None):
-        check(self._lib.ztvm_embedding_affine(self.handle, D, bits, vocab, seq_len, ptr(out), ptr(input_ids), ptr(scales),
-                                              ptr(weights), ptr(biases), stream_ptr(stream)))
+        check(self._lib.ztvm_embedding_affine(self.handle, D, bits, vocab, seq_len, addr(out), addr(input_ids), addr(scales),
+                                              addr(weights), addr(biases), stream_ptr(stream)))
 
     def moe_plan_reuse(self, enable: bool):
         """Consecutive int4_matmul_moe calls over one id list share its expert-sorted plan (see the header's contract)."""
         check(self._lib.ztvm_moe_plan_reuse(self.handle, int(enable)))
 
     def moe_route_topk(self, E, K, norm_topk, has_shared, tokens, ids, scores, logits, stream=None):
-        check(self._lib.ztvm_moe_route_topk(self.handle, E, K, int(norm_topk), int(has_shared), tokens, ptr(ids),
-                                            ptr(scores), ptr(logits), stream_ptr(stream)))
+        check(self._lib.ztvm_moe_route_topk(self.handle, E, K, int(norm_topk), int(has_shared), tokens, addr(ids),
+                                            addr(scores), addr(logits), stream_ptr(stream)))
 
     def moe_dispatch_plan(self, ids, tokens, slots, ids_stride, experts, experts_per_rank, world, order, local_expert,
                           send_counts, stream=None):
-        check(self._lib.ztvm_moe_dispatch_plan(self.handle, ptr(ids), tokens, slots, ids_stride, experts, experts_per_rank,
-                                               world, ptr(order), ptr(local_expert), ptr(send_counts), stream_ptr(stream)))
+        check(self._lib.ztvm_moe_dispatch_plan(self.handle, addr(ids), tokens, slots, ids_stride, experts, experts_per_rank,
+                                               world, addr(order), addr(local_expert), addr(send_counts), stream_ptr(stream)))
 
     def moe_ep_dispatch(self, layout: MoeEpLayout, ids, tokens, top_k, has_shared, ids_stride, x, d, x_tok_stride, stream=None):
-        check(self._lib.ztvm_moe_ep_dispatch(self.handle, C.byref(layout), ptr(ids), tokens, top_k, int(has_shared), ids_stride,
-                                             ptr(x), d, x_tok_stride, stream_ptr(stream)))
+        check(self._lib.ztvm_moe_ep_dispatch(self.handle, C.byref(layout), addr(ids), tokens, top_k, int(has_shared), ids_stride,
+                                             addr(x), d, x_tok_stride, stream_ptr(stream)))
 
     def int4_matmul_moe_ep(self, desc: MoeDesc, rows: MoeEpRows, y, x, scales, packed_w, biases, ids, stream=None):
-        check(self._lib.ztvm_int4_matmul_moe_ep(self.handle, C.byref(desc), C.byref(rows), ptr(y), ptr(x), ptr(scales),
-                                                ptr(packed_w), ptr(biases), ptr(ids), stream_ptr(stream)))
+        check(self._lib.ztvm_int4_matmul_moe_ep(self.handle, C.byref(desc), C.byref(rows), addr(y), addr(x), addr(scales),
+                                                addr(packed_w), addr(biases), addr(ids), stream_ptr(stream)))
 
     def peer_barrier(self, flags, world, rank, stream=None):
         """flags: every rank's flag-array address as mapped in this process (ints)."""
@@ -239,37 +251,37 @@ class Context:
         """ztvm_int4_matmul_multi + ztvm_peer_barrier: y_dsts / flags are every rank's addresses as mapped here (ints)."""
         ya = (C.c_void_p * 8)(*[int(v) for v in y_dsts])
         fa = (C.c_void_p * 8)(*[int(v) for v in flags])
-        check(self._lib.ztvm_int4_matmul_nshard(self.handle, C.byref(desc), ya, world, rank, y_row_stride, ptr(x), ptr(scales),
-                                                ptr(packed_w), ptr(biases), fa, stream_ptr(stream)))
+        check(self._lib.ztvm_int4_matmul_nshard(self.handle, C.byref(desc), ya, world, rank, y_row_stride, addr(x), addr(scales),
+                                                addr(packed_w), addr(biases), fa, stream_ptr(stream)))
 
     def moe_ffn_ep(self, args: "MoeFfnEpArgs", stream=None):
         check(self._lib.ztvm_moe_ffn_ep(self.handle, C.byref(args), stream_ptr(stream)))
 
     def silu_mul_rows(self, rows: MoeEpRows, ffn, h, gate_up, stream=None):
-        check(self._lib.ztvm_silu_mul_rows(self.handle, C.byref(rows), ffn, ptr(h), ptr(gate_up), stream_ptr(stream)))
+        check(self._lib.ztvm_silu_mul_rows(self.handle, C.byref(rows), ffn, addr(h), addr(gate_up), stream_ptr(stream)))
 
     def fused_ffn(self, desc: MmDesc, h, x, scales, packed_w, biases=None, stream=None):
         """h = f16(up * silu(gate)) for the [2 * desc.N, K] stack of gate and up rows (desc.N = ffn)."""
-        check(self._lib.ztvm_fused_ffn(self.handle, C.byref(desc), ptr(h), ptr(x), ptr(scales), ptr(packed_w), ptr(biases),
+        check(self._lib.ztvm_fused_ffn(self.handle, C.byref(desc), addr(h), addr(x), addr(scales), addr(packed_w), addr(biases),
                                        stream_ptr(stream)))
 
     def silu_mul(self, rows, ffn, h, gate_up, stream=None):
-        check(self._lib.ztvm_silu_mul(self.handle, rows, ffn, ptr(h), ptr(gate_up), stream_ptr(stream)))
+        check(self._lib.ztvm_silu_mul(self.handle, rows, ffn, addr(h), addr(gate_up), stream_ptr(stream)))
 
     def moe_combine(self, tokens, slots, d, out, y_slots, scores, stream=None):
-        check(self._lib.ztvm_moe_combine(self.handle, tokens, slots, d, ptr(out), ptr(y_slots), ptr(scores),
+        check(self._lib.ztvm_moe_combine(self.handle, tokens, slots, d, addr(out), addr(y_slots), addr(scores),
                                          stream_ptr(stream)))
 
     def unpack_codes(self, desc: MmDesc, codes, packed_w, stream=None):
-        check(self._lib.ztvm_unpack_codes(self.handle, C.byref(desc), ptr(codes), ptr(packed_w), stream_ptr(stream)))
+        check(self._lib.ztvm_unpack_codes(self.handle, C.byref(desc), addr(codes), addr(packed_w), stream_ptr(stream)))
 
     def unpack_codes_streamed(self, desc: MmDesc, codes, packed_w, stream=None):
         """Codes as the streaming matrix-unit kernels consume them (in-place f16 subnormals scaled back to integers)."""
-        check(self._lib.ztvm_unpack_codes_streamed(self.handle, C.byref(desc), ptr(codes), ptr(packed_w), stream_ptr(stream)))
+        check(self._lib.ztvm_unpack_codes_streamed(self.handle, C.byref(desc), addr(codes), addr(packed_w), stream_ptr(stream)))
 
     def dequant(self, desc: MmDesc, w_out, as_f16, scales, packed_w, biases=None, stream=None):
-        check(self._lib.ztvm_dequant(self.handle, C.byref(desc), ptr(w_out), int(as_f16), ptr(scales),
-                                     ptr(packed_w), ptr(biases), stream_ptr(stream)))
+        check(self._lib.ztvm_dequant(self.handle, C.byref(desc), addr(w_out), int(as_f16), addr(scales),
+                                     addr(packed_w), addr(biases), stream_ptr(stream)))
 
     def device_errors(self, stream=None) -> int:
         n = C.c_uint32(0)

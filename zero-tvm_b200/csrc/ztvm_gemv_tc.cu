@@ -18,10 +18,11 @@ bool gemv_tc_supported(const GemvParams& p, int bits, int sm_count) {
   if (p.pair_rows && (p.N != 2 * p.pair_rows || p.out_f32 || p.n_more)) return false;
   if (p.x_row_stride % 8 || (reinterpret_cast<uintptr_t>(p.X) & 15u)) return false;
   if ((reinterpret_cast<uintptr_t>(p.W) & 15u) || ((reinterpret_cast<uintptr_t>(p.S) | reinterpret_cast<uintptr_t>(p.B)) & 7u)) return false;
-  // One row over a K that ends in part of a slice: the last K tile leaves most warps idle, and the CUDA-core kernel, which
-  // deals K in 32-code units, is faster (9000 x 2112: 5.6 against 7.0 us; 14717 x 5056: 13.9 against 20 us). From two rows
-  // on the matrix unit wins everywhere (14717 x 5056, 4 rows: 20.9 against 42.5 us).
-  if (bits == 4 && p.M == 1 && p.K % 256u && !p.pair_rows) return false;
+  // One row: over a K that ends in part of a slice the last K tile leaves most warps idle, and groups of 32 fold twice as
+  // often; the CUDA-core kernel, which deals K in 32-code units, is faster there (9000 x 2112: 5.6 against 7.0 us;
+  // 14717 x 5056: 13.9 against 20 us; groups of 32, 3072 x 8192: 8.0 against 8.7 us). From two rows on the matrix unit
+  // wins everywhere (14717 x 5056, 4 rows: 20.9 against 42.5 us).
+  if (bits == 4 && p.M == 1 && (p.K % 256u || p.group_shift == 5) && !p.pair_rows) return false;
   if (bits == 8) return gemv_tc_fits_w8(p, sm_count);
   return p.group_shift == 5 ? gemv_tc_fits_w4g32(p, sm_count) : p.B ? gemv_tc_fits_w4(p, sm_count) : gemv_tc_fits_w4sym(p, sm_count);
 }
