@@ -1,38 +1,48 @@
-// Prefill GEMM, M > 8, 4-bit weights: y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS AS THE
+// Prefill GEMM, M > 16, 4-bit weights: y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS AS THE
 // A OPERAND IN TENSOR MEMORY (replaces the matrix-unit GEMMs of int4_matmul.gen.ts:1058-1456; contract of
-// ztvm_int4_matmul for M > 8).
+// ztvm_int4_matmul for M > 16). W16 = f16_rne(fl32(s * q + b)) (or s * (q - 7)), the value the reference's numpy
+// dequantiser produces (scripts/make-dsv2-layer-ref.py:108-116); f32 accumulation in tensor memory.
 //
-// Why this orientation. With both operands in shared memory a 128 x 128 x 16 tcgen05.mma reads 8 KB per ~68 cycles,
-// close to the shared-memory port's whole rate, next to the dequantisers' stores and the TMA writes (ztvm_gemm.cu).
-// Here the weights take the M side of the MMA (128 weight rows = 128 TMEM
-// lanes) and go from the dequantisers' registers straight into tensor memory with tcgen05.st; the activations take
-// the N side (256 tokens per instruction) and are the only operand read from shared memory: 32 KB per k block
-// instead of 64 + 16. D is [weight row][token] in tensor memory; the epilogue writes it transposed (a warp's 32 lanes
-// are 32 consecutive output columns of one token: 64-byte stores).
+// Why this orientation. The weights take the M side of the MMA (128 weight rows = 128 TMEM lanes) and go from the
+// dequantisers' registers straight into tensor memory with tcgen05.st; the activations take the N side (up to 256 tokens
+// per instruction) and are the only operand read from shared memory: 32 KB per k block instead of 64 + 16 with both
+// operands there. D is [weight row][token] in tensor memory.
 //
-// Roles (352 threads): warp 0 TMA-loads activation tiles (NT tokens x 64 k, 128-byte swizzle); warp 2 TMA-loads
-// packed weight tiles (128 rows x 32 words = four k blocks); warps 3..10 dequantise: warp w may touch TMEM lanes
-// 32 (w % 4) .. +31, so it owns those 32 weight rows, and the two warps that share a lane quarter split the k block
-// in halves (16 TMEM columns each); warp 1 allocates tensor memory and issues the MMAs. Every wait is bounded
-// (status word, as in ztvm_gemm.cu).
-#include <type_traits>
+// Roles (640 threads): warp 0 TMA-loads activation tiles (NT tokens x 64 k, 128-byte swizzle); warp 1 allocates tensor
+// memory and issues the MMAs; warp 2 TMA-loads packed weight tiles (128 rows x 32 words = four k blocks); warps 3..18
+// dequantise: warp w may touch TMEM lanes 32 (w % 4) .. +31, so it owns those 32 weight rows; warp 19 stages scales and biases, eight k
+// blocks at a time, as the 8-byte words around each row's groups: rows whose group count is odd (K = 64 x odd) or groups of
+// 32 cost the same as aligned groups of 64. (Loading them from global memory in the dequantisers cost a DRAM or L2 latency
+// per k block wherever a row's groups did not come as aligned 16-byte vectors: 43 us per 9216 x 3072 launch at 77 rows.)
+// Every wait is bounded (status word); on expiry the roles stop and copies in flight are waited for.
+//
+// Few tiles (short prompts, small N): the K range is split over a cluster of CTAs. Each CTA keeps the k blocks of its
+// share; at the end every CTA sends its f32 partial sums of token slice j to CTA j through distributed shared memory, and
+// each reduces and stores its own slice, in CTA order.
 #include "ztvm_kernels.h"
 #include "ztvm_tc.cuh"
 
 namespace ztvm {
 
-constexpr int kTaStages = 4;        // activation tiles in shared memory and weight slices in tensor memory
+constexpr int kTaStages = 4;        // weight slices in tensor memory
 constexpr int kTaWStages = 3;       // packed-weight ring (each slot holds four k blocks)
 constexpr int kTaWChunk = 4;
-constexpr int kTaDqWarps = 16;      // two teams of eight: a team takes every other k block
-constexpr int kTaThreads = 96 + kTaDqWarps * 32;
+constexpr int kTaSbStages = 2;      // scales ring (each stage holds eight k blocks)
+constexpr int kTaSbChunk = 8;
+constexpr int kTaSbMaxPitch = 40;   // bytes of one row's scales (or biases) in a stage: groups of 32
+constexpr int kTaTeamWarps = 4;     // dequantiser warps of a k block (128 rows)
+constexpr int kTaDqWarps = 16;      // four teams: team t takes block t of every packed-weight slot, and stage t
+constexpr int kTaThreads = 96 + kTaDqWarps * 32 + 32;
 constexpr int kTaRows = 128;        // weight rows per CTA = TMEM lanes
+constexpr int kTaMaxSplit = 8;
 
 struct GemmTaParams {
   const __half* S;
   const __half* B;   // nullptr: symmetric
   void* Y;
   uint32_t M, N, K, SPR, group_shift, out_f32;
+  uint32_t sb_pitch;   // 8 x an odd number: half of the banks apart for neighbouring rows
+  uint32_t x_tx_bytes; // bytes one activation stage receives (the boxes hold no more rows than there are)
   uint32_t* status;
 };
 
@@ -40,10 +50,22 @@ template <int NT>
 struct GemmTaSmem {
   static constexpr int kXBytes = NT * kGemmBK * 2;            // per stage
   static constexpr int kWBytes = kTaRows * 128;               // per packed-weight slot
+  static constexpr int kSbBytes = 2 * kTaRows * kTaSbMaxPitch;
   static constexpr int kOffW = kTaStages * kXBytes;
-  static constexpr int kOffBar = kOffW + kTaWStages * kWBytes;
+  static constexpr int kOffSb = kOffW + kTaWStages * kWBytes;
+  static constexpr int kOffBar = kOffSb + kTaSbStages * kSbBytes;
   static constexpr int kTotal = kOffBar + 256;
 };
+
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr) : "memory");
+}
 
 template <int NT, bool AFFINE>
 __global__ void __launch_bounds__(kTaThreads, 1)
@@ -58,7 +80,10 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   auto bar_empty = [&](int s) { return bars + 8u * (kTaStages + s); };
   auto bar_w_full = [&](int s) { return bars + 8u * (2 * kTaStages + s); };
   auto bar_w_empty = [&](int s) { return bars + 8u * (2 * kTaStages + kTaWStages + s); };
-  constexpr int kNumBars = 2 * kTaStages + 2 * kTaWStages + 1;
+  auto bar_sb_full = [&](int s) { return bars + 8u * (2 * kTaStages + 2 * kTaWStages + s); };
+  auto bar_sb_empty = [&](int s) { return bars + 8u * (2 * kTaStages + 2 * kTaWStages + kTaSbStages + s); };
+  constexpr int kNumBars = 2 * kTaStages + 2 * kTaWStages + 2 * kTaSbStages + 1;
+  static_assert(8 * kNumBars + 8 <= 256, "barrier block");
   const uint32_t bar_accum = bars + 8u * (kNumBars - 1);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen_base + L::kOffBar + 8 * kNumBars);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
@@ -66,17 +91,38 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n0 = blockIdx.x * kTaRows;
   const uint32_t m0 = blockIdx.y * NT;
-  const uint32_t num_kb = p.K / kGemmBK;
+  const uint32_t mrows = p.M - m0 < (uint32_t)NT ? p.M - m0 : (uint32_t)NT;     // tokens of this tile
+  // k blocks of this CTA: whole scale stages, so that every share starts on a multiple of eight
+  const uint32_t split = gridDim.z, kz = blockIdx.z;
+  const uint32_t all_kb = p.K / kGemmBK, units = (all_kb + kTaSbChunk - 1) / kTaSbChunk;
+  const uint32_t kb_first = kz * units / split * kTaSbChunk;
+  const uint32_t kb_last = kz + 1 == split ? all_kb : (kz + 1) * units / split * kTaSbChunk;
+  const uint32_t num_kb = kb_last - kb_first;
   constexpr uint32_t kColA = NT;                                 // weight slices start after the accumulator columns
   constexpr uint32_t kTmemCols = NT + kTaStages * 32 <= 256 ? 256 : 512;
+  const uint32_t nbox = (mrows + 127u) / 128u;                   // 128-token boxes of the tile
 
   if (threadIdx.x == 32) { tma_prefetch_desc(&tmap_x); tma_prefetch_desc(&tmap_w); }
+  auto load_x = [&](uint32_t s, uint32_t kb) {
+    // a box holds p.x_tx_bytes / 128 rows; of a 256-token tile whose second half is empty only the first box is fetched
+    mbar_arrive_expect_tx(bar_full((int)s), nbox * p.x_tx_bytes);
+    for (uint32_t b = 0; b < nbox; ++b)
+      tma_load_2d(x_ring + s * L::kXBytes + b * (128 * kGemmBK * 2), &tmap_x, bar_full((int)s), (int)((kb_first + kb) * kGemmBK), (int)(m0 + b * 128));
+  };
+  auto load_w = [&](uint32_t s, uint32_t c) {
+    mbar_arrive_expect_tx(bar_w_full((int)s), (uint32_t)L::kWBytes);
+    tma_load_2d(w_ring + s * L::kWBytes, &tmap_w, bar_w_full((int)s), (int)(kb_first * 8u + c * 32u), (int)n0);
+  };
   // Each TMA producer initialises the barriers its own copies signal and starts its first loads before the block
   // barrier: they fly while tensor memory is allocated.
   if (threadIdx.x == 0) {
     for (int s = 0; s < kTaStages; ++s) {
-      mbar_init(bar_full(s), 1 + (kTaDqWarps / 2) * 32);   // the activation tile (with its byte count) + every thread of the team that writes the slice
+      mbar_init(bar_full(s), 1 + kTaTeamWarps);   // the activation tile (with its byte count) + every warp of the team that writes the slice
       mbar_init(bar_empty(s), 1);
+    }
+    for (int s = 0; s < kTaSbStages; ++s) {
+      mbar_init(bar_sb_full(s), 32);
+      mbar_init(bar_sb_empty(s), kTaDqWarps);
     }
     mbar_init(bar_accum, 1);
     *abort_flag = 0u;
@@ -84,12 +130,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     // Programmatic dependent launch: everything before this point (and the weight / scale loads of the other warps)
     // touches nothing the previous kernel in the stream may write; the activations may be its output.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (uint32_t kb = 0; kb < (uint32_t)kTaStages && kb < num_kb; ++kb) {
-      mbar_arrive_expect_tx(bar_full((int)kb), (uint32_t)L::kXBytes);
-#pragma unroll
-      for (int b = 0; b < NT / 128; ++b)
-        tma_load_2d(x_ring + kb * L::kXBytes + b * (128 * kGemmBK * 2), &tmap_x, bar_full((int)kb), (int)(kb * kGemmBK), (int)(m0 + b * 128));
-    }
+    for (uint32_t kb = 0; kb < (uint32_t)kTaStages && kb < num_kb; ++kb) load_x(kb, kb);
   }
   if (threadIdx.x == 64) {
     for (int s = 0; s < kTaWStages; ++s) {
@@ -98,50 +139,55 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     const uint32_t nc = (num_kb + kTaWChunk - 1) / kTaWChunk;
-    for (uint32_t c = 0; c < (uint32_t)kTaWStages && c < nc; ++c) {
-      mbar_arrive_expect_tx(bar_w_full((int)c), (uint32_t)L::kWBytes);
-      tma_load_2d(w_ring + c * L::kWBytes, &tmap_w, bar_w_full((int)c), (int)(c * 32), (int)n0);
-    }
+    for (uint32_t c = 0; c < (uint32_t)kTaWStages && c < nc; ++c) load_w(c, c);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish();
   }
-  // The dequantisers' first scales and biases (16 groups of this thread's row) are requested before the block barrier:
-  // weights are not written by the previous kernel in the stream, and the DRAM latency of these loads would otherwise
-  // sit between the barrier and the first dequantised stage.
-  uint4 sv_pre0 = make_uint4(0, 0, 0, 0), bv_pre0 = sv_pre0, sv_pre1 = sv_pre0, bv_pre1 = sv_pre0;
-  const bool vec_sb_all = p.group_shift == 6 && (p.SPR % 8u) == 0 &&
-                          ((reinterpret_cast<uintptr_t>(p.S) | reinterpret_cast<uintptr_t>(p.B)) & 15u) == 0;
-  if (warp >= 3 && vec_sb_all) {
-    const uint32_t row_pre = min(n0 + (uint32_t)((warp & 3) * 32 + lane), p.N - 1);
-    const unsigned short* sp = reinterpret_cast<const unsigned short*>(p.S) + (size_t)row_pre * p.SPR;
-    const unsigned short* bp = reinterpret_cast<const unsigned short*>(p.B) + (size_t)row_pre * p.SPR;
-    sv_pre0 = __ldg(reinterpret_cast<const uint4*>(sp));
-    if (AFFINE) bv_pre0 = __ldg(reinterpret_cast<const uint4*>(bp));
-    if (num_kb > 8u) {
-      sv_pre1 = __ldg(reinterpret_cast<const uint4*>(sp + 8));
-      if (AFFINE) bv_pre1 = __ldg(reinterpret_cast<const uint4*>(bp + 8));
+  // scales: the 8-byte words around the groups of eight k blocks of each row
+  const uint32_t sb_groups = (uint32_t)(kTaSbChunk * kGemmBK) >> p.group_shift;       // 16, 8 or 4 per row and stage
+  auto load_sb = [&](uint32_t s, uint32_t ch) {
+    const uint32_t g0 = ((kb_first + ch * kTaSbChunk) * (uint32_t)kGemmBK) >> p.group_shift;
+    const uint32_t have = p.SPR - g0 < sb_groups ? p.SPR - g0 : sb_groups;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t r = (uint32_t)lane + 32u * i;
+      const size_t off = (size_t)min(n0 + r, p.N - 1) * p.SPR + g0;
+      const uint32_t odd = ((uint32_t)off & 3u) * 2u, end = odd + have * 2u;             // tables start on 8-byte boundaries
+#pragma unroll
+      for (int tb = 0; tb < (AFFINE ? 2 : 1); ++tb) {
+        const uint8_t* src = reinterpret_cast<const uint8_t*>((tb ? p.B : p.S) + off) - odd;
+        const uint32_t dst = base + L::kOffSb + s * L::kSbBytes + ((uint32_t)tb * kTaRows + r) * p.sb_pitch;
+        for (uint32_t b = 0; b < end; b += 8u)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + b), "l"(src + b), "r"(min(8u, end - b)) : "memory");
+      }
     }
-  }
+  };
+  const uint32_t sb_chunks = (num_kb + kTaSbChunk - 1) / kTaSbChunk;
+  if (warp == 3 + kTaDqWarps) load_sb(0, 0);       // before the block barrier: weights are not written by the previous kernel
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+  const int quarter = warp & 3;                       // TMEM lanes this warp may touch: [32 * quarter, +32)
+  const uint32_t wpart = (uint32_t)(warp - 3) >> 2;   // dequantisers: 0..3
+  const uint32_t r_tile = (uint32_t)(quarter * 32 + lane);
+  const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+  const bool is_dq = warp >= 3 && warp < 3 + kTaDqWarps;
+  bool acc_ok = false;
+
   if (warp == 0) {
     // ================= TMA producer: activations =================
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t issued = num_kb < (uint32_t)kTaStages ? num_kb : (uint32_t)kTaStages;
       for (uint32_t kb = issued; kb < num_kb; ++kb) {
         const int s = kb % kTaStages;
         const uint32_t ph = (kb / kTaStages) & 1u;
         if (!mbar_wait(bar_empty(s), ph ^ 1u, p.status, 1u, abort_flag)) break;
-        mbar_arrive_expect_tx(bar_full(s), (uint32_t)L::kXBytes);
-#pragma unroll
-        for (int b = 0; b < NT / 128; ++b)
-          tma_load_2d(x_ring + s * L::kXBytes + b * (128 * kGemmBK * 2), &tmap_x, bar_full(s), (int)(kb * kGemmBK), (int)(m0 + b * 128));
+        load_x((uint32_t)s, kb);
         issued = kb + 1;
       }
       if (*abort_flag) {   // the consumer stopped: wait (bounded) until the copies already issued have landed
@@ -155,8 +201,8 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
   } else if (warp == 1) {
     // ================= MMA issuer =================
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_f16(NT);
+    if (elect_one()) {
+      const uint32_t idesc = idesc_f16((int)((mrows + 15u) & ~15u));
       const uint64_t b0 = smem_desc_sw128(x_ring);
       uint32_t s = 0, ph = 0;
       // The thread is held at each tcgen05.mma until the pipe takes it, so a barrier poll between two k blocks would
@@ -183,15 +229,14 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
   } else if (warp == 2) {
     // ================= TMA producer: packed weights =================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t num_chunks = (num_kb + kTaWChunk - 1) / kTaWChunk;
       uint32_t issued = num_chunks < (uint32_t)kTaWStages ? num_chunks : (uint32_t)kTaWStages;
       for (uint32_t c = issued; c < num_chunks; ++c) {
         const int s = c % kTaWStages;
         const uint32_t ph = (c / kTaWStages) & 1u;
         if (!mbar_wait(bar_w_empty(s), ph ^ 1u, p.status, 6u, abort_flag)) break;
-        mbar_arrive_expect_tx(bar_w_full(s), (uint32_t)L::kWBytes);
-        tma_load_2d(w_ring + s * L::kWBytes, &tmap_w, bar_w_full(s), (int)(c * 32), (int)n0);
+        load_w((uint32_t)s, c);
         issued = c + 1;
       }
       if (*abort_flag) {
@@ -203,107 +248,81 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         }
       }
     }
+  } else if (!is_dq) {
+    // ================= scales and biases =================
+    for (uint32_t ch = 0; ch < sb_chunks; ++ch) {
+      const uint32_t s = ch % kTaSbStages;
+      bool ok = true;
+      if (ch >= (uint32_t)kTaSbStages) ok = mbar_wait(bar_sb_empty((int)s), ((ch / kTaSbStages) & 1u) ^ 1u, p.status, 8u, abort_flag, 400u);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (ch) load_sb(s, ch);
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_sb_full((int)s)) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
-    // ================= dequantisers (warps 3..18), then epilogue =================
-    // Two teams of eight warps take the k blocks in turn (team = k block mod 2). Inside a team, thread
-    // (quarter, lane) of half h owns weight row 32 quarter + lane and the 32-code half h of the block. A warp runs its
-    // block as one dependent chain (wait, load, dequantise, store to tensor memory, wait for the store, arrive), about
-    // twice as long as the tensor pipe needs for the block's MMAs: with one team the pipe idles half of the time, with
-    // two the chains of consecutive blocks overlap.
-    const int quarter = warp & 3;                       // TMEM lanes this warp may touch: [32 * quarter, +32)
-    const uint32_t wpart = (uint32_t)(warp - 3) >> 2;   // 0..3
-    const uint32_t part = wpart & 1u;                   // which half of the k block
-    const uint32_t team = wpart >> 1;
-    const uint32_t r_tile = (uint32_t)(quarter * 32 + lane);
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const int gshift = (int)p.group_shift;
-    const uint32_t row = min(n0 + r_tile, p.N - 1);
-    const unsigned short* srow = reinterpret_cast<const unsigned short*>(p.S) + (size_t)row * p.SPR;
-    const unsigned short* brow = reinterpret_cast<const unsigned short*>(p.B) + (size_t)row * p.SPR;
-    bool ok = true;
-    // group 64: eight groups per 16-byte load, fetched eight k blocks ahead; scalar loads otherwise
-    const bool vec_sb = vec_sb_all;
-    uint4 sv_cur = sv_pre0, bv_cur = bv_pre0, sv_nxt = sv_pre1, bv_nxt = bv_pre1;
-    auto load_sb8 = [&](uint4& sv, uint4& bv, uint32_t kb8) {
-      if (kb8 >= num_kb) return;
-      sv = __ldg(reinterpret_cast<const uint4*>(srow + kb8));
-      if (AFFINE) bv = __ldg(reinterpret_cast<const uint4*>(brow + kb8));
-    };
-    auto pick16 = [](const uint4& v, int i) -> unsigned short {
-      const uint32_t wsel = (i >> 1) == 0 ? v.x : (i >> 1) == 1 ? v.y : (i >> 1) == 2 ? v.z : v.w;
-      return (unsigned short)((i & 1) ? (wsel >> 16) : (wsel & 0xFFFFu));
-    };
-
+    // ================= dequantisers (warps 3..18) =================
+    // Four teams of four warps; thread (quarter, lane) of team t dequantises the 64 codes of weight row 32 quarter + lane
+    // in block t of every slot. Issue slots bound this part: a whole row of a block per thread (instead of half, with
+    // teams of eight) halves the waits, scale look-ups and guards per code, and four blocks are in flight at once, so a
+    // team's chain of wait, load, dequantise, store, arrive may take as long as four blocks.
+    static_assert(kTaStages == kTaWChunk && kTaDqWarps == kTaWChunk * kTaTeamWarps, "a team per stage");
+    const uint32_t team = wpart;
     const uint8_t* const wrow_sm = gen_base + L::kOffW + (r_tile >> 3) * 1024 + (r_tile & 7) * 128;
-    constexpr int kUnroll = 8;
-    auto run = [&](auto team_c) {
-      constexpr int TEAM = decltype(team_c)::value;
-      for (uint32_t kb0 = 0; kb0 < num_kb && ok; kb0 += kUnroll) {
-#pragma unroll
-        for (int i = TEAM; i < kUnroll; i += 2) {
-          const uint32_t kb = kb0 + i;
-          if (kb >= num_kb || !ok) break;
-          const int s = (int)(kb % kTaStages);
-          const uint32_t ph = (kb / kTaStages) & 1u;
-          const uint32_t c = kb / kTaWChunk;
-          const int ws = (int)(c % kTaWStages);
-          const int j = i % kTaWChunk;
-          if (j == TEAM) ok = mbar_wait(bar_w_full(ws), (c / kTaWStages) & 1u, p.status, 7u, abort_flag);
-          uint4 wv = make_uint4(0, 0, 0, 0);
-          if (ok) wv = *reinterpret_cast<const uint4*>(wrow_sm + ws * L::kWBytes + ((((uint32_t)j * 2 + part) ^ (r_tile & 7)) << 4));
-          // the TMEM slice of stage s was last read by the MMAs of k block kb - kTaStages
-          if (ok && kb >= (uint32_t)kTaStages) {
-            ok = mbar_wait(bar_empty(s), ph ^ 1u, p.status, 4u, abort_flag);
-            tc_fence_after();
+    const uint32_t w_at0 = ((team * 2u) ^ (r_tile & 7)) << 4, w_at1 = ((team * 2u + 1u) ^ (r_tile & 7)) << 4;
+    const uint32_t sb_odd = (uint32_t)(((size_t)min(n0 + r_tile, p.N - 1) * p.SPR) & 3u) * 2u;   // (stages start on multiples of four groups)
+    const uint8_t* const sb_row = gen_base + L::kOffSb + r_tile * p.sb_pitch + sb_odd;
+    const uint32_t b_delta = (uint32_t)kTaRows * p.sb_pitch;
+    const uint32_t st_at = tmem_base + lane_base + kColA + team * 32u;
+    bool ok = true;
+    uint32_t ws = 0, wph = 0, ss = 0, sph = 0;          // slot and phase of the packed ring and of the scales ring
+    for (uint32_t c = 0; c * kTaWChunk < num_kb; ++c) {
+      if (c * kTaWChunk + team < num_kb) {
+        if (ok && (c & 1u) == 0u) ok = mbar_wait(bar_sb_full((int)ss), sph, p.status, 9u, abort_flag);
+        if (ok) ok = mbar_wait(bar_w_full((int)ws), wph, p.status, 7u, abort_flag);
+        uint32_t a[32];
+        if (ok) {
+          const uint8_t* const wl = wrow_sm + ws * L::kWBytes;
+          const uint4 w0 = *reinterpret_cast<const uint4*>(wl + w_at0), w1 = *reinterpret_cast<const uint4*>(wl + w_at1);
+          const uint32_t k0 = ((c & 1u) * kTaWChunk + team) * (uint32_t)kGemmBK;
+          const uint8_t* const sp = sb_row + ss * L::kSbBytes + (k0 >> p.group_shift) * 2u;
+          const DqGroup dq = dq_group<AFFINE>(*reinterpret_cast<const unsigned short*>(sp),
+                                              AFFINE ? *reinterpret_cast<const unsigned short*>(sp + b_delta) : (unsigned short)0);
+          dequant_words_w16<AFFINE>(w0, dq, a);
+          if (p.group_shift == 5) {                     // the second half of the block is the next group
+            const DqGroup dq2 = dq_group<AFFINE>(*reinterpret_cast<const unsigned short*>(sp + 2),
+                                                 AFFINE ? *reinterpret_cast<const unsigned short*>(sp + b_delta + 2) : (unsigned short)0);
+            dequant_words_w16<AFFINE>(w1, dq2, a + 16);
+          } else {
+            dequant_words_w16<AFFINE>(w1, dq, a + 16);
           }
-          if (ok) {
-            unsigned short s16, b16 = 0;
-            if (vec_sb) {
-              s16 = pick16(sv_cur, i);
-              if (AFFINE) b16 = pick16(bv_cur, i);
-            } else {
-              const uint32_t g = (kb * kGemmBK + part * 32) >> gshift;
-              s16 = __ldg(srow + g);
-              if (AFFINE) b16 = __ldg(brow + g);
-            }
-            const DqGroup dq = dq_group<AFFINE>(s16, b16);
-            const uint32_t words[4] = {wv.x, wv.y, wv.z, wv.w};
-            uint32_t a[16];
-#pragma unroll
-            for (int wi = 0; wi < 4; ++wi) {
-              const uint4 v = dequant_word_w16<AFFINE>(words[wi], dq);
-              a[4 * wi] = v.x; a[4 * wi + 1] = v.y; a[4 * wi + 2] = v.z; a[4 * wi + 3] = v.w;
-            }
-            // 32 weights of this row = 16 TMEM columns (two k-adjacent f16 per column) of this thread's lane
-            tmem_st16(tmem_base + lane_base + kColA + (uint32_t)s * 32u + part * 16u, a);
-            tmem_st_wait();
-          }
-          // the packed slot goes back to the producer only after the stores that consumed its words; a warp signals
-          // after its team's last k block of the slot
-          if (j + 2 >= kTaWChunk || kb + 2 >= num_kb) {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_w_empty(ws));
-          }
-          tc_fence_before();
-          mbar_arrive(bar_full(s));   // every thread arrives itself (also on abort)
         }
-        if (vec_sb) {
-          sv_cur = sv_nxt; bv_cur = bv_nxt;
-          load_sb8(sv_nxt, bv_nxt, kb0 + 2 * kUnroll);
+        // the TMEM slice of this stage was last read by the MMAs of the block one slot back
+        if (ok && c > 0) {
+          ok = mbar_wait(bar_empty((int)team), (c & 1u) ^ 1u, p.status, 4u, abort_flag);
+          tc_fence_after();
         }
-      }
-      // a last slot that holds one k block only has nothing for the second team: it still hands the slot back
-      if (TEAM == 1 && (num_kb % kTaWChunk) == 1u) {
-        const uint32_t c = (num_kb - 1u) / kTaWChunk;
-        const int ws = (int)(c % kTaWStages);
-        if (ok) ok = mbar_wait(bar_w_full(ws), (c / kTaWStages) & 1u, p.status, 7u, abort_flag);
+        if (ok) {
+          // 64 weights of this row = 32 TMEM columns (two k-adjacent f16 per column) of this thread's lane
+          tmem_st32(st_at, a);
+          tmem_st_wait();
+        }
+        // every lane's stores to tensor memory are complete; one lane signals for the warp (also on abort)
+        tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_w_empty(ws));
+        if (lane == 0) mbar_arrive(bar_full((int)team));
       }
-    };
-    if (team == 0) run(std::integral_constant<int, 0>{}); else run(std::integral_constant<int, 1>{});
+      // The slots go back to the producers only after the stores that consumed their words. A team without a block in a
+      // short last slot hands them back all the same.
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(bar_w_empty((int)ws));
+        if ((c & 1u) || (c + 1) * kTaWChunk >= num_kb) mbar_arrive(bar_sb_empty((int)ss));
+      }
+      if (++ws == (uint32_t)kTaWStages) { ws = 0; wph ^= 1u; }
+      if (c & 1u) { if (++ss == (uint32_t)kTaSbStages) { ss = 0; sph ^= 1u; } }
+    }
     // ---- epilogue: D[weight row][token] in TMEM -> y[token][weight row] ------------------------------------------
-    const bool acc_ok = ok && mbar_wait(bar_accum, 0u, p.status, 5u, abort_flag);
+    acc_ok = ok && mbar_wait(bar_accum, 0u, p.status, 5u, abort_flag);
     tc_fence_after();
     asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be read by the previous kernel in the stream
     // f16 rows of whole 16-byte pieces: the tile is turned round in the (now idle) activation ring. Phase 1: a thread
@@ -312,11 +331,14 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     // All sixteen warps reach the named barrier (also when a wait ran out: they then skip the memory work).
     static_assert(NT * kTaRows * 2 <= kTaStages * L::kXBytes, "the output stage lives in the activation ring");
     const bool staged = !p.out_f32 && (p.N % 8u) == 0;
-    if (staged) {
+    const int ncb = (int)((mrows + 31u) / 32u);
+    if (split > 1) {
+      // below, with the whole cluster
+    } else if (staged) {
       const uint32_t stage = x_ring;
       if (acc_ok) {
 #pragma unroll 1
-        for (int cb = (int)wpart; cb < NT / 32; cb += 4) {
+        for (int cb = (int)wpart; cb < ncb; cb += 4) {
           uint32_t v[32];
           tmem_ld32(tmem_base + lane_base + (uint32_t)(cb * 32), v);
           tmem_ld_wait();
@@ -335,17 +357,16 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const uint32_t n = n0 + piece * 8u;
         const uint4* const stage_g = reinterpret_cast<const uint4*>(gen_base);
 #pragma unroll 4
-        for (uint32_t t = w16 * 2u + sub; t < (uint32_t)NT; t += 2u * kTaDqWarps) {
-          const uint32_t m = m0 + t;
-          if (m < p.M && n < p.N)
-            *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.Y) + (size_t)m * p.N + n) = stage_g[t * (kTaRows * 2u / 16u) + piece];
+        for (uint32_t t = w16 * 2u + sub; t < mrows; t += 2u * kTaDqWarps) {
+          if (n < p.N)
+            *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.Y) + (size_t)(m0 + t) * p.N + n) = stage_g[t * (kTaRows * 2u / 16u) + piece];
         }
       }
     } else if (acc_ok) {
       const uint32_t n = n0 + r_tile;
       // the four warps of a quarter take the 32-token blocks in turn
 #pragma unroll 1
-      for (int cb = (int)wpart; cb < NT / 32; cb += 4) {
+      for (int cb = (int)wpart; cb < ncb; cb += 4) {
         uint32_t v[32];
         tmem_ld32(tmem_base + lane_base + (uint32_t)(cb * 32), v);
         tmem_ld_wait();
@@ -362,6 +383,61 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             for (int i = 0; i < 32; ++i)
               if (m_first + i < p.M) dst[(size_t)i * p.N] = __float2half_rn(__uint_as_float(v[i]));
           }
+        }
+      }
+    }
+  }
+  if (split > 1) {
+    // ---- K shares meet: token blocks of eight, dealt to the CTAs in runs of `per`; partial sums as [sender][block][row][8
+    // tokens] in the receiver's idle rings. Every thread of the cluster takes both barriers, whatever became of its waits.
+    const uint32_t nb = (mrows + 7u) / 8u, per = (nb + split - 1) / split;
+    static_assert((NT + 56) * kTaRows * 4 <= kTaStages * L::kXBytes + kTaWStages * L::kWBytes, "partial sums of the other CTAs fit the rings");
+    __syncwarp();
+    cluster_sync_all();                                  // every CTA's MMAs have read its rings for the last time
+    if (is_dq && acc_ok) {
+      for (uint32_t b = wpart; b < nb; b += 4u) {
+        const uint32_t to = b / per;
+        if (to == kz) continue;
+        uint32_t v[8];
+        tmem_ld8(tmem_base + lane_base + b * 8u, v);
+        tmem_ld_wait();
+        const uint32_t slot = kz < to ? kz : kz - 1u;     // the receiver's own sums stay in its tensor memory
+        uint32_t dst;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(base + (((slot * per + b - to * per) * kTaRows + r_tile) * 32u)), "r"(to));
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16u * i), "r"(v[4 * i]), "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3]) : "memory");
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (is_dq && acc_ok) {
+      const uint32_t n = n0 + r_tile;
+      for (uint32_t b = kz * per + wpart; b < nb && b < (kz + 1) * per; b += 4u) {
+        uint32_t v[8];
+        tmem_ld8(tmem_base + lane_base + b * 8u, v);
+        tmem_ld_wait();
+        if (n >= p.N) continue;
+        float r[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = 0.f;
+        for (uint32_t z = 0; z < split; ++z) {              // in CTA order, wherever this CTA stands in it
+          if (z == kz) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i] += __uint_as_float(v[i]);
+          } else {
+            const float4* const got = reinterpret_cast<const float4*>(gen_base) + (((z < kz ? z : z - 1u) * per + b - kz * per) * kTaRows + r_tile) * 2u;
+            const float4 g0 = got[0], g1 = got[1];
+            r[0] += g0.x; r[1] += g0.y; r[2] += g0.z; r[3] += g0.w;
+            r[4] += g1.x; r[5] += g1.y; r[6] += g1.z; r[7] += g1.w;
+          }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+          if (b * 8u + i >= mrows) break;
+          const size_t o = (size_t)(m0 + b * 8u + i) * p.N + n;
+          if (p.out_f32) reinterpret_cast<float*>(p.Y)[o] = r[i];
+          else reinterpret_cast<__half*>(p.Y)[o] = __float2half_rn(r[i]);
         }
       }
     }
@@ -388,39 +464,93 @@ static TaEncodeFn ta_encode_fn() {
 }
 
 template <int NT, bool AFFINE>
-static cudaError_t launch_ta_one(const CUtensorMap& tx, const CUtensorMap& tw, const GemmTaParams& p, cudaStream_t st) {
-  auto kern = gemm_w4_ta_kernel<NT, AFFINE>;
-  constexpr int smem = GemmTaSmem<NT>::kTotal + 1024;
+static cudaError_t ta_kernel_ready() {
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 16 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
-  }
+  if (dev < 16 && attr_set[dev]) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_w4_ta_kernel<NT, AFFINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmTaSmem<NT>::kTotal + 1024);
+  if (e == cudaSuccess && dev < 16) attr_set[dev] = true;
+  return e;
+}
+struct TaLaunch {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((p.N + kTaRows - 1) / kTaRows, (p.M + NT - 1) / NT);
-  cfg.blockDim = dim3(kTaThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tx, tw, p);
+  cudaLaunchAttribute attr[2];
+  TaLaunch(dim3 grid, int smem, cudaStream_t st) {
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kTaThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = grid.z;
+    cfg.attrs = attr;
+    cfg.numAttrs = grid.z > 1 ? 2 : 1;
+  }
+};
+template <int NT, bool AFFINE>
+static cudaError_t launch_ta_one(const CUtensorMap& tx, const CUtensorMap& tw, const GemmTaParams& p, uint32_t split, cudaStream_t st) {
+  const cudaError_t e = ta_kernel_ready<NT, AFFINE>();
+  if (e != cudaSuccess) return e;
+  TaLaunch l(dim3((p.N + kTaRows - 1) / kTaRows, (p.M + NT - 1) / NT, split), GemmTaSmem<NT>::kTotal + 1024, st);
+  return cudaLaunchKernelEx(&l.cfg, gemm_w4_ta_kernel<NT, AFFINE>, tx, tw, p);
+}
+// Clusters of `split` CTAs that the device holds at once (a cluster sits inside one GPC, so this is less than SMs / split).
+template <int NT>
+static uint32_t ta_clusters(uint32_t split, int sm_count) {
+  if (split == 1) return (uint32_t)sm_count;
+  static int known[16][kTaMaxSplit + 1] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 16) return 1;
+  int n = known[dev][split];
+  if (n == 0) {
+    TaLaunch l(dim3(1, 1, split), GemmTaSmem<NT>::kTotal + 1024, nullptr);
+    if (ta_kernel_ready<NT, true>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_w4_ta_kernel<NT, true>, &l.cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = 1;
+    }
+    known[dev][split] = n;
+  }
+  return (uint32_t)n;
+}
+
+bool gemm_w4_supported(int bits, uint32_t group, uint32_t K) {
+  return bits == 4 && (group == 32 || group == 64 || group == 128) && K % kGemmBK == 0;
 }
 
 cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M,
-                              uint32_t N, uint32_t K, uint32_t group_shift, bool out_f32, uint32_t* status, cudaStream_t st) {
+                              uint32_t N, uint32_t K, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count, cudaStream_t st) {
   TaEncodeFn enc = ta_encode_fn();
   if (!enc) return cudaErrorNotSupported;
+  // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 8192 x 2048 .. 3072 x 8192:
+  // a k block takes 340 + 1.4 per token (at least 390), a CTA 8500 to start, fill its rings and store, the exchange of
+  // a cluster 5300 + 12 per token. Clusters run in as many waves as the device can place.
+  const uint32_t units = (K / kGemmBK + kTaSbChunk - 1) / kTaSbChunk;
+  uint32_t nt = 64, split = 1;
+  uint64_t best = ~0ull;
+  for (uint32_t t : {64u, 128u, 256u}) {
+    if (t > 64u && t / 2 >= M) continue;
+    const uint64_t tiles = (uint64_t)((N + kTaRows - 1) / kTaRows) * ((M + t - 1) / t);
+    const uint32_t live = M < t ? M : t, block = live < 36u ? 390u : 340u + live * 14u / 10u;
+    for (uint32_t z = 1; z <= (uint32_t)kTaMaxSplit && z <= units; ++z) {
+      if (z > 1 && tiles * z > (uint64_t)sm_count) break;
+      const uint32_t at_once = t == 64u ? ta_clusters<64>(z, sm_count) : t == 128u ? ta_clusters<128>(z, sm_count) : ta_clusters<256>(z, sm_count);
+      const uint64_t waves = (tiles + at_once - 1) / at_once;
+      const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + 8500u + (z > 1 ? 5300u + 12u * live : 0u));
+      if (cost < best) { best = cost; nt = t; split = z; }
+    }
+  }
   const cuuint32_t estr[2] = {1, 1};
   CUtensorMap tx, tw;
   const cuuint64_t xdims[2] = {K, M};
   const cuuint64_t xstrides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t xbox[2] = {(cuuint32_t)kGemmBK, 128};
+  // a box much taller than the tensor makes every load slow (22 against 13 us per launch at M = 17): no more rows than there are
+  const uint32_t box_rows = M >= 128u && nt >= 128u ? 128u : M >= 64u && nt == 64u ? 64u : (M + 7u) & ~7u;
+  const cuuint32_t xbox[2] = {(cuuint32_t)kGemmBK, box_rows};
   CUresult r = enc(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(X), xdims, xstrides, xbox, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -436,13 +566,13 @@ cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* 
   p.S = S; p.B = B; p.Y = Y;
   p.M = M; p.N = N; p.K = K; p.SPR = K >> group_shift; p.group_shift = group_shift;
   p.out_f32 = out_f32 ? 1u : 0u;
+  p.sb_pitch = group_shift == 5 ? 40u : 24u;
+  p.x_tx_bytes = box_rows * (uint32_t)(kGemmBK * 2);
   p.status = status;
   const bool affine = B != nullptr;
-  // 256 tokens per instruction unless that leaves most SMs without a tile (M = 256 on 8192 rows: 64 CTAs of 256 tokens
-  // or 128 CTAs of 128)
-  const uint64_t ctas256 = (uint64_t)((N + kTaRows - 1) / kTaRows) * ((M + 255) / 256);
-  if (M > 128 && (M > 256 || ctas256 >= 111)) return affine ? launch_ta_one<256, true>(tx, tw, p, st) : launch_ta_one<256, false>(tx, tw, p, st);
-  return affine ? launch_ta_one<128, true>(tx, tw, p, st) : launch_ta_one<128, false>(tx, tw, p, st);
+  if (nt == 256) return affine ? launch_ta_one<256, true>(tx, tw, p, split, st) : launch_ta_one<256, false>(tx, tw, p, split, st);
+  if (nt == 128) return affine ? launch_ta_one<128, true>(tx, tw, p, split, st) : launch_ta_one<128, false>(tx, tw, p, split, st);
+  return affine ? launch_ta_one<64, true>(tx, tw, p, split, st) : launch_ta_one<64, false>(tx, tw, p, split, st);
 }
 
 }  // namespace ztvm

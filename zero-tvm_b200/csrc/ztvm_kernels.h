@@ -65,11 +65,13 @@ bool batch_moe_supported(const GemvParams& g, int bits);
 uint32_t batch_moe_tile_rows(uint32_t experts, uint64_t pairs);
 cudaError_t launch_batch_moe(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan);
 
-// 4-bit weights, M > 8: tcgen05 GEMM with TMEM accumulators (ztvm_gemm.cu). status[0] receives a non-zero code
-// if a pipeline wait inside the kernel ran out.
+// 4-bit weights, M > 16: tcgen05 GEMM with the dequantised weights as the A operand in tensor memory and the activations
+// as the only shared-memory operand (ztvm_gemm_ta.cu). status[0] receives a non-zero code if a pipeline wait inside the
+// kernel ran out.
 bool gemm_w4_supported(int bits, uint32_t group, uint32_t K);
-cudaError_t launch_gemm_w4(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M,
-                           uint32_t N, uint32_t K, uint32_t group_shift, bool out_f32, uint32_t* status, cudaStream_t st);
+cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M,
+                              uint32_t N, uint32_t K, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count,
+                              cudaStream_t st);
 
 // Grouped MoE expert matmul (ztvm_moe_gemm.cu): pairs sorted by expert, tcgen05 tiles. `scratch` holds the plan
 // (moe_grouped_scratch_bytes), `status[0]` receives a non-zero code if a bounded wait ran out.
@@ -100,11 +102,6 @@ cudaError_t launch_moe_grouped_static(const GemvParams& g, uint32_t tokens, uint
 cudaError_t launch_moe_tc_static(const GemvParams& g, uint32_t tokens, uint32_t slots, int sm_count, cudaStream_t st);
 cudaError_t launch_moe_ta_static(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* status, int sm_count,
                                  cudaStream_t st);
-
-// The same GEMM with the dequantised weights as the A operand in tensor memory and the activations as the only
-// shared-memory operand (ztvm_gemm_ta.cu): the default for M > 8; launch_gemm_w4 stays selectable for comparison.
-cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M,
-                              uint32_t N, uint32_t K, uint32_t group_shift, bool out_f32, uint32_t* status, cudaStream_t st);
 
 // Dispatch step of the expert-parallel MoE block (ztvm_moe_ep.cu): pair rows stored straight into the owners' receive
 // buffers (peer-mapped addresses), one region per source rank.
