@@ -156,7 +156,7 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
 
   if (warp == 0) {
     // ================= TMA producer: packed weights, rows [expert * N + n0, +256) as two boxes of 128 ============
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t gc = 0, issued = 0;
       bool ok = true;
       for (uint32_t ui = 0; ui < my_units && ok; ++ui) {
@@ -182,7 +182,7 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
     }
   } else if (warp == 1) {
     // ================= MMA issuer =================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t b0 = smem_desc_sw128(x_ring);
       uint32_t gst = 0;
       bool ok = true;
@@ -287,13 +287,8 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
               b16 = __ldg(brow + kb);
             }
             const DqGroup dq = dq_group<true>(s16, b16);
-            const uint32_t words[4] = {wv.x, wv.y, wv.z, wv.w};
             uint32_t a[16];
-#pragma unroll
-            for (int wi = 0; wi < 4; ++wi) {
-              const uint4 v = dequant_word_w16<true>(words[wi], dq);
-              a[4 * wi] = v.x; a[4 * wi + 1] = v.y; a[4 * wi + 2] = v.z; a[4 * wi + 3] = v.w;
-            }
+            dequant_words_w16<true>(wv, dq, a);
             // 32 weights of this row = 16 TMEM columns (two k-adjacent f16 per column) of this thread's lane
             tmem_st16(tmem_base + lane_base + kMtaColA + s * 64u + half * 32u + khalf * 16u, a);
             tmem_st_wait();
