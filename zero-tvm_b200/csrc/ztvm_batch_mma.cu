@@ -14,7 +14,7 @@
 // CTA: eight warps as WM x WN x WK; a warp owns 32 weight rows x 8 NBW tokens (n blocks wn, wn + WN, ...: live blocks
 // spread evenly when the tile is not full) and every WK-th run. Stages of RUNS runs (weights ROWS x 64 RUNS codes,
 // activations TOK x 64 RUNS f16) go through a cp.async ring, swizzled so that fragment loads hit all banks. The sums
-// of x that multiply the biases are formed once per stage from shared memory, one stage ahead of their use.
+// of x that multiply the biases come from the matrix unit as well, one stage ahead of their use.
 #include <cstring>
 
 #include "ztvm_frag.cuh"
@@ -43,7 +43,9 @@ struct BatchCfg {
   static constexpr int kRows = WM * 32, kTok = WN * NBW * 8;
   static constexpr int kRowBytes = RUNS * Frag<BITS>::kRunBytes;
   static constexpr int kWBytes = kRows * kRowBytes, kXBytes = kTok * RUNS * 128;
-  static constexpr int kStageBytes = kWBytes + kXBytes;
+  // scales and biases of a row in a stage: the aligned 4-byte words around its RUNS values
+  static constexpr int kSbSlot = RUNS * 2 + 4, kSbBytes = 2 * kRows * kSbSlot;
+  static constexpr int kStageBytes = (kWBytes + kXBytes + kSbBytes + 127) / 128 * 128;
   static constexpr int kStages = 4 * kStageBytes <= 104 * 1024 ? 4 : 3;   // two CTAs per SM
   static constexpr int kOffXs = kStages * kStageBytes;                 // float [2][RUNS][kTok]
   static constexpr int kOffRow = kOffXs + 2 * RUNS * kTok * 4;         // uint64 [2][kTok]: input / output row offsets (grouped form)
@@ -52,8 +54,20 @@ struct BatchCfg {
   static_assert(kTok * kOutPitch * 4 <= kOffXs, "the output tile reuses the ring");
 };
 
-template <int BITS, int WM, int WN, int WK, int NBW, int RUNS, bool MOE>
-__global__ void __launch_bounds__(256, 2)
+__device__ __forceinline__ void bm_mma0(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f), "f"(0.f), "f"(0.f), "f"(0.f));
+}
+__device__ __forceinline__ void bm_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// W16: weight rows are whole 16-byte pieces (always, but for 3-bit rows of an odd number of runs).
+template <int BITS, int WM, int WN, int WK, int NBW, int RUNS, bool MOE, bool W16>
+__global__ void __launch_bounds__(256, NBW == 8 ? 1 : 2)
 batch_mma_kernel(const BatchParams p) {
   using C = BatchCfg<BITS, WM, WN, WK, NBW, RUNS>;
   using F = Frag<BITS>;
@@ -70,12 +84,14 @@ batch_mma_kernel(const BatchParams p) {
   const uint32_t* W = p.W;
   const __half *S = p.S, *B = p.B;
   uint32_t ntok, t0 = blockIdx.x * C::kTok;
+  uint32_t sb_odd0 = 0u;             // tables start on 8-byte boundaries; an expert's slice may start on an odd group
   if constexpr (MOE) {
     asm volatile("griddepcontrol.wait;" ::: "memory");     // the plan comes from the kernel before
     if (blockIdx.x >= *p.sc.ntiles) return;
     const uint32_t* tile = p.sc.tiles + (size_t)blockIdx.x * 3;
     const uint32_t expert = tile[0], first = tile[1];
     ntok = tile[2];
+    sb_odd0 = expert & p.N & p.SPR & 1u;
     W += (size_t)expert * p.N * p.KP;
     S += (size_t)expert * p.N * p.SPR;
     B += (size_t)expert * p.N * p.SPR;
@@ -91,97 +107,113 @@ batch_mma_kernel(const BatchParams p) {
   }
   const uint32_t stages = (p.SPR + RUNS - 1) / RUNS;
 
-  // ---- producer: this thread's pieces of a stage -----------------------------------------------------------------
+  // ---- producer: this thread's pieces of a stage. Where they come from and go to is worked out once; a stage costs an add
+  // and a copy per piece (computing rows and pieces afresh took more issue slots than the multiplications). -------------
+  constexpr uint32_t WP = W16 ? 16 : 8, CH = C::kRowBytes / WP, NW = (C::kRows * CH + 255) / 256;
+  const uint8_t* const w_tile = reinterpret_cast<const uint8_t*>(W + (size_t)n0 * p.KP);
+  uint32_t w_off[NW], w_dst[NW], w_on = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < NW; ++i) {
+    const uint32_t idx = tid + 256u * i, row = idx / CH, q = idx - row * CH, run = q * WP / F::kRunBytes;
+    const uint32_t sw = BITS == 3 ? 0u : BITS == 8 ? row & 1u : RUNS == 2 ? (row >> 1) & 1u : row & 3u;
+    w_off[i] = row * (p.KP * 4u) + q * WP;
+    w_dst[i] = row * C::kRowBytes + (BITS == 3 ? q * WP : (run ^ sw) * F::kRunBytes + q * WP % F::kRunBytes);
+    if (idx < (uint32_t)C::kRows * CH && n0 + row < p.N) w_on |= 1u << i;
+  }
   auto issue_w = [&](uint32_t st) {
     const uint32_t dst0 = sm + (st % C::kStages) * C::kStageBytes;
+    const uint8_t* const src0 = w_tile + (size_t)st * C::kRowBytes;
     const uint32_t live = p.SPR - st * RUNS;                       // runs that exist from here on
-    if constexpr (BITS == 3) {                                     // 24-byte runs: 8-byte pieces unless rows are 16-aligned
-      constexpr uint32_t CH = C::kRowBytes / 8;
-      for (uint32_t i = tid; i < (uint32_t)C::kRows * CH; i += 256) {
-        const uint32_t row = i / CH, q = i - row * CH;
-        if (n0 + row < p.N && q / 3 < live)
-          cp_async8_s(dst0 + row * C::kRowBytes + q * 8, reinterpret_cast<const uint8_t*>(W + (size_t)(n0 + row) * p.KP) + (size_t)st * C::kRowBytes + q * 8);
-      }
-    } else {
-      constexpr uint32_t CH = C::kRowBytes / 16, CPR = F::kRunBytes / 16;
 #pragma unroll
-      for (uint32_t i = tid; i < (uint32_t)C::kRows * CH; i += 256) {
-        const uint32_t row = i / CH, q = i % CH, run = q / CPR;
-        const uint32_t sw = BITS == 4 ? (RUNS == 2 ? (row >> 1) & 1u : row & 3u) : row & 1u;
-        if (n0 + row < p.N && run < live)
-          cp_async16_s(dst0 + row * C::kRowBytes + (run ^ sw) * F::kRunBytes + (q % CPR) * 16,
-                       reinterpret_cast<const uint8_t*>(W + (size_t)(n0 + row) * p.KP) + (size_t)st * C::kRowBytes + q * 16);
+    for (uint32_t i = 0; i < NW; ++i)
+      if ((w_on >> i & 1u) && (live >= (uint32_t)RUNS || ((tid + 256u * i) % CH) * WP / F::kRunBytes < live)) {
+        if constexpr (W16) cp_async16_s(dst0 + w_dst[i], src0 + w_off[i]);
+        else cp_async8_s(dst0 + w_dst[i], src0 + w_off[i]);
       }
+  };
+  // scales and biases: thread = (table, row)
+  constexpr uint32_t NSB = (2 * C::kRows + 255) / 256;
+  const uint32_t spr_odd = p.SPR & 1u;
+  auto issue_sb = [&](uint32_t st) {
+    const uint32_t dst0 = sm + (st % C::kStages) * C::kStageBytes + C::kWBytes + C::kXBytes;
+    const uint32_t g0 = st * RUNS, have = p.SPR - g0 < (uint32_t)RUNS ? p.SPR - g0 : (uint32_t)RUNS;
+#pragma unroll
+    for (uint32_t i = 0; i < NSB; ++i) {
+      const uint32_t idx = tid + 256u * i, row = idx % C::kRows;
+      if (idx >= 2u * C::kRows || n0 + row >= p.N) continue;
+      const __half* src = (idx >= (uint32_t)C::kRows ? B : S) + (size_t)(n0 + row) * p.SPR + g0;
+      const uint32_t odd = (uint32_t)(reinterpret_cast<uintptr_t>(src) >> 1) & 1u, end = 2u * (odd + have);
+#pragma unroll
+      for (uint32_t w = 0; w <= (uint32_t)RUNS / 2; ++w)
+        if (w * 4u < end)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst0 + idx * C::kSbSlot + w * 4u),
+                       "l"(src - odd + 2 * w), "r"(end - w * 4u < 4u ? end - w * 4u : 4u) : "memory");
     }
   };
+  // activations: thread = (token mod XT, 16-byte piece)
+  constexpr uint32_t XC = RUNS * 8, XT = 256 / XC, NX = C::kTok / XT;
+  static_assert(C::kTok % XT == 0 && XT % 8 == 0, "tokens of a thread share their swizzle");
+  const uint32_t x_q = tid % XC, x_tok = tid / XC;
+  const uint32_t x_dst = C::kWBytes + x_tok * (RUNS * 128) + ((x_q ^ (x_tok & 7u)) << 4);
+  const __half* x_src[MOE ? NX : 1];
+  uint32_t x_on = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < NX; ++i) {
+    const uint32_t tok = x_tok + XT * i;
+    if (tok < ntok) x_on |= 1u << i;
+    if constexpr (MOE) x_src[i] = p.X + (tok < ntok ? in_off[tok] : 0ull) + x_q * 8;
+  }
+  if constexpr (!MOE) x_src[0] = p.X + (size_t)(t0 + x_tok) * p.x_row_stride + x_q * 8;
+  const size_t x_step = (size_t)XT * p.x_row_stride;
   auto issue_x = [&](uint32_t st) {
-    const uint32_t dst0 = sm + (st % C::kStages) * C::kStageBytes + C::kWBytes;
-    const uint32_t live = p.SPR - st * RUNS;
+    const uint32_t dst0 = sm + (st % C::kStages) * C::kStageBytes + x_dst;
+    if ((x_q >> 3) >= p.SPR - st * RUNS) return;                   // past the last run
 #pragma unroll
-    for (uint32_t i = tid; i < (uint32_t)C::kTok * RUNS * 8; i += 256) {
-      const uint32_t tok = i / (RUNS * 8), q = i % (RUNS * 8);
-      if (tok < ntok && (q >> 3) < live) {
-        const __half* src = MOE ? p.X + in_off[tok] : p.X + (size_t)(t0 + tok) * p.x_row_stride;
-        cp_async16_s(dst0 + tok * (RUNS * 128) + ((q ^ (tok & 7u)) << 4), src + (size_t)st * (RUNS * 64) + q * 8);
-      }
-    }
+    for (uint32_t i = 0; i < NX; ++i)
+      if (x_on >> i & 1u)
+        cp_async16_s(dst0 + i * (XT * RUNS * 128), (MOE ? x_src[MOE ? i : 0] : x_src[0] + i * x_step) + (size_t)st * (RUNS * 64));
   };
-  // sums of x per (run, token) of a landed stage
-  auto sums = [&](uint32_t st) {
-    const uint32_t src0 = sm + (st % C::kStages) * C::kStageBytes + C::kWBytes;
-    float* dst = xs_sm + (st & 1u) * (RUNS * C::kTok);
-    for (uint32_t i = tid; i < (uint32_t)RUNS * C::kTok; i += 256) {
-      const uint32_t tok = i % C::kTok, run = i / C::kTok;
-      if (tok >= ntok) continue;
-      float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-      for (uint32_t q = 0; q < 8; ++q) {
-        const uint4 v = tc_lds128(src0 + tok * (RUNS * 128) + (((run * 8 + q) ^ (tok & 7u)) << 4));
-        const float2 a = __half22float2(u32_as_h2(v.x)), b = __half22float2(u32_as_h2(v.y)),
-                     d = __half22float2(u32_as_h2(v.z)), e = __half22float2(u32_as_h2(v.w));
-        s0 += (a.x + a.y) + (b.x + b.y);
-        s1 += (d.x + d.y) + (e.x + e.y);
+  // A landed stage's activations, a warp per (run, eight tokens): their sums per token by the matrix unit (rows of ones), and
+  // the pairs of values put into the order of the code pairs, in place, so that the main loop loads B registers as they are.
+  auto prepare_x = [&](uint32_t st) {
+    uint8_t* const src0 = bm_smem + (st % C::kStages) * C::kStageBytes + C::kWBytes;
+    float* const dst = xs_sm + (st & 1u) * (RUNS * C::kTok);
+    constexpr uint32_t kOnes = 0x3C003C00u;
+#pragma unroll 1
+    for (uint32_t i = warp; i < (uint32_t)RUNS * (C::kTok / 8); i += 8) {
+      const uint32_t nb = i % (C::kTok / 8), run = i / (C::kTok / 8);
+      if (nb * 8 >= ntok) continue;
+      uint8_t* const row = src0 + (nb * 8 + (uint32_t)g) * (RUNS * 128);
+      uint4* const p0 = reinterpret_cast<uint4*>(row + (((run * 8 + 2 * c) ^ (uint32_t)g) << 4));
+      uint4* const p1 = reinterpret_cast<uint4*>(row + (((run * 8 + 2 * c + 1) ^ (uint32_t)g) << 4));
+      uint32_t b[8];
+      F::b(*p0, *p1, b);
+      float d[4];
+      bm_mma0(d, kOnes, kOnes, kOnes, kOnes, b[0], b[1]);
+      bm_mma(d, kOnes, kOnes, kOnes, kOnes, b[2], b[3]);
+      bm_mma(d, kOnes, kOnes, kOnes, kOnes, b[4], b[5]);
+      bm_mma(d, kOnes, kOnes, kOnes, kOnes, b[6], b[7]);
+      if (g == 0) *reinterpret_cast<float2*>(dst + run * C::kTok + nb * 8 + 2 * c) = make_float2(d[0], d[1]);
+      if constexpr (BITS != 8) {
+        *p0 = make_uint4(b[0], b[1], b[2], b[3]);
+        *p1 = make_uint4(b[4], b[5], b[6], b[7]);
       }
-      dst[i] = s0 + s1;
     }
   };
 
-  // ---- scales and biases of this warp's rows (g, g + 8, g + 16, g + 24) for its runs of the next stage ------------
   constexpr int RPW = RUNS / WK;
   static_assert(RPW >= 1 && RPW * WK == RUNS, "runs per warp");
-  const unsigned short* srow[4];
-  size_t brow_delta = reinterpret_cast<const unsigned short*>(B) - reinterpret_cast<const unsigned short*>(S);
-#pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    const uint32_t row = min(n0 + (uint32_t)(wm * 32 + g + 8 * h), p.N - 1);
-    srow[h] = reinterpret_cast<const unsigned short*>(S) + (size_t)row * p.SPR;
-  }
-  uint32_t sb_nxt[RPW][4];             // scale in the low half, bias in the high half
-  auto load_sb = [&](uint32_t st) {
-#pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-      const uint32_t grp = st * RUNS + (uint32_t)(r * WK + wk);
-      if (grp >= p.SPR) continue;
-#pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const uint32_t s = __ldg(srow[h] + grp), b = __ldg(srow[h] + brow_delta + grp);
-        sb_nxt[r][h] = s | (b << 16);
-      }
-    }
-  };
-
-  unsigned long long acc[2][NBW][2];
+  float acc[2][NBW][4];
 #pragma unroll
   for (int t = 0; t < 2; ++t)
 #pragma unroll
-    for (int j = 0; j < NBW; ++j) acc[t][j][0] = acc[t][j][1] = 0ull;
-  const float kZero[4] = {0.f, 0.f, 0.f, 0.f};
-  const unsigned long long kR = tc_pk(F::kRatio, F::kRatio);
+    for (int j = 0; j < NBW; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[t][j][e] = 0.f;
 
 #pragma unroll
   for (int s = 0; s < C::kStages - 1; ++s)
-    if ((uint32_t)s < stages) issue_w((uint32_t)s);
-  load_sb(0);
+    if ((uint32_t)s < stages) { issue_w((uint32_t)s); issue_sb((uint32_t)s); }
   if constexpr (!MOE) asm volatile("griddepcontrol.wait;" ::: "memory");   // weights first, then what a kernel before may have written
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll
@@ -191,30 +223,31 @@ batch_mma_kernel(const BatchParams p) {
   }
   asm volatile("cp.async.wait_group %0;" ::"n"(C::kStages - 2) : "memory");
   __syncthreads();
-  sums(0);
+  prepare_x(0);
 
   for (uint32_t st = 0; st < stages; ++st) {
     asm volatile("cp.async.wait_group %0;" ::"n"(C::kStages - 3) : "memory");   // stage st + 1 has landed
-    __syncthreads();                                                              // stage st - 1 is free, sums(st) are visible
-    if (st + C::kStages - 1 < stages) { issue_w(st + C::kStages - 1); issue_x(st + C::kStages - 1); }
+    __syncthreads();                                                              // stage st - 1 is free, the activations of stage st are prepared
+    if (st + C::kStages - 1 < stages) { issue_w(st + C::kStages - 1); issue_sb(st + C::kStages - 1); issue_x(st + C::kStages - 1); }
     tc_commit();
-    float sc[RPW][4], bi[RPW][4];
-#pragma unroll
-    for (int r = 0; r < RPW; ++r)
-#pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const float2 v = __half22float2(u32_as_h2(sb_nxt[r][h]));
-        sc[r][h] = v.x * F::kUnit; bi[r][h] = v.y;
-      }
-    load_sb(st + 1);
-    if (st + 1 < stages) sums(st + 1);
+    if (st + 1 < stages) prepare_x(st + 1);
 
-    const uint32_t wbase = sm + (st % C::kStages) * C::kStageBytes, xbase = wbase + C::kWBytes;
-    const float* xs = xs_sm + (st & 1u) * (RUNS * C::kTok);
+    const uint8_t* const wst = bm_smem + (st % C::kStages) * C::kStageBytes;
+    const uint8_t* const xst = wst + C::kWBytes;
+    const float* const xs = xs_sm + (st & 1u) * (RUNS * C::kTok);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
       const uint32_t run = (uint32_t)(r * WK + wk);
       if (st * RUNS + run >= p.SPR) break;
+      float sc[4], bi[4];              // of rows g, g + 8, g + 16, g + 24
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const uint32_t row = (uint32_t)(wm * 32 + g + 8 * h);
+        const uint32_t odd = (sb_odd0 + ((n0 + row) & spr_odd)) & 1u;        // a stage starts on an even group
+        const uint8_t* const at = xst + C::kXBytes + row * C::kSbSlot + (odd + run) * 2u;
+        sc[h] = __half2float(*reinterpret_cast<const __half*>(at)) * F::kUnit;
+        bi[h] = __half2float(*reinterpret_cast<const __half*>(at + C::kRows * C::kSbSlot));
+      }
       uint32_t a[2][2][8];             // [row tile][row g | g + 8][register]
 #pragma unroll
       for (int t = 0; t < 2; ++t)
@@ -224,35 +257,28 @@ batch_mma_kernel(const BatchParams p) {
           uint32_t pos = run;
           if constexpr (BITS == 4) pos = run ^ (RUNS == 2 ? (row >> 1) & 1u : row & 3u);
           if constexpr (BITS == 8) pos = run ^ (row & 1u);
-          F::a(F::load(bm_smem + (wbase - sm) + row * C::kRowBytes + pos * F::kRunBytes + F::lane_byte(c), c), a[t][h]);
+          F::a(F::load(wst + row * C::kRowBytes + pos * F::kRunBytes + F::lane_byte(c), c), a[t][h]);
         }
 #pragma unroll
       for (int j = 0; j < NBW; ++j) {
         const uint32_t nb = (uint32_t)(wn + WN * j);
         if (nb * 8 >= ntok) break;     // warp-uniform: the rest of the tile is empty
-        const uint32_t xrow = xbase + (nb * 8 + (uint32_t)g) * (RUNS * 128);
-        const uint4 x0 = tc_lds128(xrow + (((run * 8 + 2 * c) ^ (uint32_t)g) << 4));
-        const uint4 x1 = tc_lds128(xrow + (((run * 8 + 2 * c + 1) ^ (uint32_t)g) << 4));
-        uint32_t b[8];
-        F::b(x0, x1, b);
+        const uint8_t* const xrow = xst + (nb * 8 + (uint32_t)g) * (RUNS * 128);
+        const uint4 b0 = *reinterpret_cast<const uint4*>(xrow + (((run * 8 + 2 * c) ^ (uint32_t)g) << 4));
+        const uint4 b1 = *reinterpret_cast<const uint4*>(xrow + (((run * 8 + 2 * c + 1) ^ (uint32_t)g) << 4));
         const float2 xsv = *reinterpret_cast<const float2*>(xs + run * C::kTok + nb * 8 + 2 * c);
-        const unsigned long long xs2 = tc_pk(xsv.x, xsv.y);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          float d0[4], d1[4];
-          tc_mma(d0, a[t][0][0], a[t][1][0], a[t][0][1], a[t][1][1], b[0], b[1], kZero);
-          tc_mma(d1, a[t][0][4], a[t][1][4], a[t][0][5], a[t][1][5], b[4], b[5], kZero);
-          tc_mma(d0, a[t][0][2], a[t][1][2], a[t][0][3], a[t][1][3], b[2], b[3], d0);
-          tc_mma(d1, a[t][0][6], a[t][1][6], a[t][0][7], a[t][1][7], b[6], b[7], d1);
+          float d0[4], d1[4];          // 8-bit codes have one class: a single chain
+          bm_mma0(d0, a[t][0][0], a[t][1][0], a[t][0][1], a[t][1][1], b0.x, b0.y);
+          bm_mma(d0, a[t][0][2], a[t][1][2], a[t][0][3], a[t][1][3], b0.z, b0.w);
+          if constexpr (F::kTwoClasses) bm_mma0(d1, a[t][0][4], a[t][1][4], a[t][0][5], a[t][1][5], b1.x, b1.y);
+          else bm_mma(d0, a[t][0][4], a[t][1][4], a[t][0][5], a[t][1][5], b1.x, b1.y);
+          bm_mma(F::kTwoClasses ? d1 : d0, a[t][0][6], a[t][1][6], a[t][0][7], a[t][1][7], b1.z, b1.w);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            unsigned long long v;
-            if constexpr (F::kTwoClasses) v = tc_ffma2(tc_pk(d0[2 * h], d0[2 * h + 1]), kR, tc_pk(d1[2 * h], d1[2 * h + 1]));
-            else v = tc_pk(d0[2 * h] + d1[2 * h], d0[2 * h + 1] + d1[2 * h + 1]);
-            const float s = sc[r][2 * t + h], bb = bi[r][2 * t + h];
-            unsigned long long q = acc[t][j][h];
-            q = tc_ffma2(tc_pk(s, s), v, q);
-            acc[t][j][h] = tc_ffma2(tc_pk(bb, bb), xs2, q);
+          for (int e = 0; e < 4; ++e) {
+            const float v = F::kTwoClasses ? fmaf(d0[e], F::kRatio, d1[e]) : d0[e];
+            acc[t][j][e] = fmaf(bi[2 * t + (e >> 1)], (e & 1) ? xsv.y : xsv.x, fmaf(sc[2 * t + (e >> 1)], v, acc[t][j][e]));
           }
         }
       }
@@ -273,7 +299,7 @@ batch_mma_kernel(const BatchParams p) {
         for (int j = 0; j < NBW; ++j)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const float2 v = tc_unpk(acc[t][j][h]);
+            const float2 v = make_float2(acc[t][j][2 * h], acc[t][j][2 * h + 1]);
             float* d = out + (size_t)((wn + WN * j) * 8 + 2 * c) * C::kOutPitch + wm * 32 + t * 16 + h * 8 + g;
             d[0] = k ? d[0] + v.x : v.x;
             d[C::kOutPitch] = k ? d[C::kOutPitch] + v.y : v.y;
@@ -306,10 +332,10 @@ batch_mma_kernel(const BatchParams p) {
 }
 
 // ---- host side -------------------------------------------------------------------------------------------------------
-template <int BITS, int WM, int WN, int WK, int NBW, int RUNS, bool MOE>
+template <int BITS, int WM, int WN, int WK, int NBW, int RUNS, bool MOE, bool W16 = true>
 static cudaError_t launch_cfg(const BatchParams& p, uint32_t token_tiles, cudaStream_t st) {
   using C = BatchCfg<BITS, WM, WN, WK, NBW, RUNS>;
-  auto kern = batch_mma_kernel<BITS, WM, WN, WK, NBW, RUNS, MOE>;
+  auto kern = batch_mma_kernel<BITS, WM, WN, WK, NBW, RUNS, MOE, W16>;
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -352,10 +378,17 @@ bool batch_mma_supported(const GemvParams& g, int bits) {
 
 template <int BITS>
 static cudaError_t launch_dense(const BatchParams& p, int sm_count, cudaStream_t st) {
-  // 128 x 64 tiles (a larger tile re-reads weights and activations less often) while they give every SM a CTA; with
-  // fewer, the K loop is the time and the tiles whose warps split K four ways have the shortest.
-  const uint64_t tiles = (uint64_t)((p.N + 127) / 128) * ((p.M + 63) / 64);
-  if (p.M > 32 && tiles >= (uint64_t)sm_count) return launch_cfg<BITS, 4, 2, 1, 4, 2, false>(p, (p.M + 63) / 64, st);
+  // Tile by the work of the busiest SM: tiles dealt to it x their area x what a tile costs per element of its area. Larger
+  // tiles unpack a code and load an activation for more products (4096 x 4096 x 1024: 128 x 128 tiles 183 us, 128 x 64
+  // 201 us); the smallest, whose warps split K four ways, fill the chip with few rows.
+  const uint64_t sm = (uint64_t)sm_count;
+  auto cost = [&](uint32_t rows, uint32_t tok, uint32_t weight) {
+    const uint64_t tiles = (uint64_t)((p.N + rows - 1) / rows) * ((p.M + tok - 1) / tok);
+    return (tiles + sm - 1) / sm * rows * tok * weight;
+  };
+  const uint64_t big = p.M > 64 ? cost(128, 128, 88) : ~0ull, mid = p.M > 32 ? cost(128, 64, 100) : ~0ull, small = cost(64, 32, 125);
+  if (big <= mid && big <= small) return launch_cfg<BITS, 4, 2, 1, 8, 2, false>(p, (p.M + 127) / 128, st);
+  if (mid <= small) return launch_cfg<BITS, 4, 2, 1, 4, 2, false>(p, (p.M + 63) / 64, st);
   return launch_cfg<BITS, 2, 1, 4, 4, 4, false>(p, (p.M + 31) / 32, st);
 }
 cudaError_t launch_batch_mma(const GemvParams& g, int bits, int sm_count, cudaStream_t st) {
@@ -382,6 +415,11 @@ cudaError_t launch_batch_moe(const GemvParams& g, uint32_t tokens, uint32_t slot
   if (e != cudaSuccess) return e;
   const uint64_t by_rows = (uint64_t)(P + tok - 1) / tok + g.experts;
   const uint32_t max_tiles = (uint32_t)(by_rows < P ? by_rows : P);   // the kernel reads the real count
+  if (p.KP % 4u) {
+    if (tok == 16) return launch_cfg<3, 4, 1, 2, 2, 4, true, false>(p, max_tiles, st);
+    if (tok == 32) return launch_cfg<3, 4, 1, 2, 4, 4, true, false>(p, max_tiles, st);
+    return launch_cfg<3, 4, 2, 1, 4, 2, true, false>(p, max_tiles, st);
+  }
   if (tok == 16) return launch_cfg<3, 4, 1, 2, 2, 4, true>(p, max_tiles, st);
   if (tok == 32) return launch_cfg<3, 4, 1, 2, 4, 4, true>(p, max_tiles, st);
   return launch_cfg<3, 4, 2, 1, 4, 2, true>(p, max_tiles, st);

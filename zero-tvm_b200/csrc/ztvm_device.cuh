@@ -98,9 +98,9 @@ __device__ __forceinline__ void codes8_f32(uint32_t w0, uint32_t w1, float q[8])
   }
 }
 
-// In place for the matrix unit: bytes 0, 2 and bytes 1, 3 of a word as pairs of f16 subnormals q * 2^-24.
-__device__ __forceinline__ uint32_t codes8_inplace_even(uint32_t w) { return w & 0x00FF00FFu; }
-__device__ __forceinline__ uint32_t codes8_inplace_odd(uint32_t w) { return (w >> 8) & 0x00FF00FFu; }
+// For the matrix unit: bytes 0, 1 and bytes 2, 3 of a word as pairs of f16 subnormals q * 2^-24.
+__device__ __forceinline__ uint32_t codes8_pair01(uint32_t w) { return __byte_perm(w, 0u, 0x4140); }
+__device__ __forceinline__ uint32_t codes8_pair23(uint32_t w) { return __byte_perm(w, 0u, 0x4342); }
 
 // ---- 3-bit codes ---------------------------------------------------------------------------
 // A row is one LSB-first bitstream; 32 codes occupy exactly three words. Codes 8b..8b+7 of such a

@@ -51,13 +51,12 @@ struct Frag<8> {
   __device__ __forceinline__ static void a(const Raw& v, uint32_t (&r)[8]) {
     const uint32_t w[4] = {v.w.x, v.w.y, v.w.z, v.w.w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { r[2 * j] = codes8_inplace_even(w[j]); r[2 * j + 1] = codes8_inplace_odd(w[j]); }
+    for (int j = 0; j < 4; ++j) { r[2 * j] = codes8_pair01(w[j]); r[2 * j + 1] = codes8_pair23(w[j]); }
   }
+  // the activations as they lie in memory
   __device__ __forceinline__ static void b(const uint4& x0, const uint4& x1, uint32_t (&r)[8]) {
-    r[0] = __byte_perm(x0.x, x0.y, 0x5410); r[1] = __byte_perm(x0.x, x0.y, 0x7632);
-    r[2] = __byte_perm(x0.z, x0.w, 0x5410); r[3] = __byte_perm(x0.z, x0.w, 0x7632);
-    r[4] = __byte_perm(x1.x, x1.y, 0x5410); r[5] = __byte_perm(x1.x, x1.y, 0x7632);
-    r[6] = __byte_perm(x1.z, x1.w, 0x5410); r[7] = __byte_perm(x1.z, x1.w, 0x7632);
+    r[0] = x0.x; r[1] = x0.y; r[2] = x0.z; r[3] = x0.w;
+    r[4] = x1.x; r[5] = x1.y; r[6] = x1.z; r[7] = x1.w;
   }
 };
 
