@@ -9,6 +9,13 @@
 
 namespace ztvm {
 
+// ---- programmatic dependent launch -------------------------------------------------------------
+// Every kernel of a step is launched with programmatic stream serialisation (launch_chained): it lets the next one start as
+// soon as all its own blocks run, and waits for the one before -- its end, and its writes -- ahead of its first read or
+// write of anything but weights. A chain of short kernels then pays no launch latency between them.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- loads ---------------------------------------------------------------------------------
 // Streaming 128-bit load: weights are read exactly once, so they bypass L1 allocation.
 __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {

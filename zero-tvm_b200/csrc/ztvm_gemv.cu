@@ -28,6 +28,8 @@ template <int BITS, int MT, int ROWS, bool MOE>
 __global__ void __launch_bounds__(kGemvWarps * 32)
 gemv_kernel(const GemvParams p) {
   extern __shared__ float4 smem_f4[];
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   constexpr int WPU = BITS;  // words per 32-code unit: 8 bits -> 8, 4 bits -> 4, 3 bits -> 3
@@ -35,7 +37,7 @@ gemv_kernel(const GemvParams p) {
   const uint32_t* __restrict__ W = p.W;
   const __half* __restrict__ S = p.S;
   const __half* __restrict__ Bv = p.B;
-  const __half* __restrict__ X = p.X;
+  const __half* X = p.X;   // (not restrict: a read-only load could move ahead of pdl_wait)
   size_t out_base = 0;
   if (MOE) {
     const uint32_t token = blockIdx.y, slot = blockIdx.z;
@@ -219,6 +221,8 @@ template <int ROWS, bool MOE>
 __global__ void __launch_bounds__(kGemvWarps * 32)
 gemv_fma_m1_kernel(const GemvParams p) {
   extern __shared__ float4 smem_f4[];
+  pdl_launch_dependents();
+  pdl_wait();
   uint4* xsm = reinterpret_cast<uint4*>(smem_f4);
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -226,7 +230,7 @@ gemv_fma_m1_kernel(const GemvParams p) {
   const uint32_t* __restrict__ W = p.W;
   const __half* __restrict__ S = p.S;
   const __half* __restrict__ Bv = p.B;
-  const __half* __restrict__ X = p.X;
+  const __half* X = p.X;   // (not restrict: a read-only load could move ahead of pdl_wait)
   size_t out_base = 0;
   if (MOE) {
     const uint32_t token = blockIdx.y, slot = blockIdx.z;
@@ -354,9 +358,6 @@ gemv_fma_m1_kernel(const GemvParams p) {
 // (the first weight loads) is issued before griddepcontrol.wait; activations are read and outputs are
 // written only after it, and dependents are released as soon as the activations are staged.
 constexpr int kPersistWarps = 8;
-
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Weights travel global -> shared with per-lane 16-byte cp.async copies into a ring of DEPTH stages per
 // warp: the bytes in flight are bounded by shared memory (DEPTH x ROWS x 512 B per warp), not by
@@ -549,8 +550,7 @@ static cudaError_t launch_one(const GemvParams& p, dim3 grid, size_t smem, cudaS
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  kern<<<grid, kGemvWarps * 32, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_chained(kern, grid, dim3(kGemvWarps * 32), smem, st, p);
 }
 
 template <int ROWS, bool MOE>
@@ -566,8 +566,7 @@ static cudaError_t launch_fma_m1(const GemvParams& p, dim3 grid, cudaStream_t st
   }
   const uint32_t units = p.K >> 5, units_up = (units + 31) & ~31u;
   const size_t smem = (size_t)units_up * 64 + (size_t)units_up * 4;
-  kern<<<grid, kGemvWarps * 32, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_chained(kern, grid, dim3(kGemvWarps * 32), smem, st, p);
 }
 
 template <int ROWS, int DEPTH>

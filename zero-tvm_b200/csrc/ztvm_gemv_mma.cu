@@ -71,6 +71,8 @@ template <int WPL, int NTOK, bool MOE>
 __global__ void __launch_bounds__(kMmaMaxWarps * 32)
 gemv_mma_kernel(const GemvParams p) {
   extern __shared__ uint4 smem_u4[];
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int GROUP = WPL * 32;
   constexpr int NV = NTOK <= 1 ? 1 : 2;  // tokens per lane that can be live: (2c) and (2c+1)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -79,7 +81,7 @@ gemv_mma_kernel(const GemvParams p) {
   const uint32_t* __restrict__ W = p.W;
   const __half* __restrict__ S = p.S;
   const __half* __restrict__ Bv = p.B;
-  const __half* __restrict__ X = p.X;
+  const __half* X = p.X;   // (not restrict: a read-only load could move ahead of pdl_wait)
   size_t out_base = 0;
   if (MOE) {
     const uint32_t token = blockIdx.y, slot = blockIdx.z;
@@ -286,8 +288,7 @@ static cudaError_t launch_mma_one(const GemvParams& p, dim3 grid, int threads, s
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  kern<<<grid, threads, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_chained(kern, grid, dim3(threads), smem, st, p);
 }
 
 template <int WPL, bool MOE>

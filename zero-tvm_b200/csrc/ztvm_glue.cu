@@ -188,11 +188,13 @@ cudaError_t launch_dequant(const uint32_t* W, const __half* S, const __half* B, 
 // out[t][:] = the dequantised row input_ids[t] of an affine-quantised table, f16: the canonical W16 (what the vendor
 // dequantiser stores), through the same word dequantiser as the GEMMs for 4-bit codes. One thread per 8 values.
 template <int BITS>
-__global__ void embedding_affine_kernel(const int32_t* __restrict__ input_ids, const uint32_t* __restrict__ W,
-                                        const __half* __restrict__ S, const __half* __restrict__ B, __half* __restrict__ out,
+__global__ void embedding_affine_kernel(const int32_t* input_ids, const uint32_t* W,
+                                        const __half* S, const __half* B, __half* out,
                                         uint32_t seq_len, uint32_t D, uint32_t vocab, uint32_t* err) {
   const uint32_t nblk = D >> 3, KP = D * BITS / 32, SPR = D >> 6;
   const size_t total = (size_t)seq_len * nblk;
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const uint32_t t = (uint32_t)(i / nblk), blk = (uint32_t)(i - (size_t)t * nblk);
     const int32_t id = input_ids[t];
@@ -223,9 +225,8 @@ cudaError_t launch_embedding_affine(const int32_t* input_ids, const uint32_t* W,
                                     uint32_t seq_len, uint32_t D, uint32_t vocab, int bits, uint32_t* err, cudaStream_t st) {
   const size_t total = (size_t)seq_len * (D >> 3);
   if (total == 0) return cudaSuccess;
-  if (bits == 4) embedding_affine_kernel<4><<<grid_for(total, 256), 256, 0, st>>>(input_ids, W, S, B, out, seq_len, D, vocab, err);
-  else embedding_affine_kernel<8><<<grid_for(total, 256), 256, 0, st>>>(input_ids, W, S, B, out, seq_len, D, vocab, err);
-  return cudaGetLastError();
+  return launch_chained(bits == 4 ? embedding_affine_kernel<4> : embedding_affine_kernel<8>, dim3(grid_for(total, 256)), dim3(256), 0, st,
+                        input_ids, W, S, B, out, seq_len, D, vocab, err);
 }
 
 // ---- f16 matvec with f32 accumulation and f32 output (moe_router_logits_f16.wgsl) -------------------------------
@@ -283,11 +284,13 @@ cudaError_t launch_f16_matvec(const __half* x, const __half* w, float* y, uint32
 constexpr int kTopkPerLane = 32;
 
 template <int PER>
-__global__ void __launch_bounds__(128) route_topk_kernel(const float* __restrict__ logits, uint32_t* __restrict__ ids,
-                                                          float* __restrict__ scores, uint32_t tokens, uint32_t E,
+__global__ void __launch_bounds__(128) route_topk_kernel(const float* logits, uint32_t* ids,
+                                                          float* scores, uint32_t tokens, uint32_t E,
                                                           uint32_t K, uint32_t norm_topk, uint32_t has_shared) {
   const int lane = threadIdx.x & 31;
   const uint32_t tok = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  pdl_launch_dependents();
+  pdl_wait();
   if (tok >= tokens) return;
   const float* l = logits + (size_t)tok * (E + has_shared);
   const size_t obase = (size_t)tok * (K + has_shared);
@@ -322,12 +325,11 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const float* __restrict
     for (int i = 0; i < PER; ++i) {  // ascending expert index within the lane: strict > keeps the lower one
       if (pv[i] > bv) { bv = pv[i]; bi = (uint32_t)i * 32 + lane; }
     }
-    float best = bv;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
-    uint32_t widx = bv == best ? bi : 0xffffffffu;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) widx = min(widx, __shfl_xor_sync(0xffffffffu, widx, o));
+    // non-negative floats order like their bits, and the -1 of a taken expert is a negative integer: two warp-wide integer
+    // reductions find the winner (shuffles took ten dependent steps per round)
+    const int best_bits = __reduce_max_sync(0xffffffffu, __float_as_int(bv));
+    const float best = __int_as_float(best_bits);
+    const uint32_t widx = __reduce_min_sync(0xffffffffu, __float_as_int(bv) == best_bits ? bi : 0xffffffffu);
     total += best;
     if ((uint32_t)lane == k) my_top = best;
 #pragma unroll
@@ -346,9 +348,8 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const float* __restrict
 cudaError_t launch_route_topk(const float* logits, uint32_t* ids, float* scores, uint32_t tokens, uint32_t E,
                               uint32_t K, bool norm_topk, bool has_shared, cudaStream_t st) {
   const unsigned grid = (tokens + 3) / 4;
-  if (E <= 256) route_topk_kernel<8><<<grid, 128, 0, st>>>(logits, ids, scores, tokens, E, K, norm_topk, has_shared);
-  else route_topk_kernel<kTopkPerLane><<<grid, 128, 0, st>>>(logits, ids, scores, tokens, E, K, norm_topk, has_shared);
-  return cudaGetLastError();
+  return launch_chained(E <= 256 ? route_topk_kernel<8> : route_topk_kernel<kTopkPerLane>, dim3(grid), dim3(128), 0, st, logits, ids, scores,
+                        tokens, E, K, norm_topk, has_shared);
 }
 
 // ---- SiLU * up -----------------------------------------------------------------------------------
@@ -359,10 +360,12 @@ __device__ __forceinline__ float silu_mul_one(float g, float u) {
 }
 // VEC = 8: eight elements per thread (16-byte loads and stores; ffn % 8 == 0, 16-byte aligned buffers), else one.
 template <int VEC>
-__global__ void silu_mul_kernel(const __half* __restrict__ gate_up, __half* __restrict__ h, uint32_t rows, uint32_t ffn,
-                                const uint32_t* __restrict__ seg_counts, uint32_t seg_cap) {
+__global__ void silu_mul_kernel(const __half* gate_up, __half* h, uint32_t rows, uint32_t ffn,
+                                const uint32_t* seg_counts, uint32_t seg_cap) {
   const uint32_t per_row = ffn / VEC;
   const size_t total = (size_t)rows * per_row;
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / per_row, c = (i - r * per_row) * VEC;
     if (seg_counts && (uint32_t)(r % seg_cap) >= seg_counts[r / seg_cap]) continue;   // past the region's live rows
@@ -390,15 +393,16 @@ cudaError_t launch_silu_mul(const __half* gate_up, __half* h, uint32_t rows, uin
   const size_t total = (size_t)rows * ffn;
   if (total == 0) return cudaSuccess;
   const bool vec = ffn % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(h)) & 15u) == 0;
-  if (vec) silu_mul_kernel<8><<<grid_for(total / 8, 256), 256, 0, st>>>(gate_up, h, rows, ffn, seg_counts, seg_cap ? seg_cap : 1u);
-  else silu_mul_kernel<1><<<grid_for(total, 256), 256, 0, st>>>(gate_up, h, rows, ffn, seg_counts, seg_cap ? seg_cap : 1u);
-  return cudaGetLastError();
+  return launch_chained(vec ? silu_mul_kernel<8> : silu_mul_kernel<1>, dim3(grid_for(vec ? total / 8 : total, 256)), dim3(256), 0, st, gate_up, h,
+                        rows, ffn, seg_counts, seg_cap ? seg_cap : 1u);
 }
 
 // The same over f32 [gate(ffn) | up(ffn)] rows: the second step of the fused FFN on shapes the paired GEMV does not
 // take (fused_ffn.wgsl keeps both dot products in f32 up to the final store).
-__global__ void silu_mul_f32_kernel(const float* __restrict__ gate_up, __half* __restrict__ h, uint32_t rows, uint32_t ffn) {
+__global__ void silu_mul_f32_kernel(const float* gate_up, __half* h, uint32_t rows, uint32_t ffn) {
   const size_t total = (size_t)rows * ffn;
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / ffn, c = i - r * ffn;
     h[i] = __float2half_rn(silu_mul_one(gate_up[r * 2 * ffn + c], gate_up[r * 2 * ffn + ffn + c]));
@@ -407,37 +411,47 @@ __global__ void silu_mul_f32_kernel(const float* __restrict__ gate_up, __half* _
 cudaError_t launch_silu_mul_f32(const float* gate_up, __half* h, uint32_t rows, uint32_t ffn, cudaStream_t st) {
   const size_t total = (size_t)rows * ffn;
   if (total == 0) return cudaSuccess;
-  silu_mul_f32_kernel<<<grid_for(total, 256), 256, 0, st>>>(gate_up, h, rows, ffn);
-  return cudaGetLastError();
+  return launch_chained(silu_mul_f32_kernel, dim3(grid_for(total, 256)), dim3(256), 0, st, gate_up, h, rows, ffn);
 }
 
 // ---- weighted combine -----------------------------------------------------------------------------
 // out[t][i] = f16(sum_s score[t][s] * f32(y[t][s][i])), slots added in index order (moe_combine.wgsl:39-43).
 template <int VEC>
-__global__ void moe_combine_kernel(const __half* __restrict__ y, const float* __restrict__ scores, __half* __restrict__ out,
+__global__ void moe_combine_kernel(const __half* y, const float* scores, __half* out,
                                    uint32_t tokens, uint32_t slots, uint32_t d) {
   const uint32_t per_row = d / VEC;
   const size_t total = (size_t)tokens * per_row;
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t t = i / per_row, c = (i - t * per_row) * VEC;
     float acc[VEC];
 #pragma unroll
     for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
-    for (uint32_t s = 0; s < slots; ++s) {
-      const float sc = scores[t * slots + s];
-      const __half* src = y + (t * slots + s) * d + c;
-      if constexpr (VEC == 8) {
-        const uint4 v = *reinterpret_cast<const uint4*>(src);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const __half* const src = y + t * slots * d + c;
+    const float* const sc = scores + t * slots;
+    if constexpr (VEC == 8) {
+      // four slots' rows are in flight together; they are added in index order
+      for (uint32_t s = 0; s < slots; s += 4) {
+        uint4 v[4];
+        float f[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 f = __half22float2(u32_as_h2(w[k]));
-          acc[2 * k] = __fadd_rn(acc[2 * k], __fmul_rn(sc, f.x));
-          acc[2 * k + 1] = __fadd_rn(acc[2 * k + 1], __fmul_rn(sc, f.y));
+        for (uint32_t u = 0; u < 4; ++u)
+          if (s + u < slots) { v[u] = *reinterpret_cast<const uint4*>(src + (size_t)(s + u) * d); f[u] = sc[s + u]; }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+          if (s + u >= slots) break;
+          const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 h2 = __half22float2(u32_as_h2(w[k]));
+            acc[2 * k] = __fadd_rn(acc[2 * k], __fmul_rn(f[u], h2.x));
+            acc[2 * k + 1] = __fadd_rn(acc[2 * k + 1], __fmul_rn(f[u], h2.y));
+          }
         }
-      } else {
-        acc[0] = __fadd_rn(acc[0], __fmul_rn(sc, __half2float(src[0])));
       }
+    } else {
+      for (uint32_t s = 0; s < slots; ++s) acc[0] = __fadd_rn(acc[0], __fmul_rn(sc[s], __half2float(src[(size_t)s * d])));
     }
     if constexpr (VEC == 8) {
       uint32_t ow[4];
@@ -457,9 +471,8 @@ cudaError_t launch_moe_combine(const __half* y_slots, const float* scores, __hal
   const size_t total = (size_t)tokens * d;
   if (total == 0) return cudaSuccess;
   const bool vec = d % 8 == 0 && ((reinterpret_cast<uintptr_t>(y_slots) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
-  if (vec) moe_combine_kernel<8><<<grid_for(total / 8, 256), 256, 0, st>>>(y_slots, scores, out, tokens, slots, d);
-  else moe_combine_kernel<1><<<grid_for(total, 256), 256, 0, st>>>(y_slots, scores, out, tokens, slots, d);
-  return cudaGetLastError();
+  return launch_chained(vec ? moe_combine_kernel<8> : moe_combine_kernel<1>, dim3(grid_for(vec ? total / 8 : total, 256)), dim3(256), 0, st,
+                        y_slots, scores, out, tokens, slots, d);
 }
 
 }  // namespace ztvm

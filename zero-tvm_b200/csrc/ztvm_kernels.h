@@ -6,6 +6,23 @@
 
 namespace ztvm {
 
+// Launch with programmatic stream serialisation: for kernels that call pdl_wait() (ztvm_device.cuh) before they touch what
+// the kernel before may write or still read.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 struct GemvParams {
   const uint32_t* W;   // packed codes [N][KP] (MoE: [experts][N][KP])
   const __half* S;     // scales [N][SPR]

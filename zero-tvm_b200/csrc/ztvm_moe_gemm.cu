@@ -110,12 +110,14 @@ __device__ __forceinline__ uint32_t moe_agg_add(uint32_t* cnt, uint32_t key, boo
 // same scans, same tables. Pairs are walked slot-major (a warp sees 32 tokens of one slot), so the pairs of a slot
 // that always carries the same expert (the shared expert) aggregate into one atomic per warp.
 constexpr uint32_t kPlanSmallMax = 32768;   // pairs the one-block plan takes: 32 per thread, kept in registers
-__global__ void __launch_bounds__(1024) moe_plan_small_kernel(const uint32_t* __restrict__ ids, uint32_t tokens, uint32_t slots,
+__global__ void __launch_bounds__(1024) moe_plan_small_kernel(const uint32_t* ids, uint32_t tokens, uint32_t slots,
                                                               uint32_t ids_stride, uint32_t E, uint32_t tile_rows,
                                                               MoeScratch sc, uint32_t* err, MoeSegs segs) {
   __shared__ uint32_t cnt_sm[1024], cur_sm[1024], warp_sums[32];
   const uint32_t e = threadIdx.x, P = tokens * slots;
   cnt_sm[e] = 0u;
+  pdl_launch_dependents();
+  pdl_wait();
   // every id of this thread is loaded up front (independent loads in flight together), then counted, then scattered
   uint32_t xs[kPlanSmallMax / 1024];
 #pragma unroll
@@ -407,8 +409,8 @@ cudaError_t launch_moe_plan(const GemvParams& g, uint32_t tokens, uint32_t slots
   const uint32_t P = tokens * slots, E = g.experts;
   const MoeSegs segs{g.seg_counts, g.seg_cap ? g.seg_cap : 1u};
   if (P <= kPlanSmallMax) {   // short lists: one block does it all, nothing to clear beforehand
-    moe_plan_small_kernel<<<1, 1024, 0, st>>>(g.ids, tokens, slots, g.ids_stride, E, tile_rows, sc, g.err_counter, segs);
-    return cudaGetLastError();
+    return launch_chained(moe_plan_small_kernel, dim3(1), dim3(1024), 0, st, g.ids, tokens, slots, g.ids_stride, E, tile_rows, sc,
+                          g.err_counter, segs);
   }
   cudaError_t e = cudaMemsetAsync(sc.counts, 0, ((size_t)E * 3 + 4) * 4, st);   // counts, offsets, cursor, ntiles
   if (e != cudaSuccess) return e;

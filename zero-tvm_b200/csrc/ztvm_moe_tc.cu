@@ -36,6 +36,8 @@ struct MoeTcParams {
 __global__ void __launch_bounds__(kTcWarps * 32, 1)
 moe_tc_kernel(const MoeTcParams p) {
   extern __shared__ __align__(128) uint8_t mt_smem[];
+  pdl_launch_dependents();
+  pdl_wait();                                            // the plan may come from the kernel before
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, c = lane & 3;
 
@@ -235,8 +237,7 @@ cudaError_t launch_moe_tc(const GemvParams& g, uint32_t tokens, uint32_t slots, 
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  moe_tc_kernel<<<sm_count, kTcWarps * 32, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_chained(moe_tc_kernel, dim3(sm_count), dim3(kTcWarps * 32), smem, st, p);
 }
 
 }  // namespace ztvm
