@@ -55,22 +55,23 @@ def test_router_logits_many_tokens(bits, T, rows, D, backend, dev):
     assert np.abs(got - ref).max() <= 1e-5 * np.sqrt(np.mean(ref * ref))
 
 
-@pytest.mark.parametrize("T,E,d,ffn,slots", [(9, 40, 192, 72, 4), (40, 12, 320, 136, 4), (97, 3, 256, 200, 2)])   # tiles of 16, 32, 64 pairs
-def test_grouped_3bit_experts(T, E, d, ffn, slots, backend, dev, oracle_c):
-    """3-bit experts through the grouped form: rows that fill no 128-row block, K of 3, 5 and 4 scale groups, ragged
+@pytest.mark.parametrize("bits,T,E,d,ffn,slots", [(3, 9, 40, 192, 72, 4), (3, 40, 12, 320, 136, 4), (3, 97, 3, 256, 200, 2),   # tiles of 16, 32, 64 pairs
+                                                  (4, 33, 40, 192, 72, 4), (4, 20, 9, 448, 136, 4)])    # K the streaming kernel does not take
+def test_grouped_experts(bits, T, E, d, ffn, slots, backend, dev, oracle_c):
+    """Experts through the grouped form: rows that fill no 128-row block, K of 3, 5 and 4 scale groups, ragged
     last tiles, a skewed expert, gate (shared input) and down (input per slot)."""
     rng = np.random.default_rng(T + E)
     ids = rng.integers(0, E, size=(T, slots), dtype=np.uint32)
     ids[:, 0] = 1
     for N, K, per_slot in ((ffn, d, False), (d, 64 * ((ffn + 63) // 64), True)):
-        _, W, s, b = z.synth.make_weights(rng, N, K, bits=3, sigma_s=0.02, lead=(E,))
+        _, W, s, b = z.synth.make_weights(rng, N, K, bits=bits, sigma_s=0.02, lead=(E,))
         x = z.synth.make_x(rng, T * slots if per_slot else T, K)
         y = dev.empty((T, slots, N), np.float16, fill=float("nan"))
-        desc = z.MoeDesc(z.MmDesc(K, N, 1, 64, 3, 1, 0), E, slots, T, K if per_slot else 0, N, slots * K if per_slot else K, slots * N, slots)
+        desc = z.MoeDesc(z.MmDesc(K, N, 1, 64, bits, 1, 0), E, slots, T, K if per_slot else 0, N, slots * K if per_slot else K, slots * N, slots)
         backend.ctx.int4_matmul_moe(desc, y, dev.put(x), dev.put(s), dev.put(W), dev.put(b), dev.put(ids))
         got = dev.get(y)
         assert backend.ctx.device_errors() == 0 and np.isfinite(got).all()
-        ref = oracle_c.moe_matmul_f64(x, W, s, b, ids, N, K, 64, 3, in_per_slot=per_slot)
+        ref = oracle_c.moe_matmul_f64(x, W, s, b, ids, N, K, 64, bits, in_per_slot=per_slot)
         record_parity(zo.rel_err_scaled(got, ref, 1e-3), zo.rel_err(got, ref))
-        mags = oracle_c.moe_matmul_f64(np.abs(x), W, s, np.abs(b), ids, N, K, 64, 3, in_per_slot=per_slot)
+        mags = oracle_c.moe_matmul_f64(np.abs(x), W, s, np.abs(b), ids, N, K, 64, bits, in_per_slot=per_slot)
         assert (np.abs(got - ref) <= f16_bound(ref, mags, K)).all()

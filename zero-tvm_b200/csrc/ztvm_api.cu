@@ -537,6 +537,9 @@ static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::Ge
   // for both keeps the three projections of a block on one kernel, whose plan they can then share.
   const bool few_per_expert = pairs < 10ull * md->experts;
   if (d->bits == 3) return ztvm::batch_moe_supported(p, 3) ? 4 : 0;    // exact codes at every pair count
+  // A K that the streaming kernel does not take: the batched kernel holds its place below the same crossing (2240 x 512
+  // experts, 576 pairs: 45 against 96 us per projection).
+  if (forced < 0 && !stream_ok && few_per_expert && !p.dst_index && !p.seg_counts && ztvm::batch_moe_supported(p, 4)) return 4;
   if (forced == 1) return tiles ? tiles : stream_ok ? 2 : 0;
   if (forced == 2) return stream_ok ? 2 : tiles;
   return (stream_ok && (few_per_expert || !tiles)) ? 2 : tiles;
@@ -582,11 +585,13 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
   // expert's weights once (streaming kernel); with many pairs per expert it is a real contraction (tensor-core tiles,
   // each expert's weights dequantised once per 128 pairs).
   const uint64_t pairs = (uint64_t)md->tokens * md->slots;
-  const bool want_grouped = ctx->moe_grouped < 0 ? pairs >= (d->bits == 3 ? 32u : 128u) : ctx->moe_grouped >= 1;
+  // (3-bit codes, whose per-pair kernel is slow, from 32 pairs on; the exact-code grouped kernels of 4-bit ones from 64 on.)
+  const bool want_grouped = ctx->moe_grouped < 0 ? pairs >= (d->bits == 3 ? 32u : 64u) : ctx->moe_grouped >= 1;
   if (want_grouped && pairs < (1ull << 31)) {
     const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
     const int pick = moe_pick(ctx, md, p, y);
-    if (pick) {
+    const bool f16_weights = pick == 1 || pick == 3;
+    if (pick && !(ctx->moe_grouped < 0 && f16_weights && pairs < 128)) {
       const size_t need = ztvm::moe_grouped_scratch_bytes(md->experts, (uint32_t)pairs);
       if (ctx->d_ws_bytes < need) {
         ZTVM_CUDA(cudaDeviceSynchronize());
@@ -599,7 +604,7 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
       const bool reuse = ctx->plan_reuse && pick != 3 && ctx->plan_ids == ids && ctx->plan_segs == nullptr &&
                          ctx->plan_tokens == md->tokens && ctx->plan_slots == md->slots && ctx->plan_stride == md->ids_stride &&
                          ctx->plan_tile_rows == tile_rows && ctx->plan_experts == md->experts;
-      if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe(p, md->tokens, md->slots, ws, st, reuse));
+      if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe(p, (int)d->bits, md->tokens, md->slots, ws, st, reuse));
       else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
       else if (pick == 1) ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, md->slots, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
       else ZTVM_CUDA(ztvm::launch_moe_grouped(p, md->tokens, md->slots, ws, ctx->err_counter + 1, st));
@@ -654,11 +659,12 @@ ztvm_status ztvm_int4_matmul_moe_noalloc(ztvm_ctx* ctx, const ztvm_moe_desc* md,
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
   const int pick = moe_pick(ctx, md, p, y);   // the same choice ztvm_int4_matmul_moe makes
-  if (!pick || pick == 4)
+  if (!pick || d->bits != 4)
     return fail(ZTVM_ERR_UNSUPPORTED,
                 "this entry point runs the grouped kernels only: bits=4, group=64, K %% 64 == 0, N %% 8 == 0 "
                 "(got bits=%u group=%u K=%u N=%u)", d->bits, d->group, d->K, d->N);
-  if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc_static(p, md->tokens, md->slots, ctx->sm_count, st));
+  if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe_static(p, (int)d->bits, md->tokens, md->slots, st));
+  else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc_static(p, md->tokens, md->slots, ctx->sm_count, st));
   else if (pick == 1) ZTVM_CUDA(ztvm::launch_moe_ta_static(p, md->tokens, md->slots, ctx->err_counter + 1, ctx->sm_count, st));
   else ZTVM_CUDA(ztvm::launch_moe_grouped_static(p, md->tokens, md->slots, ctx->err_counter + 1, st));
   return ZTVM_OK;

@@ -2,7 +2,7 @@
 // activation rows, dense or grouped by expert, where the weights may not be rounded to f16 first:
 //   * router logits (moe_router_logits.wgsl: f32 sums over exact codes feed a softmax and a top-k),
 //   * 8-bit projections of more than eight rows (int8_affine_batched.wgsl),
-//   * 3-bit expert matmuls (int4_matmul.gen.ts:229-254, :409-448).
+//   * 3-bit expert matmuls (int4_matmul.gen.ts:229-254, :409-448), and 4-bit ones of few pairs per expert over a ragged K.
 // Those used to run as slabs of eight rows (or, for experts, one GEMV per pair) on the CUDA cores.
 //
 // Codes enter the MMA as f16 subnormals masked in place (ztvm_frag.cuh): no dequantisation, exact products, one f32
@@ -399,12 +399,12 @@ cudaError_t launch_batch_mma(const GemvParams& g, int bits, int sm_count, cudaSt
 // Grouped by expert. Tile width by the average number of pairs an expert has: a tile's weights are streamed once for
 // its whole token tile, its MMAs run over the token blocks that exist.
 bool batch_moe_supported(const GemvParams& g, int bits) {
-  return bits == 3 && batch_common_ok(g) && (g.in_slot_stride | g.in_tok_stride) % 8u == 0 && g.experts <= 1024 && !g.dst_index;
+  return (bits == 3 || bits == 4) && batch_common_ok(g) && (g.in_slot_stride | g.in_tok_stride) % 8u == 0 && g.experts <= 1024 && !g.dst_index;
 }
 uint32_t batch_moe_tile_rows(uint32_t experts, uint64_t pairs) {
   return pairs <= 10ull * experts ? 16u : pairs <= 24ull * experts ? 32u : 64u;
 }
-cudaError_t launch_batch_moe(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan) {
+cudaError_t launch_batch_moe(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan) {
   const uint32_t P = tokens * slots, tok = batch_moe_tile_rows(g.experts, P);
   BatchParams p = batch_params(g);
   p.slots = slots;
@@ -415,6 +415,11 @@ cudaError_t launch_batch_moe(const GemvParams& g, uint32_t tokens, uint32_t slot
   if (e != cudaSuccess) return e;
   const uint64_t by_rows = (uint64_t)(P + tok - 1) / tok + g.experts;
   const uint32_t max_tiles = (uint32_t)(by_rows < P ? by_rows : P);   // the kernel reads the real count
+  if (bits == 4) {
+    if (tok == 16) return launch_cfg<4, 4, 1, 2, 2, 4, true>(p, max_tiles, st);
+    if (tok == 32) return launch_cfg<4, 4, 1, 2, 4, 4, true>(p, max_tiles, st);
+    return launch_cfg<4, 4, 2, 1, 4, 2, true>(p, max_tiles, st);
+  }
   if (p.KP % 4u) {
     if (tok == 16) return launch_cfg<3, 4, 1, 2, 2, 4, true, false>(p, max_tiles, st);
     if (tok == 32) return launch_cfg<3, 4, 1, 2, 4, 4, true, false>(p, max_tiles, st);

@@ -245,8 +245,11 @@ gemv_fma_m1_kernel(const GemvParams p) {
     X += (size_t)token * p.in_tok_stride + (size_t)slot * p.in_slot_stride;
     out_base = (size_t)token * p.out_tok_stride + (size_t)slot * p.out_slot_stride;
   }
-  const uint32_t row0 = (blockIdx.x * kGemvWarps + warp) * ROWS;
+  // A K of 16 units or fewer (512 codes) would leave half of the lanes without work: each half of the warp takes a row of its own
   const uint32_t units = p.K >> 5;
+  const uint32_t sub = units <= 16u ? 2u : 1u, span = 32u / sub;
+  const uint32_t lane_u = (uint32_t)lane & (span - 1u), lane_r = (uint32_t)lane / span;
+  const uint32_t row0 = (blockIdx.x * kGemvWarps + warp) * ROWS * sub + lane_r;
   const uint32_t units_up = (units + 31) & ~31u;
   const int gshift = p.group_shift - 5;
   const uint32_t* wrow[ROWS];
@@ -254,7 +257,7 @@ gemv_fma_m1_kernel(const GemvParams p) {
   const __half* brow[ROWS];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    const uint32_t row = min(row0 + r, p.N - 1);
+    const uint32_t row = min(row0 + r * sub, p.N - 1);
     wrow[r] = W + (size_t)row * p.KP;
     srow[r] = S + (size_t)row * p.SPR;
     brow[r] = Bv ? Bv + (size_t)row * p.SPR : nullptr;
@@ -262,7 +265,7 @@ gemv_fma_m1_kernel(const GemvParams p) {
   // first round of weights goes out before the activations are staged
   uint4 wcur[ROWS];
   {
-    const uint32_t u = min((uint32_t)lane, units - 1);
+    const uint32_t u = min(lane_u, units - 1);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) wcur[r] = ld_stream_u4(wrow[r] + (size_t)u * 4);
   }
@@ -295,10 +298,10 @@ gemv_fma_m1_kernel(const GemvParams p) {
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) acc[r] = 0.f;
 
-  for (uint32_t u = lane; u < units; u += 32) {
+  for (uint32_t u = lane_u; u < units; u += span) {
     uint4 wnext[ROWS];
     {
-      const uint32_t un = min(u + 32, units - 1);
+      const uint32_t un = min(u + span, units - 1);
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) wnext[r] = ld_stream_u4(wrow[r] + (size_t)un * 4);
     }
@@ -340,9 +343,12 @@ gemv_fma_m1_kernel(const GemvParams p) {
   }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    const float v = warp_sum(acc[r]);
-    const uint32_t row = row0 + r;
-    if (lane == 0 && row < p.N) {
+    float v = acc[r];
+    if (sub == 1u) v += __shfl_xor_sync(0xffffffffu, v, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const uint32_t row = row0 + r * sub;
+    if (lane_u == 0 && row < p.N) {
       const size_t o = MOE ? out_base + row : (size_t)row;
       if (p.out_f32) reinterpret_cast<float*>(p.Y)[o] = v;
       else reinterpret_cast<__half*>(p.Y)[o] = __float2half_rn(v);
@@ -618,7 +624,7 @@ cudaError_t launch_gemv(GemvParams p, int bits, bool moe, uint32_t tokens, uint3
   // rows per warp: 4 when that still leaves every SM several CTAs, else fewer
   const uint64_t pairs = moe ? (uint64_t)tokens * slots : 1;
   int rows = 4;
-  while (rows > 1 && ((uint64_t)(p.N + kGemvWarps * rows - 1) / (kGemvWarps * rows)) * pairs < (uint64_t)sm_count * 4)
+  while (rows > 1 && ((uint64_t)(p.N + kGemvWarps * rows - 1) / (kGemvWarps * rows)) * pairs < (uint64_t)sm_count * (moe ? 1 : 4))
     rows >>= 1;
   if ((mt == 8 || bits == 8) && rows > 2) rows = 2;  // register pressure
   const uint32_t units = p.K >> 5;
@@ -634,6 +640,8 @@ cudaError_t launch_gemv(GemvParams p, int bits, bool moe, uint32_t tokens, uint3
     return launch_fma_m1_persist<4, 4>(p, sm_count, st);
   }
   if (bits == 4 && mt == 1 && p.K <= 40960) {  // 4-bit decode row: the conversion-free FMA kernel
+    const uint32_t per_cta = (uint32_t)(kGemvWarps * rows) * (units <= 16 ? 2u : 1u);
+    grid.x = (p.N + per_cta - 1) / per_cta;
     if (moe) return rows == 4 ? launch_fma_m1<4, true>(p, grid, st) : rows == 2 ? launch_fma_m1<2, true>(p, grid, st) : launch_fma_m1<1, true>(p, grid, st);
     return rows == 4 ? launch_fma_m1<4, false>(p, grid, st) : rows == 2 ? launch_fma_m1<2, false>(p, grid, st) : launch_fma_m1<1, false>(p, grid, st);
   }

@@ -77,10 +77,10 @@ cudaError_t launch_gemv_tc3(const GemvParams& p, int sm_count, cudaStream_t st);
 // (ztvm_batch_mma.cu).
 bool batch_mma_supported(const GemvParams& p, int bits);
 cudaError_t launch_batch_mma(const GemvParams& p, int bits, int sm_count, cudaStream_t st);
-// The grouped form for 3-bit experts: pairs sorted by expert, tiles of batch_moe_tile_rows pairs.
+// The grouped form for 3-bit (and 4-bit) experts: pairs sorted by expert, tiles of batch_moe_tile_rows pairs.
 bool batch_moe_supported(const GemvParams& g, int bits);
 uint32_t batch_moe_tile_rows(uint32_t experts, uint64_t pairs);
-cudaError_t launch_batch_moe(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan);
+cudaError_t launch_batch_moe(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan);
 
 // 4-bit weights, M > 16: tcgen05 GEMM with the dequantised weights as the A operand in tensor memory and the activations
 // as the only shared-memory operand (ztvm_gemm_ta.cu). status[0] receives a non-zero code if a pipeline wait inside the
@@ -117,6 +117,7 @@ bool moe_static_scratch_fits(uint32_t experts, uint64_t pairs);
 cudaError_t launch_moe_grouped_static(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* status,
                                       cudaStream_t st);
 cudaError_t launch_moe_tc_static(const GemvParams& g, uint32_t tokens, uint32_t slots, int sm_count, cudaStream_t st);
+cudaError_t launch_batch_moe_static(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, cudaStream_t st);
 cudaError_t launch_moe_ta_static(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* status, int sm_count,
                                  cudaStream_t st);
 

@@ -581,4 +581,12 @@ cudaError_t launch_moe_tc_static(const GemvParams& g, uint32_t tokens, uint32_t 
   return launch_moe_tc(g, tokens, slots, scratch, sm_count, st);   // its plan launch clears what must start at zero
 }
 
+cudaError_t launch_batch_moe_static(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, cudaStream_t st) {
+  if (!moe_static_scratch_fits(g.experts, (uint64_t)tokens * slots)) return cudaErrorInvalidValue;
+  uint32_t* scratch = nullptr;
+  const cudaError_t e = moe_static_scratch_ptr(&scratch);
+  if (e != cudaSuccess) return e;
+  return launch_batch_moe(g, bits, tokens, slots, scratch, st, false);
+}
+
 }  // namespace ztvm
