@@ -25,8 +25,7 @@
 namespace ztvm {
 
 constexpr int kTaStages = 4;        // weight slices in tensor memory
-constexpr int kTaWStages = 3;       // packed-weight ring (each slot holds four k blocks)
-constexpr int kTaWChunk = 4;
+constexpr int kTaWChunk = 4;        // k blocks of a slot of the packed-weight ring
 constexpr int kTaSbStages = 2;      // scales ring (each stage holds eight k blocks)
 constexpr int kTaSbChunk = 8;
 constexpr int kTaSbMaxPitch = 40;   // bytes of one row's scales (or biases) in a stage: groups of 32
@@ -42,7 +41,8 @@ struct GemmTaParams {
   void* Y;
   uint32_t M, N, K, SPR, group_shift, out_f32;
   uint32_t sb_pitch;   // 8 x an odd number: half of the banks apart for neighbouring rows
-  uint32_t x_tx_bytes; // bytes one activation stage receives (the boxes hold no more rows than there are)
+  uint32_t tile_m;     // tokens of a tile (the last tile of M may hold fewer)
+  uint32_t box_rows;   // rows of one activation box: a stage receives whole boxes
   uint32_t* status;
 };
 
@@ -50,9 +50,11 @@ template <int NT>
 struct GemmTaSmem {
   static constexpr int kXBytes = NT * kGemmBK * 2;            // per stage
   static constexpr int kWBytes = kTaRows * 128;               // per packed-weight slot
-  static constexpr int kSbBytes = 2 * kTaRows * kTaSbMaxPitch;
+  // the widest tile leaves room for two packed-weight slots and for one table of groups of 32 or two of wider groups
+  static constexpr int kWStages = NT > 256 ? 2 : 3;
+  static constexpr int kSbBytes = NT > 256 ? 2 * kTaRows * 24 : 2 * kTaRows * kTaSbMaxPitch;
   static constexpr int kOffW = kTaStages * kXBytes;
-  static constexpr int kOffSb = kOffW + kTaWStages * kWBytes;
+  static constexpr int kOffSb = kOffW + kWStages * kWBytes;
   static constexpr int kOffBar = kOffSb + kTaSbStages * kSbBytes;
   static constexpr int kTotal = kOffBar + 256;
 };
@@ -73,6 +75,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                   const GemmTaParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using L = GemmTaSmem<NT>;
+  constexpr int kTaWStages = L::kWStages;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t x_ring = base, w_ring = base + L::kOffW, bars = base + L::kOffBar;
@@ -90,8 +93,8 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n0 = blockIdx.x * kTaRows;
-  const uint32_t m0 = blockIdx.y * NT;
-  const uint32_t mrows = p.M - m0 < (uint32_t)NT ? p.M - m0 : (uint32_t)NT;     // tokens of this tile
+  const uint32_t m0 = blockIdx.y * p.tile_m;
+  const uint32_t mrows = p.M - m0 < p.tile_m ? p.M - m0 : p.tile_m;     // tokens of this tile
   // k blocks of this CTA: whole scale stages, so that every share starts on a multiple of eight
   const uint32_t split = gridDim.z, kz = blockIdx.z;
   const uint32_t all_kb = p.K / kGemmBK, units = (all_kb + kTaSbChunk - 1) / kTaSbChunk;
@@ -100,14 +103,13 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const uint32_t num_kb = kb_last - kb_first;
   constexpr uint32_t kColA = NT;                                 // weight slices start after the accumulator columns
   constexpr uint32_t kTmemCols = NT + kTaStages * 32 <= 256 ? 256 : 512;
-  const uint32_t nbox = (mrows + 127u) / 128u;                   // 128-token boxes of the tile
+  const uint32_t nbox = mrows > p.box_rows ? 2u : 1u, box_bytes = p.box_rows * (uint32_t)(kGemmBK * 2);
 
   if (threadIdx.x == 32) { tma_prefetch_desc(&tmap_x); tma_prefetch_desc(&tmap_w); }
   auto load_x = [&](uint32_t s, uint32_t kb) {
-    // a box holds p.x_tx_bytes / 128 rows; of a 256-token tile whose second half is empty only the first box is fetched
-    mbar_arrive_expect_tx(bar_full((int)s), nbox * p.x_tx_bytes);
+    mbar_arrive_expect_tx(bar_full((int)s), nbox * box_bytes);
     for (uint32_t b = 0; b < nbox; ++b)
-      tma_load_2d(x_ring + s * L::kXBytes + b * (128 * kGemmBK * 2), &tmap_x, bar_full((int)s), (int)((kb_first + kb) * kGemmBK), (int)(m0 + b * 128));
+      tma_load_2d(x_ring + s * L::kXBytes + b * box_bytes, &tmap_x, bar_full((int)s), (int)((kb_first + kb) * kGemmBK), (int)(m0 + b * p.box_rows));
   };
   auto load_w = [&](uint32_t s, uint32_t c) {
     mbar_arrive_expect_tx(bar_w_full((int)s), (uint32_t)L::kWBytes);
@@ -202,7 +204,9 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   } else if (warp == 1) {
     // ================= MMA issuer =================
     if (elect_one()) {
-      const uint32_t idesc = idesc_f16((int)((mrows + 15u) & ~15u));
+      // an instruction takes up to 256 tokens: a wider tile is two column ranges of the accumulator
+      const uint32_t cols = (mrows + 15u) & ~15u, cols_a = cols > 256u ? (cols / 2u + 15u) & ~15u : cols;
+      const uint32_t idesc = idesc_f16((int)cols_a), idesc_b = idesc_f16((int)(cols - cols_a));
       const uint64_t b0 = smem_desc_sw128(x_ring);
       uint32_t s = 0, ph = 0;
       // The thread is held at each tcgen05.mma until the pipe takes it, so a barrier poll between two k blocks would
@@ -220,6 +224,8 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         for (int k = 0; k < kGemmBK / 16; ++k) {   // 16 k elements: 8 TMEM columns of A, 32 bytes along the swizzled B row
           if (k == kGemmBK / 16 - 1 && kb + 1 < num_kb) next_ready = mbar_try_wait(bar_full((int)s1), ph1);
           umma_f16_ta(tmem_base, a_tmem + (uint32_t)(8 * k), bdesc + (uint64_t)(2 * k), idesc, (kb | (uint32_t)k) ? 1u : 0u);
+          if (NT > 256 && cols > cols_a)
+            umma_f16_ta(tmem_base + cols_a, a_tmem + (uint32_t)(8 * k), bdesc + (uint64_t)(cols_a * 8u + 2 * k), idesc_b, (kb | (uint32_t)k) ? 1u : 0u);
         }
         umma_commit(bar_empty((int)s));   // the activation tile and the weight slice are free once these MMAs have read them
         if (!next_ready) ok = mbar_wait(bar_full((int)s1), ph1, p.status, 2u, abort_flag);
@@ -376,12 +382,12 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             float* dst = reinterpret_cast<float*>(p.Y) + (size_t)m_first * p.N + n;
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (m_first + i < p.M) dst[(size_t)i * p.N] = __uint_as_float(v[i]);
+              if (cb * 32 + i < (int)mrows) dst[(size_t)i * p.N] = __uint_as_float(v[i]);
           } else {
             __half* dst = reinterpret_cast<__half*>(p.Y) + (size_t)m_first * p.N + n;
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (m_first + i < p.M) dst[(size_t)i * p.N] = __float2half_rn(__uint_as_float(v[i]));
+              if (cb * 32 + i < (int)mrows) dst[(size_t)i * p.N] = __float2half_rn(__uint_as_float(v[i]));
           }
         }
       }
@@ -391,7 +397,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     // ---- K shares meet: token blocks of eight, dealt to the CTAs in runs of `per`; partial sums as [sender][block][row][8
     // tokens] in the receiver's idle rings. Every thread of the cluster takes both barriers, whatever became of its waits.
     const uint32_t nb = (mrows + 7u) / 8u, per = (nb + split - 1) / split;
-    static_assert((NT + 56) * kTaRows * 4 <= kTaStages * L::kXBytes + kTaWStages * L::kWBytes, "partial sums of the other CTAs fit the rings");
+    static_assert((NT + 56) * kTaRows * 4 <= kTaStages * L::kXBytes + L::kWStages * L::kWBytes, "partial sums of the other CTAs fit the rings");
     __syncwarp();
     cluster_sync_all();                                  // every CTA's MMAs have read its rings for the last time
     if (is_dq && acc_ok) {
@@ -495,7 +501,7 @@ template <int NT, bool AFFINE>
 static cudaError_t launch_ta_one(const CUtensorMap& tx, const CUtensorMap& tw, const GemmTaParams& p, uint32_t split, cudaStream_t st) {
   const cudaError_t e = ta_kernel_ready<NT, AFFINE>();
   if (e != cudaSuccess) return e;
-  TaLaunch l(dim3((p.N + kTaRows - 1) / kTaRows, (p.M + NT - 1) / NT, split), GemmTaSmem<NT>::kTotal + 1024, st);
+  TaLaunch l(dim3((p.N + kTaRows - 1) / kTaRows, (p.M + p.tile_m - 1) / p.tile_m, split), GemmTaSmem<NT>::kTotal + 1024, st);
   return cudaLaunchKernelEx(&l.cfg, gemm_w4_ta_kernel<NT, AFFINE>, tx, tw, p);
 }
 // Clusters of `split` CTAs that the device holds at once (a cluster sits inside one GPC, so this is less than SMs / split).
@@ -528,28 +534,32 @@ cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* 
   if (!enc) return cudaErrorNotSupported;
   // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 8192 x 2048 .. 3072 x 8192:
   // a k block takes 340 + 1.4 per token (at least 390), a CTA 8500 to start, fill its rings and store, the exchange of
-  // a cluster 5300 + 12 per token. Clusters run in as many waves as the device can place.
-  const uint32_t units = (K / kGemmBK + kTaSbChunk - 1) / kTaSbChunk;
-  uint32_t nt = 64, split = 1;
+  // a cluster 5300 + 12 per token. Clusters run in as many waves as the device can place. The tokens are dealt evenly to
+  // the tiles. (Groups of 32 with biases do not fit beside the widest tile.)
+  const uint32_t units = (K / kGemmBK + kTaSbChunk - 1) / kTaSbChunk, n_tiles = (N + kTaRows - 1) / kTaRows;
+  const uint32_t widest = B && group_shift == 5 ? 256u : 352u;
+  uint32_t tile_m = 0, split = 1;
   uint64_t best = ~0ull;
-  for (uint32_t t : {64u, 128u, 256u}) {
-    if (t > 64u && t / 2 >= M) continue;
-    const uint64_t tiles = (uint64_t)((N + kTaRows - 1) / kTaRows) * ((M + t - 1) / t);
-    const uint32_t live = M < t ? M : t, block = live < 36u ? 390u : 340u + live * 14u / 10u;
+  for (uint32_t t = 64; t <= widest; t += 32) {
+    if (t > 64u && t - 32u >= M) break;
+    const uint32_t m_tiles = (M + t - 1) / t, tm = ((M + m_tiles - 1) / m_tiles + 15u) & ~15u;
+    const uint64_t tiles = (uint64_t)n_tiles * m_tiles;
+    const uint32_t live = M < tm ? M : tm, block = live < 36u ? 390u : 340u + live * 14u / 10u;
     for (uint32_t z = 1; z <= (uint32_t)kTaMaxSplit && z <= units; ++z) {
       if (z > 1 && tiles * z > (uint64_t)sm_count) break;
-      const uint32_t at_once = t == 64u ? ta_clusters<64>(z, sm_count) : t == 128u ? ta_clusters<128>(z, sm_count) : ta_clusters<256>(z, sm_count);
+      const uint32_t at_once = tm <= 64u ? ta_clusters<64>(z, sm_count) : tm <= 128u ? ta_clusters<128>(z, sm_count)
+                               : tm <= 256u ? ta_clusters<256>(z, sm_count) : ta_clusters<352>(z, sm_count);
       const uint64_t waves = (tiles + at_once - 1) / at_once;
       const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + 8500u + (z > 1 ? 5300u + 12u * live : 0u));
-      if (cost < best) { best = cost; nt = t; split = z; }
+      if (cost < best) { best = cost; tile_m = tm; split = z; }
     }
   }
   const cuuint32_t estr[2] = {1, 1};
   CUtensorMap tx, tw;
   const cuuint64_t xdims[2] = {K, M};
   const cuuint64_t xstrides[1] = {(cuuint64_t)K * 2};
-  // a box much taller than the tensor makes every load slow (22 against 13 us per launch at M = 17): no more rows than there are
-  const uint32_t box_rows = M >= 128u && nt >= 128u ? 128u : M >= 64u && nt == 64u ? 64u : (M + 7u) & ~7u;
+  // boxes no taller than the tile: a box much taller than the tensor makes every load slow (22 against 13 us per launch at M = 17)
+  const uint32_t box_rows = tile_m > 128u ? (tile_m / 2u + 7u) & ~7u : tile_m < M ? tile_m : (M + 7u) & ~7u;
   const cuuint32_t xbox[2] = {(cuuint32_t)kGemmBK, box_rows};
   CUresult r = enc(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(X), xdims, xstrides, xbox, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -567,11 +577,12 @@ cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* 
   p.M = M; p.N = N; p.K = K; p.SPR = K >> group_shift; p.group_shift = group_shift;
   p.out_f32 = out_f32 ? 1u : 0u;
   p.sb_pitch = group_shift == 5 ? 40u : 24u;
-  p.x_tx_bytes = box_rows * (uint32_t)(kGemmBK * 2);
+  p.tile_m = tile_m; p.box_rows = box_rows;
   p.status = status;
   const bool affine = B != nullptr;
-  if (nt == 256) return affine ? launch_ta_one<256, true>(tx, tw, p, split, st) : launch_ta_one<256, false>(tx, tw, p, split, st);
-  if (nt == 128) return affine ? launch_ta_one<128, true>(tx, tw, p, split, st) : launch_ta_one<128, false>(tx, tw, p, split, st);
+  if (tile_m > 256u) return affine ? launch_ta_one<352, true>(tx, tw, p, split, st) : launch_ta_one<352, false>(tx, tw, p, split, st);
+  if (tile_m > 128u) return affine ? launch_ta_one<256, true>(tx, tw, p, split, st) : launch_ta_one<256, false>(tx, tw, p, split, st);
+  if (tile_m > 64u) return affine ? launch_ta_one<128, true>(tx, tw, p, split, st) : launch_ta_one<128, false>(tx, tw, p, split, st);
   return affine ? launch_ta_one<64, true>(tx, tw, p, split, st) : launch_ta_one<64, false>(tx, tw, p, split, st);
 }
 
