@@ -75,3 +75,26 @@ def test_grouped_experts(bits, T, E, d, ffn, slots, backend, dev, oracle_c):
         record_parity(zo.rel_err_scaled(got, ref, 1e-3), zo.rel_err(got, ref))
         mags = oracle_c.moe_matmul_f64(np.abs(x), W, s, np.abs(b), ids, N, K, 64, bits, in_per_slot=per_slot)
         assert (np.abs(got - ref) <= f16_bound(ref, mags, K)).all()
+
+
+@pytest.mark.parametrize("K", [64, 192, 320, 576, 896])
+def test_tensor_memory_tiles_over_several_units_per_cta(K, dev, oracle_c, monkeypatch):
+    """The f16-weight tiles with more units than two per SM and K of 1, 3, 5, 9 and 14 stages: the stages of a unit start on
+    either parity, and the last packed slot holds one, two or three of them. Bound: the MMA's inputs are the oracle's own
+    f16 weights, so only the f32 sums and the f16 result differ (f16_bound)."""
+    monkeypatch.setenv("ZTVM_MOE_GROUPED", "1")
+    be = z.backend.CudaMatmulBackend(0)
+    E, T, N = 20, 1500, 2104
+    rng = np.random.default_rng(K)
+    ids = rng.integers(0, E, size=(T, 1), dtype=np.uint32)
+    _, W, s, b = z.synth.make_weights(rng, N, K, bits=4, sigma_s=0.02, lead=(E,))
+    x = z.synth.make_x(rng, T, K)
+    y = dev.empty((T, 1, N), np.float16, fill=float("nan"))
+    desc = z.MoeDesc(z.MmDesc(K, N, 1, 64, 4, 1, 0), E, 1, T, 0, N, K, N, 1)
+    be.ctx.int4_matmul_moe(desc, y, dev.put(x), dev.put(s), dev.put(W), dev.put(b), dev.put(ids))
+    got = dev.get(y)
+    assert be.ctx.device_errors() == 0 and np.isfinite(got).all()
+    ref = oracle_c.moe_matmul_f64(x, W, s, b, ids, N, K, 64, 4, in_per_slot=False, w16=True)
+    mags = oracle_c.moe_matmul_f64(np.abs(x), W, s, np.abs(b), ids, N, K, 64, 4, in_per_slot=False)
+    assert (np.abs(got - ref) <= f16_bound(ref, mags, K)).all()
+    be.close()

@@ -148,6 +148,7 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
   }
 }
 
+constexpr size_t kFillThreads = 148 * 256;   // threads from which on a row-wise kernel gives each of them eight elements
 static inline unsigned grid_for(size_t total, int block) {
   size_t g = (total + block - 1) / block;
   return (unsigned)(g > 148 * 32 ? 148 * 32 : (g ? g : 1));
@@ -358,7 +359,9 @@ __device__ __forceinline__ float silu_mul_one(float g, float u) {
   const float sg = g * (1.0f / (1.0f + expf(-g)));
   return u * sg;
 }
-// VEC = 8: eight elements per thread (16-byte loads and stores; ffn % 8 == 0, 16-byte aligned buffers), else one.
+// VEC elements per thread: eight (16-byte loads and stores; ffn % 8 == 0, 16-byte aligned buffers) where that still fills
+// the chip; two (ffn even, 4-byte aligned) for a few rows, whose time is one thread's chain of exponentials and divisions;
+// else one.
 template <int VEC>
 __global__ void silu_mul_kernel(const __half* gate_up, __half* h, uint32_t rows, uint32_t ffn,
                                 const uint32_t* seg_counts, uint32_t seg_cap) {
@@ -381,6 +384,10 @@ __global__ void silu_mul_kernel(const __half* gate_up, __half* h, uint32_t rows,
         ow[k] = *reinterpret_cast<const uint32_t*>(&o);
       }
       *reinterpret_cast<uint4*>(h + r * ffn + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    } else if constexpr (VEC == 2) {
+      const float2 g2 = __half22float2(*reinterpret_cast<const __half2*>(gate_up + r * 2 * ffn + c));
+      const float2 u2 = __half22float2(*reinterpret_cast<const __half2*>(gate_up + r * 2 * ffn + ffn + c));
+      *reinterpret_cast<__half2*>(h + r * ffn + c) = __floats2half2_rn(silu_mul_one(g2.x, u2.x), silu_mul_one(g2.y, u2.y));
     } else {
       const float g = __half2float(gate_up[r * 2 * ffn + c]);
       const float u = __half2float(gate_up[r * 2 * ffn + ffn + c]);
@@ -392,9 +399,10 @@ cudaError_t launch_silu_mul(const __half* gate_up, __half* h, uint32_t rows, uin
                             const uint32_t* seg_counts, uint32_t seg_cap) {
   const size_t total = (size_t)rows * ffn;
   if (total == 0) return cudaSuccess;
-  const bool vec = ffn % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(h)) & 15u) == 0;
-  return launch_chained(vec ? silu_mul_kernel<8> : silu_mul_kernel<1>, dim3(grid_for(vec ? total / 8 : total, 256)), dim3(256), 0, st, gate_up, h,
-                        rows, ffn, seg_counts, seg_cap ? seg_cap : 1u);
+  const uintptr_t lows = reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(h);
+  const int vec = ffn % 8 == 0 && (lows & 15u) == 0 && total / 8 >= kFillThreads ? 8 : ffn % 2 == 0 && (lows & 3u) == 0 ? 2 : 1;
+  return launch_chained(vec == 8 ? silu_mul_kernel<8> : vec == 2 ? silu_mul_kernel<2> : silu_mul_kernel<1>, dim3(grid_for(total / vec, 256)),
+                        dim3(256), 0, st, gate_up, h, rows, ffn, seg_counts, seg_cap ? seg_cap : 1u);
 }
 
 // The same over f32 [gate(ffn) | up(ffn)] rows: the second step of the fused FFN on shapes the paired GEMV does not
@@ -450,6 +458,22 @@ __global__ void moe_combine_kernel(const __half* y, const float* scores, __half*
           }
         }
       }
+    } else if constexpr (VEC == 2) {
+      // a few tokens: one round of loads for up to twelve slots, added in index order
+      for (uint32_t s = 0; s < slots; s += 12) {
+        __half2 v[12];
+        float f[12];
+#pragma unroll
+        for (uint32_t u = 0; u < 12; ++u)
+          if (s + u < slots) { v[u] = *reinterpret_cast<const __half2*>(src + (size_t)(s + u) * d); f[u] = sc[s + u]; }
+#pragma unroll
+        for (uint32_t u = 0; u < 12; ++u) {
+          if (s + u >= slots) break;
+          const float2 h2 = __half22float2(v[u]);
+          acc[0] = __fadd_rn(acc[0], __fmul_rn(f[u], h2.x));
+          acc[1] = __fadd_rn(acc[1], __fmul_rn(f[u], h2.y));
+        }
+      }
     } else {
       for (uint32_t s = 0; s < slots; ++s) acc[0] = __fadd_rn(acc[0], __fmul_rn(sc[s], __half2float(src[(size_t)s * d])));
     }
@@ -461,6 +485,8 @@ __global__ void moe_combine_kernel(const __half* y, const float* scores, __half*
         ow[k] = *reinterpret_cast<const uint32_t*>(&o);
       }
       *reinterpret_cast<uint4*>(out + t * d + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    } else if constexpr (VEC == 2) {
+      *reinterpret_cast<__half2*>(out + t * d + c) = __floats2half2_rn(acc[0], acc[1]);
     } else {
       out[t * d + c] = __float2half_rn(acc[0]);
     }
@@ -470,9 +496,10 @@ cudaError_t launch_moe_combine(const __half* y_slots, const float* scores, __hal
                                uint32_t slots, uint32_t d, cudaStream_t st) {
   const size_t total = (size_t)tokens * d;
   if (total == 0) return cudaSuccess;
-  const bool vec = d % 8 == 0 && ((reinterpret_cast<uintptr_t>(y_slots) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
-  return launch_chained(vec ? moe_combine_kernel<8> : moe_combine_kernel<1>, dim3(grid_for(vec ? total / 8 : total, 256)), dim3(256), 0, st,
-                        y_slots, scores, out, tokens, slots, d);
+  const uintptr_t lows = reinterpret_cast<uintptr_t>(y_slots) | reinterpret_cast<uintptr_t>(out);
+  const int vec = d % 8 == 0 && (lows & 15u) == 0 && total / 8 >= kFillThreads ? 8 : d % 2 == 0 && (lows & 3u) == 0 ? 2 : 1;
+  return launch_chained(vec == 8 ? moe_combine_kernel<8> : vec == 2 ? moe_combine_kernel<2> : moe_combine_kernel<1>, dim3(grid_for(total / vec, 256)),
+                        dim3(256), 0, st, y_slots, scores, out, tokens, slots, d);
 }
 
 }  // namespace ztvm

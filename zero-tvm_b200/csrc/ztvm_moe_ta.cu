@@ -15,8 +15,8 @@
 //
 // Roles (832 threads): warp 0 TMA-loads packed weights (two boxes of 128 rows x 32 words = four k blocks per slot);
 // warp 1 owns tensor memory and issues the MMAs (eight per 64-element stage, one commit); warps 2..17 dequantise
-// (warp w touches TMEM lanes 32 (w % 4) .. +31; the four warps of a lane quarter take the two row halves x the two
-// 32-code halves of a stage); warps 18..21 gather activations; warps 22..25 read finished accumulators and scatter
+// (warp w touches TMEM lanes 32 (w % 4) .. +31; the four warps of a lane quarter take the two row halves x the even
+// and odd stages: a whole 64-code row of a stage per thread halves the waits, scale look-ups and guards per code); warps 18..21 gather activations; warps 22..25 read finished accumulators and scatter
 // them to where each pair lives (or, in the expert-parallel form, to the rank it came from). One arrival per warp on
 // the shared-memory barriers. Every wait is bounded: on expiry a status word is raised, the roles stop, copies in
 // flight are waited for, TMEM is freed.
@@ -109,7 +109,7 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMtaStages; ++s) {
-      mbar_init(bar_full(s), kMtaDqWarps);   // one arrival per dequantiser warp
+      mbar_init(bar_full(s), kMtaDqWarps / 2);   // one arrival per dequantiser warp of the stage's parity
       mbar_init(bar_empty(s), 1);
     }
     for (int s = 0; s < kMtaXStages; ++s) {
@@ -220,11 +220,11 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
     }
   } else if (warp < 2 + kMtaDqWarps) {
     // ================= dequantisers (warps 2..17) =================
-    // Thread (quarter, lane) of part p owns weight row 128 (p / 2) + 32 quarter + lane of the unit and the 32-code half
-    // p % 2 of every stage: 4 words in, 16 columns of tensor memory out.
+    // Thread (quarter, lane) of part p owns weight row 128 (p / 2) + 32 quarter + lane of the unit in every stage whose
+    // running number has the parity p % 2: 8 words in, 32 columns of tensor memory out.
     const int quarter = warp & 3;                       // TMEM lanes this warp may touch: [32 * quarter, +32)
     const uint32_t part = (uint32_t)(warp - 2) >> 2;    // 0..3
-    const uint32_t half = part >> 1, khalf = part & 1u;
+    const uint32_t half = part >> 1, par = part & 1u;
     const uint32_t r_half = (uint32_t)(quarter * 32 + lane);            // row inside the half
     const uint32_t r_unit = half * kMtaRows + r_half;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
@@ -247,10 +247,6 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
       sv = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.S) + off));
       bv = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.B) + off));
     };
-    auto pick16 = [](const uint4& v, uint32_t i) -> unsigned short {
-      const uint32_t wsel = (i >> 1) == 0 ? v.x : (i >> 1) == 1 ? v.y : (i >> 1) == 2 ? v.z : v.w;
-      return (unsigned short)((i & 1) ? (wsel >> 16) : (wsel & 0xFFFFu));
-    };
     uint4 sv_cur = make_uint4(0, 0, 0, 0), bv_cur = sv_cur, sv_nxt = sv_cur, bv_nxt = sv_cur;
     load_sb8(sv_cur, bv_cur, 0);
     load_sb8(sv_nxt, bv_nxt, 1);
@@ -260,18 +256,22 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
       const size_t row = row_of(ui);
       const unsigned short* srow = reinterpret_cast<const unsigned short*>(p.S) + row * p.SPR;
       const unsigned short* brow = reinterpret_cast<const unsigned short*>(p.B) + row * p.SPR;
+      const uint32_t off = (gst + par) & 1u;                        // this warp's stages of the unit: off, off + 2, ...
       for (uint32_t kb0 = 0; kb0 < num_kb && ok; kb0 += 8) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t kb = kb0 + i;
+        for (int ii = 0; ii < 4; ++ii) {
+          const uint32_t kb = kb0 + 2u * ii + off;
           if (kb >= num_kb || !ok) break;
           const uint32_t g = gst + kb;
           const uint32_t s = g % kMtaStages, ph = (g / kMtaStages) & 1u;
           const uint32_t c = gc + kb / kMtaWChunk, ws = c % kMtaWStages;
-          const uint32_t j = (uint32_t)i % kMtaWChunk;              // kb0 is a multiple of 8
-          if (j == 0) ok = mbar_wait(bar_w_full(ws), (c / kMtaWStages) & 1u, p.status, 7u, abort_flag);
-          uint4 wv = make_uint4(0, 0, 0, 0);   // 16-byte chunk 2 j + khalf of this row's 128 bytes of the slot, swizzled by the row
-          if (ok) wv = *reinterpret_cast<const uint4*>(wrow_sm + ws * L::kWBytes + (((2u * j + khalf) ^ (r_half & 7)) << 4));
+          const uint32_t j = 2u * (ii & 1) + off;                   // kb0 is a multiple of 8
+          if ((ii & 1) == 0) ok = mbar_wait(bar_w_full(ws), (c / kMtaWStages) & 1u, p.status, 7u, abort_flag);
+          uint4 wv[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};   // 16-byte chunks 2 j, 2 j + 1 of this row's 128 bytes of the slot, swizzled by the row
+          if (ok) {
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) wv[h] = *reinterpret_cast<const uint4*>(wrow_sm + ws * L::kWBytes + (((2u * j + h) ^ (r_half & 7)) << 4));
+          }
           // the TMEM slices of stage s were last read by the MMAs of stage g - kMtaStages
           if (ok && g >= (uint32_t)kMtaStages) {
             ok = mbar_wait(bar_empty(s), ph ^ 1u, p.status, 4u, abort_flag);
@@ -280,21 +280,26 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
           if (ok) {
             unsigned short s16, b16;
             if (vec_sb) {
-              s16 = pick16(sv_cur, (uint32_t)i);
-              b16 = pick16(bv_cur, (uint32_t)i);
+              const uint32_t s2 = ii == 0 ? sv_cur.x : ii == 1 ? sv_cur.y : ii == 2 ? sv_cur.z : sv_cur.w;
+              const uint32_t b2 = ii == 0 ? bv_cur.x : ii == 1 ? bv_cur.y : ii == 2 ? bv_cur.z : bv_cur.w;
+              s16 = (unsigned short)(s2 >> (16u * off));
+              b16 = (unsigned short)(b2 >> (16u * off));
             } else {
               s16 = __ldg(srow + kb);
               b16 = __ldg(brow + kb);
             }
             const DqGroup dq = dq_group<true>(s16, b16);
-            uint32_t a[16];
-            dequant_words_w16<true>(wv, dq, a);
-            // 32 weights of this row = 16 TMEM columns (two k-adjacent f16 per column) of this thread's lane
-            tmem_st16(tmem_base + lane_base + kMtaColA + s * 64u + half * 32u + khalf * 16u, a);
+            // 64 weights of this row = 32 TMEM columns (two k-adjacent f16 per column) of this thread's lane, in two stores
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+              uint32_t a[16];
+              dequant_words_w16<true>(wv[h], dq, a);
+              tmem_st16(tmem_base + lane_base + kMtaColA + s * 64u + half * 32u + h * 16u, a);
+            }
             tmem_st_wait();
           }
           // the packed slot goes back to the producer only after the stores that consumed its words
-          if (j == kMtaWChunk - 1 || kb + 1 == num_kb) {
+          if ((ii & 1) == 1 || kb + 2 >= num_kb) {
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_w_empty(ws));
           }
@@ -307,6 +312,13 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
         sv_cur = sv_nxt; bv_cur = bv_nxt;
         load_sb8(sv_nxt, bv_nxt, item + 2u);
         ++item;
+      }
+      // a last slot without a stage of this warp's is handed back all the same
+      if (ok && (num_chunks - 1) * kMtaWChunk + off >= num_kb) {
+        const uint32_t c = gc + num_chunks - 1, ws = c % kMtaWStages;
+        ok = mbar_wait(bar_w_full(ws), (c / kMtaWStages) & 1u, p.status, 7u, abort_flag);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_w_empty(ws));
       }
       gst += num_kb;
       gc += num_chunks;
