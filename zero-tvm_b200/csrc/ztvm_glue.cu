@@ -185,6 +185,9 @@ cudaError_t launch_dequant(const uint32_t* W, const __half* S, const __half* B, 
   return cudaGetLastError();
 }
 
+// i / n, in 32 bits where that holds it: a 64-bit division would be most of what a row-wise kernel executes per element
+__device__ __forceinline__ size_t row_of(size_t i, uint32_t n) { return i >> 32 ? i / n : (uint32_t)i / n; }
+
 // ---- embedding rows (embedding_affine.wgsl:38-57, embedding_affine_int8.wgsl) ------------------------------
 // out[t][:] = the dequantised row input_ids[t] of an affine-quantised table, f16: the canonical W16 (what the vendor
 // dequantiser stores), through the same word dequantiser as the GEMMs for 4-bit codes. One thread per 8 values.
@@ -197,7 +200,7 @@ __global__ void embedding_affine_kernel(const int32_t* input_ids, const uint32_t
   pdl_launch_dependents();
   pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t t = (uint32_t)(i / nblk), blk = (uint32_t)(i - (size_t)t * nblk);
+    const uint32_t t = (uint32_t)row_of(i, nblk), blk = (uint32_t)(i - (size_t)t * nblk);
     const int32_t id = input_ids[t];
     if (id < 0 || (uint32_t)id >= vocab) {          // counted, the row is left untouched
       if (blk == 0) atomicAdd(err, 1u);
@@ -370,7 +373,7 @@ __global__ void silu_mul_kernel(const __half* gate_up, __half* h, uint32_t rows,
   pdl_launch_dependents();
   pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = i / per_row, c = (i - r * per_row) * VEC;
+    const size_t r = row_of(i, per_row), c = (i - r * per_row) * VEC;
     if (seg_counts && (uint32_t)(r % seg_cap) >= seg_counts[r / seg_cap]) continue;   // past the region's live rows
     if constexpr (VEC == 8) {
       const uint4 gv = *reinterpret_cast<const uint4*>(gate_up + r * 2 * ffn + c);
@@ -432,7 +435,7 @@ __global__ void moe_combine_kernel(const __half* y, const float* scores, __half*
   pdl_launch_dependents();
   pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t t = i / per_row, c = (i - t * per_row) * VEC;
+    const size_t t = row_of(i, per_row), c = (i - t * per_row) * VEC;
     float acc[VEC];
 #pragma unroll
     for (int k = 0; k < VEC; ++k) acc[k] = 0.f;
