@@ -15,6 +15,40 @@ from __future__ import annotations
 
 from typing import Callable, List, Tuple
 
+from .backend import _decode_matmul
+
+
+def _span(buf):
+    """Byte range of a bound buffer from its address on, or None where its size is unknown."""
+    if hasattr(buf, "data_ptr"):
+        return buf.data_ptr(), buf.data_ptr() + buf.numel() * buf.element_size()
+    return None
+
+
+def _independent_pair(be, a, b):
+    """Whether two consecutive recorded calls are the gate and the up projection of one MoE block: same entry, PODArgs,
+    activations, ids and grid, outputs that share no element, and so few pairs that neither needs the expert-sorted plan
+    (whose work buffer the first would fill for the second)."""
+    if a[0] != be.dispatch or b[0] != be.dispatch:
+        return False
+    (ea, ba, ga), (eb, bb, gb) = a[1], b[1]
+    if ea != eb or ga != gb or len(ga) < 3 or len(ba) != 7 or len(bb) != 7 or list(ba[4]) != list(bb[4]):
+        return False
+    spans = [_span(t) for t in (ba[0], bb[0], ba[1], bb[1], ba[6], bb[6])]
+    if None in spans or spans[2] != spans[3] or spans[4] != spans[5]:
+        return False
+    _, moe, desc = _decode_matmul(ea, tuple(ba[4]))
+    if not moe or desc is None or ga[1] * ga[2] >= (64 if desc[0].bits == 4 else 32):   # (from there on calls are grouped)
+        return False
+    rows, (_in_slot, out_slot, _in_tok, out_tok, _ids) = desc[0].N, desc[1]
+    slots, tokens = ga[2], ga[1]
+    lo, hi = sorted((spans[0][0], spans[1][0]))
+    reach = 2 * ((tokens - 1) * out_tok + (slots - 1) * out_slot + rows)          # bytes from a call's first to its last element
+    beside = rows * 2 <= hi - lo <= (out_slot - rows) * 2 and out_tok >= slots * out_slot   # rows of one in the gaps of the other
+    if not (beside or hi - lo >= reach):
+        return False
+    return all(s[1] <= out or s[0] >= out + reach for s in (spans[2], spans[4]) for out in (lo, hi))   # neither writes what the other reads
+
 
 class DecodeRecorder:
     def __init__(self, backend):
@@ -49,6 +83,25 @@ class DecodeRecorder:
         for fn, args, kw in self._calls:
             fn(*args, stream=stream, **kw)
 
+    def _run_captured(self, main, side):
+        """The sequence inside the capture. The gate and up projections of a decoded token are a few CTAs each and read the
+        same inputs: as two branches of the graph they run side by side (four blocks of one token, 256 experts of
+        2048 x 512: 89 -> 73 us)."""
+        import torch
+        i = 0
+        while i < len(self._calls):
+            fn, args, kw = self._calls[i]
+            if i + 1 < len(self._calls) and _independent_pair(self.be, self._calls[i], self._calls[i + 1]):
+                side.wait_event(main.record_event())
+                fn(*args, stream=main.cuda_stream, **kw)
+                fn, args, kw = self._calls[i + 1]
+                fn(*args, stream=side.cuda_stream, **kw)
+                main.wait_event(side.record_event())
+                i += 2
+                continue
+            fn(*args, stream=main.cuda_stream, **kw)
+            i += 1
+
     def run_eager(self, stream=None):
         """The recorded sequence as plain launches on `stream` (default: torch's current stream)."""
         import torch
@@ -72,7 +125,7 @@ class DecodeRecorder:
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g, stream=self._stream):
                     self.be.ctx.moe_plan_reuse(plan_reuse)          # drops any plan: the captured step builds its own
-                    self._run(self._stream.cuda_stream)
+                    self._run_captured(self._stream, torch.cuda.Stream())
                 self._stream.synchronize()
         finally:
             self.be.ctx.moe_plan_reuse(False)
