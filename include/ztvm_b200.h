@@ -164,8 +164,8 @@ ZTVM_API ztvm_status ztvm_moe_plan_reuse(ztvm_ctx* ctx, int32_t enable);
  *    bits 4, group 64, K % 64 == 0, N % 8 == 0, input strides multiples of 8 elements. Anything else is
  *    ZTVM_ERR_UNSUPPORTED / ZTVM_ERR_ALIGNMENT. From 128 pairs on
  *    (and with the ZTVM_MOE_GROUPED knob unset) the kernel is chosen exactly as ztvm_int4_matmul_moe chooses it, so
- *    the results are those of that call on the same inputs, bit for bit; below 128 pairs that call runs the per-pair
- *    GEMV instead, and the two agree within the path's tolerance only.
+ *    the results are those of that call on the same inputs, bit for bit; below 128 pairs that call may run the per-pair
+ *    GEMV instead (always below 64), and the two agree within the path's tolerance only.
  *  - The first call on a device looks up the array's device address and loads the kernels: make one call
  *    per device at start-up, before any stream capture.
  *  - There is ONE array per device, shared by every context and stream: two calls that overlap in time on

@@ -32,7 +32,7 @@ struct ztvm_ctx {
   void* d_ws; size_t d_ws_bytes;
   void* d_ffn; size_t d_ffn_bytes;      // f32 gate/up rows of ztvm_fused_ffn's two-launch form
   // env ZTVM_MOE_GROUPED (a measurement knob): 0 forces the per-pair GEMV, 1 the tensor-core tiles, 2 the streaming
-  // grouped kernel; unset = by size (below 128 pairs per-pair; then streaming while an expert sees few pairs)
+  // grouped kernel; unset = by size (few pairs per-pair; then the exact-code kernels while an expert sees few of them)
   int moe_grouped;
   // what the plan in d_ws was built from (ztvm_int4_matmul_moe_ep reuse_plan)
   const void* plan_ids; const void* plan_segs; uint32_t plan_tokens, plan_tile_rows, plan_experts, plan_slots, plan_stride;

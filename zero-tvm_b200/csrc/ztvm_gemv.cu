@@ -246,6 +246,7 @@ gemv_fma_m1_kernel(const GemvParams p) {
     out_base = (size_t)token * p.out_tok_stride + (size_t)slot * p.out_slot_stride;
   }
   // A K of 16 units or fewer (512 codes) would leave half of the lanes without work: each half of the warp takes a row of its own
+  // (2048 x 512, nine pairs: 5.6 -> 4.1 us)
   const uint32_t units = p.K >> 5;
   const uint32_t sub = units <= 16u ? 2u : 1u, span = 32u / sub;
   const uint32_t lane_u = (uint32_t)lane & (span - 1u), lane_r = (uint32_t)lane / span;

@@ -1,5 +1,5 @@
 // Persistent decode GEMV for 3-bit / group-64 weights, M = 1 (the q3 GEMV body, int4_matmul.gen.ts:409-448): the design
-// of ztvm_gemv_tc.cu — one CTA per SM, K cut in 256-code slices owned by warps, per-warp cp.async ring, activations as
+// of ztvm_gemv_tc.cuh — one CTA per SM, K cut in 256-code slices owned by warps, per-warp cp.async ring, activations as
 // MMA B fragments in registers, fixed-order meeting of the K-slice partials — with an unpack made for a bit stream
 // whose codes do not sit on nibble boundaries.
 //

