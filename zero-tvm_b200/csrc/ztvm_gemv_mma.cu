@@ -71,7 +71,7 @@ template <int WPL, int NTOK, bool MOE>
 __global__ void __launch_bounds__(kMmaMaxWarps * 32)
 gemv_mma_kernel(const GemvParams p) {
   extern __shared__ uint4 smem_u4[];
-  pdl_launch_dependents();
+  if (MOE) pdl_launch_dependents();   // (a dense grid does not: see gemv_kernel)
   pdl_wait();
   constexpr int GROUP = WPL * 32;
   constexpr int NV = NTOK <= 1 ? 1 : 2;  // tokens per lane that can be live: (2c) and (2c+1)
