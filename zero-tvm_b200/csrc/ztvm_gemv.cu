@@ -28,8 +28,8 @@ template <int BITS, int MT, int ROWS, bool MOE>
 __global__ void __launch_bounds__(kGemvWarps * 32)
 gemv_kernel(const GemvParams p) {
   extern __shared__ float4 smem_f4[];
-  // A dense grid fills the chip in CTAs of a fixed share each: the next launch's CTAs, let in early, would be dealt to whatever
-  // slots are free and leave its SMs unevenly loaded (3-bit 3003 x 4416 back to back: 10.3 us, let in early 12.7)
+  // A dense grid fills the chip in CTAs of a fixed share each: CTAs let in early would be dealt to whatever slots are free and
+  // leave its SMs unevenly loaded (3-bit 3003 x 4416 back to back: 9.7 us, let in early 12.7)
   if (MOE) pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -559,7 +559,9 @@ static cudaError_t launch_one(const GemvParams& p, dim3 grid, size_t smem, cudaS
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  return launch_chained(kern, grid, dim3(kGemvWarps * 32), smem, st, p);
+  if (MOE) return launch_chained(kern, grid, dim3(kGemvWarps * 32), smem, st, p);
+  kern<<<grid, kGemvWarps * 32, smem, st>>>(p);   // a dense grid neither comes in early (see the kernel) nor lets the next one in
+  return cudaGetLastError();
 }
 
 template <int ROWS, bool MOE>
@@ -575,7 +577,9 @@ static cudaError_t launch_fma_m1(const GemvParams& p, dim3 grid, cudaStream_t st
   }
   const uint32_t units = p.K >> 5, units_up = (units + 31) & ~31u;
   const size_t smem = (size_t)units_up * 64 + (size_t)units_up * 4;
-  return launch_chained(kern, grid, dim3(kGemvWarps * 32), smem, st, p);
+  if (MOE) return launch_chained(kern, grid, dim3(kGemvWarps * 32), smem, st, p);
+  kern<<<grid, kGemvWarps * 32, smem, st>>>(p);   // a dense grid neither comes in early (see the kernel) nor lets the next one in
+  return cudaGetLastError();
 }
 
 template <int ROWS, int DEPTH>

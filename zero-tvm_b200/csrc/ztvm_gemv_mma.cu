@@ -288,7 +288,9 @@ static cudaError_t launch_mma_one(const GemvParams& p, dim3 grid, int threads, s
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  return launch_chained(kern, grid, dim3(threads), smem, st, p);
+  if (MOE) return launch_chained(kern, grid, dim3(threads), smem, st, p);
+  kern<<<grid, threads, smem, st>>>(p);
+  return cudaGetLastError();
 }
 
 template <int WPL, bool MOE>
