@@ -145,6 +145,15 @@ ZTVM_API ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* de
                                  const void* scales, const void* packed_w, const void* biases,
                                  const uint32_t* ids, void* stream);
 
+/* Whether ztvm_int4_matmul_moe, called with these arguments on this context, sorts the pairs by expert into the plan that
+ * the context keeps (uses_plan = 1), or reads ids directly and touches no state of the context but the error counter
+ * (uses_plan = 0). Two calls that use no plan and share no output may run side by side, as branches of a captured graph
+ * for instance. Same argument checks as the call; nothing is launched and no buffer is read. No counterpart in the
+ * reference. */
+ZTVM_API ztvm_status ztvm_int4_matmul_moe_uses_plan(ztvm_ctx* ctx, const ztvm_moe_desc* desc, const void* y, const void* x,
+                                 const void* scales, const void* packed_w, const void* biases,
+                                 const uint32_t* ids, uint32_t* uses_plan);
+
 /* The gate, up and down matmuls of one step walk the same id list, and each ztvm_int4_matmul_moe call sorts it by
  * expert again (the plan). With reuse enabled, a call whose ids address, tokens, slots, ids_stride and expert count
  * equal the previous call's uses that call's plan. The caller then promises that the id list changes only through

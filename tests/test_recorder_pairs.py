@@ -49,3 +49,91 @@ def test_separate_outputs_may_run_side_by_side():
 ])
 def test_overlapping_calls_stay_in_sequence(change):
     assert not calls(3, 4, **change)
+
+
+class FakeStream:
+    """Notes what a capture puts on it."""
+
+    def __init__(self, name, log):
+        self.cuda_stream, self.log = name, log
+
+    def record_event(self):
+        return self.cuda_stream
+
+    def wait_event(self, event):
+        self.log.append((self.cuda_stream, "waits for", event))
+
+
+def recorded_token(be, tokens=1, slots=9):
+    gu, x = torch.zeros(tokens, slots, 2 * FFN, dtype=torch.float16), torch.zeros(tokens, D, dtype=torch.float16)
+    w, s = torch.zeros(E, FFN, D // 8, dtype=torch.int32), torch.zeros(E, FFN, D // 64, dtype=torch.float16)
+    ids, pod = torch.zeros(tokens, slots, dtype=torch.int32), moe_gate_pod_args(D, FFN, slots)
+    rec = DecodeRecorder(be)
+    for out in (gu, gu.view(-1)[FFN:]):
+        rec.dispatch("int4_matmul_tiled_affine_moe", [out, x, s, w, pod, s, ids], (16, tokens, slots))
+    return rec
+
+
+@pytest.mark.parametrize("plan,want", [
+    (False, [("side", "waits for", "main"), ("main", "runs"), ("side", "runs"), ("main", "waits for", "side")]),
+    (True, [("main", "runs"), ("main", "runs")]),
+])
+def test_calls_that_use_the_plan_are_captured_in_sequence(plan, want):
+    """A context may group any number of pairs (its MoE kernel knob): only the library knows, and what shares its plan
+    buffer must not become two branches."""
+    log = []
+
+    class Backend:
+        def dispatch(self, entry, bindings, grid, stream=None):
+            log.append((stream, "runs"))
+
+        def uses_moe_plan(self, entry, bindings, grid):
+            return plan
+
+    recorded_token(Backend())._run_captured(FakeStream("main", log), FakeStream("side", log))
+    assert log == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("knob,tokens,want", [(None, 1, False), (None, 16, True), ("0", 64, False), ("1", 1, True), ("2", 1, True)])
+def test_the_library_says_which_calls_use_the_plan(knob, tokens, want, dev, monkeypatch):
+    if knob is None:
+        monkeypatch.delenv("ZTVM_MOE_GROUPED", raising=False)
+    else:
+        monkeypatch.setenv("ZTVM_MOE_GROUPED", knob)
+    be = z.backend.CudaMatmulBackend(0)
+    for _, (entry, bindings, grid), _ in recorded_token(be, tokens)._calls:
+        bindings = [t.cuda() if torch.is_tensor(t) and t.storage_offset() == 0 else torch.zeros(t.numel() + FFN, dtype=t.dtype, device="cuda")[FFN:]
+                    if torch.is_tensor(t) else t for t in bindings]
+        assert be.uses_moe_plan(entry, bindings, grid) is want
+    be.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("knob", [None, "1", "2"])
+def test_replayed_token_under_the_kernel_knob(knob, dev, monkeypatch):
+    """Gate and up of one token, captured and replayed on other ids each time, give what plain launches give."""
+    import numpy as np
+    monkeypatch.setenv("ZTVM_MOE_GROUPED", knob) if knob else monkeypatch.delenv("ZTVM_MOE_GROUPED", raising=False)
+    be = z.backend.CudaMatmulBackend(0)
+    rng = np.random.default_rng(3)
+    slots, (_, W, s, b) = 9, z.synth.make_weights(rng, FFN, D, bits=4, sigma_s=0.02, lead=(E,))
+    x, gu = dev.put(z.synth.make_x(rng, 1, D)), dev.empty((1, slots, 2 * FFN), np.float16, fill=0.0)
+    w, s, b = dev.put(W), dev.put(s), dev.put(b)
+    ids, pod, rec = dev.empty((1, slots), np.uint32, fill=0), moe_gate_pod_args(D, FFN, slots), DecodeRecorder(be)
+    for out in (gu, gu.view(-1)[FFN:]):
+        rec.dispatch("int4_matmul_tiled_affine_moe", [out, x, s, w, pod, b, ids], (16, 1, slots))
+    step = rec.capture()
+    for k in range(4):
+        ids.copy_(torch.tensor(rng.integers(0, E, (1, slots)).astype(np.int32)))
+        gu.fill_(float("nan"))
+        torch.cuda.synchronize()
+        step.replay()
+        torch.cuda.synchronize()
+        got = gu.clone()
+        gu.fill_(float("nan"))
+        torch.cuda.synchronize()
+        rec.run_eager()
+        torch.cuda.synchronize()
+        assert torch.equal(got, gu) and torch.isfinite(gu.float()).all()
+    be.close()

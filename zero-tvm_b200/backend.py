@@ -296,10 +296,19 @@ class CudaMatmulBackend:
         ids = bindings[6] if len(bindings) > 6 else None
         if desc is None or ids is None:
             raise ValueError(f"{entry}: MoE variants need 8 PODArgs fields and ids at slot 6")
+        self.ctx.int4_matmul_moe(self._moe_desc(desc, weights, grid), out, x, scales, weights, biases, ids, stream)
+
+    def uses_moe_plan(self, entry: str, bindings: Sequence, grid: Sequence[int] = (1, 1, 1)) -> bool:
+        """Whether `dispatch` of these arguments, a complete MoE bind group, builds or reads the expert-sorted plan that
+        the context keeps."""
+        out, x, scales, weights, pod, biases, ids = bindings[:7]
+        desc = _decode_matmul(entry, tuple(pod))[2]
+        return self.ctx.int4_matmul_moe_uses_plan(self._moe_desc(desc, weights, grid), out, x, scales, weights, biases, ids)
+
+    def _moe_desc(self, desc, weights, grid: Sequence[int]) -> MoeDesc:
         mm, strides, k_packed = desc
         _gx, gy, gz = (list(grid) + [1, 1, 1])[:3]
-        self.ctx.int4_matmul_moe(MoeDesc(mm, self._experts_of(weights, mm.N, k_packed), gz, gy, *strides), out, x, scales, weights,
-                                 biases, ids, stream)
+        return MoeDesc(mm, self._experts_of(weights, mm.N, k_packed), gz, gy, *strides)
 
     @staticmethod
     def _experts_of(weights, n: int, k_packed: int) -> int:

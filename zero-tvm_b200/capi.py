@@ -15,7 +15,7 @@ LIB_PATH = os.environ.get("ZTVM_LIB") or os.path.join(_HERE, "lib", "libztvm_b20
 # every symbol include/ztvm_b200.h declares
 SYMBOLS = [
     "ztvm_version", "ztvm_status_string", "ztvm_init", "ztvm_destroy", "ztvm_last_error", "ztvm_sync",
-    "ztvm_int4_matmul", "ztvm_int4_matmul_multi", "ztvm_int4_matmul_host", "ztvm_int4_matmul_host_async", "ztvm_host_wait", "ztvm_int4_matmul_moe", "ztvm_int4_matmul_moe_noalloc",
+    "ztvm_int4_matmul", "ztvm_int4_matmul_multi", "ztvm_int4_matmul_host", "ztvm_int4_matmul_host_async", "ztvm_host_wait", "ztvm_int4_matmul_moe", "ztvm_int4_matmul_moe_uses_plan", "ztvm_int4_matmul_moe_noalloc",
     "ztvm_moe_router_logits", "ztvm_embedding_affine", "ztvm_moe_plan_reuse", "ztvm_moe_route_topk", "ztvm_moe_dispatch_plan", "ztvm_moe_ep_dispatch", "ztvm_int4_matmul_moe_ep", "ztvm_silu_mul_rows", "ztvm_peer_barrier", "ztvm_moe_ffn_ep", "ztvm_int4_matmul_nshard",
     "ztvm_fused_ffn",
     "ztvm_silu_mul",
@@ -90,6 +90,7 @@ def load() -> C.CDLL:
         "ztvm_int4_matmul_host_async": [vp, C.POINTER(MmDesc), vp, vp, vp, vp, vp],
         "ztvm_host_wait": [vp],
         "ztvm_int4_matmul_moe": [vp, C.POINTER(MoeDesc), vp, vp, vp, vp, vp, vp, vp],
+        "ztvm_int4_matmul_moe_uses_plan": [vp, C.POINTER(MoeDesc), vp, vp, vp, vp, vp, vp, C.POINTER(u32)],
         "ztvm_int4_matmul_moe_noalloc": [vp, C.POINTER(MoeDesc), vp, vp, vp, vp, vp, vp, vp],
         "ztvm_moe_router_logits": [vp, u32, u32, u32, u32, vp, vp, vp, vp, vp, vp],
         "ztvm_embedding_affine": [vp, u32, u32, u32, u32, vp, vp, vp, vp, vp, vp],
@@ -207,6 +208,13 @@ class Context:
     def int4_matmul_moe(self, desc: MoeDesc, y, x, scales, packed_w, biases, ids, stream=None):
         check(self._lib.ztvm_int4_matmul_moe(self.handle, C.byref(desc), addr(y), addr(x), addr(scales),
                                              addr(packed_w), addr(biases), addr(ids), stream_ptr(stream)))
+
+    def int4_matmul_moe_uses_plan(self, desc: MoeDesc, y, x, scales, packed_w, biases, ids) -> bool:
+        """Whether int4_matmul_moe would run these arguments on the context's expert-sorted plan."""
+        n = C.c_uint32(0)
+        check(self._lib.ztvm_int4_matmul_moe_uses_plan(self.handle, C.byref(desc), addr(y), addr(x), addr(scales),
+                                                       addr(packed_w), addr(biases), addr(ids), C.byref(n)))
+        return bool(n.value)
 
     def int4_matmul_moe_noalloc(self, desc: MoeDesc, y, x, scales, packed_w, biases, ids, stream=None):
         """The grouped MoE matmul with its plan in a fixed device array (no allocation; limits in the header)."""

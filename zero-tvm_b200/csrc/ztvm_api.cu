@@ -559,10 +559,23 @@ static ztvm::GemvParams moe_params(ztvm_ctx* ctx, const ztvm_moe_desc* md, void*
   return p;
 }
 
-ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y, const void* x, const void* scales,
-                                 const void* packed_w, const void* biases, const uint32_t* ids, void* stream) {
-  ztvm_status s = check_ctx(ctx);
-  if (s) return s;
+// The kernel ztvm_int4_matmul_moe runs a call on: one of moe_pick's grouped kernels, which read an expert-sorted plan, or 0
+// for the per-pair GEMV. Many pairs are sorted by expert: while an expert sees only a few of them the job is bound by
+// streaming each active expert's weights once, with many it is a real contraction.
+// (3-bit codes, whose per-pair kernel is slow, from 32 pairs on; the exact-code grouped kernels of 4-bit ones from 64 on,
+// the tiles with f16 weights from 128 on.)
+static int moe_route(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::GemvParams& p, const void* y) {
+  const uint64_t pairs = (uint64_t)md->tokens * md->slots;
+  if (pairs >= (1ull << 31)) return 0;
+  if (ctx->moe_grouped >= 0) return ctx->moe_grouped ? moe_pick(ctx, md, p, y) : 0;
+  if (pairs < (md->mm.bits == 3 ? 32u : 64u)) return 0;
+  const int pick = moe_pick(ctx, md, p, y);
+  return (pick == 1 || pick == 3) && pairs < 128 ? 0 : pick;
+}
+
+static ztvm_status check_moe(const ztvm_moe_desc* md, const void* y, const void* x, const void* scales, const void* packed_w,
+                             const void* biases, const uint32_t* ids) {
+  ztvm_status s;
   if (!md) return fail(ZTVM_ERR_NULL_POINTER, "desc is NULL");
   const ztvm_mm_desc* d = &md->mm;
   if ((s = check_desc(d, false))) return s;
@@ -578,55 +591,62 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
   if (md->ids_stride < md->slots) return fail(ZTVM_ERR_BAD_DIMS, "ids_stride=%u < slots=%u", md->ids_stride, md->slots);
   if ((md->in_slot_stride | md->in_tok_stride) % 8)
     return fail(ZTVM_ERR_ALIGNMENT, "input strides must be multiples of 8 elements (16-byte activation loads)");
+  return ZTVM_OK;
+}
+
+ztvm_status ztvm_int4_matmul_moe_uses_plan(ztvm_ctx* ctx, const ztvm_moe_desc* md, const void* y, const void* x,
+                                           const void* scales, const void* packed_w, const void* biases,
+                                           const uint32_t* ids, uint32_t* uses_plan) {
+  ztvm_status s = check_ctx(ctx);
+  if (s) return s;
+  if (!uses_plan) return fail(ZTVM_ERR_NULL_POINTER, "uses_plan is NULL");
+  if ((s = check_moe(md, y, x, scales, packed_w, biases, ids))) return s;
+  *uses_plan = 0;
+  if (md->tokens)
+    *uses_plan = moe_route(ctx, md, moe_params(ctx, md, const_cast<void*>(y), x, scales, packed_w, biases, ids), y) != 0;
+  return ZTVM_OK;
+}
+
+ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y, const void* x, const void* scales,
+                                 const void* packed_w, const void* biases, const uint32_t* ids, void* stream) {
+  ztvm_status s = check_ctx(ctx);
+  if (s) return s;
+  if ((s = check_moe(md, y, x, scales, packed_w, biases, ids))) return s;
+  if (md->tokens == 0) return ZTVM_OK;
+  const ztvm_mm_desc* d = &md->mm;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  ztvm_mm_desc dd = *d;
-  dd.M = 1;
-  // Many pairs: sort them by expert. While an expert sees only a few pairs the job is bound by streaming each active
-  // expert's weights once (streaming kernel); with many pairs per expert it is a real contraction (tensor-core tiles,
-  // each expert's weights dequantised once per 128 pairs).
   const uint64_t pairs = (uint64_t)md->tokens * md->slots;
-  // (3-bit codes, whose per-pair kernel is slow, from 32 pairs on; the exact-code grouped kernels of 4-bit ones from 64 on.)
-  const bool want_grouped = ctx->moe_grouped < 0 ? pairs >= (d->bits == 3 ? 32u : 64u) : ctx->moe_grouped >= 1;
-  if (want_grouped && pairs < (1ull << 31)) {
-    const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
-    const int pick = moe_pick(ctx, md, p, y);
-    const bool f16_weights = pick == 1 || pick == 3;
-    if (pick && !(ctx->moe_grouped < 0 && f16_weights && pairs < 128)) {
-      const size_t need = ztvm::moe_grouped_scratch_bytes(md->experts, (uint32_t)pairs);
-      if (ctx->d_ws_bytes < need) {
-        ZTVM_CUDA(cudaDeviceSynchronize());
-        if ((s = grow(&ctx->d_ws, &ctx->d_ws_bytes, need, false))) return s;
-        ctx->plan_ids = nullptr;
-      }
-      uint32_t* ws = static_cast<uint32_t*>(ctx->d_ws);
-      const uint32_t tile_rows = pick == 4 ? ztvm::batch_moe_tile_rows(md->experts, pairs) : pick == 2 ? ztvm::kMoeTcTileRows : ztvm::kMoeTaTileRows;
-      // gate, up and down of one step walk the same id list: with ztvm_moe_plan_reuse on, its plan is built once
-      const bool reuse = ctx->plan_reuse && pick != 3 && ctx->plan_ids == ids && ctx->plan_segs == nullptr &&
-                         ctx->plan_tokens == md->tokens && ctx->plan_slots == md->slots && ctx->plan_stride == md->ids_stride &&
-                         ctx->plan_tile_rows == tile_rows && ctx->plan_experts == md->experts;
-      if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe(p, (int)d->bits, md->tokens, md->slots, ws, st, reuse));
-      else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
-      else if (pick == 1) ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, md->slots, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
-      else ZTVM_CUDA(ztvm::launch_moe_grouped(p, md->tokens, md->slots, ws, ctx->err_counter + 1, st));
-      ctx->plan_ids = pick != 3 ? ids : nullptr; ctx->plan_segs = nullptr; ctx->plan_tokens = md->tokens; ctx->plan_slots = md->slots;
-      ctx->plan_stride = md->ids_stride; ctx->plan_tile_rows = tile_rows; ctx->plan_experts = md->experts;
-      return ZTVM_OK;
+  const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
+  if (const int pick = moe_route(ctx, md, p, y)) {
+    const size_t need = ztvm::moe_grouped_scratch_bytes(md->experts, (uint32_t)pairs);
+    if (ctx->d_ws_bytes < need) {
+      ZTVM_CUDA(cudaDeviceSynchronize());
+      if ((s = grow(&ctx->d_ws, &ctx->d_ws_bytes, need, false))) return s;
+      ctx->plan_ids = nullptr;
     }
+    uint32_t* ws = static_cast<uint32_t*>(ctx->d_ws);
+    const uint32_t tile_rows = pick == 4 ? ztvm::batch_moe_tile_rows(md->experts, pairs) : pick == 2 ? ztvm::kMoeTcTileRows : ztvm::kMoeTaTileRows;
+    // gate, up and down of one step walk the same id list: with ztvm_moe_plan_reuse on, its plan is built once
+    const bool reuse = ctx->plan_reuse && pick != 3 && ctx->plan_ids == ids && ctx->plan_segs == nullptr &&
+                       ctx->plan_tokens == md->tokens && ctx->plan_slots == md->slots && ctx->plan_stride == md->ids_stride &&
+                       ctx->plan_tile_rows == tile_rows && ctx->plan_experts == md->experts;
+    if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe(p, (int)d->bits, md->tokens, md->slots, ws, st, reuse));
+    else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
+    else if (pick == 1) ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, md->slots, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
+    else ZTVM_CUDA(ztvm::launch_moe_grouped(p, md->tokens, md->slots, ws, ctx->err_counter + 1, st));
+    ctx->plan_ids = pick != 3 ? ids : nullptr; ctx->plan_segs = nullptr; ctx->plan_tokens = md->tokens; ctx->plan_slots = md->slots;
+    ctx->plan_stride = md->ids_stride; ctx->plan_tile_rows = tile_rows; ctx->plan_experts = md->experts;
+    return ZTVM_OK;
   }
   // grid.y carries the token: split very long token lists into slabs of 65535
   for (uint32_t t0 = 0; t0 < md->tokens; t0 += 65535) {
     const uint32_t nt = md->tokens - t0 < 65535 ? md->tokens - t0 : 65535;
-    ztvm::GemvParams p = gemv_params(ctx, &dd, y, x, scales, packed_w, biases);
-    p.X = static_cast<const __half*>(x) + (size_t)t0 * md->in_tok_stride;
-    p.Y = static_cast<__half*>(y) + (size_t)t0 * md->out_tok_stride;
-    p.ids = ids + (size_t)t0 * md->ids_stride;
-    p.experts = md->experts;
-    p.in_slot_stride = md->in_slot_stride; p.out_slot_stride = md->out_slot_stride;
-    p.in_tok_stride = md->in_tok_stride; p.out_tok_stride = md->out_tok_stride;
-    p.ids_stride = md->ids_stride;
-    p.err_counter = ctx->err_counter;
-    if (use_mma(ctx, d, 1)) ZTVM_CUDA(ztvm::launch_gemv_mma(p, true, nt, md->slots, st));
-    else ZTVM_CUDA(ztvm::launch_gemv(p, (int)d->bits, true, nt, md->slots, ctx->sm_count, st));
+    ztvm::GemvParams q = p;
+    q.X = p.X + (size_t)t0 * md->in_tok_stride;
+    q.Y = static_cast<__half*>(y) + (size_t)t0 * md->out_tok_stride;
+    q.ids = ids + (size_t)t0 * md->ids_stride;
+    if (use_mma(ctx, d, 1)) ZTVM_CUDA(ztvm::launch_gemv_mma(q, true, nt, md->slots, st));
+    else ZTVM_CUDA(ztvm::launch_gemv(q, (int)d->bits, true, nt, md->slots, ctx->sm_count, st));
   }
   return ZTVM_OK;
 }

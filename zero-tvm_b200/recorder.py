@@ -26,9 +26,9 @@ def _span(buf):
 
 
 def _independent_pair(be, a, b):
-    """Whether two consecutive recorded calls are the gate and the up projection of one MoE block: same entry, PODArgs,
-    activations, ids and grid, outputs that share no element, and so few pairs that neither needs the expert-sorted plan
-    (whose work buffer the first would fill for the second)."""
+    """Whether two consecutive recorded calls are the gate and the up projection of one MoE block of a few pairs: same
+    entry, PODArgs, activations, ids and grid, and outputs that share no element. (Whether the library runs them without
+    the plan that calls of a context share is the library's to say: DecodeRecorder._side_by_side.)"""
     if a[0] != be.dispatch or b[0] != be.dispatch:
         return False
     (ea, ba, ga), (eb, bb, gb) = a[1], b[1]
@@ -38,7 +38,7 @@ def _independent_pair(be, a, b):
     if None in spans or spans[2] != spans[3] or spans[4] != spans[5]:
         return False
     _, moe, desc = _decode_matmul(ea, tuple(ba[4]))
-    if not moe or desc is None or ga[1] * ga[2] >= (64 if desc[0].bits == 4 else 32):   # (from there on calls are grouped)
+    if not moe or desc is None or ga[1] * ga[2] >= (64 if desc[0].bits == 4 else 32):   # (more pairs fill the chip by themselves)
         return False
     rows, (_in_slot, out_slot, _in_tok, out_tok, _ids) = desc[0].N, desc[1]
     slots, tokens = ga[2], ga[1]
@@ -83,6 +83,11 @@ class DecodeRecorder:
         for fn, args, kw in self._calls:
             fn(*args, stream=stream, **kw)
 
+    def _side_by_side(self, a, b):
+        """Two calls become branches of the graph only where the library runs both on the kernel that reads ids directly:
+        the expert-sorted plan is one buffer, which the first call would fill while the second reads or fills it."""
+        return _independent_pair(self.be, a, b) and not self.be.uses_moe_plan(*a[1]) and not self.be.uses_moe_plan(*b[1])
+
     def _run_captured(self, main, side):
         """The sequence inside the capture. The gate and up projections of a decoded token are a few CTAs each and read the
         same inputs: as two branches of the graph they run side by side (four blocks of one token, 256 experts of
@@ -91,7 +96,7 @@ class DecodeRecorder:
         i = 0
         while i < len(self._calls):
             fn, args, kw = self._calls[i]
-            if i + 1 < len(self._calls) and _independent_pair(self.be, self._calls[i], self._calls[i + 1]):
+            if i + 1 < len(self._calls) and self._side_by_side(self._calls[i], self._calls[i + 1]):
                 side.wait_event(main.record_event())
                 fn(*args, stream=main.cuda_stream, **kw)
                 fn, args, kw = self._calls[i + 1]
