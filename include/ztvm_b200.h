@@ -20,6 +20,11 @@
  *    The context's own stream is non-blocking: it is NOT ordered against the legacy default stream.
  *    A caller whose other work runs on the legacy default stream passes cudaStreamLegacy (handle 1),
  *    not NULL, to have the call ordered with that work.
+ *  - Work buffers: the calls that need device memory of their own (the grouped MoE matmul for its plan, the two-launch fused
+ *    FFN) take it from the context. Calls on different streams use different buffers. A captured call uses one that belongs
+ *    to its graph, which no other call touches and which the context gets back when the graph and its executables are
+ *    gone. A buffer is allocated when a stream or a capture first needs it, or needs more (a stream synchronises for that;
+ *    a capture is not disturbed).
  *  - Layouts: packed weights u32[N][K*bits/32], 4-bit code i of a word at bits [4i,4i+4)
  *    (src/compiler/shaders/int4_matmul.gen.ts:157-167); 3-bit code i of a row at bit 3i of the
  *    row's LSB-first bitstream (int4_matmul.gen.ts:115-131); scales / biases f16[N][K/group];
@@ -166,7 +171,7 @@ ZTVM_API ztvm_status ztvm_moe_plan_reuse(ztvm_ctx* ctx, int32_t enable);
  * (WebGPU buffers are all created up front there); it exists for hosts whose device memory is entirely handed
  * to their own pool, or whose serving loop cannot take the device-wide synchronisation that growing a work
  * buffer costs. ztvm_int4_matmul_moe keeps its plan (expert histogram, tile table, sorted pair list) in a
- * buffer that grows on demand; this entry point keeps it in a fixed array inside the library's device image
+ * work buffer of the context; this entry point keeps it in a fixed array inside the library's device image
  * and makes no allocating call at all.
  *  - Limits: tokens*slots <= ZTVM_MOE_NOALLOC_MAX_PAIRS and experts <= ZTVM_MOE_NOALLOC_MAX_EXPERTS, else
  *    ZTVM_ERR_TOO_LARGE. Only the grouped kernels run here (there is no fall-back to the per-pair kernel):
@@ -318,8 +323,7 @@ ZTVM_API ztvm_status ztvm_int4_matmul_nshard(ztvm_ctx* ctx, const ztvm_mm_desc* 
  * lacks (src/zero-tvm/engine-core.ts:2513-2519 pays gate_up matmul + silu_mul on affine models).
  * 4-bit, group 64, K % 256 == 0, M <= 8: ONE launch of the persistent GEMV, whose CTAs own gate and up tiles of the
  * same output rows. Other shapes (group 32 / 128, 3-bit, 8-bit, M > 8): the 2 * ffn-row matmul into an f32 buffer of
- * the context (grown on demand: device synchronise + cudaMalloc when a call needs more than any before it), then the
- * activation -- same arithmetic, two launches. desc->out_f32 must be 0. */
+ * the context (a work buffer: see the conventions), then the activation -- same arithmetic, two launches. desc->out_f32 must be 0. */
 ZTVM_API ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* desc, void* h, const void* x, const void* scales,
                            const void* packed_w, const void* biases, void* stream);
 

@@ -8,6 +8,7 @@
 
 #include "../../include/ztvm_b200.h"
 #include "ztvm_kernels.h"
+#include "ztvm_workbuf.h"
 
 struct ztvm_ctx {
   uint32_t magic;
@@ -27,15 +28,10 @@ struct ztvm_ctx {
   struct HostLane { cudaStream_t stream; void* d_x; size_t d_x_bytes; void* d_y; size_t d_y_bytes; } lanes[3];
   uint32_t next_lane;
   void* d_y; size_t d_y_bytes;
-  // plan scratch of the grouped MoE matmul (grown on demand: a call that needs more synchronises the device,
-  // reallocates and goes on; make one call at the largest size before capturing a graph)
-  void* d_ws; size_t d_ws_bytes;
-  void* d_ffn; size_t d_ffn_bytes;      // f32 gate/up rows of ztvm_fused_ffn's two-launch form
+  ztvm::WorkBufs* work;   // plans of the grouped MoE matmul, f32 gate/up rows of ztvm_fused_ffn's two-launch form
   // env ZTVM_MOE_GROUPED (a measurement knob): 0 forces the per-pair GEMV, 1 the tensor-core tiles, 2 the streaming
   // grouped kernel; unset = by size (few pairs per-pair; then the exact-code kernels while an expert sees few of them)
   int moe_grouped;
-  // what the plan in d_ws was built from (ztvm_int4_matmul_moe_ep reuse_plan)
-  const void* plan_ids; const void* plan_segs; uint32_t plan_tokens, plan_tile_rows, plan_experts, plan_slots, plan_stride;
   int plan_reuse;   // ztvm_moe_plan_reuse: consecutive ztvm_int4_matmul_moe calls over one id list share its plan
   int moe_tiles_sm; // env ZTVM_MOE_TILES=sm: the grouped MoE tiles with both operands in shared memory (a measurement knob)
 };
@@ -192,6 +188,8 @@ ztvm_status ztvm_init(int32_t device_ordinal, ztvm_ctx** out_ctx) {
   ztvm_ctx* c = new (std::nothrow) ztvm_ctx();
   if (!c) return fail(ZTVM_ERR_CUDA, "out of host memory");
   memset(c, 0, sizeof(*c));
+  c->work = new (std::nothrow) ztvm::WorkBufs();
+  if (!c->work) { delete c; return fail(ZTVM_ERR_CUDA, "out of host memory"); }
   c->device = device_ordinal;
   c->sm_count = prop.multiProcessorCount;
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
@@ -199,6 +197,7 @@ ztvm_status ztvm_init(int32_t device_ordinal, ztvm_ctx** out_ctx) {
   if (e == cudaSuccess) e = cudaMemset(c->err_counter, 0, 256);
   if (e != cudaSuccess) {
     if (c->stream) cudaStreamDestroy(c->stream);
+    delete c->work;
     delete c;
     return cuda_fail(e, "context set-up");
   }
@@ -222,8 +221,8 @@ ztvm_status ztvm_destroy(ztvm_ctx* ctx) {
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
   if (ctx->d_x) cudaFree(ctx->d_x);
   if (ctx->d_y) cudaFree(ctx->d_y);
-  if (ctx->d_ws) cudaFree(ctx->d_ws);
-  if (ctx->d_ffn) cudaFree(ctx->d_ffn);
+  ctx->work->free_all();
+  delete ctx->work;
   for (auto& l : ctx->lanes) {
     if (l.stream) { cudaStreamSynchronize(l.stream); cudaStreamDestroy(l.stream); }
     if (l.d_x) cudaFree(l.d_x);
@@ -378,13 +377,11 @@ ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* h, const 
     }
   }
   const size_t need = (size_t)d->M * gu.N * sizeof(float);
-  if (ctx->d_ffn_bytes < need) {
-    ZTVM_CUDA(cudaDeviceSynchronize());
-    if ((s = grow(&ctx->d_ffn, &ctx->d_ffn_bytes, need, false))) return s;
-  }
+  ztvm::WorkBuf* rows = nullptr;
+  ZTVM_CUDA(ctx->work->get(ztvm::WorkBufs::kFfnRows, need, st, &rows));
   gu.out_f32 = 1;
-  if ((s = ztvm_int4_matmul(ctx, &gu, ctx->d_ffn, x, scales, packed_w, biases, st))) return s;
-  ZTVM_CUDA(ztvm::launch_silu_mul_f32(static_cast<const float*>(ctx->d_ffn), static_cast<__half*>(h), d->M, d->N, st));
+  if ((s = ztvm_int4_matmul(ctx, &gu, rows->p, x, scales, packed_w, biases, st))) return s;
+  ZTVM_CUDA(ztvm::launch_silu_mul_f32(static_cast<const float*>(rows->p), static_cast<__half*>(h), d->M, d->N, st));
   return ZTVM_OK;
 }
 
@@ -618,24 +615,19 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
   const uint64_t pairs = (uint64_t)md->tokens * md->slots;
   const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
   if (const int pick = moe_route(ctx, md, p, y)) {
-    const size_t need = ztvm::moe_grouped_scratch_bytes(md->experts, (uint32_t)pairs);
-    if (ctx->d_ws_bytes < need) {
-      ZTVM_CUDA(cudaDeviceSynchronize());
-      if ((s = grow(&ctx->d_ws, &ctx->d_ws_bytes, need, false))) return s;
-      ctx->plan_ids = nullptr;
-    }
-    uint32_t* ws = static_cast<uint32_t*>(ctx->d_ws);
+    ztvm::WorkBuf* buf = nullptr;
+    ZTVM_CUDA(ctx->work->get(ztvm::WorkBufs::kPlan, ztvm::moe_grouped_scratch_bytes(md->experts, (uint32_t)pairs), st, &buf));
+    uint32_t* ws = static_cast<uint32_t*>(buf->p);
     const uint32_t tile_rows = pick == 4 ? ztvm::batch_moe_tile_rows(md->experts, pairs) : pick == 2 ? ztvm::kMoeTcTileRows : ztvm::kMoeTaTileRows;
     // gate, up and down of one step walk the same id list: with ztvm_moe_plan_reuse on, its plan is built once
-    const bool reuse = ctx->plan_reuse && pick != 3 && ctx->plan_ids == ids && ctx->plan_segs == nullptr &&
-                       ctx->plan_tokens == md->tokens && ctx->plan_slots == md->slots && ctx->plan_stride == md->ids_stride &&
-                       ctx->plan_tile_rows == tile_rows && ctx->plan_experts == md->experts;
+    const ztvm::PlanKey key = {ids, nullptr, md->tokens, md->slots, md->ids_stride, tile_rows, md->experts};
+    const bool reuse = ctx->plan_reuse && pick != 3 && buf->plan == key;
+    buf->plan.ids = nullptr;
     if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe(p, (int)d->bits, md->tokens, md->slots, ws, st, reuse));
     else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
     else if (pick == 1) ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, md->slots, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
     else ZTVM_CUDA(ztvm::launch_moe_grouped(p, md->tokens, md->slots, ws, ctx->err_counter + 1, st));
-    ctx->plan_ids = pick != 3 ? ids : nullptr; ctx->plan_segs = nullptr; ctx->plan_tokens = md->tokens; ctx->plan_slots = md->slots;
-    ctx->plan_stride = md->ids_stride; ctx->plan_tile_rows = tile_rows; ctx->plan_experts = md->experts;
+    if (pick != 3) buf->plan = key;
     return ZTVM_OK;
   }
   // grid.y carries the token: split very long token lists into slabs of 65535
@@ -694,7 +686,7 @@ ztvm_status ztvm_moe_plan_reuse(ztvm_ctx* ctx, int32_t enable) {
   ztvm_status s = check_ctx(ctx);
   if (s) return s;
   ctx->plan_reuse = enable ? 1 : 0;
-  ctx->plan_ids = nullptr;
+  ctx->work->drop_plans();
   return ZTVM_OK;
 }
 
@@ -707,7 +699,7 @@ ztvm_status ztvm_moe_route_topk(ztvm_ctx* ctx, uint32_t E, uint32_t K, uint32_t 
   if (K == 0 || K > 32 || K > E) return fail(ZTVM_ERR_BAD_DIMS, "K=%u: need 1 <= K <= min(32, E)", K);
   if (tokens == 0) return ZTVM_OK;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  ctx->plan_ids = nullptr;   // a new id list: whatever plan the context holds describes the old one
+  ctx->work->drop_plans();   // a new id list: whatever plans the context holds describe the old one
   ZTVM_CUDA(ztvm::launch_route_topk(logits, ids, scores, tokens, E, K, norm_topk != 0, has_shared != 0, st));
   return ZTVM_OK;
 }
@@ -729,19 +721,16 @@ ztvm_status ztvm_moe_dispatch_plan(ztvm_ctx* ctx, const uint32_t* ids, uint32_t 
     ZTVM_CUDA(cudaMemsetAsync(send_counts, 0, (size_t)world * 8, st));
     return ZTVM_OK;
   }
-  const size_t need = ztvm::moe_grouped_scratch_bytes(experts, (uint32_t)pairs);
-  if (ctx->d_ws_bytes < need) {
-    ZTVM_CUDA(cudaDeviceSynchronize());
-    if ((s = grow(&ctx->d_ws, &ctx->d_ws_bytes, need, false))) return s;
-  }
-  ctx->plan_ids = nullptr;
+  ztvm::WorkBuf* buf = nullptr;
+  ZTVM_CUDA(ctx->work->get(ztvm::WorkBufs::kPlan, ztvm::moe_grouped_scratch_bytes(experts, (uint32_t)pairs), st, &buf));
+  buf->plan.ids = nullptr;
   ztvm::GemvParams p;
   memset(&p, 0, sizeof(p));
   p.ids = ids;
   p.experts = experts;
   p.ids_stride = ids_stride;
   p.err_counter = ctx->err_counter;
-  ZTVM_CUDA(ztvm::launch_moe_dispatch_plan(p, tokens, slots, experts_per_rank, world, static_cast<uint32_t*>(ctx->d_ws),
+  ZTVM_CUDA(ztvm::launch_moe_dispatch_plan(p, tokens, slots, experts_per_rank, world, static_cast<uint32_t*>(buf->p),
                                            reinterpret_cast<long long*>(order), local_expert,
                                            reinterpret_cast<long long*>(send_counts), st));
   return ZTVM_OK;
@@ -813,20 +802,16 @@ ztvm_status ztvm_int4_matmul_moe_ep(ztvm_ctx* ctx, const ztvm_moe_desc* md, cons
   if (pick != 1 && pick != 2)
     return fail(ZTVM_ERR_UNSUPPORTED, "the expert-parallel form runs the grouped kernels only: bits=4, group=64, K %% 64 == 0 "
                 "(got bits=%u group=%u K=%u N=%u)", d->bits, d->group, d->K, d->N);
-  const size_t need = ztvm::moe_grouped_scratch_bytes(md->experts, md->tokens);
-  if (ctx->d_ws_bytes < need) {
-    ZTVM_CUDA(cudaDeviceSynchronize());
-    if ((s = grow(&ctx->d_ws, &ctx->d_ws_bytes, need, false))) return s;
-    ctx->plan_ids = nullptr;
-  }
-  const uint32_t tile_rows = pick == 1 ? ztvm::kMoeTaTileRows : ztvm::kMoeTcTileRows;
-  const bool reuse = rows->reuse_plan && ctx->plan_ids == ids && ctx->plan_segs == rows->seg_counts &&
-                     ctx->plan_tokens == md->tokens && ctx->plan_tile_rows == tile_rows && ctx->plan_experts == md->experts;
-  uint32_t* ws = static_cast<uint32_t*>(ctx->d_ws);
+  ztvm::WorkBuf* buf = nullptr;
+  ZTVM_CUDA(ctx->work->get(ztvm::WorkBufs::kPlan, ztvm::moe_grouped_scratch_bytes(md->experts, md->tokens), st, &buf));
+  const ztvm::PlanKey key = {ids, rows->seg_counts, md->tokens, 1, md->ids_stride, pick == 1 ? ztvm::kMoeTaTileRows : ztvm::kMoeTcTileRows,
+                             md->experts};
+  const bool reuse = rows->reuse_plan && buf->plan == key;
+  buf->plan.ids = nullptr;
+  uint32_t* ws = static_cast<uint32_t*>(buf->p);
   if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, 1, ws, ctx->sm_count, st, reuse));
   else ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, 1, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
-  ctx->plan_ids = ids; ctx->plan_segs = rows->seg_counts; ctx->plan_tokens = md->tokens; ctx->plan_slots = 1;
-  ctx->plan_stride = md->ids_stride; ctx->plan_tile_rows = tile_rows; ctx->plan_experts = md->experts;
+  buf->plan = key;
   return ZTVM_OK;
 }
 

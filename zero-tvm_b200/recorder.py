@@ -5,7 +5,7 @@ the C ABI is captured once into a CUDA graph and replayed per token, so a step c
     rec = DecodeRecorder(backend)
     rec.dispatch("int4_matmul_sg_tiled_vec4h_affine", [qkv, x, s, W, pod, b], grid)   # any method of the backend
     rec.router_logits("moe_router_logits", [...], grid); rec.router_topk(...); ...
-    step = rec.capture()        # one eager pass first (function attributes, work buffers), then the capture
+    step = rec.capture()        # one eager pass first (kernels loaded, bad calls rejected), then the capture
     step.replay()               # every buffer is bound by address, as in the engine's bind groups
 
 Only calls of this library are recorded; whatever else a step needs (attention, norms) would be captured by its own
@@ -114,7 +114,7 @@ class DecodeRecorder:
         self._run(s.cuda_stream if s.cuda_stream else 1)
 
     def capture(self, plan_reuse: bool = True):
-        """One eager pass (sets kernel attributes, grows the context's work buffers: neither may happen inside a
+        """One eager pass (loads the kernels and sets their attributes; what it rejects is rejected before a
         capture), then the capture. plan_reuse: the MoE matmuls of the step share one expert-sorted plan per id list
         (valid because, inside the recorded sequence, only the recorded router writes the id list)."""
         import torch
