@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
     (65, 1001, 2176, False), (77, 2176, 3072, False), (128, 392, 8192, True),                           # 128
     (129, 250, 4224, False), (200, 5000, 1152, False), (257, 9600, 640, False), (300, 2048, 4096, False),  # 256, one to many shares
     (273, 12200, 1088, False), (700, 6200, 2176, True), (1000, 5900, 320, False), (352, 130, 4160, False),  # up to 352
-    (1000, 6100, 1088, False), (700, 6200, 2176, True), (50, 20000, 1664, False), (260, 19900, 640, False),  # whole waves and a rest
+    (1000, 6100, 1088, False), (300, 1003, 4096, True), (350, 20011, 128, False), (50, 20000, 1664, False), (260, 19900, 640, False),  # whole waves and a rest
 ])
 def test_tiles_and_shares(group, affine, M, N, K, f32, backend, dev, oracle_c):
     if K % group:

@@ -335,6 +335,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
     // ---- epilogue: D[weight row][token] in TMEM -> y[token][weight row] ------------------------------------------
     acc_ok = ok && mbar_wait(bar_accum, 0u, p.status, 5u, abort_flag);
+    acc_ok = __all_sync(0xffffffffu, acc_ok);            // the loads from tensor memory below are the whole warp's
     tc_fence_after();
     asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be read by the previous kernel in the stream
     // f16 rows of whole 16-byte pieces: the tile is turned round in the (now idle) activation ring. Phase 1: a thread
@@ -396,6 +397,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
               if (cb * 32 + i < (int)mrows) dst[(size_t)i * p.N] = __float2half_rn(__uint_as_float(v[i]));
           }
         }
+        __syncwarp();   // lanes past N are back before the next load, which takes the whole warp
       }
     }
   }
@@ -429,28 +431,30 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         uint32_t v[8];
         tmem_ld8(tmem_base + lane_base + b * 8u, v);
         tmem_ld_wait();
-        if (n >= p.N) continue;
-        float r[8];
+        if (n < p.N) {
+          float r[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = 0.f;
-        for (uint32_t z = 0; z < split; ++z) {              // in CTA order, wherever this CTA stands in it
-          if (z == kz) {
+          for (int i = 0; i < 8; ++i) r[i] = 0.f;
+          for (uint32_t z = 0; z < split; ++z) {              // in CTA order, wherever this CTA stands in it
+            if (z == kz) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) r[i] += __uint_as_float(v[i]);
-          } else {
-            const float4* const got = reinterpret_cast<const float4*>(gen_base) + (((z < kz ? z : z - 1u) * per + b - kz * per) * kTaRows + r_tile) * 2u;
-            const float4 g0 = got[0], g1 = got[1];
-            r[0] += g0.x; r[1] += g0.y; r[2] += g0.z; r[3] += g0.w;
-            r[4] += g1.x; r[5] += g1.y; r[6] += g1.z; r[7] += g1.w;
+              for (int i = 0; i < 8; ++i) r[i] += __uint_as_float(v[i]);
+            } else {
+              const float4* const got = reinterpret_cast<const float4*>(gen_base) + (((z < kz ? z : z - 1u) * per + b - kz * per) * kTaRows + r_tile) * 2u;
+              const float4 g0 = got[0], g1 = got[1];
+              r[0] += g0.x; r[1] += g0.y; r[2] += g0.z; r[3] += g0.w;
+              r[4] += g1.x; r[5] += g1.y; r[6] += g1.z; r[7] += g1.w;
+            }
+          }
+#pragma unroll
+          for (uint32_t i = 0; i < 8; ++i) {
+            if (b * 8u + i >= mrows) break;
+            const size_t o = (size_t)(m0 + b * 8u + i) * p.N + n;
+            if (p.out_f32) reinterpret_cast<float*>(p.Y)[o] = r[i];
+            else reinterpret_cast<__half*>(p.Y)[o] = __float2half_rn(r[i]);
           }
         }
-#pragma unroll
-        for (uint32_t i = 0; i < 8; ++i) {
-          if (b * 8u + i >= mrows) break;
-          const size_t o = (size_t)(m0 + b * 8u + i) * p.N + n;
-          if (p.out_f32) reinterpret_cast<float*>(p.Y)[o] = r[i];
-          else reinterpret_cast<__half*>(p.Y)[o] = __float2half_rn(r[i]);
-        }
+        __syncwarp();     // lanes past N are back before the next load, which takes the whole warp
       }
     }
   }

@@ -394,6 +394,7 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeGemmPara
             for (int i = 0; i < 32 && n + i < p.N; ++i) dst_row[n + i] = __float2half_rn(__uint_as_float(v[i]));
           }
         }
+        __syncwarp();   // lanes without a row are back before the next load, which takes the whole warp
       }
     }
   }
