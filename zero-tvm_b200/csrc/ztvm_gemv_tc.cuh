@@ -53,9 +53,9 @@ __device__ __forceinline__ void tc_cp4_zfill(uint32_t dst, const void* src, uint
 // by each of them: lane (g, c) owns columns 2c and 2c + 1.
 // AL: K is whole slices and the tables allow a slice's scales to be copied in one piece.
 // W = warps per CTA: 16 (one CTA per SM, the whole shared memory as its ring) for projections that keep an SM busy for
-// tens of microseconds; 8 (two CTAs fit an SM: registers and shared memory halve) for small ones, so that the CTAs of
-// the NEXT launch in the stream -- already started under programmatic dependent launch -- sit beside this launch's and
-// stream their first weights while it finishes, instead of waiting for the SM to empty.
+// tens of microseconds; 8 (registers and shared memory halve) for small ones, so that a CTA of the NEXT launch in the stream
+// -- already started under programmatic dependent launch -- can sit beside this launch's and stream its first weights while it
+// finishes, instead of waiting for the SM to empty. Two CTAs of ONE launch must not: each has a fixed share of the rows.
 template <int BITS, bool G32, int NT, bool AFFINE, bool AL, int W>
 __global__ void __launch_bounds__(W * 32, 16 / W)
 gemv_tc_kernel(const GemvParams p) {
@@ -435,7 +435,7 @@ inline size_t tc_smem(const GemvParams& p, int sm_count, int warps) {
   return n;
 }
 constexpr size_t tc_smem_limit(int warps) { return warps == 8 ? 112 * 1024 : 227 * 1024; }
-// warps per CTA for a problem: 8 (two CTAs per SM) while an SM's share of the weights is small, else 16
+// warps per CTA for a problem: 8 while an SM's share of the weights is small, else 16
 template <int BITS, bool G32>
 inline int tc_warps_for(const GemvParams& p, int sm_count) {
   const bool small = tc_slices<BITS>(p) <= 8u && (uint64_t)p.N * p.KP * 4 / (uint64_t)sm_count <= 384u * 1024u;   // one K tile only
@@ -454,14 +454,18 @@ cudaError_t launch_tc_one(const GemvParams& p, unsigned grid, size_t smem, cudaS
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 16 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_limit(W));
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W == 8 ? kOnePerSmSmem : tc_smem_limit(W)));
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(W * 32);
-  cfg.dynamicSmemBytes = smem;
+  static_assert(tc_smem_limit(8) <= kOnePerSmSmem, "the padding holds what eight warps use");
+  // One share per SM (4-bit row, hidden 1536, ffn 3072, a step of four layers: 90 us without, 80 us with). Shares of a few rows, a
+  // router's, may as well sit side by side (router of 94 rows in a recorded MoE token: 35.8 us a step kept apart, 35.3 us).
+  const uint32_t out_rows = p.pair_rows ? p.pair_rows : p.N;
+  cfg.dynamicSmemBytes = W == 8 && out_rows > 4u * grid ? kOnePerSmSmem : smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

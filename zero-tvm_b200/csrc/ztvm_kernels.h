@@ -23,6 +23,14 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// Shared memory that a launch of one CTA per SM asks for at least. Such a grid gives each CTA a fixed share of the rows. Started
+// early, behind kernels that still hold SMs, its CTAs go to whatever slots come free first; where an SM has room for two of
+// them, some get two shares and others none (a recorded 4-bit row, hidden 3648, ffn 10944: the down projections behind a
+// SiLU that had let them in early made it 263 us, 212 us with one share per SM; 225 us before the SiLU let them in). More
+// than half of an SM's 228 KB (with the 1 KB that each CTA takes beside its own) keeps them apart; 112 KB stay for a CTA of
+// the launch before or after.
+constexpr size_t kOnePerSmSmem = 114 * 1024;
+
 struct GemvParams {
   const uint32_t* W;   // packed codes [N][KP] (MoE: [experts][N][KP])
   const __half* S;     // scales [N][SPR]
