@@ -22,8 +22,8 @@
  *    not NULL, to have the call ordered with that work.
  *  - Work buffers: the calls that need device memory of their own (the grouped MoE matmul for its plan, the two-launch fused
  *    FFN) take it from the context. Calls on different streams use different buffers. A captured call uses one that belongs
- *    to its graph, which no other call touches and which the context gets back when the graph and its executables are
- *    gone. A buffer is allocated when a stream or a capture first needs it, or needs more (a stream synchronises for that;
+ *    to its graph, which no other call touches; beyond the first 64 MB of those the context gets one back when the graph and
+ *    its executables are gone. A buffer is allocated when a stream or a capture first needs it, or needs more (a stream synchronises for that;
  *    a capture is not disturbed).
  *  - Layouts: packed weights u32[N][K*bits/32], 4-bit code i of a word at bits [4i,4i+4)
  *    (src/compiler/shaders/int4_matmul.gen.ts:157-167); 3-bit code i of a row at bit 3i of the
