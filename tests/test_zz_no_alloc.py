@@ -118,3 +118,17 @@ def test_noalloc_refuses_what_does_not_fit_or_is_not_a_tile_shape(backend, dev):
             call(**kw)
         assert e.value.status == code and word in str(e.value), (kw, e.value)
     backend.ctx.sync()
+
+
+def test_noalloc_refuses_rows_that_are_no_multiple_of_eight(backend, dev):
+    """... at every K, also one that only the batched kernel takes (which would accept any N)."""
+    mb = z.synth.moe_block(2, E=8, hidden=256, ffn=128, seed=1)
+    gw, gs, gb = (dev.put(a) for a in mb["gate"])
+    x, y, ids = dev.put(mb["x"]), dev.empty((2, 3, 128), np.float16, fill=-7.0), dev.put(np.zeros((2, 3), dtype=np.uint32))
+    for K in (256, 192):
+        with pytest.raises(z.ZtvmError) as e:
+            backend.ctx.int4_matmul_moe_noalloc(moe_desc(K, 100, 9, 3, 2, 0, 128, 256, 384), y, x, gs, gw, gb, ids)
+        assert e.value.status == z.capi.ERR_UNSUPPORTED and "N=100" in str(e.value)
+    assert (dev.get(y) == -7.0).all()
+    backend.ctx.int4_matmul_moe_noalloc(moe_desc(192, 104, 9, 3, 2, 0, 128, 256, 384), y, x, gs, gw, gb, ids)
+    backend.ctx.sync()

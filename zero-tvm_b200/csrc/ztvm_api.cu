@@ -671,7 +671,8 @@ ztvm_status ztvm_int4_matmul_moe_noalloc(ztvm_ctx* ctx, const ztvm_moe_desc* md,
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   const ztvm::GemvParams p = moe_params(ctx, md, y, x, scales, packed_w, biases, ids);
   const int pick = moe_pick(ctx, md, p, y);   // the same choice ztvm_int4_matmul_moe makes
-  if (!pick || d->bits != 4)
+  // (moe_pick may also name the batched kernel, which takes 3-bit codes and any N: this entry point's contract does not)
+  if (!pick || d->bits != 4 || d->N % 8)
     return fail(ZTVM_ERR_UNSUPPORTED,
                 "this entry point runs the grouped kernels only: bits=4, group=64, K %% 64 == 0, N %% 8 == 0 "
                 "(got bits=%u group=%u K=%u N=%u)", d->bits, d->group, d->K, d->N);
