@@ -4,7 +4,9 @@ import ctypes
 import os
 import re
 
+import numpy as np
 import pytest
+import torch
 
 import zero_tvm_b200 as z
 from zero_tvm_b200.backend import (Int4MatmulOpts, int4_matmul_entry, moe_down_pod_args, moe_gate_pod_args,
@@ -168,6 +170,29 @@ def test_backend_dispatch_argument_errors_need_no_gpu():
         be.dispatch("int4_matmul_tiled_affine_moe", [1, 2, 3, 4, [256, 32, 8], 5])  # no ids / short PODArgs
     with pytest.raises(ValueError):
         be.dispatch("int4_matmul_batched_dyn_affine", [1, 2, 3, 4, [256, 32, 8], 5])  # no M_ROWS
+
+
+@pytest.mark.parametrize("make", [list, tuple, np.array, lambda v: np.array(v, dtype=np.uint32), lambda v: torch.tensor(v),
+                                  lambda v: [torch.tensor(x) for x in v], lambda v: [float(x) for x in v], lambda v: list(v) + [None]])
+def test_podargs_of_any_container_decode_alike_and_are_kept_once(make, monkeypatch):
+    from zero_tvm_b200 import backend as zb
+    for entry, pod in (("int4_matmul_batched_dyn_affine", [256, 32, 64, 5]), ("int4_matmul_tiled_affine_moe", [64, 8, 72, 0, 144, 512, 1296, 9])):
+        monkeypatch.setattr(zb, "_DECODED", {})
+        want = zb._decode_matmul(entry, pod)
+        for _ in range(5):
+            affine, moe, desc = zb._decode_matmul(entry, make(pod))
+            assert (affine, moe) == want[:2] and list(zb._DECODED) == [(entry, *pod)]
+            got, ref = (desc[0], want[2][0]) if moe else (desc, want[2])
+            assert bytes(got) == bytes(ref) and (not moe or desc[1:] == want[2][1:])
+
+
+def test_decoded_podargs_are_bounded(monkeypatch):
+    from zero_tvm_b200 import backend as zb
+    monkeypatch.setattr(zb, "_DECODED", {})
+    monkeypatch.setattr(zb, "_DECODED_MAX", 8)
+    for n in range(1, 40):
+        assert zb._decode_matmul("int4_matmul_batched_dyn", [256, 32, n, 3])[2].N == n
+    assert len(zb._DECODED) <= 8
 
 
 def test_bench_workload_parsing_and_algorithmic_bytes():

@@ -236,11 +236,31 @@ def pick_chunk_gemm(requested: Optional[str], *, affine: bool, K: int, cap: int 
 
 
 # ---- the dispatch surface ---------------------------------------------------------------------------
-@functools.lru_cache(maxsize=4096)
+_DECODED: dict = {}          # (entry name, *fields) -> what they decode to; plain integers only, at most _DECODED_MAX
+_DECODED_MAX = 4096
+
+
 def _decode_matmul(entry: str, pod: Sequence):
     """(affine, moe, descriptor) of an entry name and its PODArgs; MoE: (mm, strides, K_PACKED), the rest is per call.
     Decoding costs more than the launch (a dispatch took 8 us without the cache), and a call site passes the same name and
-    PODArgs for ever."""
+    PODArgs for ever. PODArgs may hold anything with an integer value: a tensor's elements hash by identity, so what is
+    kept is kept under the integers."""
+    try:
+        return _DECODED[(entry, *pod)]
+    except (KeyError, TypeError):            # not seen yet; fields that do not hash
+        pass
+    known = _decode_fields(entry, pod)
+    try:
+        key = (entry, *(int(v) for v in pod))
+    except (TypeError, ValueError):          # something that no decoder reads, behind the fields
+        return known
+    if len(_DECODED) >= _DECODED_MAX:
+        _DECODED.clear()
+    _DECODED[key] = known
+    return known
+
+
+def _decode_fields(entry: str, pod: Sequence):
     info = parse_entry(entry)
     k_packed, spr, n = int(pod[0]), int(pod[1]), int(pod[2])
     if k_packed <= 0 or spr <= 0 or (k_packed * 32) % info.bits:
@@ -281,11 +301,10 @@ class CudaMatmulBackend:
             parse_entry(entry)
             raise ValueError("bind group needs [out, in, scales, weights, PODArgs, ...]")
         out, x, scales, weights, pod = bindings[:5]
-        try:
-            known = _decode_matmul(entry, tuple(pod))
-        except TypeError:                        # PODArgs that do not hash
-            known = _decode_matmul.__wrapped__(entry, pod)
-        affine, moe, desc = known
+        try:                                     # (as in _decode_matmul, without the call)
+            affine, moe, desc = _DECODED[(entry, *pod)]
+        except (KeyError, TypeError):
+            affine, moe, desc = _decode_matmul(entry, pod)
         biases = bindings[5] if len(bindings) > 5 else None
         if affine and biases is None:
             raise ValueError(f"{entry}: affine variants bind biases at slot 5")
@@ -302,7 +321,7 @@ class CudaMatmulBackend:
         """Whether `dispatch` of these arguments, a complete MoE bind group, builds or reads the expert-sorted plan that
         the context keeps."""
         out, x, scales, weights, pod, biases, ids = bindings[:7]
-        desc = _decode_matmul(entry, tuple(pod))[2]
+        desc = _decode_matmul(entry, pod)[2]
         return self.ctx.int4_matmul_moe_uses_plan(self._moe_desc(desc, weights, grid), out, x, scales, weights, biases, ids)
 
     def _moe_desc(self, desc, weights, grid: Sequence[int]) -> MoeDesc:

@@ -37,7 +37,7 @@ def _independent_pair(be, a, b):
     spans = [_span(t) for t in (ba[0], bb[0], ba[1], bb[1], ba[6], bb[6])]
     if None in spans or spans[2] != spans[3] or spans[4] != spans[5]:
         return False
-    _, moe, desc = _decode_matmul(ea, tuple(ba[4]))
+    _, moe, desc = _decode_matmul(ea, ba[4])
     if not moe or desc is None or ga[1] * ga[2] >= (64 if desc[0].bits == 4 else 32):   # (more pairs fill the chip by themselves)
         return False
     rows, (_in_slot, out_slot, _in_tok, out_tok, _ids) = desc[0].N, desc[1]
