@@ -1,5 +1,6 @@
-"""GPU parity of the prefill GEMM where its tiles and K shares can go wrong: every token tile (64, 128, 256), one to eight
-K shares (also uneven ones, and more shares than token blocks), scale groups of 32, 64 and 128 with rows off their 8- and
+"""GPU parity of the prefill GEMM where its tiles and K shares can go wrong: every token tile (64, 128, 256, 352), one to eight
+K shares (also uneven ones, and more shares than token blocks), scale groups of 32 (without biases and with:
+two tables at the widest pitch, tiles of at most 256 tokens), 64 and 128 with rows off their 8- and
 16-byte alignment (K = 64 x odd), rows past M, N that is no multiple of 8 or 128, f32 output."""
 import numpy as np
 import pytest
@@ -12,7 +13,7 @@ from test_gpu_gemm import FLOOR_FRAC, TOL
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("group,affine", [(64, True), (32, False), (128, True)])
+@pytest.mark.parametrize("group,affine", [(64, True), (32, False), (128, True), (32, True)])
 @pytest.mark.parametrize("M,N,K,f32", [
     (17, 128, 128, False), (24, 40, 4096, False), (33, 3072, 1664, False), (64, 1000, 5120, True),      # 64-token tiles
     (65, 1001, 2176, False), (77, 2176, 3072, False), (128, 392, 8192, True),                           # 128

@@ -618,7 +618,7 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
     ztvm::WorkBuf* buf = nullptr;
     ZTVM_CUDA(ctx->work->get(ztvm::WorkBufs::kPlan, ztvm::moe_grouped_scratch_bytes(md->experts, (uint32_t)pairs), st, &buf));
     uint32_t* ws = static_cast<uint32_t*>(buf->p);
-    const uint32_t tile_rows = pick == 4 ? ztvm::batch_moe_tile_rows(md->experts, pairs) : pick == 2 ? ztvm::kMoeTcTileRows : ztvm::kMoeTaTileRows;
+    const uint32_t tile_rows = pick == 4 ? ztvm::batch_moe_tile_rows((int)d->bits, md->experts, pairs) : pick == 2 ? ztvm::kMoeTcTileRows : ztvm::kMoeTaTileRows;
     // gate, up and down of one step walk the same id list: with ztvm_moe_plan_reuse on, its plan is built once
     const ztvm::PlanKey key = {ids, nullptr, md->tokens, md->slots, md->ids_stride, tile_rows, md->experts};
     const bool reuse = ctx->plan_reuse && pick != 3 && buf->plan == key;
@@ -824,7 +824,7 @@ ztvm_status ztvm_silu_mul_rows(ztvm_ctx* ctx, const ztvm_moe_ep_rows* rows, uint
   if (ffn == 0 || !rows->seg_counts || rows->seg_cap == 0) return fail(ZTVM_ERR_BAD_DIMS, "ffn, seg_counts and seg_cap must be set");
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   ZTVM_CUDA(ztvm::launch_silu_mul(static_cast<const __half*>(gate_up), static_cast<__half*>(h), rows->segments * rows->seg_cap,
-                                  ffn, st, rows->seg_counts, rows->seg_cap));
+                                  ffn, ctx->sm_count, st, rows->seg_counts, rows->seg_cap));
   return ZTVM_OK;
 }
 
@@ -834,7 +834,7 @@ ztvm_status ztvm_silu_mul(ztvm_ctx* ctx, uint32_t rows, uint32_t ffn, void* h, c
   if (!h || !gate_up) return fail(ZTVM_ERR_NULL_POINTER, "h/gate_up must be non-NULL");
   if (ffn == 0) return fail(ZTVM_ERR_BAD_DIMS, "ffn=0");
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  ZTVM_CUDA(ztvm::launch_silu_mul(static_cast<const __half*>(gate_up), static_cast<__half*>(h), rows, ffn, st));
+  ZTVM_CUDA(ztvm::launch_silu_mul(static_cast<const __half*>(gate_up), static_cast<__half*>(h), rows, ffn, ctx->sm_count, st));
   return ZTVM_OK;
 }
 
@@ -846,7 +846,7 @@ ztvm_status ztvm_moe_combine(ztvm_ctx* ctx, uint32_t tokens, uint32_t slots, uin
   if (slots == 0 || d == 0) return fail(ZTVM_ERR_BAD_DIMS, "slots and d must be non-zero");
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   ZTVM_CUDA(ztvm::launch_moe_combine(static_cast<const __half*>(y_slots), scores, static_cast<__half*>(out), tokens,
-                                     slots, d, st));
+                                     slots, d, ctx->sm_count, st));
   return ZTVM_OK;
 }
 

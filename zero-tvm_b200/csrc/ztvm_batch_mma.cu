@@ -397,15 +397,15 @@ cudaError_t launch_batch_mma(const GemvParams& g, int bits, int sm_count, cudaSt
 }
 
 // Grouped by expert. Tile width by the average number of pairs an expert has: a tile's weights are streamed once for
-// its whole token tile, its MMAs run over the token blocks that exist.
+// its whole token tile, its MMAs run over the token blocks that exist. (4-bit codes come here with few pairs only.)
 bool batch_moe_supported(const GemvParams& g, int bits) {
   return (bits == 3 || bits == 4) && batch_common_ok(g) && (g.in_slot_stride | g.in_tok_stride) % 8u == 0 && g.experts <= 1024 && !g.dst_index;
 }
-uint32_t batch_moe_tile_rows(uint32_t experts, uint64_t pairs) {
-  return pairs <= 10ull * experts ? 16u : pairs <= 24ull * experts ? 32u : 64u;
+uint32_t batch_moe_tile_rows(int bits, uint32_t experts, uint64_t pairs) {
+  return bits == 4 || pairs <= 10ull * experts ? 16u : pairs <= 24ull * experts ? 32u : 64u;
 }
 cudaError_t launch_batch_moe(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan) {
-  const uint32_t P = tokens * slots, tok = batch_moe_tile_rows(g.experts, P);
+  const uint32_t P = tokens * slots, tok = batch_moe_tile_rows(bits, g.experts, P);
   BatchParams p = batch_params(g);
   p.slots = slots;
   p.in_slot_stride = g.in_slot_stride; p.out_slot_stride = g.out_slot_stride;
@@ -415,11 +415,7 @@ cudaError_t launch_batch_moe(const GemvParams& g, int bits, uint32_t tokens, uin
   if (e != cudaSuccess) return e;
   const uint64_t by_rows = (uint64_t)(P + tok - 1) / tok + g.experts;
   const uint32_t max_tiles = (uint32_t)(by_rows < P ? by_rows : P);   // the kernel reads the real count
-  if (bits == 4) {
-    if (tok == 16) return launch_cfg<4, 4, 1, 2, 2, 4, true>(p, max_tiles, st);
-    if (tok == 32) return launch_cfg<4, 4, 1, 2, 4, 4, true>(p, max_tiles, st);
-    return launch_cfg<4, 4, 2, 1, 4, 2, true>(p, max_tiles, st);
-  }
+  if (bits == 4) return launch_cfg<4, 4, 1, 2, 2, 4, true>(p, max_tiles, st);
   if (p.KP % 4u) {
     if (tok == 16) return launch_cfg<3, 4, 1, 2, 2, 4, true, false>(p, max_tiles, st);
     if (tok == 32) return launch_cfg<3, 4, 1, 2, 4, 4, true, false>(p, max_tiles, st);

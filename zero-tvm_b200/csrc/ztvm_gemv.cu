@@ -247,10 +247,11 @@ gemv_fma_m1_kernel(const GemvParams p) {
     X += (size_t)token * p.in_tok_stride + (size_t)slot * p.in_slot_stride;
     out_base = (size_t)token * p.out_tok_stride + (size_t)slot * p.out_slot_stride;
   }
-  // A K of 16 units or fewer (512 codes) would leave half of the lanes without work: each half of the warp takes a row of its own
+  // An expert's K of 16 units or fewer (512 codes) would leave half of the lanes without work: each half of the warp takes a row of
+  // its own. (Dense rows come here with a K beyond the persistent kernel's only.)
   // (2048 x 512, nine pairs: 5.6 -> 4.1 us)
   const uint32_t units = p.K >> 5;
-  const uint32_t sub = units <= 16u ? 2u : 1u, span = 32u / sub;
+  const uint32_t sub = MOE && units <= 16u ? 2u : 1u, span = 32u / sub;
   const uint32_t lane_u = (uint32_t)lane & (span - 1u), lane_r = (uint32_t)lane / span;
   const uint32_t row0 = (blockIdx.x * kGemvWarps + warp) * ROWS * sub + lane_r;
   const uint32_t units_up = (units + 31) & ~31u;
@@ -645,12 +646,10 @@ cudaError_t launch_gemv(GemvParams p, int bits, bool moe, uint32_t tokens, uint3
   const size_t smem = (size_t)mt * tile_units * (128 + 4);
   dim3 grid((p.N + kGemvWarps * rows - 1) / (kGemvWarps * rows), moe ? tokens : 1, moe ? slots : 1);
   if (bits == 4 && mt == 1 && !moe && p.K <= 20480) {  // dense 4-bit decode row: persistent FMA kernel
-    const uint32_t rows_per_warp = p.N / ((uint32_t)sm_count * 2 * kPersistWarps);
-    (void)rows_per_warp;
     return launch_fma_m1_persist<4, 4>(p, sm_count, st);
   }
   if (bits == 4 && mt == 1 && p.K <= 40960) {  // 4-bit decode row: the conversion-free FMA kernel
-    const uint32_t per_cta = (uint32_t)(kGemvWarps * rows) * (units <= 16 ? 2u : 1u);
+    const uint32_t per_cta = (uint32_t)(kGemvWarps * rows) * (moe && units <= 16 ? 2u : 1u);
     grid.x = (p.N + per_cta - 1) / per_cta;
     if (moe) return rows == 4 ? launch_fma_m1<4, true>(p, grid, st) : rows == 2 ? launch_fma_m1<2, true>(p, grid, st) : launch_fma_m1<1, true>(p, grid, st);
     return rows == 4 ? launch_fma_m1<4, false>(p, grid, st) : rows == 2 ? launch_fma_m1<2, false>(p, grid, st) : launch_fma_m1<1, false>(p, grid, st);

@@ -148,7 +148,8 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
   }
 }
 
-constexpr size_t kFillThreads = 148 * 256;   // threads from which on a row-wise kernel gives each of them eight elements
+// threads from which on a row-wise kernel gives each of them eight elements: a block on every SM
+static inline size_t fill_threads(int sm_count) { return (size_t)sm_count * 256; }
 static inline unsigned grid_for(size_t total, int block) {
   size_t g = (total + block - 1) / block;
   return (unsigned)(g > 148 * 32 ? 148 * 32 : (g ? g : 1));
@@ -398,12 +399,12 @@ __global__ void silu_mul_kernel(const __half* gate_up, __half* h, uint32_t rows,
     }
   }
 }
-cudaError_t launch_silu_mul(const __half* gate_up, __half* h, uint32_t rows, uint32_t ffn, cudaStream_t st,
+cudaError_t launch_silu_mul(const __half* gate_up, __half* h, uint32_t rows, uint32_t ffn, int sm_count, cudaStream_t st,
                             const uint32_t* seg_counts, uint32_t seg_cap) {
   const size_t total = (size_t)rows * ffn;
   if (total == 0) return cudaSuccess;
   const uintptr_t lows = reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(h);
-  const int vec = ffn % 8 == 0 && (lows & 15u) == 0 && total / 8 >= kFillThreads ? 8 : ffn % 2 == 0 && (lows & 3u) == 0 ? 2 : 1;
+  const int vec = ffn % 8 == 0 && (lows & 15u) == 0 && total / 8 >= fill_threads(sm_count) ? 8 : ffn % 2 == 0 && (lows & 3u) == 0 ? 2 : 1;
   return launch_chained(vec == 8 ? silu_mul_kernel<8> : vec == 2 ? silu_mul_kernel<2> : silu_mul_kernel<1>, dim3(grid_for(total / vec, 256)),
                         dim3(256), 0, st, gate_up, h, rows, ffn, seg_counts, seg_cap ? seg_cap : 1u);
 }
@@ -496,11 +497,11 @@ __global__ void moe_combine_kernel(const __half* y, const float* scores, __half*
   }
 }
 cudaError_t launch_moe_combine(const __half* y_slots, const float* scores, __half* out, uint32_t tokens,
-                               uint32_t slots, uint32_t d, cudaStream_t st) {
+                               uint32_t slots, uint32_t d, int sm_count, cudaStream_t st) {
   const size_t total = (size_t)tokens * d;
   if (total == 0) return cudaSuccess;
   const uintptr_t lows = reinterpret_cast<uintptr_t>(y_slots) | reinterpret_cast<uintptr_t>(out);
-  const int vec = d % 8 == 0 && (lows & 15u) == 0 && total / 8 >= kFillThreads ? 8 : d % 2 == 0 && (lows & 3u) == 0 ? 2 : 1;
+  const int vec = d % 8 == 0 && (lows & 15u) == 0 && total / 8 >= fill_threads(sm_count) ? 8 : d % 2 == 0 && (lows & 3u) == 0 ? 2 : 1;
   return launch_chained(vec == 8 ? moe_combine_kernel<8> : vec == 2 ? moe_combine_kernel<2> : moe_combine_kernel<1>, dim3(grid_for(total / vec, 256)),
                         dim3(256), 0, st, y_slots, scores, out, tokens, slots, d);
 }

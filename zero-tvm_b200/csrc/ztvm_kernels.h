@@ -87,7 +87,7 @@ bool batch_mma_supported(const GemvParams& p, int bits);
 cudaError_t launch_batch_mma(const GemvParams& p, int bits, int sm_count, cudaStream_t st);
 // The grouped form for 3-bit (and 4-bit) experts: pairs sorted by expert, tiles of batch_moe_tile_rows pairs.
 bool batch_moe_supported(const GemvParams& g, int bits);
-uint32_t batch_moe_tile_rows(uint32_t experts, uint64_t pairs);
+uint32_t batch_moe_tile_rows(int bits, uint32_t experts, uint64_t pairs);
 cudaError_t launch_batch_moe(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan);
 
 // 4-bit weights, M > 16: tcgen05 GEMM with the dequantised weights as the A operand in tensor memory and the activations
@@ -165,10 +165,10 @@ cudaError_t launch_f16_matvec(const __half* x, const __half* w, float* y, uint32
 cudaError_t launch_route_topk(const float* logits, uint32_t* ids, float* scores, uint32_t tokens, uint32_t E,
                               uint32_t K, bool norm_topk, bool has_shared, cudaStream_t st);
 // seg_counts != nullptr: rows come in regions of seg_cap, only the first seg_counts[region] of each are computed
-cudaError_t launch_silu_mul(const __half* gate_up, __half* h, uint32_t rows, uint32_t ffn, cudaStream_t st,
+cudaError_t launch_silu_mul(const __half* gate_up, __half* h, uint32_t rows, uint32_t ffn, int sm_count, cudaStream_t st,
                             const uint32_t* seg_counts = nullptr, uint32_t seg_cap = 1);
 cudaError_t launch_silu_mul_f32(const float* gate_up, __half* h, uint32_t rows, uint32_t ffn, cudaStream_t st);
 cudaError_t launch_moe_combine(const __half* y_slots, const float* scores, __half* out, uint32_t tokens,
-                               uint32_t slots, uint32_t d, cudaStream_t st);
+                               uint32_t slots, uint32_t d, int sm_count, cudaStream_t st);
 
 }  // namespace ztvm
