@@ -74,3 +74,35 @@ def test_decode_step_graph_matches_eager(backend, dev):
     for k in want2:
         assert np.array_equal(got2[k], want2[k]), k
     assert backend.ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("bits,symmetric", [(4, False), (4, True), (3, False), (8, False)])
+@pytest.mark.parametrize("hidden,ffn", [(1088, 2240), (2112, 4928)])
+def test_ragged_one_row_step_replays_bit_for_bit(bits, symmetric, hidden, ffn, backend, dev):
+    """Widths that are no multiple of 256: the one-row kernels of those, started early behind one another."""
+    import torch
+    rng = np.random.default_rng(hidden + bits)
+    group, rec, outs = 32 if symmetric else 64, z.recorder.DecodeRecorder(backend), []
+    for layer in range(2):
+        x, gu, h, y = (dev.empty((1, n), np.float16, fill=0.0) for n in (hidden, 2 * ffn, ffn, hidden))
+        x.copy_(dev.put(z.synth.make_x(rng, 1, hidden)))
+        for out, inp, n, k in ((gu, x, 2 * ffn, hidden), (y, h, hidden, ffn)):
+            _, W, s, b = z.synth.make_weights(rng, n, k, bits=bits, group=group, sigma_s=0.01 * 15 / (2**bits - 1))
+            entry = "int8_affine_matvec" if bits == 8 else resolve_matmul(affine=not symmetric, K=k, q3=bits == 3)
+            rec.dispatch(entry, [out, inp, dev.put(s), dev.put(W), pod_args(k, n, bits=bits, group=group)] + ([] if symmetric else [dev.put(b)]))
+            if out is gu:
+                rec.silu_mul(h, gu, 1, ffn)
+        outs += [gu, h, y]
+    torch.cuda.synchronize()
+    rec.run_eager()
+    torch.cuda.synchronize()
+    want = [t.clone() for t in outs]
+    step = rec.capture()
+    for _ in range(5):
+        for t in outs:
+            t.fill_(float("nan"))
+        torch.cuda.synchronize()
+        step.replay()
+        step.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(t, w) and torch.isfinite(t.float()).all() for t, w in zip(outs, want))
