@@ -95,8 +95,9 @@ typedef struct ztvm_mm_desc {
  * int4_matmul_batched_dyn[_affine] and the tiled / subgroup-matrix prefill GEMMs
  * (src/compiler/shaders/int4_matmul.gen.ts:170-571, :580-695, :805-1456; call sites
  * src/zero-tvm/engine-core.ts:2290, :2312, :2517-2519, :2543-2549, :4280-4293).
- * M <= 8 runs the bandwidth-bound GEMV, M <= 16 two slabs of it; larger M runs the tensor-core GEMM (which multiplies
- * f16-rounded weights f16(s*q+b), like the reference's matrix-unit GEMMs). */
+ * M <= 8 runs the bandwidth-bound GEMV, M <= 16 two slabs of it; larger M of 4-bit weights runs the tensor-core GEMM (which
+ * multiplies f16-rounded weights f16(s*q+b), like the reference's matrix-unit GEMMs). 8-bit weights keep exact codes at
+ * every M: from nine rows on a batched kernel (groups of 64), else slabs; 3-bit ones run as slabs. */
 ZTVM_API ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* desc, void* y, const void* x,
                              const void* scales, const void* packed_w, const void* biases, void* stream);
 
@@ -321,8 +322,8 @@ ZTVM_API ztvm_status ztvm_int4_matmul_nshard(ztvm_ctx* ctx, const ztvm_mm_desc* 
  * weight, scales and biases hold 2 * ffn rows, gate rows first. Replaces fused_ffn (src/compiler/shaders/fused_ffn.wgsl:
  * bindings [output, input, scales, weights, PODArgs]; symmetric group 32 there) and is the affine sibling the engine
  * lacks (src/zero-tvm/engine-core.ts:2513-2519 pays gate_up matmul + silu_mul on affine models).
- * 4-bit, group 64, K % 256 == 0, M <= 8: ONE launch of the persistent GEMV, whose CTAs own gate and up tiles of the
- * same output rows. Other shapes (group 32 / 128, 3-bit, 8-bit, M > 8): the 2 * ffn-row matmul into an f32 buffer of
+ * 4-bit groups of 64, symmetric groups of 32 and 8-bit, K % 64 == 0, M <= 8: ONE launch of the persistent GEMV, whose CTAs
+ * own gate and up tiles of the same output rows. Other shapes (affine groups of 32, groups of 128, 3-bit, M > 8): the 2 * ffn-row matmul into an f32 buffer of
  * the context (a work buffer: see the conventions), then the activation -- same arithmetic, two launches. desc->out_f32 must be 0. */
 ZTVM_API ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* desc, void* h, const void* x, const void* scales,
                            const void* packed_w, const void* biases, void* stream);

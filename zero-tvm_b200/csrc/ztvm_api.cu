@@ -12,7 +12,7 @@
 
 struct ztvm_ctx {
   uint32_t magic;
-  int no_gemm;    // env ZTVM_NO_GEMM=1: keep M > 8 on GEMV slabs (a measurement knob)
+  int no_gemm;    // env ZTVM_NO_GEMM=1: M > 8 on the exact-code kernels (batched, else GEMV slabs), a measurement knob
   // 0 auto: the persistent matrix-unit GEMV where its shape rules allow, else M = 1 on the CUDA-core FMA GEMV and
   // M = 2..8 on the tiled matrix-unit GEMV; 1: FMA always; 2: tiled matrix unit always; 3: like 0 but M = 1 stays on
   // the FMA GEMV (env ZTVM_GEMV_PATH=fma|mma|tc|tc_m2, a measurement knob)
@@ -249,10 +249,10 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
   if ((s = check_desc(d, true))) return s;
   if ((s = check_buffers(d, y, x, scales, packed_w, biases))) return s;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  // Up to 16 rows the GEMV in slabs of eight wins: it re-streams the weights once per slab at HBM speed, while the
-  // tensor-core kernels dequantise every code once at ~12 codes per clock and SM whatever M is (measured on
-  // 8192 x 2048: 9.4 us against 21 us at M = 16, 14 against 13 us at M = 24). It is also the reference's choice for
-  // short chunks (runtime-M matvec, exact codes and f32 weights; its GEMMs start at 64 rows).
+  // Up to 16 rows the GEMV in slabs of eight: exact codes and f32 weights, the reference's choice for short chunks (runtime-M
+  // matvec; its GEMMs start at 64 rows). From 17 on a third slab costs more than the GEMM at every width. Weight sets from HBM,
+  // GEMM against slabs, us: 8192 x 2048 9.8 : 11.1 at 16 rows, 10.1 : 15.8 at 17; 24576 x 4096 40.7 : 34.2 and 40.8 : 48.0;
+  // 4096 x 12288 18.6 : 24.2 and 19.0 : 35.6. (The GEMM is ahead at 9..16 rows too where K is long, but rounds the weights to f16.)
   if (d->M > 16 && ztvm::gemm_w4_supported((int)d->bits, d->group, d->K) && !ctx->no_gemm) {
     if (!aligned(y, 16)) return fail(ZTVM_ERR_ALIGNMENT, "y must be 16-byte aligned for the GEMM path");
     ZTVM_CUDA(ztvm::launch_gemm_w4_ta(static_cast<const uint32_t*>(packed_w), static_cast<const __half*>(scales),
@@ -385,7 +385,7 @@ ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* h, const 
   return ZTVM_OK;
 }
 
-// One router logit per (token, row): the exact-code GEMV in slabs of eight tokens for quantised routers (never the f16
+// One router logit per (token, row): the exact-code kernels for quantised routers, GEMV or batched (never the f16
 // tensor-core GEMM: logits feed a softmax and a top-k, so they keep the f32-accumulated exact-code arithmetic of the
 // reference's matvec whatever the token count), a plain f16 matvec for routers stored in f16.
 ztvm_status ztvm_moe_router_logits(ztvm_ctx* ctx, uint32_t D, uint32_t rows, uint32_t tokens, uint32_t bits, float* logits,
@@ -517,7 +517,7 @@ ztvm_status ztvm_host_wait(ztvm_ctx* ctx) {
 
 // Which grouped kernel serves a MoE launch: 0 none (per-pair GEMV), 1 tensor-core tiles with the weights in tensor
 // memory, 2 streaming kernel, 3 tensor-core tiles with both operands in shared memory (ZTVM_MOE_TILES=sm, or shapes
-// only it takes), 4 the exact-code batched kernel (3-bit experts). `forced` is the context's ZTVM_MOE_GROUPED knob (-1 = by size).
+// only it takes), 4 the exact-code batched kernel (3-bit experts; 4-bit ones of few pairs over a K that 2 does not take). `forced` is the context's ZTVM_MOE_GROUPED knob (-1 = by size).
 static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::GemvParams& p, const void* y) {
   const int forced = ctx->moe_grouped;
   const ztvm_mm_desc* d = &md->mm;
@@ -527,15 +527,16 @@ static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::Ge
                      ztvm::moe_grouped_supported((int)d->bits, d->group, d->K, d->N, md->experts);
   const int tiles = ctx->moe_tiles_sm ? (sm_ok ? 3 : ta_ok ? 1 : 0) : (ta_ok ? 1 : sm_ok ? 3 : 0);
   const bool stream_ok = ztvm::moe_tc_supported(p, (int)d->bits) && !p.dst_index;
-  // Where the two grouped kernels cross (measured on the 257-expert block, hidden 2048, ffn 512): the tiles cost the same
-  // whatever the pair count (every expert's weights are dequantised once: ~100 us per projection), the streaming kernel
-  // grows with the 8-pair chunks it walks (gate: 35 us + 0.020 us per pair; down, with its short K: 48 us + 0.028 us per
-  // pair). They meet near 12.6 pairs per expert for the long-K projections and 6.6 for the short-K one; one threshold
-  // for both keeps the three projections of a block on one kernel, whose plan they can then share.
+  // The tiles cost the same whatever the pair count (every expert's weights are dequantised once), the streaming kernel grows
+  // with the 8-pair chunks it walks. 257 experts, plan kept, us: gate / up, 512 x 2048: tiles 69, streaming 49 / 54 / 68 / 80 / 91
+  // at 4 / 6 / 8 / 10 / 12 pairs per expert; down, 2048 x 512: tiles 68, streaming 58 / 69 / 80 / 98 / 115 at 2 / 4 / 6 / 8 / 10.
+  // (64 experts: 21 against 18 / 19 / 21 / 25 at 4 / 6 / 8 / 10, 22 against 22 / 24 / 28 / 35.) So they meet at eight and four
+  // pairs per expert. The line is at ten for all three projections of a block: below it they keep exact codes and f32 weights,
+  // which the tiles round to f16, and one kernel, whose plan they share.
   const bool few_per_expert = pairs < 10ull * md->experts;
   if (d->bits == 3) return ztvm::batch_moe_supported(p, 3) ? 4 : 0;    // exact codes at every pair count
-  // A K that the streaming kernel does not take: the batched kernel holds its place below the same crossing (2240 x 512
-  // experts, 576 pairs: 45 against 96 us per projection).
+  // A K that the streaming kernel does not take: the batched kernel, exact codes as well, holds its place (257 experts of 512 x
+  // 2240, us: 55 / 63 / 67 at 4 / 8 / 10 pairs per expert against 80 on the tiles).
   if (forced < 0 && !stream_ok && few_per_expert && !p.dst_index && !p.seg_counts && ztvm::batch_moe_supported(p, 4)) return 4;
   if (forced == 1) return tiles ? tiles : stream_ok ? 2 : 0;
   if (forced == 2) return stream_ok ? 2 : tiles;

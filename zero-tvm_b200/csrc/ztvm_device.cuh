@@ -10,9 +10,17 @@
 namespace ztvm {
 
 // ---- programmatic dependent launch -------------------------------------------------------------
-// Every kernel of a step is launched with programmatic stream serialisation (launch_chained): it lets the next one start as
-// soon as all its own blocks run, and waits for the one before -- its end, and its writes -- ahead of its first read or
-// write of anything but weights. A chain of short kernels then pays no launch latency between them.
+// Most kernels of a step are launched with programmatic stream serialisation: such a launch starts as soon as every CTA of the
+// launch before has let it in (or is gone), and each of its CTAs waits -- for the end of the launch before and its writes --
+// ahead of its first read or write of anything but weights. All CTAs wait, so the end of a launch means the end of all before it.
+//   * The row-wise kernels, the plan, the per-pair MoE forms and the streaming MoE kernel let the next launch in at once; the
+//     persistent GEMVs when their activations are in place; the tiled kernels (prefill GEMM, batched, MoE tiles) when their
+//     first copies are under way.
+//   * Grids of one CTA per SM keep their CTAs apart (kOnePerSmSmem, ztvm_kernels.h): let in early, they are dealt to whatever
+//     slots come free first.
+//   * In plain stream order, neither early nor letting in: the dense gemv_kernel, gemv_fma_m1_kernel and gemv_mma_kernel, whose
+//     many CTAs of a fixed share each filled the SMs unevenly when let in early (3-bit 3003 x 4416: 9.7 us, 12.7 us), the f16
+//     router matvec, the earlier MoE tiles, the plan of long lists, the expert-parallel dispatch and barrier, and the parity hooks.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
