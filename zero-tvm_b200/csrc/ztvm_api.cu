@@ -33,6 +33,8 @@ struct ztvm_ctx {
   // grouped kernel; unset = by size (few pairs per-pair; then the exact-code kernels while an expert sees few of them)
   int moe_grouped;
   int plan_reuse;   // ztvm_moe_plan_reuse: consecutive ztvm_int4_matmul_moe calls over one id list share its plan
+  // The last call's last launch, for HalfSm: its weight bytes if it was a half-SM one, and its stream. `call`: the call being made.
+  struct { uint64_t half; cudaStream_t st; } call, last;
   int moe_tiles_sm; // env ZTVM_MOE_TILES=sm: the grouped MoE tiles with both operands in shared memory (a measurement knob)
 };
 
@@ -63,7 +65,20 @@ ztvm_status check_ctx(ztvm_ctx* ctx) {
   int dev = -1;
   ZTVM_CUDA(cudaGetDevice(&dev));
   if (dev != ctx->device) ZTVM_CUDA(cudaSetDevice(ctx->device));
+  ctx->last = ctx->call;         // every entry point comes through here
+  ctx->call.half = 0;
   return ZTVM_OK;
+}
+
+// What a GEMV launch on `st` finds before it, and what it leaves for the next call.
+ztvm::HalfSm half_before(const ztvm_ctx* ctx, cudaStream_t st) {
+  ztvm::HalfSm h;
+  h.before = ctx->last.st == st ? ctx->last.half : 0;
+  return h;
+}
+void half_after(ztvm_ctx* ctx, const ztvm::HalfSm& h, cudaStream_t st) {
+  ctx->call.half = h.now;
+  ctx->call.st = st;
 }
 
 // True when `p` is page-locked host memory known to the runtime (cudaHostAlloc / cudaHostRegister).
@@ -271,6 +286,7 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
     }
   }
   // Otherwise rows are processed in slabs of at most 8 by the GEMV.
+  ztvm::HalfSm half = half_before(ctx, st);
   for (uint32_t m0 = 0; m0 < d->M; m0 += 8) {
     ztvm_mm_desc dd = *d;
     dd.M = d->M - m0 < 8 ? d->M - m0 : 8;
@@ -279,11 +295,14 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
     p.Y = d->out_f32 ? static_cast<void*>(static_cast<float*>(y) + (size_t)m0 * d->N)
                      : static_cast<void*>(static_cast<__half*>(y) + (size_t)m0 * d->N);
     const bool want_tc = ctx->gemv_path == 0 || (ctx->gemv_path == 3 && dd.M > 1);
-    if (want_tc && ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st));
+    if (want_tc && ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st, &half));
     else if (want_tc && ztvm::gemv_tc3_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc3(p, ctx->sm_count, st));
     else if (use_mma(ctx, d, dd.M)) ZTVM_CUDA(ztvm::launch_gemv_mma(p, false, 1, 1, st));
-    else ZTVM_CUDA(ztvm::launch_gemv(p, (int)d->bits, false, 1, 1, ctx->sm_count, st));
+    else ZTVM_CUDA(ztvm::launch_gemv(p, (int)d->bits, false, 1, 1, ctx->sm_count, st, &half));
+    half = {half.now, 0};
   }
+  half.now = half.before;
+  half_after(ctx, half, st);
   return ZTVM_OK;
 }
 
@@ -372,7 +391,9 @@ ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* h, const 
     p.pair_rows = d->N;
     p.y_row_stride = d->N;
     if (ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) {
-      ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st));
+      ztvm::HalfSm half = half_before(ctx, st);
+      ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st, &half));
+      half_after(ctx, half, st);
       return ZTVM_OK;
     }
   }
@@ -451,7 +472,9 @@ ztvm_status ztvm_int4_matmul_multi(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* c
     return fail(ZTVM_ERR_UNSUPPORTED,
                 "the multi-destination form runs the persistent GEMV only: bits=4, group=64, K %% 256 == 0, 16-byte aligned "
                 "x and weights (got bits=%u group=%u K=%u)", d->bits, d->group, d->K);
-  ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st));
+  ztvm::HalfSm half = half_before(ctx, st);
+  ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st, &half));
+  half_after(ctx, half, st);
   return ZTVM_OK;
 }
 
@@ -639,7 +662,7 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
     q.Y = static_cast<__half*>(y) + (size_t)t0 * md->out_tok_stride;
     q.ids = ids + (size_t)t0 * md->ids_stride;
     if (use_mma(ctx, d, 1)) ZTVM_CUDA(ztvm::launch_gemv_mma(q, true, nt, md->slots, st));
-    else ZTVM_CUDA(ztvm::launch_gemv(q, (int)d->bits, true, nt, md->slots, ctx->sm_count, st));
+    else ZTVM_CUDA(ztvm::launch_gemv(q, (int)d->bits, true, nt, md->slots, ctx->sm_count, st, nullptr));
   }
   return ZTVM_OK;
 }

@@ -16,8 +16,8 @@ namespace ztvm {
 //   * The row-wise kernels, the plan, the per-pair MoE forms and the streaming MoE kernel let the next launch in at once; the
 //     persistent GEMVs when their activations are in place; the tiled kernels (prefill GEMM, batched, MoE tiles) when their
 //     first copies are under way.
-//   * Grids of one CTA per SM keep their CTAs apart (kOnePerSmSmem, ztvm_kernels.h): let in early, they are dealt to whatever
-//     slots come free first.
+//   * Grids of one CTA per SM with room for two keep their CTAs apart where it matters (HalfSm, ztvm_kernels.h): let in early,
+//     they are dealt to whatever slots come free first.
 //   * In plain stream order, neither early nor letting in: the dense gemv_kernel, gemv_fma_m1_kernel and gemv_mma_kernel, whose
 //     many CTAs of a fixed share each filled the SMs unevenly when let in early (3-bit 3003 x 4416: 9.7 us, 12.7 us), the f16
 //     router matvec, the earlier MoE tiles, the plan of long lists, the expert-parallel dispatch and barrier, and the parity hooks.

@@ -584,7 +584,7 @@ static cudaError_t launch_fma_m1(const GemvParams& p, dim3 grid, cudaStream_t st
 }
 
 template <int ROWS, int DEPTH>
-static cudaError_t launch_fma_m1_persist(const GemvParams& p, int sm_count, cudaStream_t st) {
+static cudaError_t launch_fma_m1_persist(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half) {
   auto kern = gemv_fma_m1_persist_kernel<ROWS, DEPTH>;
   static bool attr_set[16] = {};
   int dev = 0;
@@ -612,7 +612,9 @@ static cudaError_t launch_fma_m1_persist(const GemvParams& p, int sm_count, cuda
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kPersistWarps * 32);
-  cfg.dynamicSmemBytes = grid <= (uint32_t)sm_count && smem < kOnePerSmSmem ? kOnePerSmSmem : smem;
+  const bool apart = grid <= (uint32_t)sm_count && !half_sm_behind(*half, p);
+  half->now = grid == (uint32_t)sm_count ? half_sm_bytes(p) : 0;
+  cfg.dynamicSmemBytes = apart && smem < kOnePerSmSmem ? kOnePerSmSmem : smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -630,7 +632,7 @@ static cudaError_t launch_rows(const GemvParams& p, int rows, dim3 grid, size_t 
 }
 
 cudaError_t launch_gemv(GemvParams p, int bits, bool moe, uint32_t tokens, uint32_t slots, int sm_count,
-                        cudaStream_t st) {
+                        cudaStream_t st, HalfSm* half) {
   const int mt = p.M <= 1 ? 1 : p.M <= 2 ? 2 : p.M <= 4 ? 4 : 8;
   // rows per warp: 4 when that still leaves every SM several CTAs, else fewer
   const uint64_t pairs = moe ? (uint64_t)tokens * slots : 1;
@@ -646,7 +648,7 @@ cudaError_t launch_gemv(GemvParams p, int bits, bool moe, uint32_t tokens, uint3
   const size_t smem = (size_t)mt * tile_units * (128 + 4);
   dim3 grid((p.N + kGemvWarps * rows - 1) / (kGemvWarps * rows), moe ? tokens : 1, moe ? slots : 1);
   if (bits == 4 && mt == 1 && !moe && p.K <= 20480) {  // dense 4-bit decode row: persistent FMA kernel
-    return launch_fma_m1_persist<4, 4>(p, sm_count, st);
+    return launch_fma_m1_persist<4, 4>(p, sm_count, st, half);
   }
   if (bits == 4 && mt == 1 && p.K <= 40960) {  // 4-bit decode row: the conversion-free FMA kernel
     const uint32_t per_cta = (uint32_t)(kGemvWarps * rows) * (moe && units <= 16 ? 2u : 1u);

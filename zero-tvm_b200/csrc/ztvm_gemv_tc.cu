@@ -4,13 +4,13 @@
 namespace ztvm {
 
 bool gemv_tc_fits_w4(const GemvParams& p, int sm_count);
-cudaError_t launch_gemv_tc_w4(const GemvParams& p, int sm_count, cudaStream_t st);
+cudaError_t launch_gemv_tc_w4(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half);
 bool gemv_tc_fits_w4sym(const GemvParams& p, int sm_count);
-cudaError_t launch_gemv_tc_w4sym(const GemvParams& p, int sm_count, cudaStream_t st);
+cudaError_t launch_gemv_tc_w4sym(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half);
 bool gemv_tc_fits_w4g32(const GemvParams& p, int sm_count);
-cudaError_t launch_gemv_tc_w4g32(const GemvParams& p, int sm_count, cudaStream_t st);
+cudaError_t launch_gemv_tc_w4g32(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half);
 bool gemv_tc_fits_w8(const GemvParams& p, int sm_count);
-cudaError_t launch_gemv_tc_w8(const GemvParams& p, int sm_count, cudaStream_t st);
+cudaError_t launch_gemv_tc_w8(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half);
 
 bool gemv_tc_supported(const GemvParams& p, int bits, int sm_count) {
   if (bits == 3 || p.M < 1 || p.M > 8 || p.K % 64u || p.K == 0 || p.N == 0) return false;
@@ -27,9 +27,9 @@ bool gemv_tc_supported(const GemvParams& p, int bits, int sm_count) {
   return p.group_shift == 5 ? gemv_tc_fits_w4g32(p, sm_count) : p.B ? gemv_tc_fits_w4(p, sm_count) : gemv_tc_fits_w4sym(p, sm_count);
 }
 
-cudaError_t launch_gemv_tc(const GemvParams& p, int bits, int sm_count, cudaStream_t st) {
-  if (bits == 8) return launch_gemv_tc_w8(p, sm_count, st);
-  return p.group_shift == 5 ? launch_gemv_tc_w4g32(p, sm_count, st) : p.B ? launch_gemv_tc_w4(p, sm_count, st) : launch_gemv_tc_w4sym(p, sm_count, st);
+cudaError_t launch_gemv_tc(const GemvParams& p, int bits, int sm_count, cudaStream_t st, HalfSm* half) {
+  if (bits == 8) return launch_gemv_tc_w8(p, sm_count, st, half);
+  return p.group_shift == 5 ? launch_gemv_tc_w4g32(p, sm_count, st, half) : p.B ? launch_gemv_tc_w4(p, sm_count, st, half) : launch_gemv_tc_w4sym(p, sm_count, st, half);
 }
 
 }  // namespace ztvm

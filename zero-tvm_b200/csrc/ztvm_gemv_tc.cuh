@@ -448,7 +448,7 @@ inline bool tc_fits(const GemvParams& p, int sm_count) {
 }
 
 template <int BITS, bool G32, int NT, bool AFFINE, bool AL, int W>
-cudaError_t launch_tc_one(const GemvParams& p, unsigned grid, size_t smem, cudaStream_t st) {
+cudaError_t launch_tc_one(const GemvParams& p, unsigned grid, size_t smem, int sm_count, cudaStream_t st, HalfSm* half) {
   auto kern = gemv_tc_kernel<BITS, G32, NT, AFFINE, AL, W>;
   static bool attr_set[16] = {};
   int dev = 0;
@@ -462,10 +462,12 @@ cudaError_t launch_tc_one(const GemvParams& p, unsigned grid, size_t smem, cudaS
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(W * 32);
   static_assert(tc_smem_limit(8) <= kOnePerSmSmem, "the padding holds what eight warps use");
-  // One share per SM (4-bit row, hidden 1536, ffn 3072, a step of four layers: 90 us without, 80 us with). Shares of a few rows, a
-  // router's, may as well sit side by side (router of 94 rows in a recorded MoE token: 35.8 us a step kept apart, 35.3 us).
+  // Shares of a few rows, a router's, may as well sit side by side (94 rows in a recorded MoE token: 35.8 us a step kept apart,
+  // 35.3 us)
   const uint32_t out_rows = p.pair_rows ? p.pair_rows : p.N;
-  cfg.dynamicSmemBytes = W == 8 && out_rows > 4u * grid ? kOnePerSmSmem : smem;
+  const bool behind = half_sm_behind(*half, p), apart = W == 8 && !behind && out_rows > 4u * grid;
+  half->now = W == 8 && grid == (unsigned)sm_count && (behind || apart) ? half_sm_bytes(p) : 0;
+  cfg.dynamicSmemBytes = apart ? kOnePerSmSmem : smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -476,22 +478,22 @@ cudaError_t launch_tc_one(const GemvParams& p, unsigned grid, size_t smem, cudaS
 }
 
 template <int BITS, bool G32, bool AFFINE, bool AL, int W>
-cudaError_t launch_tc_w(const GemvParams& p, int sm_count, cudaStream_t st) {
+cudaError_t launch_tc_w(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half) {
   const unsigned grid = tc_grid_for(p, sm_count);
   const size_t smem = tc_smem<BITS, G32>(p, sm_count, W);
   switch (tc_tokens(p)) {
-    case 1: return launch_tc_one<BITS, G32, 1, AFFINE, AL, W>(p, grid, smem, st);
-    case 2: return launch_tc_one<BITS, G32, 2, AFFINE, AL, W>(p, grid, smem, st);
-    case 4: return launch_tc_one<BITS, G32, 4, AFFINE, AL, W>(p, grid, smem, st);
-    default: return launch_tc_one<BITS, G32, 8, AFFINE, AL, W>(p, grid, smem, st);
+    case 1: return launch_tc_one<BITS, G32, 1, AFFINE, AL, W>(p, grid, smem, sm_count, st, half);
+    case 2: return launch_tc_one<BITS, G32, 2, AFFINE, AL, W>(p, grid, smem, sm_count, st, half);
+    case 4: return launch_tc_one<BITS, G32, 4, AFFINE, AL, W>(p, grid, smem, sm_count, st, half);
+    default: return launch_tc_one<BITS, G32, 8, AFFINE, AL, W>(p, grid, smem, sm_count, st, half);
   }
 }
 template <int BITS, bool G32, bool AFFINE>
-cudaError_t launch_tc_format(const GemvParams& p, int sm_count, cudaStream_t st) {
+cudaError_t launch_tc_format(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half) {
   const bool al = tc_aligned<BITS, G32>(p);
   if (tc_warps_for<BITS, G32>(p, sm_count) == 8)
-    return al ? launch_tc_w<BITS, G32, AFFINE, true, 8>(p, sm_count, st) : launch_tc_w<BITS, G32, AFFINE, false, 8>(p, sm_count, st);
-  return al ? launch_tc_w<BITS, G32, AFFINE, true, 16>(p, sm_count, st) : launch_tc_w<BITS, G32, AFFINE, false, 16>(p, sm_count, st);
+    return al ? launch_tc_w<BITS, G32, AFFINE, true, 8>(p, sm_count, st, half) : launch_tc_w<BITS, G32, AFFINE, false, 8>(p, sm_count, st, half);
+  return al ? launch_tc_w<BITS, G32, AFFINE, true, 16>(p, sm_count, st, half) : launch_tc_w<BITS, G32, AFFINE, false, 16>(p, sm_count, st, half);
 }
 
 }  // namespace ztvm

@@ -2,5 +2,5 @@
 
 namespace ztvm {
 bool gemv_tc_fits_w4g32(const GemvParams& p, int sm_count) { return tc_fits<4, true>(p, sm_count); }
-cudaError_t launch_gemv_tc_w4g32(const GemvParams& p, int sm_count, cudaStream_t st) { return launch_tc_format<4, true, false>(p, sm_count, st); }
+cudaError_t launch_gemv_tc_w4g32(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half) { return launch_tc_format<4, true, false>(p, sm_count, st, half); }
 }  // namespace ztvm

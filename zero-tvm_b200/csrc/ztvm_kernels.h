@@ -23,13 +23,20 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
-// Shared memory that a launch of one CTA per SM asks for at least. Such a grid gives each CTA a fixed share of the rows. Started
-// early, behind kernels that still hold SMs, its CTAs go to whatever slots come free first; where an SM has room for two of
-// them, some get two shares and others none (a recorded 4-bit row, hidden 3648, ffn 10944: the down projections behind a
-// SiLU that had let them in early made it 263 us, 212 us with one share per SM; 225 us before the SiLU let them in). More
-// than half of an SM's 228 KB (with the 1 KB that each CTA takes beside its own) keeps them apart; 112 KB stay for a CTA of
-// the launch before or after.
+// Grids of one CTA per SM, each CTA with a fixed share of the rows and room for two of them on an SM ("half-SM" launches: the
+// eight-warp matrix-unit GEMV, the CUDA-core GEMV's smaller grid). Started early, their CTAs go to whatever slots come free
+// first. Behind another half-SM launch that is one slot on every SM, as long as its CTAs are all still at work. Behind
+// anything else, or behind a launch much shorter than itself, some SMs may be free as a whole: they get two shares, others
+// none (a recorded 4-bit row, hidden 3648, ffn 10944: the down projections behind a SiLU that let them in early made it
+// 263 us, 212 us with one share per SM; hidden 1024: an lm_head behind a down projection of a tenth of its size, 75 and 68 us).
+// Such a launch asks for more than half of an SM's 228 KB (with the 1 KB that each CTA takes beside its own), which keeps its
+// CTAs apart and leaves 112 KB for a CTA of the next launch -- but not for one that asks for as much itself, so launches behind
+// a half-SM one of their own size don't (8192 x 2048 back to back: 4.2 us, 4.8 us if all of them did).
 constexpr size_t kOnePerSmSmem = 114 * 1024;
+struct HalfSm {
+  uint64_t before = 0;   // in: weight bytes of the launch before on the stream if it was one, else 0
+  uint64_t now = 0;      // out: the same of this launch
+};
 
 struct GemvParams {
   const uint32_t* W;   // packed codes [N][KP] (MoE: [experts][N][KP])
@@ -65,8 +72,12 @@ struct GemvParams {
   uint32_t pair_rows;
 };
 
+inline uint64_t half_sm_bytes(const GemvParams& p) { return (uint64_t)p.N * p.KP * 4; }
+// whether the launch before leaves one slot on every SM
+inline bool half_sm_behind(const HalfSm& h, const GemvParams& p) { return 2 * h.before >= half_sm_bytes(p); }
+
 cudaError_t launch_gemv(GemvParams p, int bits, bool moe, uint32_t tokens, uint32_t slots, int sm_count,
-                        cudaStream_t st);
+                        cudaStream_t st, HalfSm* half);
 
 // 4-bit weights on the warp-level matrix unit (ztvm_gemv_mma.cu); M <= 8.
 bool gemv_mma_supported(int bits, uint32_t group);
@@ -75,7 +86,7 @@ cudaError_t launch_gemv_mma(GemvParams p, bool moe, uint32_t tokens, uint32_t sl
 // Persistent matrix-unit GEMV, M <= 8: 4-bit groups of 64 / 32 and 8-bit groups of 64 (ztvm_gemv_tc.cuh).
 // `gemv_tc_supported` checks shape and alignment; anything it refuses goes to the kernels above.
 bool gemv_tc_supported(const GemvParams& p, int bits, int sm_count);
-cudaError_t launch_gemv_tc(const GemvParams& p, int bits, int sm_count, cudaStream_t st);
+cudaError_t launch_gemv_tc(const GemvParams& p, int bits, int sm_count, cudaStream_t st, HalfSm* half);
 
 // 3-bit / group-64 weights, M = 1, persistent matrix-unit GEMV (ztvm_gemv_tc3.cu).
 bool gemv_tc3_supported(const GemvParams& p, int bits, int sm_count);
