@@ -56,7 +56,7 @@ def test_router_logits_many_tokens(bits, T, rows, D, backend, dev):
     assert np.abs(got - ref).max() <= 1e-5 * np.sqrt(np.mean(ref * ref))
 
 
-@pytest.mark.parametrize("bits,T,E,d,ffn,slots", [(3, 9, 40, 192, 72, 4), (3, 40, 12, 320, 136, 4), (3, 97, 3, 256, 200, 2),   # tiles of 16, 32, 64 pairs
+@pytest.mark.parametrize("bits,T,E,d,ffn,slots", [(3, 9, 40, 192, 72, 4), (3, 19, 40, 192, 72, 4), (3, 40, 12, 320, 136, 4), (3, 97, 3, 256, 200, 2),   # tiles of 16, 32, 64 pairs
                                                   (4, 33, 40, 192, 72, 4), (4, 20, 9, 448, 136, 4)])    # K the streaming kernel does not take
 def test_grouped_experts(bits, T, E, d, ffn, slots, backend, dev, oracle_c):
     """Experts through the grouped form: rows that fill no 128-row block, K of 3, 5 and 4 scale groups, ragged

@@ -137,3 +137,24 @@ def test_replayed_token_under_the_kernel_knob(knob, dev, monkeypatch):
         torch.cuda.synchronize()
         assert torch.equal(got, gu) and torch.isfinite(gu.float()).all()
     be.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits,E_,tokens,slots,K,N,shared,own", [
+    (4, 64, 8, 8, 512, 64, True, False), (4, 64, 12, 8, 512, 64, True, True),       # K > N: from 3/2 pairs per expert on
+    (4, 64, 8, 8, 192, 256, True, True), (4, 200, 16, 8, 512, 64, True, True),      # K < N; 128 pairs
+    (4, 64, 7, 9, 192, 256, False, False),
+    (3, 64, 8, 8, 512, 64, True, False), (3, 64, 9, 8, 512, 64, True, True), (3, 16, 10, 4, 512, 64, True, True),
+    (3, 64, 8, 4, 64, 192, True, True), (3, 64, 8, 4, 128, 192, True, False), (3, 64, 10, 4, 128, 192, True, True), (3, 64, 31, 1, 64, 192, False, False),
+])
+def test_a_plan_of_one_call_needs_more_pairs(bits, E_, tokens, slots, K, N, shared, own, backend, dev):
+    x, y = torch.zeros(tokens, K, dtype=torch.float16, device="cuda"), torch.zeros(tokens, slots, N, dtype=torch.float16, device="cuda")
+    w, s = torch.zeros(E_, N, K * bits // 32, dtype=torch.int32, device="cuda"), torch.zeros(E_, N, K // 64, dtype=torch.float16, device="cuda")
+    ids = torch.zeros(tokens, slots, dtype=torch.int32, device="cuda")
+    desc = z.MoeDesc(z.MmDesc(K, N, 1, 64, bits, 1, 0), E_, slots, tokens, 0, N, K, slots * N, slots)
+    try:
+        for reuse, want in ((True, shared), (False, own)):
+            backend.ctx.moe_plan_reuse(reuse)
+            assert backend.ctx.int4_matmul_moe_uses_plan(desc, y, x, s, w, s, ids) is want
+    finally:
+        backend.ctx.moe_plan_reuse(False)

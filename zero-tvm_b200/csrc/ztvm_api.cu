@@ -589,7 +589,21 @@ static int moe_route(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::G
   const uint64_t pairs = (uint64_t)md->tokens * md->slots;
   if (pairs >= (1ull << 31)) return 0;
   if (ctx->moe_grouped >= 0) return ctx->moe_grouped ? moe_pick(ctx, md, p, y) : 0;
-  if (pairs < (md->mm.bits == 3 ? 32u : 64u)) return 0;
+  const ztvm_mm_desc* d = &md->mm;
+  if (pairs < (d->bits == 3 ? 32u : 64u)) return 0;
+  // A plan that no other call shares (5 to 8 us of its own, for one projection instead of a block's three) pays where the pairs
+  // are more, where they share experts, or where K is shorter than N, which the per-pair kernels are slow at. Per-pair against
+  // grouped with its plan, us: 4-bit, 257 experts of 512 x 2048: 12.5 : 18.9 at 64 pairs, 21.7 : 26.0 at 126, 29.8 : 28.6 at 160
+  // (64 experts 15.4 : 18.5 at 80, 21.8 : 20.4 at 126; 16 experts 12.2 : 11.5 at 64), of 2048 x 512: 24.7 : 23.4 at 64. 3-bit,
+  // 257 experts of 512 x 2048: 15.4 : 21.0 at 44, 24.2 : 21.4 at 80 (16 experts 15.5 : 15.4 at 44), of 1408 x 704: 14.8 : 17.3
+  // at 32, 19.4 : 19.7 at 44, of 2048 x 512: 19.8 : 14.6 at 32.
+  if (!ctx->plan_reuse) {
+    if (d->bits == 3) {
+      if (pairs < (3ull * d->K <= d->N ? 32u : d->K < d->N ? 40u : 72u) && 2 * pairs < 5ull * md->experts) return 0;
+    } else if (pairs < 128 && d->K >= d->N && 2 * pairs < 3ull * md->experts) {
+      return 0;
+    }
+  }
   const int pick = moe_pick(ctx, md, p, y);
   return (pick == 1 || pick == 3) && pairs < 128 ? 0 : pick;
 }
