@@ -328,6 +328,16 @@ ZTVM_API ztvm_status ztvm_int4_matmul_nshard(ztvm_ctx* ctx, const ztvm_mm_desc* 
 ZTVM_API ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* desc, void* h, const void* x, const void* scales,
                            const void* packed_w, const void* biases, void* stream);
 
+/* A step of many small calls: between begin and end, one-row ztvm_int4_matmul calls with f16 results on `stream`, and a ztvm_silu_mul over the
+ * result of the one just before, are held back and launched together, as one kernel in which a matmul waits for the earlier ones
+ * only where it reads or overwrites what they wrote. Any other call of the context, and ztvm_step_end, launches what is held back
+ * first, so the order is that of the calls, and results are theirs up to the order of f32 sums (a matmul's is the same in every
+ * step, whatever it is joined with); an error of the launch is reported by the call that made it. Events recorded and work
+ * submitted on `stream` by other means between begin and end would not find it in order: end the step before.
+ * (The reference submits a token's dispatches as one command buffer, src/zero-tvm/engine-core.ts:2194-2202.) */
+ZTVM_API ztvm_status ztvm_step_begin(ztvm_ctx* ctx, void* stream);
+ZTVM_API ztvm_status ztvm_step_end(ztvm_ctx* ctx);
+
 /* h[r][i] = f16(up * gate * 1/(1+exp(-gate))) over rows of [gate(ffn) | up(ffn)] f16.
  * Replaces silu_mul (src/compiler/shaders/silu_mul.wgsl:26-44). */
 ZTVM_API ztvm_status ztvm_silu_mul(ztvm_ctx* ctx, uint32_t rows, uint32_t ffn, void* h, const void* gate_up, void* stream);

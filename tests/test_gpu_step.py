@@ -1,0 +1,162 @@
+"""One-row matmuls of a recorded step in one launch: whatever they read and overwrite of one another, replays give what the same
+calls give as steps of one call each, bit for bit, and that is the oracle's result."""
+import numpy as np
+import pytest
+
+import zero_tvm_b200 as z
+from oracle import ztvm_oracle as zo
+from zero_tvm_b200.backend import pod_args, resolve_matmul
+
+pytestmark = pytest.mark.gpu
+
+FORMATS = [(4, False), (4, True), (3, False), (8, False)]
+
+
+class Step:
+    """Recorded calls over named one-row buffers."""
+
+    def __init__(self, backend, dev, rng, bits, symmetric):
+        self.be, self.dev, self.rng, self.bits, self.sym = backend, dev, rng, bits, symmetric
+        self.group = 32 if symmetric else 64
+        self.rec, self.bufs, self.weights = z.recorder.DecodeRecorder(backend), {}, []
+
+    def buf(self, name, n, dtype=np.float16, values=None):
+        self.bufs[name] = self.dev.empty((1, n), dtype, fill=0.0)
+        if values is not None:
+            self.bufs[name].copy_(self.dev.put(values))
+        return self.bufs[name]
+
+    def matmul(self, y, x, n, k, f32=False):
+        q, W, s, b = z.synth.make_weights(self.rng, n, k, bits=self.bits, group=self.group, sigma_s=0.01 * 15 / (2**self.bits - 1))
+        keep = np.float16(10 / np.sqrt(k))                # results about as large as their inputs, however long the chain
+        s, b = s * keep, None if self.sym else b * keep
+        entry = "int8_affine_matvec" if self.bits == 8 else resolve_matmul(affine=not self.sym, K=k, q3=self.bits == 3, out_f32=f32)
+        self.rec.dispatch(entry, [self.bufs[y], self.bufs[x], self.dev.put(s), self.dev.put(W), pod_args(k, n, bits=self.bits, group=self.group)]
+                          + ([] if b is None else [self.dev.put(b)]))
+        self.weights.append((y, x, q, s, b))
+
+    def check(self, replays=3):
+        """Results one by one, then replays of the captured step from the same buffers."""
+        import torch
+        torch.cuda.synchronize()
+        start = {k: v.clone() for k, v in self.bufs.items()}
+
+        def restore():
+            for k, v in self.bufs.items():
+                v.copy_(start[k])
+            torch.cuda.synchronize()
+
+        for fn, args, _ in self.rec._calls:            # one by one: steps of one call
+            self.be.ctx.step_begin(1)
+            fn(*args, stream=1)
+            self.be.ctx.step_end()
+        torch.cuda.synchronize()
+        want = {k: v.clone() for k, v in self.bufs.items()}
+        restore()
+        step = self.rec.capture()
+        for _ in range(replays):
+            restore()
+            step.replay()
+            torch.cuda.synchronize()
+            for k, v in self.bufs.items():
+                assert torch.equal(v, want[k]) and torch.isfinite(v.float()).all(), k
+        assert self.be.ctx.device_errors() == 0
+        return want
+
+    def against_oracle(self, want, y):
+        """Result buffer `y`, whose x no later call overwrote. f32 sums over exact codes: each of K terms rounds at 2^-24 of the
+        largest partial sum, far below the f16 store's 2^-11; graded as the other GEMV tests are."""
+        _, x, q, s, b = next(w for w in self.weights if w[0] == y)
+        w32 = zo.dequant_w32(q, s, b, self.group, affine=b is not None)
+        ref = want[x].cpu().numpy().astype(np.float64) @ w32.astype(np.float64).T
+        got = want[y].cpu().numpy().astype(np.float64)
+        assert zo.rel_err_scaled(got, ref, 1e-3) < 2e-3, y
+
+
+@pytest.mark.parametrize("bits,symmetric", FORMATS)
+@pytest.mark.parametrize("d,wide", [(64, 149), (192, 1), (320, 2368), (1024, 40), (2112, 320), (4160, 704)])
+def test_reads_and_overwrites(bits, symmetric, d, wide, backend, dev):
+    """Results read by the next call and by one further on, a buffer overwritten after it was read, one written twice; results of
+    one row, of fewer rows than SMs, and tiles that end anywhere."""
+    rng = np.random.default_rng(d + wide + bits)
+    st = Step(backend, dev, rng, bits, symmetric)
+    for name in ("a", "b", "c"):
+        st.buf(name, d, values=z.synth.make_x(rng, 1, d))
+    st.buf("n", wide)
+    st.buf("f", wide, np.float32)
+    st.buf("a2", d)
+    st.matmul("n", "a", wide, d)            # reads a
+    st.matmul("b", "a", d, d)
+    st.matmul("c", "b", d, d)               # reads the last result
+    st.matmul("a2", "b", d, d)              # ... and once more
+    st.matmul("b", "c", d, d)               # overwrites what two calls read
+    st.matmul("b", "a2", d, d)              # ... and overwrites that
+    if bits != 8:
+        st.matmul("f", "b", wide, d, f32=True)
+    want = st.check()
+    for y in ("n",) if bits == 8 else ("n", "f"):
+        st.against_oracle(want, y)
+
+
+@pytest.mark.parametrize("bits,symmetric", FORMATS)
+@pytest.mark.parametrize("hidden,ffn", [(256, 8), (448, 1096), (1088, 2240)])
+def test_activation_behind_a_matmul(bits, symmetric, hidden, ffn, backend, dev):
+    """SiLU * up joins the matmul it reads, writes both buffers, and is waited for; where it reads something else it runs alone."""
+    rng = np.random.default_rng(hidden + bits)
+    st = Step(backend, dev, rng, bits, symmetric)
+    down = ffn // 64 * 64
+    st.buf("x", hidden, values=z.synth.make_x(rng, 1, hidden))
+    for name, n in (("gu", 2 * ffn), ("h", ffn), ("gu2", 2 * ffn), ("h2", ffn), ("y", hidden), ("y2", hidden)):
+        st.buf(name, n)
+    for gu, h, y in (("gu", "h", "y"), ("gu2", "h2", "y2")):
+        st.matmul(gu, "x", 2 * ffn, hidden)
+        if gu == "gu2":
+            st.matmul("y2", "x", hidden, hidden)          # between the two
+        st.rec.silu_mul(st.bufs[h], st.bufs[gu], 1, ffn)
+        if down:
+            st.bufs[h + "_k"] = st.bufs[h][:, :down]
+            st.matmul(y, h + "_k", hidden, down)
+    want = st.check()
+    st.against_oracle(want, "gu")
+    if down:
+        st.against_oracle(want, "y")
+
+
+def test_more_calls_than_one_launch_takes_and_formats_in_turn(backend, dev):
+    rng = np.random.default_rng(1)
+    st = Step(backend, dev, rng, 4, False)
+    st.buf("v0", 256, values=z.synth.make_x(rng, 1, 256))
+    for i in range(70):
+        st.buf(f"v{i + 1}", 256)
+        st.bits = 8 if 30 <= i < 33 else 4
+        st.matmul(f"v{i + 1}", f"v{i}" if i % 4 else "v0", 256, 256)
+        if i % 8 == 7:
+            st.buf(f"w{i}", 512)
+            st.buf(f"s{i}", 256)
+            st.matmul(f"w{i}", "v0", 512, 256)
+            st.rec.silu_mul(st.bufs[f"s{i}"], st.bufs[f"w{i}"], 1, 256)
+            st.bufs[f"v{i + 1}"] = st.bufs[f"s{i}"]
+    st.check(replays=2)
+
+
+def test_two_captured_steps_replay_side_by_side(backend, dev):
+    """Each captured step counts arrivals in words of its own."""
+    import torch
+    rng = np.random.default_rng(2)
+    steps = []
+    for _ in range(2):
+        st = Step(backend, dev, rng, 4, False)
+        for i in range(4):
+            st.buf(f"v{i}", 512, values=z.synth.make_x(rng, 1, 512) * 0.1)
+        for i in range(3):
+            st.matmul(f"v{i + 1}", f"v{i}", 512, 512)
+        steps.append((st, st.check(), st.rec.capture()))
+    streams = [torch.cuda.Stream() for _ in steps]
+    for _ in range(20):
+        for s, (_, _, step) in zip(streams, steps):
+            with torch.cuda.stream(s):
+                step.replay()
+    torch.cuda.synchronize()
+    for st, want, _ in steps:
+        assert all(torch.equal(v, want[k]) for k, v in st.bufs.items())
+    assert backend.ctx.device_errors() == 0

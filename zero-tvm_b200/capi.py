@@ -18,6 +18,7 @@ SYMBOLS = [
     "ztvm_int4_matmul", "ztvm_int4_matmul_multi", "ztvm_int4_matmul_host", "ztvm_int4_matmul_host_async", "ztvm_host_wait", "ztvm_int4_matmul_moe", "ztvm_int4_matmul_moe_uses_plan", "ztvm_int4_matmul_moe_noalloc",
     "ztvm_moe_router_logits", "ztvm_embedding_affine", "ztvm_moe_plan_reuse", "ztvm_moe_route_topk", "ztvm_moe_dispatch_plan", "ztvm_moe_ep_dispatch", "ztvm_int4_matmul_moe_ep", "ztvm_silu_mul_rows", "ztvm_peer_barrier", "ztvm_moe_ffn_ep", "ztvm_int4_matmul_nshard",
     "ztvm_fused_ffn",
+    "ztvm_step_begin", "ztvm_step_end",
     "ztvm_silu_mul",
     "ztvm_moe_combine", "ztvm_unpack_codes", "ztvm_unpack_codes_streamed", "ztvm_dequant", "ztvm_device_errors",
 ]
@@ -104,6 +105,8 @@ def load() -> C.CDLL:
         "ztvm_moe_ffn_ep": [vp, C.POINTER(MoeFfnEpArgs), vp],
         "ztvm_int4_matmul_nshard": [vp, C.POINTER(MmDesc), C.POINTER(C.c_void_p), u32, u32, u32, vp, vp, vp, vp, C.POINTER(C.c_void_p), vp],
         "ztvm_fused_ffn": [vp, C.POINTER(MmDesc), vp, vp, vp, vp, vp, vp],
+        "ztvm_step_begin": [vp, vp],
+        "ztvm_step_end": [vp],
         "ztvm_silu_mul": [vp, u32, u32, vp, vp, vp],
         "ztvm_moe_combine": [vp, u32, u32, u32, vp, vp, vp, vp],
         "ztvm_unpack_codes": [vp, C.POINTER(MmDesc), vp, vp, vp],
@@ -272,6 +275,14 @@ class Context:
         """h = f16(up * silu(gate)) for the [2 * desc.N, K] stack of gate and up rows (desc.N = ffn)."""
         check(self._lib.ztvm_fused_ffn(self.handle, C.byref(desc), addr(h), addr(x), addr(scales), addr(packed_w), addr(biases),
                                        stream_ptr(stream)))
+
+    def step_begin(self, stream=None):
+        """One-row matmuls (and the SiLU behind one) called on `stream` from here on are launched together, by step_end or
+        by the next call of another kind."""
+        check(self._lib.ztvm_step_begin(self.handle, stream_ptr(stream)))
+
+    def step_end(self):
+        check(self._lib.ztvm_step_end(self.handle))
 
     def silu_mul(self, rows, ffn, h, gate_up, stream=None):
         check(self._lib.ztvm_silu_mul(self.handle, rows, ffn, addr(h), addr(gate_up), stream_ptr(stream)))

@@ -8,6 +8,7 @@
 
 #include "../../include/ztvm_b200.h"
 #include "ztvm_kernels.h"
+#include "ztvm_step.h"
 #include "ztvm_workbuf.h"
 
 struct ztvm_ctx {
@@ -35,6 +36,10 @@ struct ztvm_ctx {
   int plan_reuse;   // ztvm_moe_plan_reuse: consecutive ztvm_int4_matmul_moe calls over one id list share its plan
   // The last call's last launch, for HalfSm: its weight bytes if it was a half-SM one, and its stream. `call`: the call being made.
   struct { uint64_t half; cudaStream_t st; } call, last;
+  // ztvm_step_begin .. ztvm_step_end: one-row matmuls called on step_stream, not launched yet
+  ztvm::StepBuilder* step;
+  int step_on;
+  cudaStream_t step_stream;
   int moe_tiles_sm; // env ZTVM_MOE_TILES=sm: the grouped MoE tiles with both operands in shared memory (a measurement knob)
 };
 
@@ -59,7 +64,10 @@ ztvm_status cuda_fail(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, #call);      \
   } while (0)
 
-ztvm_status check_ctx(ztvm_ctx* ctx) {
+ztvm_status step_flush(ztvm_ctx* ctx);
+
+// `hold`: the call may join the matmuls held back (ztvm_step_begin); every other call launches them first.
+ztvm_status check_ctx(ztvm_ctx* ctx, bool hold = false) {
   if (!ctx) return fail(ZTVM_ERR_BAD_CONTEXT, "context is NULL");
   if (ctx->magic != kMagic) return fail(ZTVM_ERR_BAD_CONTEXT, "context is not live (destroyed or corrupt)");
   int dev = -1;
@@ -67,7 +75,33 @@ ztvm_status check_ctx(ztvm_ctx* ctx) {
   if (dev != ctx->device) ZTVM_CUDA(cudaSetDevice(ctx->device));
   ctx->last = ctx->call;         // every entry point comes through here
   ctx->call.half = 0;
-  return ZTVM_OK;
+  return hold || !ctx->step_on ? ZTVM_OK : step_flush(ctx);
+}
+
+// Launches what ztvm_int4_matmul and ztvm_silu_mul held back.
+ztvm_status step_flush(ztvm_ctx* ctx) {
+  if (ctx->step->size() == 0) return ZTVM_OK;
+  uint32_t* counters = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (ctx->step->waits()) {
+    ztvm::WorkBuf* buf = nullptr;
+    e = ctx->work->get(ztvm::WorkBufs::kStep, (ztvm::kStepMaxOps + 1) * sizeof(uint32_t), ctx->step_stream, &buf);
+    if (e == cudaSuccess && buf->fresh) {
+      // Zero once: every launch leaves its counters as it found them. (On the context's own stream, so that no capture sees it.)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      e = cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e == cudaSuccess) {
+        e = cudaMemsetAsync(buf->p, 0, buf->bytes, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+      }
+      if (e == cudaSuccess) buf->fresh = false;
+    }
+    if (e == cudaSuccess) counters = static_cast<uint32_t*>(buf->p);
+  }
+  if (e == cudaSuccess) e = ctx->step->launch(counters, ctx->err_counter + 1, ctx->sm_count, ctx->step_stream);
+  ctx->step->clear();
+  return e == cudaSuccess ? ZTVM_OK : cuda_fail(e, "launch of the matmuls held back");
 }
 
 // What a GEMV launch on `st` finds before it, and what it leaves for the next call.
@@ -204,7 +238,8 @@ ztvm_status ztvm_init(int32_t device_ordinal, ztvm_ctx** out_ctx) {
   if (!c) return fail(ZTVM_ERR_CUDA, "out of host memory");
   memset(c, 0, sizeof(*c));
   c->work = new (std::nothrow) ztvm::WorkBufs();
-  if (!c->work) { delete c; return fail(ZTVM_ERR_CUDA, "out of host memory"); }
+  c->step = new (std::nothrow) ztvm::StepBuilder();
+  if (!c->work || !c->step) { delete c->work; delete c->step; delete c; return fail(ZTVM_ERR_CUDA, "out of host memory"); }
   c->device = device_ordinal;
   c->sm_count = prop.multiProcessorCount;
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
@@ -213,6 +248,7 @@ ztvm_status ztvm_init(int32_t device_ordinal, ztvm_ctx** out_ctx) {
   if (e != cudaSuccess) {
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c->work;
+    delete c->step;
     delete c;
     return cuda_fail(e, "context set-up");
   }
@@ -230,7 +266,7 @@ ztvm_status ztvm_init(int32_t device_ordinal, ztvm_ctx** out_ctx) {
 }
 
 ztvm_status ztvm_destroy(ztvm_ctx* ctx) {
-  ztvm_status s = check_ctx(ctx);
+  ztvm_status s = check_ctx(ctx, true);      // (matmuls held back and never asked for are dropped)
   if (s) return s;
   cudaStreamSynchronize(ctx->stream);
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
@@ -238,6 +274,7 @@ ztvm_status ztvm_destroy(ztvm_ctx* ctx) {
   if (ctx->d_y) cudaFree(ctx->d_y);
   ctx->work->free_all();
   delete ctx->work;
+  delete ctx->step;
   for (auto& l : ctx->lanes) {
     if (l.stream) { cudaStreamSynchronize(l.stream); cudaStreamDestroy(l.stream); }
     if (l.d_x) cudaFree(l.d_x);
@@ -257,13 +294,37 @@ ztvm_status ztvm_sync(ztvm_ctx* ctx) {
   return ZTVM_OK;
 }
 
+ztvm_status ztvm_step_begin(ztvm_ctx* ctx, void* stream) {
+  ztvm_status s = check_ctx(ctx);
+  if (s) return s;
+  if (ctx->step_on) return fail(ZTVM_ERR_UNSUPPORTED, "a step is being recorded already");
+  ctx->step_stream = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  ctx->step->clear();
+  ctx->step_on = 1;
+  return ZTVM_OK;
+}
+
+ztvm_status ztvm_step_end(ztvm_ctx* ctx) {
+  ztvm_status s = check_ctx(ctx);           // launches what is held back
+  if (ctx && ctx->magic == kMagic) ctx->step_on = 0;
+  return s;
+}
+
 ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, const void* x, const void* scales,
                              const void* packed_w, const void* biases, void* stream) {
-  ztvm_status s = check_ctx(ctx);
+  ztvm_status s = check_ctx(ctx, true);
   if (s) return s;
   if ((s = check_desc(d, true))) return s;
   if ((s = check_buffers(d, y, x, scales, packed_w, biases))) return s;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  if (ctx->step_on) {
+    const bool join = d->M == 1 && st == ctx->step_stream && ctx->gemv_path == 0;
+    ztvm::GemvParams p;
+    if (join) p = gemv_params(ctx, d, y, x, scales, packed_w, biases);
+    if (join && ctx->step->add(p, (int)d->bits, ctx->sm_count)) return ZTVM_OK;
+    if ((s = step_flush(ctx))) return s;
+    if (join && ctx->step->add(p, (int)d->bits, ctx->sm_count)) return ZTVM_OK;
+  }
   // Up to 16 rows the GEMV in slabs of eight: exact codes and f32 weights, the reference's choice for short chunks (runtime-M
   // matvec; its GEMMs start at 64 rows). From 17 on a third slab costs more than the GEMM at every width. Weight sets from HBM,
   // GEMM against slabs, us: 8192 x 2048 9.8 : 11.1 at 16 rows, 10.1 : 15.8 at 17; 24576 x 4096 40.7 : 34.2 and 40.8 : 48.0;
@@ -295,7 +356,12 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
     p.Y = d->out_f32 ? static_cast<void*>(static_cast<float*>(y) + (size_t)m0 * d->N)
                      : static_cast<void*>(static_cast<__half*>(y) + (size_t)m0 * d->N);
     const bool want_tc = ctx->gemv_path == 0 || (ctx->gemv_path == 3 && dd.M > 1);
-    if (want_tc && ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st, &half));
+    if (d->M == 1 && ctx->gemv_path == 0 && ztvm::step_alone_faster((int)d->bits, d->affine != 0, d->N, d->K) &&
+        ctx->step->add(p, (int)d->bits, ctx->sm_count)) {      // (nothing is held back here)
+      const cudaError_t e = ctx->step->launch(nullptr, ctx->err_counter + 1, ctx->sm_count, st);
+      ctx->step->clear();
+      if (e != cudaSuccess) return cuda_fail(e, "one-row matmul");
+    } else if (want_tc && ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st, &half));
     else if (want_tc && ztvm::gemv_tc3_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc3(p, ctx->sm_count, st));
     else if (use_mma(ctx, d, dd.M)) ZTVM_CUDA(ztvm::launch_gemv_mma(p, false, 1, 1, st));
     else ZTVM_CUDA(ztvm::launch_gemv(p, (int)d->bits, false, 1, 1, ctx->sm_count, st, &half));
@@ -867,11 +933,15 @@ ztvm_status ztvm_silu_mul_rows(ztvm_ctx* ctx, const ztvm_moe_ep_rows* rows, uint
 }
 
 ztvm_status ztvm_silu_mul(ztvm_ctx* ctx, uint32_t rows, uint32_t ffn, void* h, const void* gate_up, void* stream) {
-  ztvm_status s = check_ctx(ctx);
+  ztvm_status s = check_ctx(ctx, true);
   if (s) return s;
   if (!h || !gate_up) return fail(ZTVM_ERR_NULL_POINTER, "h/gate_up must be non-NULL");
   if (ffn == 0) return fail(ZTVM_ERR_BAD_DIMS, "ffn=0");
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  if (ctx->step_on) {
+    if (st == ctx->step_stream && ctx->step->add_silu(gate_up, h, rows, ffn, ctx->sm_count)) return ZTVM_OK;
+    if ((s = step_flush(ctx))) return s;
+  }
   ZTVM_CUDA(ztvm::launch_silu_mul(static_cast<const __half*>(gate_up), static_cast<__half*>(h), rows, ffn, ctx->sm_count, st));
   return ZTVM_OK;
 }

@@ -46,6 +46,12 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// up * silu(gate) in f32 (silu_mul.wgsl:40-43).
+__device__ __forceinline__ float silu_mul_one(float g, float u) {
+  const float sg = g * (1.0f / (1.0f + expf(-g)));
+  return u * sg;
+}
+
 // ---- 4-bit codes ---------------------------------------------------------------------------
 // Code i of a word sits at bits [4i, 4i+4). The eight codes come out as four half2 holding the
 // exact integers, in the pair order (q0,q4) (q1,q5) (q2,q6) (q3,q7):

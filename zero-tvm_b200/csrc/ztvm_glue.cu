@@ -358,11 +358,7 @@ cudaError_t launch_route_topk(const float* logits, uint32_t* ids, float* scores,
 }
 
 // ---- SiLU * up -----------------------------------------------------------------------------------
-// Rows of [gate(ffn) | up(ffn)] f16 -> f16 [ffn]; f32 arithmetic (silu_mul.wgsl:40-43).
-__device__ __forceinline__ float silu_mul_one(float g, float u) {
-  const float sg = g * (1.0f / (1.0f + expf(-g)));
-  return u * sg;
-}
+// Rows of [gate(ffn) | up(ffn)] f16 -> f16 [ffn] (silu_mul_one).
 // VEC elements per thread: eight (16-byte loads and stores; ffn % 8 == 0, 16-byte aligned buffers) where that still fills
 // the chip; two (ffn even, 4-byte aligned) for a few rows, whose time is one thread's chain of exponentials and divisions
 // (9 x 512: 1.7 -> 1.3 us); else one.

@@ -1,5 +1,5 @@
 // Work buffers of the calls that need device memory of their own (the expert-sorted plan of the grouped MoE matmul, the f32
-// rows of the fused FFN's two-launch form), host side.
+// rows of the fused FFN's two-launch form, the counters of a step's matmuls in one launch), host side.
 //
 // Calls that may overlap never share a buffer:
 //   * a call outside any capture uses its stream's buffer (at most kWorkStreams of them per purpose; a further stream takes
@@ -41,13 +41,14 @@ struct WorkBuf {
   std::atomic<bool> held{false};    // a graph refers to it, or did: `held` falls only for those with a user object
   uint64_t last_use = 0;
   PlanKey plan;                     // plan.ids == nullptr: no plan
+  bool fresh = false;               // (re)allocated since its user last looked
 };
 
 class WorkBufs {
  public:
   static constexpr int kWorkStreams = 4;
   static constexpr size_t kKeptBytes = 64u << 20;
-  enum Purpose { kPlan, kFfnRows };
+  enum Purpose { kPlan, kFfnRows, kStep };
 
   // A buffer of at least `need` bytes for a call on `st`.
   cudaError_t get(Purpose purpose, size_t need, cudaStream_t st, WorkBuf** out) {
@@ -170,6 +171,7 @@ class WorkBufs {
     b->plan = PlanKey();
     const cudaError_t e = cudaMalloc(&b->p, bytes);
     if (e == cudaSuccess) b->bytes = bytes;
+    b->fresh = true;
     return e;
   }
 

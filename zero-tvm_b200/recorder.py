@@ -79,10 +79,6 @@ class DecodeRecorder:
     def __len__(self):
         return len(self._calls)
 
-    def _run(self, stream):
-        for fn, args, kw in self._calls:
-            fn(*args, stream=stream, **kw)
-
     def _side_by_side(self, a, b):
         """Two calls become branches of the graph only where the library runs both on the kernel that reads ids directly:
         the expert-sorted plan is one buffer, which the first call would fill while the second reads or fills it."""
@@ -92,26 +88,43 @@ class DecodeRecorder:
         """The sequence inside the capture. The gate and up projections of a decoded token are a few CTAs each and read the
         same inputs: as two branches of the graph they run side by side (four blocks of one token, 256 experts of
         2048 x 512: 89 -> 73 us)."""
-        import torch
         i = 0
         while i < len(self._calls):
-            fn, args, kw = self._calls[i]
             if i + 1 < len(self._calls) and self._side_by_side(self._calls[i], self._calls[i + 1]):
                 side.wait_event(main.record_event())
+                fn, args, kw = self._calls[i]
                 fn(*args, stream=main.cuda_stream, **kw)
                 fn, args, kw = self._calls[i + 1]
                 fn(*args, stream=side.cuda_stream, **kw)
                 main.wait_event(side.record_event())
                 i += 2
                 continue
-            fn(*args, stream=main.cuda_stream, **kw)
-            i += 1
+            # up to the next such pair: the library joins what it can into one launch
+            end = i + 1
+            while end < len(self._calls) and not (end + 1 < len(self._calls) and self._side_by_side(self._calls[end], self._calls[end + 1])):
+                end += 1
+            self._run_joined(main.cuda_stream, i, end)
+            i = end
+
+    def _run_joined(self, stream, first, last):
+        """Calls first..last - 1 as one step: consecutive one-row matmuls become one launch."""
+        step_begin = getattr(getattr(self.be, "ctx", None), "step_begin", None)
+        if step_begin is None or last - first < 2:
+            for fn, args, kw in self._calls[first:last]:
+                fn(*args, stream=stream, **kw)
+            return
+        step_begin(stream)
+        try:
+            for fn, args, kw in self._calls[first:last]:
+                fn(*args, stream=stream, **kw)
+        finally:
+            self.be.ctx.step_end()
 
     def run_eager(self, stream=None):
-        """The recorded sequence as plain launches on `stream` (default: torch's current stream)."""
+        """The recorded sequence launched on `stream` (default: torch's current stream), joined as in the captured step."""
         import torch
         s = stream if stream is not None else torch.cuda.current_stream()
-        self._run(s.cuda_stream if s.cuda_stream else 1)
+        self._run_joined(s.cuda_stream if s.cuda_stream else 1, 0, len(self._calls))
 
     def capture(self, plan_reuse: bool = True):
         """One eager pass (loads the kernels and sets their attributes; what it rejects is rejected before a
@@ -125,7 +138,7 @@ class DecodeRecorder:
         self.be.ctx.moe_plan_reuse(plan_reuse)
         try:
             with torch.cuda.stream(self._stream):
-                self._run(self._stream.cuda_stream)
+                self._run_joined(self._stream.cuda_stream, 0, len(self._calls))
                 self._stream.synchronize()
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g, stream=self._stream):
