@@ -329,12 +329,14 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
   // matvec; its GEMMs start at 64 rows). From 17 on a third slab costs more than the GEMM at every width. Weight sets from HBM,
   // GEMM against slabs, us: 8192 x 2048 9.8 : 11.1 at 16 rows, 10.1 : 15.8 at 17; 24576 x 4096 40.7 : 34.2 and 40.8 : 48.0;
   // 4096 x 12288 18.6 : 24.2 and 19.0 : 35.6. (The GEMM is ahead at 9..16 rows too where K is long, but rounds the weights to f16.)
-  if (d->M > 16 && ztvm::gemm_w4_supported((int)d->bits, d->group, d->K) && !ctx->no_gemm) {
+  // 8-bit weights go as two f16 terms each, exact to 2^-22; f32 results (router logits) stay with the exact-code kernel below, and so
+  // do up to 32 rows, one token tile of it (12288 x 2048: 14 us at 24 rows, the GEMM 18; at 40 rows 26, 19; 2048 x 6144 30, 20).
+  const bool two_terms = d->bits == 8 && d->M > 32 && d->affine && !d->out_f32 && aligned(y, 16);
+  if (d->M > 16 && (d->bits == 4 || two_terms) && ztvm::gemm_ta_supported((int)d->bits, d->group, d->K) && !ctx->no_gemm) {
     if (!aligned(y, 16)) return fail(ZTVM_ERR_ALIGNMENT, "y must be 16-byte aligned for the GEMM path");
-    ZTVM_CUDA(ztvm::launch_gemm_w4_ta(static_cast<const uint32_t*>(packed_w), static_cast<const __half*>(scales),
-                                      d->affine ? static_cast<const __half*>(biases) : nullptr, static_cast<const __half*>(x), y,
-                                      d->M, d->N, d->K, (uint32_t)log2_exact(d->group), d->out_f32 != 0, ctx->err_counter + 1,
-                                      ctx->sm_count, st));
+    ZTVM_CUDA(ztvm::launch_gemm_ta(static_cast<const uint32_t*>(packed_w), static_cast<const __half*>(scales),
+                                   d->affine ? static_cast<const __half*>(biases) : nullptr, static_cast<const __half*>(x), y, d->M, d->N, d->K,
+                                   (int)d->bits, (uint32_t)log2_exact(d->group), d->out_f32 != 0, ctx->err_counter + 1, ctx->sm_count, st));
     return ZTVM_OK;
   }
   // Rows whose weights may not be rounded to f16 -- 8-bit codes, and router logits at any width -- in one launch of the

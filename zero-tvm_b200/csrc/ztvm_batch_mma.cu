@@ -1,7 +1,7 @@
 // Batched exact-code matmul on the warp matrix unit: y[t, n] = sum_k x[t, k] * (s q + b)[n, k] for tens to thousands of
 // activation rows, dense or grouped by expert, where the weights may not be rounded to f16 first:
 //   * router logits (moe_router_logits.wgsl: f32 sums over exact codes feed a softmax and a top-k),
-//   * 8-bit projections of more than eight rows (int8_affine_batched.wgsl),
+//   * 8-bit projections of 9 to 32 rows, and of any more with f32 results (int8_affine_batched.wgsl),
 //   * 3-bit expert matmuls (int4_matmul.gen.ts:229-254, :409-448), and 4-bit ones of few pairs per expert over a ragged K.
 // Those used to run as slabs of eight rows (or, for experts, one GEMV per pair) on the CUDA cores.
 //

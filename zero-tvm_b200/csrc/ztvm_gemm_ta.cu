@@ -1,4 +1,4 @@
-// Prefill GEMM, M > 16, 4-bit weights: y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS AS THE
+// Prefill GEMM, M > 16, 4-bit and 8-bit weights: y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS AS THE
 // A OPERAND IN TENSOR MEMORY (replaces the matrix-unit GEMMs of int4_matmul.gen.ts:1058-1456; contract of
 // ztvm_int4_matmul for M > 16). W16 = f16_rne(fl32(s * q + b)) (or s * (q - 7)), the value the reference's numpy
 // dequantiser produces (scripts/make-dsv2-layer-ref.py:108-116); f32 accumulation in tensor memory.
@@ -21,6 +21,12 @@
 // 64 / 128 / 256 / 352 tokens: at many tokens the MMA's reads and the TMA's writes of the activations share the 128 bytes
 // per clock of shared memory, beside a fixed 0.18 us that wider tiles have less often. 24576 x 4096, 1024 tokens: 172 us
 // with tiles of 256, 154 us; 6144 x 4096 (192 tiles of 256 on 148 SMs, 144 of 352): 54, 38 us.
+//
+// 8-bit weights (int8_affine_batched.wgsl multiplies them as f32) are two f16 terms in two slices and two MMAs each: w = hi + lo holds a
+// weight to 2^-22. Stored times a power of two per row, from a scan of the row's scales and biases while the first copies fly, so
+// that neither large nor tiny scales cost anything. 200 tokens, us, against the
+// warp-level matrix unit with exact codes (ztvm_batch_mma.cu): 3072 x 2048 15.6 : 26.1, 12288 x 2048 24.8 : 80.6, 2048 x 6144 26 : 44.6; 1000
+// tokens 12288 x 2048 84 : 267.
 //
 // Few tiles (short prompts, small N): the K range is split over a cluster of CTAs. Each CTA keeps the k blocks of its
 // share; at the end every CTA sends its f32 partial sums of token slice j to CTA j through distributed shared memory, and
@@ -52,35 +58,64 @@ struct GemmTaParams {
   uint32_t* status;
 };
 
-template <int NT>
+template <int NT, int BITS>
 struct GemmTaSmem {
   static constexpr int kXBytes = NT * kGemmBK * 2;            // per stage
-  static constexpr int kWBytes = kTaRows * 128;               // per packed-weight slot
+  static constexpr int kWBytes = kTaRows * 32 * BITS;         // per packed-weight slot: four k blocks, in boxes of 128 bytes a row
   // the widest tile leaves room for two packed-weight slots and for one table of groups of 32 or two of wider groups
-  static constexpr int kWStages = NT > 256 ? 2 : 3;
+  static constexpr int kWStages = NT > 256 || (BITS == 8 && NT > 128) ? 2 : 3;
   static constexpr int kSbBytes = NT > 256 ? 2 * kTaRows * 24 : 2 * kTaRows * kTaSbMaxPitch;
   static constexpr int kOffW = kTaStages * kXBytes;
   static constexpr int kOffSb = kOffW + kWStages * kWBytes;
   static constexpr int kOffBar = kOffSb + kTaSbStages * kSbBytes;
-  static constexpr int kTotal = kOffBar + 256;
+  static constexpr int kTotal = kOffBar + 256 + (BITS == 8 ? 4 * kTaRows * 4 : 0);     // (8-bit: bounds of the rows' weights)
 };
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(taddr) : "memory");
 }
 
-template <int NT, bool AFFINE>
+// 8-bit weights may not be rounded to f16: two f16 terms each, w = hi + lo, and two MMAs.
+// Bound of a row's weights from a quarter of its groups: max |s| * 255 + |b|.
+__device__ __forceinline__ float ta_row_bound(const GemmTaParams& p, uint32_t row, uint32_t quarter) {
+  float top = 0.f;
+  const __half *const s = p.S + (size_t)row * p.SPR, *const b = p.B + (size_t)row * p.SPR;
+  const uint32_t end = (quarter + 1u) * p.SPR / 4u;
+#pragma unroll 8
+  for (uint32_t g = quarter * p.SPR / 4u; g < end; ++g) top = fmaxf(top, fmaf(255.f, fabsf(__half2float(__ldg(s + g))), fabsf(__half2float(__ldg(b + g)))));
+  return top;
+}
+// The power of two by which a row's weights are stored: top * unit < 2^15.
+__device__ __forceinline__ float ta_row_unit(float top) {
+  const uint32_t e = __float_as_uint(top) >> 23;             // top < 2^(e - 126); 0: all zeros
+  return __uint_as_float((e == 0u ? 127u : 127u + 141u - e) << 23);
+}
+// Sixteen codes: w = fl32(s q + b), hi = f16(w), lo = f16(w - hi).
+__device__ __forceinline__ void ta_terms8(const uint4& w, float s, float b, uint32_t* hi, uint32_t* lo) {
+  const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      // a byte under the exponent of 2^23 is that many units above it
+      const float q0 = __uint_as_float(__byte_perm(v[i], 0x4B000000u, j ? 0x7442 : 0x7440)) - 8388608.f;
+      const float q1 = __uint_as_float(__byte_perm(v[i], 0x4B000000u, j ? 0x7443 : 0x7441)) - 8388608.f;
+      const float w0 = fmaf(s, q0, b), w1 = fmaf(s, q1, b);
+      const __half2 h = __floats2half2_rn(w0, w1);
+      const float2 f = __half22float2(h);
+      hi[2 * i + j] = h2_as_u32(h);
+      lo[2 * i + j] = h2_as_u32(__floats2half2_rn(w0 - f.x, w1 - f.y));
+    }
+}
+
+template <int NT, bool AFFINE, int BITS>
 __global__ void __launch_bounds__(kTaThreads, 1)
-gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
+gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                   const GemmTaParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  using L = GemmTaSmem<NT>;
+  using L = GemmTaSmem<NT, BITS>;
   constexpr int kTaWStages = L::kWStages;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
@@ -108,7 +143,9 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const uint32_t kb_last = kz + 1 == split ? all_kb : (kz + 1) * units / split * kTaSbChunk;
   const uint32_t num_kb = kb_last - kb_first;
   constexpr uint32_t kColA = NT;                                 // weight slices start after the accumulator columns
-  constexpr uint32_t kTmemCols = NT + kTaStages * 32 <= 256 ? 256 : 512;
+  constexpr uint32_t kACols = BITS == 8 ? 64 : 32;               // of a stage: 64 weights of a row as f16, 8-bit ones as two terms each
+  constexpr uint32_t kTmemCols = NT + kTaStages * kACols <= 256 ? 256 : 512;
+  static_assert(NT + kTaStages * kACols <= 512, "tensor memory");
   const uint32_t nbox = mrows > p.box_rows ? 2u : 1u, box_bytes = p.box_rows * (uint32_t)(kGemmBK * 2);
 
   if (threadIdx.x == 32) { tma_prefetch_desc(&tmap_x); tma_prefetch_desc(&tmap_w); }
@@ -119,7 +156,9 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   };
   auto load_w = [&](uint32_t s, uint32_t c) {
     mbar_arrive_expect_tx(bar_w_full((int)s), (uint32_t)L::kWBytes);
-    tma_load_2d(w_ring + s * L::kWBytes, &tmap_w, bar_w_full((int)s), (int)(kb_first * 8u + c * 32u), (int)n0);
+#pragma unroll
+    for (uint32_t b = 0; b < BITS / 4; ++b)
+      tma_load_2d(w_ring + s * L::kWBytes + b * (kTaRows * 128), &tmap_w, bar_w_full((int)s), (int)(kb_first * 2u * BITS + c * 8u * BITS + b * 32u), (int)n0);
   };
   // Each TMA producer initialises the barriers its own copies signal and starts its first loads before the block
   // barrier: they fly while tensor memory is allocated.
@@ -186,6 +225,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
   const bool is_dq = warp >= 3 && warp < 3 + kTaDqWarps;
   bool acc_ok = false;
+  [[maybe_unused]] float unscale = 1.f;               // 8-bit: results are sums of stored weights
 
   if (warp == 0) {
     // ================= TMA producer: activations =================
@@ -222,7 +262,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       for (uint32_t kb = 0; kb < num_kb && ok; ++kb) {
         tc_fence_after();
         const uint64_t bdesc = b0 + (uint64_t)(s * (L::kXBytes >> 4));
-        const uint32_t a_tmem = tmem_base + kColA + s * 32u;
+        const uint32_t a_tmem = tmem_base + kColA + s * kACols;
         uint32_t s1 = s + 1u, ph1 = ph;
         if (s1 == (uint32_t)kTaStages) { s1 = 0; ph1 ^= 1u; }
         bool next_ready = true;
@@ -232,6 +272,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           umma_f16_ta(tmem_base, a_tmem + (uint32_t)(8 * k), bdesc + (uint64_t)(2 * k), idesc, (kb | (uint32_t)k) ? 1u : 0u);
           if (NT > 256 && cols > cols_a)
             umma_f16_ta(tmem_base + cols_a, a_tmem + (uint32_t)(8 * k), bdesc + (uint64_t)(cols_a * 8u + 2 * k), idesc_b, (kb | (uint32_t)k) ? 1u : 0u);
+          if (BITS == 8) umma_f16_ta(tmem_base, a_tmem + 32u + (uint32_t)(8 * k), bdesc + (uint64_t)(2 * k), idesc, 1u);   // the second terms
         }
         umma_commit(bar_empty((int)s));   // the activation tile and the weight slice are free once these MMAs have read them
         if (!next_ready) ok = mbar_wait(bar_full((int)s1), ph1, p.status, 2u, abort_flag);
@@ -280,19 +321,29 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     static_assert(kTaStages == kTaWChunk && kTaDqWarps == kTaWChunk * kTaTeamWarps, "a team per stage");
     const uint32_t team = wpart;
     const uint8_t* const wrow_sm = gen_base + L::kOffW + (r_tile >> 3) * 1024 + (r_tile & 7) * 128;
-    const uint32_t w_at0 = ((team * 2u) ^ (r_tile & 7)) << 4, w_at1 = ((team * 2u + 1u) ^ (r_tile & 7)) << 4;
+    [[maybe_unused]] const uint32_t w_at0 = ((team * 2u) ^ (r_tile & 7)) << 4, w_at1 = ((team * 2u + 1u) ^ (r_tile & 7)) << 4;
     const uint32_t sb_odd = (uint32_t)(((size_t)min(n0 + r_tile, p.N - 1) * p.SPR) & 3u) * 2u;   // (stages start on multiples of four groups)
     const uint8_t* const sb_row = gen_base + L::kOffSb + r_tile * p.sb_pitch + sb_odd;
     const uint32_t b_delta = (uint32_t)kTaRows * p.sb_pitch;
-    const uint32_t st_at = tmem_base + lane_base + kColA + team * 32u;
+    const uint32_t st_at = tmem_base + lane_base + kColA + team * kACols;
+    [[maybe_unused]] float row_unit = 1.f;                 // 8-bit: weights are stored times this power of two
+    if constexpr (BITS == 8) {
+      // ... which takes the largest weight that the row's scales allow to the top of f16's range: no weight overflows, and the two terms
+      // hold one to 2^-22 of its size or 2^-39 of that largest one
+      float* const bounds = reinterpret_cast<float*>(gen_base + L::kOffBar + 256);
+      bounds[team * kTaRows + r_tile] = ta_row_bound(p, min(n0 + r_tile, p.N - 1), team);
+      asm volatile("bar.sync 1, %0;" ::"n"(kTaDqWarps * 32) : "memory");
+      row_unit = ta_row_unit(fmaxf(fmaxf(bounds[r_tile], bounds[kTaRows + r_tile]), fmaxf(bounds[2 * kTaRows + r_tile], bounds[3 * kTaRows + r_tile])));
+      unscale = 1.f / row_unit;
+    }
     bool ok = true;
     uint32_t ws = 0, wph = 0, ss = 0, sph = 0;          // slot and phase of the packed ring and of the scales ring
     for (uint32_t c = 0; c * kTaWChunk < num_kb; ++c) {
       if (c * kTaWChunk + team < num_kb) {
         if (ok && (c & 1u) == 0u) ok = mbar_wait(bar_sb_full((int)ss), sph, p.status, 9u, abort_flag);
         if (ok) ok = mbar_wait(bar_w_full((int)ws), wph, p.status, 7u, abort_flag);
-        uint32_t a[32];
-        if (ok) {
+        uint32_t a[BITS == 8 ? 1 : 32];
+        if (BITS == 4 && ok) {
           const uint8_t* const wl = wrow_sm + ws * L::kWBytes;
           const uint4 w0 = *reinterpret_cast<const uint4*>(wl + w_at0), w1 = *reinterpret_cast<const uint4*>(wl + w_at1);
           const uint32_t k0 = ((c & 1u) * kTaWChunk + team) * (uint32_t)kGemmBK;
@@ -313,7 +364,23 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           ok = mbar_wait(bar_empty((int)team), (c & 1u) ^ 1u, p.status, 4u, abort_flag);
           tc_fence_after();
         }
-        if (ok) {
+        if (BITS == 8 && ok) {
+          const uint8_t* const wl = wrow_sm + ws * L::kWBytes + (team >> 1) * (kTaRows * 128);
+          const uint32_t k0 = ((c & 1u) * kTaWChunk + team) * (uint32_t)kGemmBK;
+          const uint8_t* const sp = sb_row + ss * L::kSbBytes + (k0 >> 6) * 2u;
+          const float sf = __half2float(*reinterpret_cast<const __half*>(sp)) * row_unit, bf = __half2float(*reinterpret_cast<const __half*>(sp + b_delta)) * row_unit;
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h) {                  // 32 codes at a time: 16 columns of each term
+            uint32_t hi[16], lo[16];
+#pragma unroll
+            for (uint32_t j = 0; j < 2; ++j)
+              ta_terms8(*reinterpret_cast<const uint4*>(wl + ((((team & 1u) * 4u + h * 2u + j) ^ (r_tile & 7)) << 4)), sf, bf, hi + 8 * j, lo + 8 * j);
+            tmem_st16(st_at + 16u * h, hi);
+            tmem_st16(st_at + 32u + 16u * h, lo);
+          }
+          tmem_st_wait();
+        }
+        if constexpr (BITS == 4) if (ok) {
           // 64 weights of this row = 32 TMEM columns (two k-adjacent f16 per column) of this thread's lane
           tmem_st32(st_at, a);
           tmem_st_wait();
@@ -355,6 +422,10 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           uint32_t v[32];
           tmem_ld32(tmem_base + lane_base + (uint32_t)(cb * 32), v);
           tmem_ld_wait();
+          if constexpr (BITS == 8) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * unscale);
+          }
           const uint32_t col = stage + (uint32_t)(cb * 32) * (kTaRows * 2u) + r_tile * 2u;
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -383,6 +454,10 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         uint32_t v[32];
         tmem_ld32(tmem_base + lane_base + (uint32_t)(cb * 32), v);
         tmem_ld_wait();
+        if constexpr (BITS == 8) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * unscale);
+        }
         const uint32_t m_first = m0 + cb * 32;
         if (n < p.N) {
           if (p.out_f32) {
@@ -449,6 +524,7 @@ gemm_w4_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 #pragma unroll
           for (uint32_t i = 0; i < 8; ++i) {
             if (b * 8u + i >= mrows) break;
+            if constexpr (BITS == 8) r[i] *= unscale;
             const size_t o = (size_t)(m0 + b * 8u + i) * p.N + n;
             if (p.out_f32) reinterpret_cast<float*>(p.Y)[o] = r[i];
             else reinterpret_cast<__half*>(p.Y)[o] = __float2half_rn(r[i]);
@@ -479,13 +555,13 @@ static TaEncodeFn ta_encode_fn() {
   return fn;
 }
 
-template <int NT, bool AFFINE>
+template <int NT, bool AFFINE, int BITS>
 static cudaError_t ta_kernel_ready() {
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 16 && attr_set[dev]) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_w4_ta_kernel<NT, AFFINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmTaSmem<NT>::kTotal + 1024);
+  const cudaError_t e = cudaFuncSetAttribute(gemm_ta_kernel<NT, AFFINE, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmTaSmem<NT, BITS>::kTotal + 1024);
   if (e == cudaSuccess && dev < 16) attr_set[dev] = true;
   return e;
 }
@@ -507,15 +583,15 @@ struct TaLaunch {
     cfg.numAttrs = grid.z > 1 ? 2 : 1;
   }
 };
-template <int NT, bool AFFINE>
+template <int NT, bool AFFINE, int BITS>
 static cudaError_t launch_ta_one(const CUtensorMap& tx, const CUtensorMap& tw, const GemmTaParams& p, uint32_t split, cudaStream_t st) {
-  const cudaError_t e = ta_kernel_ready<NT, AFFINE>();
+  const cudaError_t e = ta_kernel_ready<NT, AFFINE, BITS>();
   if (e != cudaSuccess) return e;
-  TaLaunch l(dim3((p.N + kTaRows - 1) / kTaRows, (p.M + p.tile_m - 1) / p.tile_m, split), GemmTaSmem<NT>::kTotal + 1024, st);
-  return cudaLaunchKernelEx(&l.cfg, gemm_w4_ta_kernel<NT, AFFINE>, tx, tw, p);
+  TaLaunch l(dim3((p.N + kTaRows - 1) / kTaRows, (p.M + p.tile_m - 1) / p.tile_m, split), GemmTaSmem<NT, BITS>::kTotal + 1024, st);
+  return cudaLaunchKernelEx(&l.cfg, gemm_ta_kernel<NT, AFFINE, BITS>, tx, tw, p);
 }
 // Clusters of `split` CTAs that the device holds at once (a cluster sits inside one GPC, so this is less than SMs / split).
-template <int NT>
+template <int NT, int BITS>
 static uint32_t ta_clusters(uint32_t split, int sm_count) {
   if (split == 1) return (uint32_t)sm_count;
   static int known[16][kTaMaxSplit + 1] = {};
@@ -524,8 +600,8 @@ static uint32_t ta_clusters(uint32_t split, int sm_count) {
   if (dev >= 16) return 1;
   int n = known[dev][split];
   if (n == 0) {
-    TaLaunch l(dim3(1, 1, split), GemmTaSmem<NT>::kTotal + 1024, nullptr);
-    if (ta_kernel_ready<NT, true>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_w4_ta_kernel<NT, true>, &l.cfg) != cudaSuccess || n < 1) {
+    TaLaunch l(dim3(1, 1, split), GemmTaSmem<NT, BITS>::kTotal + 1024, nullptr);
+    if (ta_kernel_ready<NT, true, BITS>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_ta_kernel<NT, true, BITS>, &l.cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       n = 1;
     }
@@ -534,33 +610,43 @@ static uint32_t ta_clusters(uint32_t split, int sm_count) {
   return (uint32_t)n;
 }
 
-bool gemm_w4_supported(int bits, uint32_t group, uint32_t K) {
+bool gemm_ta_supported(int bits, uint32_t group, uint32_t K) {
+  if (bits == 8) return group == 64 && K % kGemmBK == 0;
   return bits == 4 && (group == 32 || group == 64 || group == 128) && K % kGemmBK == 0;
 }
 
-cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M,
-                              uint32_t N, uint32_t K, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count, cudaStream_t st) {
+template <int BITS>
+static uint32_t ta_at_once(uint32_t tm, uint32_t z, int sm_count) {
+  if (tm <= 64u) return ta_clusters<64, BITS>(z, sm_count);
+  if (tm <= 128u) return ta_clusters<128, BITS>(z, sm_count);
+  if (BITS == 8 || tm <= 256u) return ta_clusters<256, BITS>(z, sm_count);
+  return ta_clusters<352, 4>(z, sm_count);
+}
+
+cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M, uint32_t N, uint32_t K,
+                           int bits, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count, cudaStream_t st) {
   TaEncodeFn enc = ta_encode_fn();
   if (!enc) return cudaErrorNotSupported;
   // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 8192 x 2048 .. 3072 x 8192:
   // a k block takes 340 + 1.4 per token (at least 390), a CTA 8500 to start, fill its rings and store, the exchange of
   // a cluster 5300 + 12 per token. Clusters run in as many waves as the device can place. The tokens are dealt evenly to
-  // the tiles. (Groups of 32 with biases do not fit beside the widest tile.)
+  // the tiles. (Groups of 32 with biases do not fit beside the widest tile.) 8-bit, whose blocks are twice the MMAs and more than twice
+  // the dequantisation: 700 + 1 per token, at least 5.5 per token; the exchange more for every share beyond two; no shares of the
+  // 256-token tiles (2048 x 6144, 200 tokens, us: two tiles in four shares 26, one in four 46, one whole 52).
   const uint32_t units = (K / kGemmBK + kTaSbChunk - 1) / kTaSbChunk, n_tiles = (N + kTaRows - 1) / kTaRows;
-  const uint32_t widest = B && group_shift == 5 ? 256u : 352u;
+  const uint32_t widest = bits == 8 || (B && group_shift == 5) ? 256u : 352u;
   uint32_t tile_m = 0, split = 1;
   uint64_t best = ~0ull;
   for (uint32_t t = 64; t <= widest; t += 32) {
     if (t > 64u && t - 32u >= M) break;
     const uint32_t m_tiles = (M + t - 1) / t, tm = ((M + m_tiles - 1) / m_tiles + 15u) & ~15u;
     const uint64_t tiles = (uint64_t)n_tiles * m_tiles;
-    const uint32_t live = M < tm ? M : tm, block = live < 36u ? 390u : 340u + live * 14u / 10u;
+    const uint32_t live = M < tm ? M : tm, block = bits == 8 ? (live < 156u ? 700u + live : live * 55u / 10u) : live < 36u ? 390u : 340u + live * 14u / 10u;
     for (uint32_t z = 1; z <= (uint32_t)kTaMaxSplit && z <= units; ++z) {
-      if (z > 1 && tiles * z > (uint64_t)sm_count) break;
-      const uint32_t at_once = tm <= 64u ? ta_clusters<64>(z, sm_count) : tm <= 128u ? ta_clusters<128>(z, sm_count)
-                               : tm <= 256u ? ta_clusters<256>(z, sm_count) : ta_clusters<352>(z, sm_count);
+      if (z > 1 && (tiles * z > (uint64_t)sm_count || (bits == 8 && tm > 128u))) break;
+      const uint32_t at_once = bits == 8 ? ta_at_once<8>(tm, z, sm_count) : ta_at_once<4>(tm, z, sm_count);
       const uint64_t waves = (tiles + at_once - 1) / at_once;
-      const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + 8500u + (z > 1 ? 5300u + 12u * live : 0u));
+      const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + 8500u + (z > 1 ? 5300u + 12u * live + (bits == 8 && z > 2 ? 28u * live * (z - 2) : 0u) : 0u));
       if (cost < best) { best = cost; tile_m = tm; split = z; }
     }
   }
@@ -575,8 +661,8 @@ cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* 
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-  const cuuint64_t wdims[2] = {K / 8, N};
-  const cuuint64_t wstrides[1] = {(cuuint64_t)(K / 8) * 4};
+  const cuuint64_t wdims[2] = {K / 32 * (uint32_t)bits, N};
+  const cuuint64_t wstrides[1] = {(cuuint64_t)(K / 32 * (uint32_t)bits) * 4};
   const cuuint32_t wbox[2] = {32, (cuuint32_t)kTaRows};
   r = enc(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint32_t*>(W), wdims, wstrides, wbox, estr,
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -589,11 +675,15 @@ cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* 
   p.sb_pitch = group_shift == 5 ? 40u : 24u;
   p.tile_m = tile_m; p.box_rows = box_rows;
   p.status = status;
+  if (bits == 8) {
+    if (tile_m > 128u) return launch_ta_one<256, true, 8>(tx, tw, p, split, st);
+    return tile_m > 64u ? launch_ta_one<128, true, 8>(tx, tw, p, split, st) : launch_ta_one<64, true, 8>(tx, tw, p, split, st);
+  }
   const bool affine = B != nullptr;
-  if (tile_m > 256u) return affine ? launch_ta_one<352, true>(tx, tw, p, split, st) : launch_ta_one<352, false>(tx, tw, p, split, st);
-  if (tile_m > 128u) return affine ? launch_ta_one<256, true>(tx, tw, p, split, st) : launch_ta_one<256, false>(tx, tw, p, split, st);
-  if (tile_m > 64u) return affine ? launch_ta_one<128, true>(tx, tw, p, split, st) : launch_ta_one<128, false>(tx, tw, p, split, st);
-  return affine ? launch_ta_one<64, true>(tx, tw, p, split, st) : launch_ta_one<64, false>(tx, tw, p, split, st);
+  if (tile_m > 256u) return affine ? launch_ta_one<352, true, 4>(tx, tw, p, split, st) : launch_ta_one<352, false, 4>(tx, tw, p, split, st);
+  if (tile_m > 128u) return affine ? launch_ta_one<256, true, 4>(tx, tw, p, split, st) : launch_ta_one<256, false, 4>(tx, tw, p, split, st);
+  if (tile_m > 64u) return affine ? launch_ta_one<128, true, 4>(tx, tw, p, split, st) : launch_ta_one<128, false, 4>(tx, tw, p, split, st);
+  return affine ? launch_ta_one<64, true, 4>(tx, tw, p, split, st) : launch_ta_one<64, false, 4>(tx, tw, p, split, st);
 }
 
 }  // namespace ztvm

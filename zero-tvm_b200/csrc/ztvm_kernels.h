@@ -101,13 +101,12 @@ bool batch_moe_supported(const GemvParams& g, int bits);
 uint32_t batch_moe_tile_rows(int bits, uint32_t experts, uint64_t pairs);
 cudaError_t launch_batch_moe(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan);
 
-// 4-bit weights, M > 16: tcgen05 GEMM with the dequantised weights as the A operand in tensor memory and the activations
+// 4-bit weights, and 8-bit ones as two f16 terms, M > 16: tcgen05 GEMM with the dequantised weights as the A operand in tensor memory and the activations
 // as the only shared-memory operand (ztvm_gemm_ta.cu). status[0] receives a non-zero code if a pipeline wait inside the
 // kernel ran out.
-bool gemm_w4_supported(int bits, uint32_t group, uint32_t K);
-cudaError_t launch_gemm_w4_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M,
-                              uint32_t N, uint32_t K, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count,
-                              cudaStream_t st);
+bool gemm_ta_supported(int bits, uint32_t group, uint32_t K);
+cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M, uint32_t N, uint32_t K,
+                           int bits, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count, cudaStream_t st);
 
 // Grouped MoE expert matmul (ztvm_moe_gemm.cu): pairs sorted by expert, tcgen05 tiles. `scratch` holds the plan
 // (moe_grouped_scratch_bytes), `status[0]` receives a non-zero code if a bounded wait ran out.
