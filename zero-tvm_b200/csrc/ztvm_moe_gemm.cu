@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t moe_agg_add(uint32_t* cnt, uint32_t key, boo
   return active ? atomicAdd(&cnt[key], 1u) : 0u;
 }
 
-// The whole plan in ONE block for pair lists up to a few tens of thousands: histogram and cursors in shared memory,
+// The whole plan in ONE block for pair lists up to a few thousand (kPlanClusterMin): histogram and cursors in shared memory,
 // same scans, same tables. Pairs are walked slot-major (a warp sees 32 tokens of one slot), so the pairs of a slot
 // that always carries the same expert (the shared expert) aggregate into one atomic per warp.
 constexpr uint32_t kPlanSmallMax = 32768;   // pairs the one-block plan takes: 32 per thread, kept in registers
@@ -403,12 +403,98 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeGemmPara
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
+// The same in a cluster of eight CTAs, each with an eighth of the pairs: one SM's shared-memory atomics and the loads of 18 ids a thread
+// bound the one-block plan (MoE block of 2048 tokens, 18432 pairs over 257 experts: 343 us a pass with it, 332 so; the one-block
+// plan is 21 of them, about 1.1 per 1024 pairs). Histograms are exchanged through distributed shared memory; every CTA
+// takes the scans for itself.
+constexpr uint32_t kPlanCtas = 8, kPlanClusterMin = 8192;
+__global__ void __launch_bounds__(1024) moe_plan_cluster_kernel(const uint32_t* ids, uint32_t tokens, uint32_t slots, uint32_t ids_stride,
+                                                                uint32_t E, uint32_t tile_rows, MoeScratch sc, uint32_t* err, MoeSegs segs) {
+  __shared__ uint32_t cnt_sm[1024], cur_sm[1024], warp_sums[32];
+  constexpr int kPer = (int)(kPlanSmallMax / (1024 * kPlanCtas));
+  const uint32_t e = threadIdx.x, P = tokens * slots, rank = blockIdx.x;      // (the grid is one cluster)
+  cnt_sm[e] = 0u;
+  pdl_launch_dependents();
+  pdl_wait();
+  uint32_t xs[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t j = rank * 1024u + threadIdx.x + 1024u * kPlanCtas * k;    // j = slot * tokens + token
+    xs[k] = 0xFFFFFFFEu;                                                       // not a pair
+    if (j < P) {
+      const uint32_t s = j / tokens, t = j - s * tokens;
+      if (segs.live(t * slots + s)) xs[k] = ids[(size_t)t * ids_stride + s];
+    }
+  }
+  __syncthreads();
+  uint32_t bad = 0;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    if (xs[k] >= E && xs[k] != 0xFFFFFFFEu) ++bad;
+    moe_agg_add(cnt_sm, xs[k], xs[k] < E);
+  }
+  if (bad) atomicAdd(err, bad);
+  cluster_sync_all();
+  uint32_t cnt = 0, before = 0;                                                // of expert e: all pairs, those of the CTAs before this one
+#pragma unroll
+  for (uint32_t r = 0; r < kPlanCtas; ++r) {
+    uint32_t at, v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(cnt_sm + e)), "r"(r));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    cnt += v;
+    if (r < rank) before += v;
+  }
+  if (e >= E) cnt = 0u;
+  cluster_sync_all();                                                          // no CTA leaves before the others have read its counts
+  const uint32_t nt = (cnt + tile_rows - 1) / tile_rows;
+  uint32_t total_pairs, total_tiles;
+  const uint32_t off = moe_block_excl_scan(cnt, warp_sums, &total_pairs);
+  const uint32_t tb = moe_block_excl_scan(nt, warp_sums, &total_tiles);
+  cur_sm[e] = off + before;
+  if (rank == 0) {
+    if (e < E) { sc.counts[e] = cnt; sc.offsets[e] = off; }
+    if (e == 0) { sc.offsets[E] = total_pairs; *sc.ntiles = total_tiles; }
+  }
+  for (uint32_t j = rank; j < nt; j += kPlanCtas) {
+    uint32_t* tt = sc.tiles + (size_t)(tb + j) * 3;
+    tt[0] = e;
+    tt[1] = off + j * tile_rows;
+    tt[2] = min(tile_rows, cnt - j * tile_rows);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t j = rank * 1024u + threadIdx.x + 1024u * kPlanCtas * k;
+    const bool ok = xs[k] < E;
+    const uint32_t pos = moe_agg_add(cur_sm, xs[k], ok);
+    if (ok) {
+      const uint32_t s = j / tokens, t = j - s * tokens;
+      sc.sorted[pos] = t * slots + s;
+    }
+  }
+}
+
 // Plan of one grouped launch: histogram of the expert ids, prefix sums + table of tiles of at most `tile_rows` pairs of
 // one expert, scatter of the pair indices into expert order. The words that must start at zero are cleared here.
 cudaError_t launch_moe_plan(const GemvParams& g, uint32_t tokens, uint32_t slots, const MoeScratch& sc, uint32_t tile_rows,
                             cudaStream_t st) {
   const uint32_t P = tokens * slots, E = g.experts;
   const MoeSegs segs{g.seg_counts, g.seg_cap ? g.seg_cap : 1u};
+  if (P > kPlanClusterMin && P <= kPlanSmallMax) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kPlanCtas);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = kPlanCtas;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, moe_plan_cluster_kernel, g.ids, tokens, slots, g.ids_stride, E, tile_rows, sc, g.err_counter, segs);
+  }
   if (P <= kPlanSmallMax) {   // short lists: one block does it all, nothing to clear beforehand
     return launch_chained(moe_plan_small_kernel, dim3(1), dim3(1024), 0, st, g.ids, tokens, slots, g.ids_stride, E, tile_rows, sc,
                           g.err_counter, segs);
