@@ -109,7 +109,7 @@ class DecodeRecorder:
     def _run_joined(self, stream, first, last):
         """Calls first..last - 1 as one step: consecutive one-row matmuls become one launch."""
         step_begin = getattr(getattr(self.be, "ctx", None), "step_begin", None)
-        if step_begin is None or last - first < 2:
+        if step_begin is None:
             for fn, args, kw in self._calls[first:last]:
                 fn(*args, stream=stream, **kw)
             return
