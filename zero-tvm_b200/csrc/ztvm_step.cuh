@@ -14,8 +14,7 @@
 //     but its launches do not join): a TMA box per stage 19.8, warps that only fetch for the others 16.0, codes
 //     straight from global memory to registers 16.4, e4m3 codes and activations (mma.sync on them is conversions and f16 MMAs here) 18.3.
 //   * K is cut into slices of a stage's width. KS of the 16 warps stand side by side along K, RG = 16 / KS groups of them take
-//     different row tiles; KS is the divisor with the fewest steps (see step_split), so that a K of 33 runs of 64 codes keeps 15
-//     warps busy and not nine.
+//     different row tiles (see step_split).
 //   * activations lie in shared memory with the sums of their scale groups; a warp turns its slice into MMA B fragments once per
 //     K tile.
 //   * codes masked where they sit are f16 subnormals (codes4_inplace, codes3_inplace, codes8_pair01): exact products; every scale

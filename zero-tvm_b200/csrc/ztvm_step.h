@@ -10,7 +10,6 @@ constexpr int kStepRounds = 4;      // row tiles of a warp between two meetings 
 constexpr int kStepPitch = 68;      // floats of a warp's partial sums: 64 rows, warps four banks apart
 constexpr int kStepMaxOps = 64;
 
-
 struct alignas(16) StepOp {
   const uint32_t* W;
   const __half* S;
