@@ -10,11 +10,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,N,K,size", [
-    (33, 128, 64, 1.0), (64, 129, 576, 1.0), (65, 2048, 2112, 1.0),        # tile widths, a last slot of one block, K shares in a cluster
+    (33, 128, 64, 1.0), (64, 129, 576, 1.0), (65, 2048, 2112, 1.0), (33, 128, 1536, 1.0), (40, 300, 1600, 2.0**-17), (40, 300, 1536, 2.0**12), (130, 300, 1728, 0.0),        # tile widths, a last slot of one block, K shares in a cluster
     (128, 1000, 1152, 1.0), (129, 257, 320, 1.0), (200, 3072, 2048, 1.0), (256, 130, 192, 1.0), (257, 20001, 128, 1.0), (700, 136, 4160, 1.0),
     (40, 300, 512, 2.0**-17), (40, 300, 512, 2.0**13), (40, 300, 64, 0.0),   # scales among f16's subnormals, weights past f16's largest
 ])
 def test_two_terms(M, N, K, size, backend, dev, oracle_c):
+    """(Those of little work over a short K run on the kernel that multiplies the codes: the same bound.)"""
     p = z.synth.projection(N, K, M=M, bits=8, seed=M + N, sigma_s=0.01 / 17)
     rng = np.random.default_rng(K)
     s, b = p["scales"].astype(np.float32), p["biases"].astype(np.float32)

@@ -25,7 +25,7 @@
 // 8-bit weights (int8_affine_batched.wgsl multiplies them as f32) are two f16 terms in two slices and two MMAs each: w = hi + lo holds a
 // weight to 2^-22. Stored times a power of two per row, from a scan of the row's scales and biases while the first copies fly, so
 // that neither large nor tiny scales cost anything. 200 tokens, us, against the
-// warp-level matrix unit with exact codes (ztvm_batch_mma.cu): 3072 x 2048 15.6 : 26.1, 12288 x 2048 24.8 : 80.6, 2048 x 6144 26 : 44.6; 1000
+// warp-level matrix unit with exact codes (ztvm_batch_mma.cu): 3072 x 2048 14.0 : 26.1, 12288 x 2048 23.2 : 80.5, 2048 x 6144 21.6 : 44.6; 1000
 // tokens 12288 x 2048 84 : 267.
 //
 // Few tiles (short prompts, small N): the K range is split over a cluster of CTAs. Each CTA keeps the k blocks of its
@@ -78,13 +78,24 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
 }
 
 // 8-bit weights may not be rounded to f16: two f16 terms each, w = hi + lo, and two MMAs.
-// Bound of a row's weights from a quarter of its groups: max |s| * 255 + |b|.
+// Bound of a row's weights from a quarter of its groups: max |s| * 255 + |b|. Tables start on 8-byte boundaries.
 __device__ __forceinline__ float ta_row_bound(const GemmTaParams& p, uint32_t row, uint32_t quarter) {
   float top = 0.f;
   const __half *const s = p.S + (size_t)row * p.SPR, *const b = p.B + (size_t)row * p.SPR;
-  const uint32_t end = (quarter + 1u) * p.SPR / 4u;
+  auto see = [&](__half sv, __half bv) { top = fmaxf(top, fmaf(255.f, fabsf(__half2float(sv)), fabsf(__half2float(bv)))); };
+  if ((p.SPR & 3u) == 0u) {                                  // four groups per load: 96 groups in one latency
+    const uint32_t fours = p.SPR / 4u, end = (quarter + 1u) * fours / 4u;
 #pragma unroll 8
-  for (uint32_t g = quarter * p.SPR / 4u; g < end; ++g) top = fmaxf(top, fmaf(255.f, fabsf(__half2float(__ldg(s + g))), fabsf(__half2float(__ldg(b + g)))));
+    for (uint32_t g = quarter * fours / 4u; g < end; ++g) {
+      const uint2 sv = __ldg(reinterpret_cast<const uint2*>(s) + g), bv = __ldg(reinterpret_cast<const uint2*>(b) + g);
+      see(__low2half(u32_as_h2(sv.x)), __low2half(u32_as_h2(bv.x))); see(__high2half(u32_as_h2(sv.x)), __high2half(u32_as_h2(bv.x)));
+      see(__low2half(u32_as_h2(sv.y)), __low2half(u32_as_h2(bv.y))); see(__high2half(u32_as_h2(sv.y)), __high2half(u32_as_h2(bv.y)));
+    }
+  } else {
+    const uint32_t end = (quarter + 1u) * p.SPR / 4u;
+#pragma unroll 8
+    for (uint32_t g = quarter * p.SPR / 4u; g < end; ++g) see(__ldg(s + g), __ldg(b + g));
+  }
   return top;
 }
 // The power of two by which a row's weights are stored: top * unit < 2^15.

@@ -403,11 +403,10 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeGemmPara
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
-// The same in a cluster of eight CTAs, each with an eighth of the pairs: one SM's shared-memory atomics and the loads of 18 ids a thread
-// bound the one-block plan (MoE block of 2048 tokens, 18432 pairs over 257 experts: 343 us a pass with it, 332 so; the one-block
-// plan is 21 of them, about 1.1 per 1024 pairs). Histograms are exchanged through distributed shared memory; every CTA
-// takes the scans for itself.
-constexpr uint32_t kPlanCtas = 8, kPlanClusterMin = 8192;
+// The same in a cluster of eight CTAs, each with an eighth of the pairs: one SM's shared-memory atomics and the loads of up to 32 ids a
+// thread bound the one-block plan (257 experts, us: 18432 pairs 21, 8.0 so; 9216 7.3, 4608 6.9 so, 2304 in one block 9.6 cold). Histograms
+// are exchanged through distributed shared memory; every CTA takes the scans for itself.
+constexpr uint32_t kPlanCtas = 8, kPlanClusterMin = 4096;
 __global__ void __launch_bounds__(1024) moe_plan_cluster_kernel(const uint32_t* ids, uint32_t tokens, uint32_t slots, uint32_t ids_stride,
                                                                 uint32_t E, uint32_t tile_rows, MoeScratch sc, uint32_t* err, MoeSegs segs) {
   __shared__ uint32_t cnt_sm[1024], cur_sm[1024], warp_sums[32];
