@@ -1,0 +1,47 @@
+"""What f32 sums leave behind, seen through f16 results: rows whose exact results are zero."""
+import numpy as np
+import pytest
+
+import zero_tvm_b200 as z
+
+pytestmark = pytest.mark.gpu
+
+
+def cancelling(seed, N, half, M, bits, group, symmetric):
+    """x, W, s, b and the size of a result's terms (2-norm). The second half of K holds the products of the first, each group in another
+    order and negated. Activations are mostly small beside a few large ones, as behind a SiLU * up."""
+    rng = np.random.default_rng(seed)
+    x1 = (rng.standard_normal((M, half)) ** 5 * 4).clip(-6e4, 6e4).astype(np.float16)
+    q1 = rng.integers(0, 1 << bits, (N, half), dtype=np.uint8)
+    order = np.concatenate([g * group + rng.permutation(group) for g in range(half // group)])
+    s1 = np.abs(rng.standard_normal((N, half // group)) * 0.01 * 15 / (2**bits - 1)).astype(np.float16)
+    b1 = (rng.standard_normal((N, half // group)) * 0.05).astype(np.float16)
+    x, q = np.concatenate([x1, -x1[:, order]], 1), np.concatenate([q1, q1[:, order]], 1)
+    s, b = np.concatenate([s1, s1], 1), None if symmetric else np.concatenate([b1, b1], 1)
+    per = np.repeat(s.astype(np.float64), group, 1)
+    terms = (per * q) ** 2 + ((7 * per) ** 2 if symmetric else np.repeat(b.astype(np.float64), group, 1) ** 2)
+    return x, z.synth.pack_codes(q, bits), s, b, np.sqrt((x.astype(np.float64) ** 2 @ terms.T).mean())
+
+
+@pytest.mark.parametrize("bits,symmetric,half,M", [
+    (4, True, 1536, 1), (4, True, 4096, 1), (4, True, 160, 1), (4, True, 1056, 1),    # groups of 32: whole and ragged slices
+])
+def test_sums_keep_f32(bits, symmetric, half, M, backend, dev):
+    """Each result passes 2 K / group folds and a few more additions, each of which rounds by at most 2^-24 of a partial sum; their signs are
+    as good as random, and a partial sum is about as large as the terms' 2-norm. By itself, and joined with another in a step."""
+    group, N = 32 if symmetric else 64, 1100
+    x, W, s, b, size = cancelling(half + M, N, half, M, bits, group, symmetric)
+    K = 2 * half
+    bound = np.sqrt(2 * K / group + 32) * 2.0**-24 * size + 2.0**-25                   # (f16 spacing near zero)
+    args = [dev.put(x), dev.put(s), dev.put(W), None if b is None else dev.put(b)]
+    desc = z.MmDesc(K, N, M, group, bits, int(not symmetric), 0)
+    ys = [dev.empty((M, N), np.float16, fill=9.0) for _ in range(3)]
+    backend.ctx.int4_matmul(desc, ys[0], *args)
+    backend.ctx.step_begin()
+    for y in ys[1:]:
+        backend.ctx.int4_matmul(desc, y, *args)
+    backend.ctx.step_end()
+    backend.ctx.sync()
+    for y in ys:
+        err = np.sqrt((dev.get(y).astype(np.float64) ** 2).mean())
+        assert err <= bound, (err / size, bound / size)

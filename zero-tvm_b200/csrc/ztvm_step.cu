@@ -72,8 +72,11 @@ bool StepBuilder::layout() {
   p.off_ops = (uint32_t)(kStepWarps * kStepDepth) * stage;
   p.off_part = p.off_ops + (p.n > 1 ? p.n * (uint32_t)sizeof(StepOp) : 0u);
   p.off_x = p.off_part + 2u * (uint32_t)(kStepWarps * kStepPitch) * 4u;
-  p.off_xsum = p.off_x + k_pad * 2u;
-  return p.off_xsum + k_pad / 32u * 4u <= 227u * 1024u;
+  const uint32_t parts = step_two_parts(format_ & 31, format_ == 4 + 32, al) ? 2u : 1u;
+  p.x_bytes = k_pad * 2u;
+  p.off_xsum = p.off_x + parts * p.x_bytes;
+  smem_ = p.off_xsum + parts * (k_pad / 32u * 4u);
+  return smem_ <= 227u * 1024u;
 }
 
 // Waits of matmul i, or false where it may not follow the earlier ones in one launch: its weights are fetched ahead of every wait.
@@ -164,15 +167,12 @@ cudaError_t StepBuilder::launch(uint32_t* counters, uint32_t* status, int sm_cou
   const bool together = waits();
   p.counters = together ? counters : nullptr;
   p.status = status;
-  uint32_t k_most = 0;
-  for (uint32_t i = 0; i < p.n; ++i) k_most = k_most < p.op[i].K ? p.op[i].K : k_most;
-  const size_t smem = p.off_xsum + (k_most + 255u) / 256u * 256u / 32u * 4u;
   const bool al = all_aligned(p, format_);
   switch (format_) {
-    case 3: return launch_step_w3(p, al, smem, sm_count, together, st);
-    case 8: return launch_step_w8(p, al, smem, sm_count, together, st);
-    case 4: return launch_step_w4(p, al, smem, sm_count, together, st);
-    default: return launch_step_w4g32(p, al, smem, sm_count, together, st);
+    case 3: return launch_step_w3(p, al, smem_, sm_count, together, st);
+    case 8: return launch_step_w8(p, al, smem_, sm_count, together, st);
+    case 4: return launch_step_w4(p, al, smem_, sm_count, together, st);
+    default: return launch_step_w4g32(p, al, smem_, sm_count, together, st);
   }
 }
 

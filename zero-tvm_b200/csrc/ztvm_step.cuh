@@ -21,6 +21,8 @@
 //     group is summed inside the matrix unit and folded into f32 accumulators, acc += s*(ratio*lo + hi) + b*sum(x). With one
 //     token the MMA's columns are the scale groups of the slice: a lane's codes belong to one group, and its activations stand in that
 //     group's column.
+//   * the unit truncates its sums. Rows that f32 FMAs would otherwise serve (step_two_parts) multiply activations in two parts, in
+//     two columns, whose sums are exact.
 //   * the K slices of a block of rows meet in shared memory in a fixed order: results are deterministic, and the same whether a
 //     matmul runs alone or among others, with or without its activation.
 //
@@ -46,7 +48,24 @@ struct StepFmt {
   static constexpr int kSbRow = (AFFINE ? 2 : 1) * kSbSlot;
   static constexpr int kStage = kCodes + 16 * kSbRow;
   static constexpr int kB = BITS == 3 ? 2 * kCodes3Views : BITS == 8 ? 16 : 32;   // registers of B fragments
+  static constexpr bool kTwo = step_two_parts(BITS, G32, AL);
+  static constexpr int kSets = kTwo && G32 ? 2 : 1;                 // accumulator sets: two parts of four groups fill the eight columns
 };
+
+// kTwo: an activation as two f16 values, x = unit * (whole + rest / 2048), with nothing lost: `unit` takes the group's largest to a whole part
+// of 2^10 .. 2^11, and the rest, at most half, keeps the bits below (an f16 of any size has eleven in all). The products of codes and whole
+// parts then sum to whole numbers below 2^24, which the matrix unit, that truncates its sums, gives exactly; what it drops of the rests' sum
+// is 2^-11 of what it would drop of the activations'.
+constexpr float kStepRest = 2048.f;
+__device__ __forceinline__ float step_group_unit(uint32_t top) {           // top: bits of the largest f16 magnitude
+  const uint32_t e = __float_as_uint(__half2float(__ushort_as_half((unsigned short)top))) >> 23;   // 0: all zeros, 255: not finite
+  return e == 0u || e == 255u ? 1.f : __uint_as_float((e - 10u) << 23);
+}
+__device__ __forceinline__ void step_parts(float x, float& whole, float& rest) {
+  whole = rintf(x);
+  const float r = (x - whole) * kStepRest;
+  rest = r == r ? r : 0.f;                                                 // (infinities: all in `whole`)
+}
 
 // Tile row of MMA row g (0..7). The 16-byte pieces of a row lie XORed with row mod 8; these orders make the rows of each phase
 // of a fragment load (four rows x 32 bytes, two rows x 64) fall on different banks.
@@ -64,6 +83,11 @@ __device__ __forceinline__ uint32_t step_ld_acquire(const uint32_t* a) {
 }
 __device__ __forceinline__ void step_cp4_zfill(uint32_t dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ unsigned long long step_mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 __device__ __forceinline__ void step_mma0(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
@@ -102,6 +126,7 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
   using C = StepFmt<BITS, G32, AFFINE, AL>;
   constexpr int G = C::kG, RPI = C::kRuns, kR = kStepRounds;
   // the sum of a run is kUnit * (kRatio * lo + hi)
+  static_assert(AFFINE || C::kTwo, "symmetric sums are taken in units of the products");
   constexpr float kRatio = BITS == 4 ? 16.f : 1.f, kUnit = BITS == 4 ? 1048576.f : 16777216.f;
   extern __shared__ __align__(128) uint8_t step_smem[];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -120,7 +145,7 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(step_smem) + warp * (kStepDepth * C::kStage);
   float* const partial = reinterpret_cast<float*>(step_smem + p.off_part);        // [2][warps][kStepPitch]
   uint8_t* const xs = step_smem + p.off_x;
-  float* const xsum = reinterpret_cast<float*>(step_smem + p.off_xsum);           // per scale group
+  float* const xsum = reinterpret_cast<float*>(step_smem + p.off_xsum);           // per scale group (kTwo: and the groups' units, behind them)
 
   // ---- producer: a stage at a time, in the order the warp consumes them ---------------------------------------------
   // This lane's pieces of a stage: 16 bytes (8 where 3-bit rows may start between them) of kPieces rows.
@@ -276,30 +301,60 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
     for (uint32_t i = tid; i < pieces; i += kStepWarps * 32u) {
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (i < have) v = __ldcg(reinterpret_cast<const uint4*>(o.X) + i);      // (other SMs may just have written it)
-      reinterpret_cast<uint4*>(xs)[i] = v;
-      const float2 x0 = __half22float2(u32_as_h2(v.x)), x1 = __half22float2(u32_as_h2(v.y)), x2 = __half22float2(u32_as_h2(v.z)),
-                   x3 = __half22float2(u32_as_h2(v.w));
-      float sum = ((x0.x + x0.y) + (x1.x + x1.y)) + ((x2.x + x2.y) + (x3.x + x3.y));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      float2 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = __half22float2(u32_as_h2(w[k]));
+      float sum = ((x[0].x + x[0].y) + (x[1].x + x[1].y)) + ((x[2].x + x[2].y) + (x[3].x + x[3].y));
       sum += __shfl_xor_sync(0xffffffffu, sum, 1);
       sum += __shfl_xor_sync(0xffffffffu, sum, 2);
       if constexpr (!G32) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-      if ((i & (G32 ? 3u : 7u)) == 0u) xsum[i / (G32 ? 4u : 8u)] = sum;
+      const bool first = (i & (G32 ? 3u : 7u)) == 0u;
+      const uint32_t grp = i / (G32 ? 4u : 8u);
+      if constexpr (C::kTwo) {
+        uint32_t top = 0u;                                    // the group's largest magnitude, as bits
+#pragma unroll
+        for (int k = 0; k < 4; ++k) top = max(max(top, w[k] & 0x7fffu), w[k] >> 16 & 0x7fffu);
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        if constexpr (!G32) top = max(top, __shfl_xor_sync(0xffffffffu, top, 4));
+        const float unit = step_group_unit(top), scale = 1.f / unit;           // powers of two
+        uint32_t whole[4], rest[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float2 a, b;
+          step_parts(x[k].x * scale, a.x, b.x);
+          step_parts(x[k].y * scale, a.y, b.y);
+          whole[k] = h2_as_u32(__floats2half2_rn(a.x, a.y));
+          rest[k] = h2_as_u32(__floats2half2_rn(b.x, b.y));
+        }
+        reinterpret_cast<uint4*>(xs)[i] = make_uint4(whole[0], whole[1], whole[2], whole[3]);
+        reinterpret_cast<uint4*>(xs + p.x_bytes)[i] = make_uint4(rest[0], rest[1], rest[2], rest[3]);
+        if (first) xsum[p.x_bytes / 64u + grp] = unit;
+        if constexpr (!AFFINE) sum *= scale;                  // (symmetric: in units, as the products)
+      } else {
+        reinterpret_cast<uint4*>(xs)[i] = v;
+      }
+      if (first) xsum[grp] = sum;
     }
     const StepShare cs = step_share(o, warp);
     const uint32_t pair = o.pair, spr = o.spr, KS = o.ks, RG = o.rg, all_rounds = ((cs.tiles + RG - 1u) * o.rg_inv) >> 16;
     __syncthreads();
 
     uint32_t xf[C::kB];                                       // B fragments of the slice
-    unsigned long long xs2 = 0ull;                            // sums of x over the groups of columns 2c, 2c + 1
+    // of columns 2c, 2c + 1, per accumulator set: the sums of x over their groups (0 with a second part) and (kTwo) their units
+    unsigned long long xs2[C::kSets], unit2[C::kSets];
     auto load_x = [&](uint32_t sl) {
-      const __half* const xr = reinterpret_cast<const __half*>(xs) + sl * (uint32_t)C::kSlice;
+      // (kTwo: columns 0..3 take the first part of four groups, 4..7 the second)
+      const __half* const xr = reinterpret_cast<const __half*>(xs + (C::kTwo && g >= 4u ? p.x_bytes : 0u)) + sl * (uint32_t)C::kSlice;
+      const uint32_t gc = C::kTwo ? g & 3u : g;               // the column's group (of its set)
       if constexpr (BITS == 3) {
-        // lane (g, c) multiplies the codes of group c, in MMA column c; a code's offset in its half goes onto its activation
+        // lane (g, c) multiplies the codes of group c, in that group's column; a code's offset in its half goes onto its activation
         __align__(16) __half h[64];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           uint4 v = make_uint4(0u, 0u, 0u, 0u);
-          if (g == c) v = *reinterpret_cast<const uint4*>(xr + 64u * c + 8 * i);
+          if (gc == c) v = *reinterpret_cast<const uint4*>(xr + 64u * c + 8 * i);
           *reinterpret_cast<uint4*>(&h[8 * i]) = v;
         }
         const __half q4 = __float2half(0.25f), q8 = __float2half(0.125f), q32 = __float2half(0.03125f), z = __float2half(0.f);
@@ -311,35 +366,51 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
         }
       } else {
         const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-        uint4 v0 = z4, v1 = z4;
-        if constexpr (G32) {
-          v0 = *reinterpret_cast<const uint4*>(xr + 32u * g + 8u * c);
-          v1 = v0;
-        } else if (g < (uint32_t)RPI) {
-          v0 = *reinterpret_cast<const uint4*>(xr + 64u * g + 16u * c);
-          v1 = *reinterpret_cast<const uint4*>(xr + 64u * g + 16u * c + 8u);
-        }
-        uint32_t b[8];
-        Frag<BITS>::b(v0, v1, b);
 #pragma unroll
-        for (int r = 0; r < RPI; ++r)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            // registers 0, 1, 4, 5 come from the first piece, the others from the second (8-bit: 0..3 and 4..7)
-            const bool second = BITS == 8 ? k >= 4 : (k & 2) != 0;
-            const uint32_t col = G32 ? 2u * r + (second ? 1u : 0u) : (uint32_t)r;
-            xf[r * 8 + k] = g == col ? b[k] : 0u;
+        for (int set = 0; set < C::kSets; ++set) {
+          constexpr int kRunsPerSet = RPI / C::kSets;
+          uint4 v0 = z4, v1 = z4;
+          if constexpr (G32) {                                 // (the two pieces of a run are groups of their own)
+            v0 = *reinterpret_cast<const uint4*>(xr + 128u * set + 32u * gc + 8u * c);
+            v1 = v0;
+          } else if (gc < (uint32_t)RPI) {
+            v0 = *reinterpret_cast<const uint4*>(xr + 64u * gc + 16u * c);
+            v1 = *reinterpret_cast<const uint4*>(xr + 64u * gc + 16u * c + 8u);
           }
+          uint32_t b[8];
+          Frag<BITS>::b(v0, v1, b);
+#pragma unroll
+          for (int r = 0; r < kRunsPerSet; ++r)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              // registers 0, 1, 4, 5 come from the first piece, the others from the second (8-bit: 0..3 and 4..7)
+              const bool second = BITS == 8 ? k >= 4 : (k & 2) != 0;
+              const uint32_t col = G32 ? 2u * r + (second ? 1u : 0u) : (uint32_t)r;
+              xf[(set * kRunsPerSet + r) * 8 + k] = gc == col ? b[k] : 0u;
+            }
+        }
       }
-      float2 s = make_float2(0.f, 0.f);
-      if (2u * c < (uint32_t)G) s = *reinterpret_cast<const float2*>(xsum + sl * (uint32_t)G + 2u * c);
-      xs2 = tc_pk(s.x * (1.f / kUnit), s.y * (1.f / kUnit));  // exact: the accumulators hold results in units of kUnit
+#pragma unroll
+      for (int set = 0; set < C::kSets; ++set) {
+        float2 s = make_float2(0.f, 0.f);
+        if constexpr (C::kTwo) {
+          const float* const at = xsum + sl * (uint32_t)G + 4u * set + 2u * (c & 1u);
+          const float2 u = *reinterpret_cast<const float2*>(at + p.x_bytes / 64u);
+          const float part = c < 2u ? kUnit : kUnit / kStepRest;
+          unit2[set] = tc_pk(u.x * part, u.y * part);
+          if (c < 2u) s = *reinterpret_cast<const float2*>(at);
+          xs2[set] = AFFINE ? tc_pk(s.x, s.y) : tc_pk(s.x * (1.f / kUnit), s.y * (1.f / kUnit));
+        } else {
+          if (2u * c < (uint32_t)G) s = *reinterpret_cast<const float2*>(xsum + sl * (uint32_t)G + 2u * c);
+          xs2[set] = tc_pk(s.x * (1.f / kUnit), s.y * (1.f / kUnit));  // exact: the accumulators hold results in units of kUnit
+        }
+      }
     };
     // (AL false) rows whose scales start on an odd group lie one value into their words; tiles start on rows of one parity
     const uint32_t odd_lo = ((cs.r0 + tr) & spr & 1u) * 2u, odd_hi = pair & spr & 1u ? odd_lo ^ 2u : odd_lo;
     // the stage at `st` times the slice, folded into `a`
     auto multiply = [&](unsigned long long (&a)[2]) {
-      float lo[4], hi[4];
+      float lo[C::kSets][4], hi[C::kSets][4];
       const uint32_t at0 = st + frag;
       if constexpr (BITS == 3) {
         uint32_t w[6], u[6];
@@ -353,9 +424,9 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
           uint32_t w0, w1, u0, u1;
           codes3_inplace(w, k, w0, w1);
           codes3_inplace(u, k, u0, u1);
-          if (k == 0) step_mma0(lo, w0, u0, w1, u1, xf[2 * k], xf[2 * k + 1]);
-          else if (k == 1) step_mma0(hi, w0, u0, w1, u1, xf[2 * k], xf[2 * k + 1]);
-          else step_mma(k & 1 ? hi : lo, w0, u0, w1, u1, xf[2 * k], xf[2 * k + 1]);
+          if (k == 0) step_mma0(lo[0], w0, u0, w1, u1, xf[2 * k], xf[2 * k + 1]);
+          else if (k == 1) step_mma0(hi[0], w0, u0, w1, u1, xf[2 * k], xf[2 * k + 1]);
+          else step_mma(k & 1 ? hi[0] : lo[0], w0, u0, w1, u1, xf[2 * k], xf[2 * k + 1]);
         }
       } else {
         using F = Frag<BITS>;
@@ -375,34 +446,42 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
           }
           uint32_t ag[8], ah[8];
           F::a(vg, ag); F::a(vh, ah);
+          constexpr int kRunsPerSet = RPI / C::kSets;
+          const int set = r / kRunsPerSet;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            if (r == 0 && h == 0) {
-              step_mma0(lo, ag[0], ah[0], ag[1], ah[1], xf[0], xf[1]);
-              step_mma0(hi, ag[4], ah[4], ag[5], ah[5], xf[4], xf[5]);
+            if (r % kRunsPerSet == 0 && h == 0) {
+              step_mma0(lo[set], ag[0], ah[0], ag[1], ah[1], xf[r * 8], xf[r * 8 + 1]);
+              step_mma0(hi[set], ag[4], ah[4], ag[5], ah[5], xf[r * 8 + 4], xf[r * 8 + 5]);
             } else {
-              step_mma(lo, ag[2 * h], ah[2 * h], ag[2 * h + 1], ah[2 * h + 1], xf[r * 8 + 2 * h], xf[r * 8 + 2 * h + 1]);
-              step_mma(hi, ag[4 + 2 * h], ah[4 + 2 * h], ag[5 + 2 * h], ah[5 + 2 * h], xf[r * 8 + 4 + 2 * h], xf[r * 8 + 5 + 2 * h]);
+              step_mma(lo[set], ag[2 * h], ah[2 * h], ag[2 * h + 1], ah[2 * h + 1], xf[r * 8 + 2 * h], xf[r * 8 + 2 * h + 1]);
+              step_mma(hi[set], ag[4 + 2 * h], ah[4 + 2 * h], ag[5 + 2 * h], ah[5 + 2 * h], xf[r * 8 + 4 + 2 * h], xf[r * 8 + 5 + 2 * h]);
             }
           }
         }
       }
-      // column 2c + v of the accumulators is one scale group (columns past the last group fold zeros with any scale)
-      const uint32_t sc = st + C::kCodes + tr * C::kSbRow + 2u * ((2u * c) % (uint32_t)G);
+      // column 2c + v of the accumulators is one scale group, or a part of one (columns past the last group fold zeros with any scale)
+      const uint32_t sc = st + C::kCodes + tr * C::kSbRow + 2u * (C::kTwo ? 2u * (c & 1u) : (2u * c) % (uint32_t)G);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t at = sc + 8u * h * C::kSbRow + (AL ? 0u : h ? odd_hi : odd_lo);
-        auto two = [&](uint32_t q) {
-          if constexpr (AL) return __half22float2(u32_as_h2(tc_lds32(q)));
-          return make_float2(__half2float(__ushort_as_half((unsigned short)tc_lds16(q))),
-                             __half2float(__ushort_as_half((unsigned short)tc_lds16(q + 2u))));
-        };
-        const float2 s = two(at);
-        float2 b;
-        if constexpr (AFFINE) b = two(at + C::kSbSlot); else b = make_float2(-7.f * s.x, -7.f * s.y);
-        const unsigned long long d = tc_ffma2(tc_pk(lo[2 * h], lo[2 * h + 1]), tc_pk(kRatio, kRatio), tc_pk(hi[2 * h], hi[2 * h + 1]));
-        a[h] = tc_ffma2(tc_pk(b.x, b.y), xs2, tc_ffma2(tc_pk(s.x, s.y), d, a[h]));
-      }
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int set = 0; set < C::kSets; ++set) {
+          const uint32_t at = sc + 8u * h * C::kSbRow + 8u * set + (AL ? 0u : h ? odd_hi : odd_lo);
+          auto two = [&](uint32_t q) {
+            if constexpr (AL) return __half22float2(u32_as_h2(tc_lds32(q)));
+            return make_float2(__half2float(__ushort_as_half((unsigned short)tc_lds16(q))),
+                               __half2float(__ushort_as_half((unsigned short)tc_lds16(q + 2u))));
+          };
+          const float2 s = two(at);
+          const unsigned long long d = tc_ffma2(tc_pk(lo[set][2 * h], lo[set][2 * h + 1]), tc_pk(kRatio, kRatio), tc_pk(hi[set][2 * h], hi[set][2 * h + 1]));
+          const unsigned long long su = C::kTwo ? step_mul2(tc_pk(s.x, s.y), unit2[set]) : tc_pk(s.x, s.y);
+          if constexpr (AFFINE) {
+            const float2 b = two(at + C::kSbSlot);
+            a[h] = tc_ffma2(tc_pk(b.x, b.y), xs2[set], tc_ffma2(su, d, a[h]));
+          } else {
+            a[h] = tc_ffma2(su, tc_ffma2(tc_pk(-7.f, -7.f), xs2[set], d), a[h]);      // s * sum((q - 7) x)
+          }
+        }
     };
     if (cs.nkt == 1u) load_x(cs.ks);
 
@@ -435,9 +514,9 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
         for (int h = 0; h < 2; ++h) {
           const float2 v2 = tc_unpk(acc[q][h]);
           float v = v2.x + v2.y;
-          if constexpr (G > 2) v += __shfl_xor_sync(0xffffffffu, v, 1);
-          if constexpr (G > 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
-          if (c == 0u) mine[q * 16 + tr + 8u * h] = v * kUnit;
+          if constexpr (C::kTwo || G > 2) v += __shfl_xor_sync(0xffffffffu, v, 1);
+          if constexpr (C::kTwo || G > 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
+          if (c == 0u) mine[q * 16 + tr + 8u * h] = C::kTwo ? v : v * kUnit;
         }
       }
       __syncthreads();
@@ -521,7 +600,7 @@ cudaError_t launch_step_format(const StepProgram& p, bool al, size_t smem, int g
   if (p.n == 1) {
     StepProgramT<1> q;
     q.op[0] = p.op[0];
-    q.n = 1; q.off_part = p.off_part; q.off_x = p.off_x; q.off_xsum = p.off_xsum;
+    q.n = 1; q.x_bytes = p.x_bytes; q.off_part = p.off_part; q.off_x = p.off_x; q.off_xsum = p.off_xsum;
     q.counters = nullptr; q.status = p.status;
     return al ? launch_step_one<BITS, G32, AFFINE, true>(q, smem, grid, false, st) : launch_step_one<BITS, G32, AFFINE, false>(q, smem, grid, false, st);
   }
