@@ -25,6 +25,7 @@ def cancelling(seed, N, half, M, bits, group, symmetric):
 
 @pytest.mark.parametrize("bits,symmetric,half,M", [
     (4, True, 1536, 1), (4, True, 4096, 1), (4, True, 160, 1), (4, True, 1056, 1),    # groups of 32: whole and ragged slices
+    (4, False, 1088, 1), (4, False, 320, 1), (4, False, 3648, 1), (3, False, 1088, 1), (3, False, 320, 1), (3, False, 3648, 1),    # K % 256
 ])
 def test_sums_keep_f32(bits, symmetric, half, M, backend, dev):
     """Each result passes 2 K / group folds and a few more additions, each of which rounds by at most 2^-24 of a partial sum; their signs are
@@ -45,3 +46,26 @@ def test_sums_keep_f32(bits, symmetric, half, M, backend, dev):
     for y in ys:
         err = np.sqrt((dev.get(y).astype(np.float64) ** 2).mean())
         assert err <= bound, (err / size, bound / size)
+
+
+@pytest.mark.parametrize("K", [64, 320, 1600, 2112])
+@pytest.mark.parametrize("size", [2.0**-10, 2.0**-14, 2.0**-20])
+def test_small_activations_of_3_bit_rows(K, size, backend, dev, oracle_c):
+    """K % 256 != 0: f32 activations whatever their size. One rounding to f16: 2^-11 of the result, 2^-25 among the subnormals."""
+    rng = np.random.default_rng(K)
+    N = 777
+    _, W, s, b = z.synth.make_weights(rng, N, K, bits=3, sigma_s=0.02)
+    x = (z.synth.make_x(rng, 1, K) * np.float32(size)).astype(np.float16)
+    s, b = s * np.float16(8), b * np.float16(8)
+    ref = oracle_c.matmul_f64(x, W, s, b, 64, 3, True)
+    args = [dev.put(x), dev.put(s), dev.put(W), dev.put(b)]
+    ys = [dev.empty((1, N), np.float16, fill=9.0) for _ in range(3)]
+    backend.ctx.int4_matmul(z.MmDesc(K, N, 1, 64, 3, 1, 0), ys[0], *args)
+    backend.ctx.step_begin()
+    for y in ys[1:]:
+        backend.ctx.int4_matmul(z.MmDesc(K, N, 1, 64, 3, 1, 0), y, *args)
+    backend.ctx.step_end()
+    backend.ctx.sync()
+    for y in ys:
+        got = dev.get(y).astype(np.float64)
+        assert np.linalg.norm(got - ref) <= 2.0**-11 * np.linalg.norm(ref) + 2.0**-25 * np.sqrt(N)

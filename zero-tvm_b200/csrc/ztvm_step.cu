@@ -121,6 +121,8 @@ bool StepBuilder::add(const GemvParams& g, int bits, int sm_count) {
   o.K = g.K; o.KP = g.KP; o.spr = g.SPR;
   o.slices = (g.K + slice_codes(format) - 1) / slice_codes(format);
   step_split(&o);
+  // (one kernel for all of a run, and a matmul's sums are the same in every run)
+  if (i && step_two_parts(bits, sym32, op_aligned(o, format)) != step_two_parts(bits, sym32, op_aligned(p.op[0], format))) return false;
   auto span = [](const void* q, uint64_t bytes) { return Span{reinterpret_cast<uintptr_t>(q), reinterpret_cast<uintptr_t>(q) + bytes}; };
   x_[i] = span(g.X, (uint64_t)g.K * 2);
   y_[i] = span(g.Y, (uint64_t)g.N * 2);

@@ -14,7 +14,7 @@ constexpr int kStepMaxOps = 64;
 // serve a matmul by itself. Error of the f32 sums against 64 bits, relative, N(0, 1) activations / a few large ones among small: groups of
 // 32, 3000 x 3072, f32 FMAs 0.96e-7 / 1.8e-7, one part 6.5e-7 / 39e-7, two 0.90e-7 / 1.5e-7. Decode of 8 layers, hidden 3072: 241 us on
 // the FMAs, 195 with one part, 218 with two.
-constexpr bool step_two_parts(int bits, bool g32, bool al) { (void)al; return bits == 4 && g32; }
+constexpr bool step_two_parts(int bits, bool g32, bool al) { return bits != 8 && (g32 || !al); }
 
 struct alignas(16) StepOp {
   const uint32_t* W;
