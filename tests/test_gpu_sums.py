@@ -69,3 +69,17 @@ def test_small_activations_of_3_bit_rows(K, size, backend, dev, oracle_c):
     for y in ys:
         got = dev.get(y).astype(np.float64)
         assert np.linalg.norm(got - ref) <= 2.0**-11 * np.linalg.norm(ref) + 2.0**-25 * np.sqrt(N)
+
+
+@pytest.mark.parametrize("symmetric,N,K", [(False, 60000, 320), (False, 9000, 2112), (False, 1200, 9024), (True, 60000, 320), (True, 4096, 8192), (True, 1200, 9024)])
+def test_single_rows_round_the_f32_result(symmetric, N, K, backend, dev):
+    """4-bit rows of K % 256 != 0 or groups of 32 by themselves: one kernel whatever the result's type, so f16 results are the f32 ones rounded."""
+    rng = np.random.default_rng(N + K)
+    group = 32 if symmetric else 64
+    _, W, s, b = z.synth.make_weights(rng, N, K, group=group, affine=not symmetric)
+    args = [dev.put(z.synth.make_x(rng, 1, K)), dev.put(s), dev.put(W), None if symmetric else dev.put(b)]
+    y16, y32 = dev.empty((1, N), np.float16, fill=9.0), dev.empty((1, N), np.float32, fill=9.0)
+    backend.ctx.int4_matmul(z.MmDesc(K, N, 1, group, 4, int(not symmetric), 0), y16, *args)
+    backend.ctx.int4_matmul(z.MmDesc(K, N, 1, group, 4, int(not symmetric), 1), y32, *args)
+    backend.ctx.sync()
+    assert (dev.get(y16) == dev.get(y32).astype(np.float16)).all()

@@ -360,7 +360,7 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
     p.Y = d->out_f32 ? static_cast<void*>(static_cast<float*>(y) + (size_t)m0 * d->N)
                      : static_cast<void*>(static_cast<__half*>(y) + (size_t)m0 * d->N);
     const bool want_tc = ctx->gemv_path == 0 || (ctx->gemv_path == 3 && dd.M > 1);
-    if (d->M == 1 && ctx->gemv_path == 0 && ztvm::step_alone_faster((int)d->bits, d->affine != 0, d->N, d->K) &&
+    if (d->M == 1 && ctx->gemv_path == 0 && ztvm::step_alone_faster((int)d->bits, d->affine != 0, d->N, d->K, ctx->sm_count) &&
         ctx->step->add(p, (int)d->bits, ctx->sm_count)) {      // (nothing is held back here)
       const cudaError_t e = ctx->step->launch(nullptr, ctx->err_counter + 1, ctx->sm_count, st);
       ctx->step->clear();

@@ -45,14 +45,18 @@ bool all_aligned(const StepProgram& p, int format) {
 
 }  // namespace
 
-// A launch of its own has nothing to join. Calls one by one, us, here against the kernels for one projection:
-//   8-bit: everywhere (4096 x 4096 6.1 : 7.0, 14717 x 5056 16.7 : 21.4, 1200 x 9024 8.5 : 12.0)
-//   3-bit: everywhere (4096 x 4096 5.3 : 5.8, 3000 x 1600 4.1 : 6.2, 14717 x 5056 16.1 : 26.7; 9216 x 3072 6.45 : 6.31)
-//   4-bit: long K, which those take in K tiles with a meeting each (1200 x 9024 9.1 : 11.1, 12000 x 8000 18.0 : 19.7, 4096 x 12288 10.1 :
-//     11.4; 14717 x 5056 14.1 : 13.2), and with biases small ones (4096 x 4096 5.1 : 5.4, 8192 x 2048 4.4 : 5.2; 9216 x 3072 6.4 : 6.1;
-//     groups of 32 8192 x 2048 4.8 : 4.1)
-bool step_alone_faster(int bits, bool affine, uint32_t N, uint32_t K) {
-  return bits != 4 || K >= 7168u || (affine && (uint64_t)N * K <= (20u << 20));
+// A launch of its own has nothing to join. Calls one after the other, us, here against the kernels for one projection:
+//   8-bit: everywhere (4096 x 4096 5.7 : 6.8, 12000 x 7936 19.4 : 22.5, 1200 x 9024 8.2 : 12.0, 1000 x 576 2.7 : 2.6)
+//   3-bit over whole slices: everywhere (1024 x 1024 3.0 : 3.5, 4096 x 4096 5.1 : 5.6, 12000 x 7936 16.3 : 16.8)
+//   4-bit with biases, whole slices: long K, which those take in K tiles with a meeting each (1200 x 8960 8.0 : 8.6, 2048 x 12288 7.1 : 9.1),
+//     and small ones (4096 x 4096 4.8 : 5.3, 1024 x 4096 3.5 : 4.0; dispatched from Python, 8192 x 2048 4.3 : 5.2; 9216 x 3072 6.4 : 6.1)
+//   3-bit in two parts: from a second tile of rows per SM on (3000 x 1600 4.3 : 4.6, 9000 x 2112 7.0 : 10.3, 3072 x 8256 14.7 : 19.9; 1000 x 576
+//     3.6 : 2.4, 2048 x 4160 7.6 : 7.5, 512 x 12352 14.1 : 13.3)
+//   4-bit in two parts: nowhere by much. K % 256: 1000 x 576 3.0 : 2.1, 9000 x 2112 6.0 : 5.4, 3072 x 8256 11.6 : 8.1, 12000 x 8000 17.7 : 18.8;
+//     groups of 32: 8192 x 2048 4.8 : 3.8, 3072 x 8192 7.7 : 7.0, 3072 x 8256 13.2 : 8.0, 4096 x 12288 10.5 : 10.7
+bool step_alone_faster(int bits, bool affine, uint32_t N, uint32_t K, int sm_count) {
+  if (step_two_parts(bits, !affine, K % 256u == 0)) return bits == 3 && N > 16u * (uint32_t)sm_count;
+  return bits != 4 || K >= 7168u || (uint64_t)N * K <= (20u << 20);
 }
 
 bool StepBuilder::waits() const {

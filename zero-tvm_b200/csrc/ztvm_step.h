@@ -69,7 +69,7 @@ class StepBuilder {
 };
 
 // Whether a one-row matmul that no run takes is faster here than on the kernels for one projection.
-bool step_alone_faster(int bits, bool affine, uint32_t N, uint32_t K);
+bool step_alone_faster(int bits, bool affine, uint32_t N, uint32_t K, int sm_count);
 
 cudaError_t launch_step_w4(const StepProgram& p, bool al, size_t smem, int grid, bool together, cudaStream_t st);
 cudaError_t launch_step_w4g32(const StepProgram& p, bool al, size_t smem, int grid, bool together, cudaStream_t st);
