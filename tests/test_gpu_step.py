@@ -160,3 +160,41 @@ def test_two_captured_steps_replay_side_by_side(backend, dev):
     for st, want, _ in steps:
         assert all(torch.equal(v, want[k]) for k, v in st.bufs.items())
     assert backend.ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("bits,symmetric", FORMATS)
+def test_other_calls_inside_a_step(bits, symmetric, backend, dev, oracle_c):
+    """A step on the context's own stream: calls that are made of a matmul have its result when they go on, and find what was called before
+    them done."""
+    import torch
+    rng = np.random.default_rng(bits)
+    K, N, group, ctx = 576, 300, 32 if symmetric else 64, backend.ctx
+    W, s, b = z.synth.make_weights(rng, N, K, bits=bits, group=group, affine=not symmetric)[1:]
+    W2, s2, b2 = z.synth.make_weights(rng, K, 320, bits=bits, group=group, affine=not symmetric)[1:]
+    desc, feed = z.MmDesc(K, N, 1, group, bits, int(not symmetric), 0), z.MmDesc(320, K, 1, group, bits, int(not symmetric), 0)
+    w = [dev.put(s), dev.put(W), None if symmetric else dev.put(b)]
+    w2 = [dev.put(s2), dev.put(W2), None if symmetric else dev.put(b2)]
+    xs = [z.synth.make_x(rng, 1, K) for _ in range(3)]
+    want = [oracle_c.matmul_f64(x, W, s, b, group, bits, not symmetric) for x in xs]
+    x0 = z.synth.make_x(rng, 1, 320)
+    got = [np.full((1, N), 7, np.float16) for _ in range(2)]
+    pinned = torch.full((1, N), 7, dtype=torch.float16).pin_memory()
+    dx, d0, mid, y, h = dev.put(xs[2]), dev.put(x0), dev.empty((1, K), np.float16), dev.empty((1, N), np.float16), dev.empty((1, N // 2), np.float16, fill=0.0)
+    ctx.step_begin()
+    try:
+        ctx.int4_matmul(desc, y, dx, *w)                       # held back
+        ctx.int4_matmul_host(desc, got[0], xs[0], *w)
+        ctx.int4_matmul(feed, mid, d0, *w2)                    # held back
+        ctx.int4_matmul_host(desc, got[1], xs[1], *w)
+        ctx.int4_matmul_host_async(desc, pinned, torch.from_numpy(xs[2]).pin_memory(), *w)
+        ctx.host_wait()
+        ctx.int4_matmul(desc, y, dx, *w)                       # held back
+        ctx.fused_ffn(z.MmDesc(K, N // 2, 1, group, bits, int(not symmetric), 0), h, dx, *w)
+    finally:
+        ctx.step_end()
+    ctx.sync()
+    for out, ref in zip(got + [pinned.numpy(), dev.get(y)], want + [want[2]]):
+        assert zo.rel_err_scaled(out.astype(np.float64), ref, 1e-3) < 2e-3
+    assert zo.rel_err_scaled(dev.get(mid).astype(np.float64), oracle_c.matmul_f64(x0, W2, s2, b2, group, bits, not symmetric), 1e-3) < 2e-3
+    gate, up = want[2][:, :N // 2], want[2][:, N // 2:]
+    assert zo.rel_err_scaled(dev.get(h).astype(np.float64), up * gate / (1 + np.exp(-gate)), 1e-2) < 4e-3

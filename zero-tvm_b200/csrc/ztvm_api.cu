@@ -306,25 +306,16 @@ ztvm_status ztvm_step_begin(ztvm_ctx* ctx, void* stream) {
 
 ztvm_status ztvm_step_end(ztvm_ctx* ctx) {
   ztvm_status s = check_ctx(ctx);           // launches what is held back
-  if (ctx && ctx->magic == kMagic) ctx->step_on = 0;
+  if (ctx && ctx->magic == kMagic) {
+    ctx->step->clear();                     // (a check that failed before the launch leaves it there)
+    ctx->step_on = 0;
+  }
   return s;
 }
 
-ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, const void* x, const void* scales,
-                             const void* packed_w, const void* biases, void* stream) {
-  ztvm_status s = check_ctx(ctx, true);
-  if (s) return s;
-  if ((s = check_desc(d, true))) return s;
-  if ((s = check_buffers(d, y, x, scales, packed_w, biases))) return s;
-  cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  if (ctx->step_on) {
-    const bool join = d->M == 1 && st == ctx->step_stream && ctx->gemv_path == 0;
-    ztvm::GemvParams p;
-    if (join) p = gemv_params(ctx, d, y, x, scales, packed_w, biases);
-    if (join && ctx->step->add(p, (int)d->bits, ctx->sm_count)) return ZTVM_OK;
-    if ((s = step_flush(ctx))) return s;
-    if (join && ctx->step->add(p, (int)d->bits, ctx->sm_count)) return ZTVM_OK;
-  }
+// ztvm_int4_matmul of checked arguments, never held back: nothing is, at this point.
+static ztvm_status matmul_now(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, const void* x, const void* scales, const void* packed_w,
+                              const void* biases, cudaStream_t st) {
   // Up to 16 rows the GEMV in slabs of eight: exact codes and f32 weights, the reference's choice for short chunks (runtime-M
   // matvec; its GEMMs start at 64 rows). From 17 on a third slab costs more than the GEMM at every width. Weight sets from HBM,
   // GEMM against slabs, us: 8192 x 2048 9.8 : 11.1 at 16 rows, 10.1 : 15.8 at 17; 24576 x 4096 40.7 : 34.2 and 40.8 : 48.0;
@@ -374,6 +365,33 @@ ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, cons
   half.now = half.before;
   half_after(ctx, half, st);
   return ZTVM_OK;
+}
+// The same as part of another call, which goes on with the result.
+static ztvm_status matmul_inside(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, const void* x, const void* scales, const void* packed_w,
+                                 const void* biases, cudaStream_t st) {
+  ctx->last = ctx->call;
+  ctx->call.half = 0;
+  ztvm_status s = check_desc(d, true);
+  if (!s) s = check_buffers(d, y, x, scales, packed_w, biases);
+  return s ? s : matmul_now(ctx, d, y, x, scales, packed_w, biases, st);
+}
+
+ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, const void* x, const void* scales,
+                             const void* packed_w, const void* biases, void* stream) {
+  ztvm_status s = check_ctx(ctx, true);
+  if (s) return s;
+  if ((s = check_desc(d, true))) return s;
+  if ((s = check_buffers(d, y, x, scales, packed_w, biases))) return s;
+  cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  if (ctx->step_on) {
+    const bool join = d->M == 1 && st == ctx->step_stream && ctx->gemv_path == 0;
+    ztvm::GemvParams p;
+    if (join) p = gemv_params(ctx, d, y, x, scales, packed_w, biases);
+    if (join && ctx->step->add(p, (int)d->bits, ctx->sm_count)) return ZTVM_OK;
+    if ((s = step_flush(ctx))) return s;
+    if (join && ctx->step->add(p, (int)d->bits, ctx->sm_count)) return ZTVM_OK;
+  }
+  return matmul_now(ctx, d, y, x, scales, packed_w, biases, st);
 }
 
 ztvm_status ztvm_peer_barrier(ztvm_ctx* ctx, uint32_t* const* flags, uint32_t world, uint32_t rank, void* stream) {
@@ -471,7 +489,7 @@ ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* h, const 
   ztvm::WorkBuf* rows = nullptr;
   ZTVM_CUDA(ctx->work->get(ztvm::WorkBufs::kFfnRows, need, st, &rows));
   gu.out_f32 = 1;
-  if ((s = ztvm_int4_matmul(ctx, &gu, rows->p, x, scales, packed_w, biases, st))) return s;
+  if ((s = matmul_inside(ctx, &gu, rows->p, x, scales, packed_w, biases, st))) return s;
   ZTVM_CUDA(ztvm::launch_silu_mul_f32(static_cast<const float*>(rows->p), static_cast<__half*>(h), d->M, d->N, st));
   return ZTVM_OK;
 }
@@ -498,7 +516,7 @@ ztvm_status ztvm_moe_router_logits(ztvm_ctx* ctx, uint32_t D, uint32_t rows, uin
   if ((s = check_buffers(&d, logits, x, scales, w, biases))) return s;
   const int keep = ctx->no_gemm;
   ctx->no_gemm = 1;
-  s = ztvm_int4_matmul(ctx, &d, logits, x, scales, w, biases, st);
+  s = matmul_inside(ctx, &d, logits, x, scales, w, biases, st);
   ctx->no_gemm = keep;
   return s;
 }
@@ -567,7 +585,7 @@ ztvm_status ztvm_int4_matmul_host(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y_
   if (!x_pinned) { memcpy(hp, x_host, xb); x_src = hp; }
   void* y_dst = y_pinned ? y_host : static_cast<void*>(hp + (x_pinned ? 0 : xb));
   ZTVM_CUDA(cudaMemcpyAsync(ctx->d_x, x_src, xb, cudaMemcpyHostToDevice, ctx->stream));
-  if ((s = ztvm_int4_matmul(ctx, d, ctx->d_y, ctx->d_x, scales, packed_w, biases, ctx->stream))) return s;
+  if ((s = matmul_inside(ctx, d, ctx->d_y, ctx->d_x, scales, packed_w, biases, ctx->stream))) return s;
   ZTVM_CUDA(cudaMemcpyAsync(y_dst, ctx->d_y, yb, cudaMemcpyDeviceToHost, ctx->stream));
   ZTVM_CUDA(cudaStreamSynchronize(ctx->stream));
   if (!y_pinned) memcpy(y_host, y_dst, yb);
@@ -595,7 +613,7 @@ ztvm_status ztvm_int4_matmul_host_async(ztvm_ctx* ctx, const ztvm_mm_desc* d, vo
     if ((s = grow(&l.d_y, &l.d_y_bytes, yb, false))) return s;
   }
   ZTVM_CUDA(cudaMemcpyAsync(l.d_x, x_host, xb, cudaMemcpyHostToDevice, l.stream));
-  if ((s = ztvm_int4_matmul(ctx, d, l.d_y, l.d_x, scales, packed_w, biases, l.stream))) return s;
+  if ((s = matmul_inside(ctx, d, l.d_y, l.d_x, scales, packed_w, biases, l.stream))) return s;
   ZTVM_CUDA(cudaMemcpyAsync(y_host, l.d_y, yb, cudaMemcpyDeviceToHost, l.stream));
   return ZTVM_OK;
 }
