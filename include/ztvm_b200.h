@@ -97,8 +97,8 @@ typedef struct ztvm_mm_desc {
  * src/zero-tvm/engine-core.ts:2290, :2312, :2517-2519, :2543-2549, :4280-4293).
  * M <= 8 runs the bandwidth-bound GEMV, M <= 16 two slabs of it; larger M of 4-bit weights runs the tensor-core GEMM (which
  * multiplies f16-rounded weights f16(s*q+b), like the reference's matrix-unit GEMMs). 8-bit weights are not rounded at any M:
- * f16 results of more than 32 rows run on the same GEMM with two f16 terms per weight (y 16-byte aligned, K >= 1536 or much work), f32
- * results and other calls of more than eight rows on a batched kernel that multiplies the codes (groups of 64), others as slabs; 3-bit ones run as slabs. */
+ * f16 results of more than 32 rows run on the tensor cores with exact codes and f32 folds of the scale groups (y 16-byte aligned, K >= 1536 or much work), f32
+ * results and other calls of more than eight rows on a batched kernel that does the same (groups of 64), others as slabs; 3-bit ones run as slabs. */
 ZTVM_API ztvm_status ztvm_int4_matmul(ztvm_ctx* ctx, const ztvm_mm_desc* desc, void* y, const void* x,
                              const void* scales, const void* packed_w, const void* biases, void* stream);
 

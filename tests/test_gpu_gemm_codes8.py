@@ -1,4 +1,4 @@
-"""Prefill GEMM on 8-bit weights: two f16 terms per weight lose nothing that an f16 result shows, whatever the size of the scales."""
+"""Prefill GEMM on 8-bit weights: exact codes, f32 folds of the scale groups, whatever the size of the scales."""
 import numpy as np
 import pytest
 
@@ -10,12 +10,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,N,K,size", [
-    (33, 128, 64, 1.0), (64, 129, 576, 1.0), (65, 2048, 2112, 1.0), (33, 128, 1536, 1.0), (40, 300, 1600, 2.0**-17), (40, 300, 1536, 2.0**12), (130, 300, 1728, 0.0),        # tile widths, a last slot of one block, K shares in a cluster
-    (128, 1000, 1152, 1.0), (129, 257, 320, 1.0), (200, 3072, 2048, 1.0), (256, 130, 192, 1.0), (257, 20001, 128, 1.0), (700, 136, 4160, 1.0),
-    (40, 300, 512, 2.0**-17), (40, 300, 512, 2.0**13), (40, 300, 64, 0.0),   # scales among f16's subnormals, weights past f16's largest
+    (33, 128, 1536, 1.0), (64, 129, 1600, 1.0), (65, 2048, 2112, 1.0), (47, 1, 1664, 1.0), (33, 17, 6144, 1.0),    # token tiles, K shares, rows past N
+    (129, 257, 1728, 1.0), (200, 3072, 2048, 1.0), (128, 1000, 6144, 1.0), (700, 136, 4160, 1.0),                  # SPR % 4 of 0 to 3, last slots of 1 to 4 blocks
+    (257, 20001, 128, 1.0), (1000, 10000, 64, 1.0), (513, 20000, 192, 1.0), (330, 8200, 320, 1.0),                # fewer blocks than teams, and few more
+    (40, 300, 1600, 2.0**-17), (40, 300, 1536, 2.0**12), (130, 300, 1728, 0.0),                                   # scales among f16's subnormals, weights past f16's largest, none
 ])
-def test_two_terms(M, N, K, size, backend, dev, oracle_c):
-    """(Those of little work over a short K run on the kernel that multiplies the codes: the same bound.)"""
+def test_codes(M, N, K, size, backend, dev, oracle_c):
     p = z.synth.projection(N, K, M=M, bits=8, seed=M + N, sigma_s=0.01 / 17)
     rng = np.random.default_rng(K)
     s, b = p["scales"].astype(np.float32), p["biases"].astype(np.float32)
@@ -34,9 +34,7 @@ def test_two_terms(M, N, K, size, backend, dev, oracle_c):
     assert np.isfinite(got).all() and np.abs(ref).max() < 65504
     record_parity(zo.rel_err_scaled(got, ref, 1e-3), zo.rel_err(got, ref))
     mags = oracle_c.matmul_f64(np.abs(x), p["W"][rows], s[rows], np.abs(b[rows]), 64, 8, True)
-    # one rounding to f16 (2^-11, absolute 2^-25); the weight as f32 and its two terms 2^-22 of |s q + b| <= the terms of `mags`; the matrix
-    # unit drops bits below 2^-23 of the largest partial sum once per 16 products, of either term; row bound 2^-39 of the row's largest
-    # possible weight (255 s + |b|) per product
-    top = np.max(255 * np.abs(s[rows].astype(np.float64)) + np.abs(b[rows].astype(np.float64)), axis=1)
-    bound = 2.0**-11 * np.abs(ref) + 2.0**-25 + (2 * K / 16 + 6) * 2.0**-23 * mags + 2.0**-38 * top[None, :] * np.abs(x).astype(np.float64).sum(1)[:, None]
+    # one rounding to f16 (2^-11, absolute 2^-25) of f32 sums: the matrix unit drops bits below 2^-23 of the largest partial sum once per 16
+    # products, the folds and the meetings of teams and K shares round three more times per 64 codes
+    bound = 2.0**-11 * np.abs(ref) + 2.0**-25 + 1.001 * (K / 16 + 3 * K / 64 + 12) * 2.0**-23 * mags
     assert (np.abs(got - ref) <= bound).all()

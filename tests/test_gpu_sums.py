@@ -25,15 +25,16 @@ def cancelling(seed, N, half, M, bits, group, symmetric):
 
 @pytest.mark.parametrize("bits,symmetric,half,M", [
     (4, True, 1536, 1), (4, True, 4096, 1), (4, True, 160, 1), (4, True, 1056, 1),    # groups of 32: whole and ragged slices
+    (8, False, 1024, 40), (8, False, 3072, 33), (8, False, 3072, 200), (8, False, 1088, 130),     # 8-bit prompts: token tiles, K shares
     (4, False, 1088, 1), (4, False, 320, 1), (4, False, 3648, 1), (3, False, 1088, 1), (3, False, 320, 1), (3, False, 3648, 1),    # K % 256
 ])
 def test_sums_keep_f32(bits, symmetric, half, M, backend, dev):
-    """Each result passes 2 K / group folds and a few more additions, each of which rounds by at most 2^-24 of a partial sum; their signs are
-    as good as random, and a partial sum is about as large as the terms' 2-norm. By itself, and joined with another in a step."""
+    """Each result passes 2 K / group folds and a few more additions, each of which rounds by at most 2^-24 of a partial sum, evenly spread;
+    a partial sum is about as large as the terms' 2-norm. By itself, and joined with another in a step."""
     group, N = 32 if symmetric else 64, 1100
     x, W, s, b, size = cancelling(half + M, N, half, M, bits, group, symmetric)
     K = 2 * half
-    bound = np.sqrt(2 * K / group + 32) * 2.0**-24 * size + 2.0**-25                   # (f16 spacing near zero)
+    bound = np.sqrt((2 * K / group + 32) / 3) * 2.0**-24 * size + 2.0**-25                   # (f16 spacing near zero)
     args = [dev.put(x), dev.put(s), dev.put(W), None if b is None else dev.put(b)]
     desc = z.MmDesc(K, N, M, group, bits, int(not symmetric), 0)
     ys = [dev.empty((M, N), np.float16, fill=9.0) for _ in range(3)]
@@ -46,6 +47,18 @@ def test_sums_keep_f32(bits, symmetric, half, M, backend, dev):
     for y in ys:
         err = np.sqrt((dev.get(y).astype(np.float64) ** 2).mean())
         assert err <= bound, (err / size, bound / size)
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 5000, 6144), (40, 25000, 4096)])
+def test_sums_of_8_bit_prompts_lean_nowhere(M, N, K, backend, dev, oracle_c):
+    """Sums that a matrix unit truncates over the whole of K come out too small. Here it has the 64 terms of a group, four truncations by 2^-24
+    of a sum, and the rounding to f16, evenly spread within 2^-11, averages out: four standard deviations of a mean."""
+    p = z.synth.projection(N, K, M=M, bits=8, seed=K, sigma_s=0.01 / 17)
+    y = dev.empty((M, N), np.float16, fill=9.0)
+    backend.ctx.int4_matmul(z.MmDesc(K, N, M, 64, 8, 1, 0), y, dev.put(p["x"]), dev.put(p["scales"]), dev.put(p["W"]), dev.put(p["biases"]))
+    ref = oracle_c.matmul_f64(p["x"], p["W"], p["scales"], p["biases"], 64, 8, True)
+    lean = (np.sign(ref) * (dev.get(y) - ref)).sum() / np.abs(ref).sum()
+    assert abs(lean) <= 4 * 2.0**-24 + 4 * 2.0**-11 / np.sqrt(3 * M * N)
 
 
 @pytest.mark.parametrize("K", [64, 320, 1600, 2112])

@@ -320,12 +320,12 @@ static ztvm_status matmul_now(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, con
   // matvec; its GEMMs start at 64 rows). From 17 on a third slab costs more than the GEMM at every width. Weight sets from HBM,
   // GEMM against slabs, us: 8192 x 2048 9.8 : 11.1 at 16 rows, 10.1 : 15.8 at 17; 24576 x 4096 40.7 : 34.2 and 40.8 : 48.0;
   // 4096 x 12288 18.6 : 24.2 and 19.0 : 35.6. (The GEMM is ahead at 9..16 rows too where K is long, but rounds the weights to f16.)
-  // 8-bit weights go as two f16 terms each, exact to 2^-22; f32 results (router logits) stay with the exact-code kernel below, and so
-  // do up to 32 rows, one token tile of it, and small matmuls over a short K, its serial part, us, GEMM against it: 12288 x 2048 18 : 14 at
-  // 24 rows, 17.3 : 26 at 40; 2048 x 6144 15 : 30 at 40; 2048 x 2048 9.2 : 10.9 at 33; 1536 x 1088 10.2 : 7.0 at 40, 10.5 : 9.6 at 200, 12.4 :
-  // 25.7 at 1000.
-  const bool two_terms = d->bits == 8 && d->M > 32 && (d->K >= 1536 || (uint64_t)d->M * d->N * d->K > 400000000ull) && d->affine && !d->out_f32 && aligned(y, 16);
-  if (d->M > 16 && (d->bits == 4 || two_terms) && ztvm::gemm_ta_supported((int)d->bits, d->group, d->K) && !ctx->no_gemm) {
+  // 8-bit weights go as exact codes, with f32 folds, like in the batched kernel below. f32 results (router logits) stay with that one, and so
+  // do up to 32 rows, one token tile of it, and small matmuls over a short K, its serial part, us, GEMM against it: 12288 x 2048 17.5 : 25.8 at
+  // 33 rows, 33.6 : 31.5 at 77, 51.7 : 80.6 at 200; 2048 x 6144 14.1 : 30.1 at 33; 2048 x 2048 9.2 : 11.0 at 33; 1536 x 1088 11.1 : 10.0 at 256,
+  // 12.3 : 16.3 at 500.
+  const bool codes8 = d->bits == 8 && d->M > 32 && (d->K >= 1536 || (uint64_t)d->M * d->N * d->K > 600000000ull) && d->affine && !d->out_f32 && aligned(y, 16);
+  if (d->M > 16 && (d->bits == 4 || codes8) && ztvm::gemm_ta_supported((int)d->bits, d->group, d->K) && !ctx->no_gemm) {
     if (!aligned(y, 16)) return fail(ZTVM_ERR_ALIGNMENT, "y must be 16-byte aligned for the GEMM path");
     ZTVM_CUDA(ztvm::launch_gemm_ta(static_cast<const uint32_t*>(packed_w), static_cast<const __half*>(scales),
                                    d->affine ? static_cast<const __half*>(biases) : nullptr, static_cast<const __half*>(x), y, d->M, d->N, d->K,

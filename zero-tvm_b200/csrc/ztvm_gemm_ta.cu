@@ -1,4 +1,4 @@
-// Prefill GEMM, M > 16, 4-bit and 8-bit weights: y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS AS THE
+// Prefill GEMM, M > 16, 4-bit weights: y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS (8-bit ones: codes) AS THE
 // A OPERAND IN TENSOR MEMORY (replaces the matrix-unit GEMMs of int4_matmul.gen.ts:1058-1456; contract of
 // ztvm_int4_matmul for M > 16). W16 = f16_rne(fl32(s * q + b)) (or s * (q - 7)), the value the reference's numpy
 // dequantiser produces (scripts/make-dsv2-layer-ref.py:108-116); f32 accumulation in tensor memory.
@@ -22,11 +22,14 @@
 // per clock of shared memory, beside a fixed 0.18 us that wider tiles have less often. 24576 x 4096, 1024 tokens: 172 us
 // with tiles of 256, 154 us; 6144 x 4096 (192 tiles of 256 on 148 SMs, 144 of 352): 54, 38 us.
 //
-// 8-bit weights (int8_affine_batched.wgsl multiplies them as f32) are two f16 terms in two slices and two MMAs each: w = hi + lo holds a
-// weight to 2^-22. Stored times a power of two per row, from a scan of the row's scales and biases while the first copies fly, so
-// that neither large nor tiny scales cost anything. 200 tokens, us, against the
-// warp-level matrix unit with exact codes (ztvm_batch_mma.cu): 3072 x 2048 14.0 : 26.1, 12288 x 2048 23.2 : 80.5, 2048 x 6144 21.6 : 44.6; 1000
-// tokens 12288 x 2048 84 : 267.
+// 8-bit weights (int8_affine_batched.wgsl multiplies them as f32) may not be rounded, and the MMA truncates its sums (over a K of 6144 3.6e-6
+// of the result, all one way). So the slices hold the codes, which f16 has exactly; a k block is one scale group, summed in an
+// accumulator of its own and folded in f32 registers, sum += s * acc + b * sum(x): 1.1e-7, as on the warp-level matrix unit (ztvm_batch_mma.cu),
+// 1.4e-7. Each of the four teams has its slice, accumulator, sums of activations and f32 sums for itself; they meet at the end.
+// Tiles of up to 64 tokens: what bounds them is issue slots (two FMAs and a load per row, token and group, 86 % of the slots of an SM that
+// has a tile) at 0.41 to 0.44 us a block. With one accumulator ring for all teams (tiles of 128) every warp waited for every block: 0.5 and
+// 0.97 us at 64 and 128 tokens. us against that kernel, 200 tokens: 3072 x 2048 18.1 : 26.4, 12288 x 2048 51.7 : 80.6, 2048 x 6144 28.2 : 44.7; 1000
+// tokens 12288 x 2048 196 : 267.
 //
 // Few tiles (short prompts, small N): the K range is split over a cluster of CTAs. Each CTA keeps the k blocks of its
 // share; at the end every CTA sends its f32 partial sums of token slice j to CTA j through distributed shared memory, and
@@ -63,12 +66,14 @@ struct GemmTaSmem {
   static constexpr int kXBytes = NT * kGemmBK * 2;            // per stage
   static constexpr int kWBytes = kTaRows * 32 * BITS;         // per packed-weight slot: four k blocks, in boxes of 128 bytes a row
   // the widest tile leaves room for two packed-weight slots and for one table of groups of 32 or two of wider groups
-  static constexpr int kWStages = NT > 256 || (BITS == 8 && NT > 128) ? 2 : 3;
+  static constexpr int kWStages = NT > 256 ? 2 : BITS == 8 ? 4 : 3;
   static constexpr int kSbBytes = NT > 256 ? 2 * kTaRows * 24 : 2 * kTaRows * kTaSbMaxPitch;
   static constexpr int kOffW = kTaStages * kXBytes;
   static constexpr int kOffSb = kOffW + kWStages * kWBytes;
   static constexpr int kOffBar = kOffSb + kTaSbStages * kSbBytes;
-  static constexpr int kTotal = kOffBar + 256 + (BITS == 8 ? 4 * kTaRows * 4 : 0);     // (8-bit: bounds of the rows' weights)
+  static constexpr int kOffXsum = kOffBar + 256;              // 8-bit: sums of a block's activations per token, two rounds of the stages
+  static constexpr int kTotal = kOffXsum + (BITS == 8 ? 2 * kTaStages * NT * 4 : 0);
+  static constexpr int kAccs = BITS == 8 ? kTaStages : 1;     // accumulators: 8-bit blocks have one each
 };
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
@@ -77,48 +82,29 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
                : "r"(taddr) : "memory");
 }
 
-// 8-bit weights may not be rounded to f16: two f16 terms each, w = hi + lo, and two MMAs.
-// Bound of a row's weights from a quarter of its groups: max |s| * 255 + |b|. Tables start on 8-byte boundaries.
-__device__ __forceinline__ float ta_row_bound(const GemmTaParams& p, uint32_t row, uint32_t quarter) {
-  float top = 0.f;
-  const __half *const s = p.S + (size_t)row * p.SPR, *const b = p.B + (size_t)row * p.SPR;
-  auto see = [&](__half sv, __half bv) { top = fmaxf(top, fmaf(255.f, fabsf(__half2float(sv)), fabsf(__half2float(bv)))); };
-  if ((p.SPR & 3u) == 0u) {                                  // four groups per load: 96 groups in one latency
-    const uint32_t fours = p.SPR / 4u, end = (quarter + 1u) * fours / 4u;
-#pragma unroll 8
-    for (uint32_t g = quarter * fours / 4u; g < end; ++g) {
-      const uint2 sv = __ldg(reinterpret_cast<const uint2*>(s) + g), bv = __ldg(reinterpret_cast<const uint2*>(b) + g);
-      see(__low2half(u32_as_h2(sv.x)), __low2half(u32_as_h2(bv.x))); see(__high2half(u32_as_h2(sv.x)), __high2half(u32_as_h2(bv.x)));
-      see(__low2half(u32_as_h2(sv.y)), __low2half(u32_as_h2(bv.y))); see(__high2half(u32_as_h2(sv.y)), __high2half(u32_as_h2(bv.y)));
-    }
-  } else {
-    const uint32_t end = (quarter + 1u) * p.SPR / 4u;
-#pragma unroll 8
-    for (uint32_t g = quarter * p.SPR / 4u; g < end; ++g) see(__ldg(s + g), __ldg(b + g));
-  }
-  return top;
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                 "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+               : "r"(taddr) : "memory");
 }
-// The power of two by which a row's weights are stored: top * unit < 2^15.
-__device__ __forceinline__ float ta_row_unit(float top) {
-  const uint32_t e = __float_as_uint(top) >> 23;             // top < 2^(e - 126); 0: all zeros
-  return __uint_as_float((e == 0u ? 127u : 127u + 141u - e) << 23);
+// two f32 at a time (fma.rn.f32x2)
+__device__ __forceinline__ unsigned long long ta_pk(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-// Sixteen codes: w = fl32(s q + b), hi = f16(w), lo = f16(w - hi).
-__device__ __forceinline__ void ta_terms8(const uint4& w, float s, float b, uint32_t* hi, uint32_t* lo) {
-  const uint32_t v[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      // a byte under the exponent of 2^23 is that many units above it
-      const float q0 = __uint_as_float(__byte_perm(v[i], 0x4B000000u, j ? 0x7442 : 0x7440)) - 8388608.f;
-      const float q1 = __uint_as_float(__byte_perm(v[i], 0x4B000000u, j ? 0x7443 : 0x7441)) - 8388608.f;
-      const float w0 = fmaf(s, q0, b), w1 = fmaf(s, q1, b);
-      const __half2 h = __floats2half2_rn(w0, w1);
-      const float2 f = __half22float2(h);
-      hi[2 * i + j] = h2_as_u32(h);
-      lo[2 * i + j] = h2_as_u32(__floats2half2_rn(w0 - f.x, w1 - f.y));
-    }
+__device__ __forceinline__ unsigned long long ta_ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// acc + the two halves of h
+__device__ __forceinline__ float ta_add2(float acc, uint32_t h) {
+  asm("{\n\t.reg .f16 a, b, one;\n\tmov.b16 one, 0x3C00;\n\tmov.b32 {a, b}, %1;\n\t"
+      "fma.rn.f32.f16 %0, a, one, %0;\n\tfma.rn.f32.f16 %0, b, one, %0;\n\t}" : "+f"(acc) : "r"(h));
+  return acc;
 }
 
 template <int NT, bool AFFINE, int BITS>
@@ -137,9 +123,12 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   auto bar_w_empty = [&](int s) { return bars + 8u * (2 * kTaStages + kTaWStages + s); };
   auto bar_sb_full = [&](int s) { return bars + 8u * (2 * kTaStages + 2 * kTaWStages + s); };
   auto bar_sb_empty = [&](int s) { return bars + 8u * (2 * kTaStages + 2 * kTaWStages + kTaSbStages + s); };
-  constexpr int kNumBars = 2 * kTaStages + 2 * kTaWStages + 2 * kTaSbStages + 1;
+  constexpr int kBarAccum = 2 * kTaStages + 2 * kTaWStages + 2 * kTaSbStages;
+  // 8-bit: activations landed (in `full` otherwise)
+  auto bar_x = [&](int s) { return BITS == 8 ? bars + 8u * (kBarAccum + 1 + s) : bars + 8u * s; };
+  constexpr int kNumBars = kBarAccum + 1 + (BITS == 8 ? kTaStages : 0);
   static_assert(8 * kNumBars + 8 <= 256, "barrier block");
-  const uint32_t bar_accum = bars + 8u * (kNumBars - 1);
+  const uint32_t bar_accum = bars + 8u * kBarAccum;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen_base + L::kOffBar + 8 * kNumBars);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
 
@@ -153,17 +142,16 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   const uint32_t kb_first = kz * units / split * kTaSbChunk;
   const uint32_t kb_last = kz + 1 == split ? all_kb : (kz + 1) * units / split * kTaSbChunk;
   const uint32_t num_kb = kb_last - kb_first;
-  constexpr uint32_t kColA = NT;                                 // weight slices start after the accumulator columns
-  constexpr uint32_t kACols = BITS == 8 ? 64 : 32;               // of a stage: 64 weights of a row as f16, 8-bit ones as two terms each
-  constexpr uint32_t kTmemCols = NT + kTaStages * kACols <= 256 ? 256 : 512;
-  static_assert(NT + kTaStages * kACols <= 512, "tensor memory");
+  constexpr uint32_t kColA = NT * L::kAccs;                      // weight slices start after the accumulator columns
+  constexpr uint32_t kTmemCols = kColA + kTaStages * 32 <= 256 ? 256 : 512;
+  static_assert(kColA + kTaStages * 32 <= 512, "tensor memory");
   const uint32_t nbox = mrows > p.box_rows ? 2u : 1u, box_bytes = p.box_rows * (uint32_t)(kGemmBK * 2);
 
   if (threadIdx.x == 32) { tma_prefetch_desc(&tmap_x); tma_prefetch_desc(&tmap_w); }
   auto load_x = [&](uint32_t s, uint32_t kb) {
-    mbar_arrive_expect_tx(bar_full((int)s), nbox * box_bytes);
+    mbar_arrive_expect_tx(bar_x((int)s), nbox * box_bytes);
     for (uint32_t b = 0; b < nbox; ++b)
-      tma_load_2d(x_ring + s * L::kXBytes + b * box_bytes, &tmap_x, bar_full((int)s), (int)((kb_first + kb) * kGemmBK), (int)(m0 + b * p.box_rows));
+      tma_load_2d(x_ring + s * L::kXBytes + b * box_bytes, &tmap_x, bar_x((int)s), (int)((kb_first + kb) * kGemmBK), (int)(m0 + b * p.box_rows));
   };
   auto load_w = [&](uint32_t s, uint32_t c) {
     mbar_arrive_expect_tx(bar_w_full((int)s), (uint32_t)L::kWBytes);
@@ -175,8 +163,10 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   // barrier: they fly while tensor memory is allocated.
   if (threadIdx.x == 0) {
     for (int s = 0; s < kTaStages; ++s) {
-      mbar_init(bar_full(s), 1 + kTaTeamWarps);   // the activation tile (with its byte count) + every warp of the team that writes the slice
-      mbar_init(bar_empty(s), 1);
+      // the activation tile (with its byte count) + every warp of the team that writes the slice
+      mbar_init(bar_full(s), BITS == 8 ? kTaTeamWarps : 1 + kTaTeamWarps);
+      if (BITS == 8) mbar_init(bar_x(s), 1);
+      mbar_init(bar_empty(s), BITS == 8 ? 2 : 1);
     }
     for (int s = 0; s < kTaSbStages; ++s) {
       mbar_init(bar_sb_full(s), 32);
@@ -236,7 +226,6 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
   const bool is_dq = warp >= 3 && warp < 3 + kTaDqWarps;
   bool acc_ok = false;
-  [[maybe_unused]] float unscale = 1.f;               // 8-bit: results are sums of stored weights
 
   if (warp == 0) {
     // ================= TMA producer: activations =================
@@ -253,7 +242,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const uint32_t first = issued > (uint32_t)kTaStages ? issued - kTaStages : 0u;
         for (uint32_t kb = first; kb < issued; ++kb) {
           const long long t0 = clock64();
-          while (!mbar_try_wait(bar_full(kb % kTaStages), (kb / kTaStages) & 1u) &&
+          while (!mbar_try_wait(bar_x(kb % kTaStages), (kb / kTaStages) & 1u) &&
                  (unsigned long long)(clock64() - t0) < kWaitCycles) {}
         }
       }
@@ -270,10 +259,26 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       // be a bubble in the pipe: the next block's barrier is polled once before the last MMA of the current block is
       // issued, in the shadow of the MMAs already queued, and waited for afterwards only if that poll failed.
       bool ok = mbar_wait(bar_full(0), 0u, p.status, 2u, abort_flag);
+      if constexpr (BITS == 8) {
+        // Each block into its stage's accumulator: the team that wrote the slice had folded what was there before.
+        for (uint32_t kb = 0; kb < num_kb && ok; ++kb) {
+          ok = mbar_wait(bar_x((int)s), ph, p.status, 3u, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t bdesc = b0 + (uint64_t)(s * (L::kXBytes >> 4));
+#pragma unroll
+          for (int k = 0; k < kGemmBK / 16; ++k)
+            umma_f16_ta(tmem_base + s * NT, tmem_base + kColA + s * 32u + (uint32_t)(8 * k), bdesc + (uint64_t)(2 * k), idesc, k ? 1u : 0u);
+          umma_commit(bar_empty((int)s));
+          mbar_arrive(bar_empty((int)s));    // (a plain arrival as well: it passes on what the team wrote to shared memory before its own)
+          if (++s == (uint32_t)kTaStages) { s = 0; ph ^= 1u; }
+          if (kb + 1 < num_kb) ok = mbar_wait(bar_full((int)s), ph, p.status, 2u, abort_flag);
+        }
+      } else {
       for (uint32_t kb = 0; kb < num_kb && ok; ++kb) {
         tc_fence_after();
         const uint64_t bdesc = b0 + (uint64_t)(s * (L::kXBytes >> 4));
-        const uint32_t a_tmem = tmem_base + kColA + s * kACols;
+        const uint32_t a_tmem = tmem_base + kColA + s * 32u;
         uint32_t s1 = s + 1u, ph1 = ph;
         if (s1 == (uint32_t)kTaStages) { s1 = 0; ph1 ^= 1u; }
         bool next_ready = true;
@@ -283,13 +288,13 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           umma_f16_ta(tmem_base, a_tmem + (uint32_t)(8 * k), bdesc + (uint64_t)(2 * k), idesc, (kb | (uint32_t)k) ? 1u : 0u);
           if (NT > 256 && cols > cols_a)
             umma_f16_ta(tmem_base + cols_a, a_tmem + (uint32_t)(8 * k), bdesc + (uint64_t)(cols_a * 8u + 2 * k), idesc_b, (kb | (uint32_t)k) ? 1u : 0u);
-          if (BITS == 8) umma_f16_ta(tmem_base, a_tmem + 32u + (uint32_t)(8 * k), bdesc + (uint64_t)(2 * k), idesc, 1u);   // the second terms
         }
         umma_commit(bar_empty((int)s));   // the activation tile and the weight slice are free once these MMAs have read them
         if (!next_ready) ok = mbar_wait(bar_full((int)s1), ph1, p.status, 2u, abort_flag);
         s = s1; ph = ph1;
       }
       if (ok) umma_commit(bar_accum);
+      }
     }
   } else if (warp == 2) {
     // ================= TMA producer: packed weights =================
@@ -336,25 +341,129 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     const uint32_t sb_odd = (uint32_t)(((size_t)min(n0 + r_tile, p.N - 1) * p.SPR) & 3u) * 2u;   // (stages start on multiples of four groups)
     const uint8_t* const sb_row = gen_base + L::kOffSb + r_tile * p.sb_pitch + sb_odd;
     const uint32_t b_delta = (uint32_t)kTaRows * p.sb_pitch;
-    const uint32_t st_at = tmem_base + lane_base + kColA + team * kACols;
-    [[maybe_unused]] float row_unit = 1.f;                 // 8-bit: weights are stored times this power of two
-    if constexpr (BITS == 8) {
-      // ... which takes the largest weight that the row's scales allow to the top of f16's range: no weight overflows, and the two terms
-      // hold one to 2^-22 of its size or 2^-39 of that largest one
-      float* const bounds = reinterpret_cast<float*>(gen_base + L::kOffBar + 256);
-      bounds[team * kTaRows + r_tile] = ta_row_bound(p, min(n0 + r_tile, p.N - 1), team);
-      asm volatile("bar.sync 1, %0;" ::"n"(kTaDqWarps * 32) : "memory");
-      row_unit = ta_row_unit(fmaxf(fmaxf(bounds[r_tile], bounds[kTaRows + r_tile]), fmaxf(bounds[2 * kTaRows + r_tile], bounds[3 * kTaRows + r_tile])));
-      unscale = 1.f / row_unit;
-    }
+    const uint32_t st_at = tmem_base + lane_base + kColA + team * 32u;
     bool ok = true;
+    if constexpr (BITS == 8) {
+      static_assert(kTaWStages == 4, "slots of the packed ring by c & 3");
+      // Codes go to tensor memory masked where they sit, as f16 subnormals (products q * 2^-24 * x, exact). A team takes its block's
+      // accumulator back and folds it into f32 registers: a thread has its weight row and all tokens of the tile. Slice, accumulator
+      // and sums of activations are the team's own, so teams wait for nothing but their own MMAs. What round c - 1 left is folded
+      // before round c overwrites it; the sums of activations alternate between two places, as a warp may be a round ahead of another.
+      float* const xsum = reinterpret_cast<float*>(gen_base + L::kOffXsum) + team * NT;
+      unsigned long long sum[NT / 2];
+#pragma unroll
+      for (int i = 0; i < NT / 2; ++i) sum[i] = 0ull;
+      for (uint32_t c = 0;; ++c) {
+        if (c > 0) {
+          const uint32_t d = c - 1u, sbs = (d >> 1) & 1u;
+          if (d * kTaWChunk + team < num_kb) {
+            if (ok && (d & 1u) == 0u) ok = mbar_wait(bar_sb_full((int)sbs), (d >> 2) & 1u, p.status, 9u, abort_flag);
+            if (ok) ok = mbar_wait(bar_empty((int)team), d & 1u, p.status, 4u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            tc_fence_after();
+            if (ok) {
+              const uint8_t* const sp = sb_row + sbs * L::kSbBytes + ((d & 1u) * kTaWChunk + team) * 2u;
+              const float sf = __half2float(*reinterpret_cast<const __half*>(sp)), bf = __half2float(*reinterpret_cast<const __half*>(sp + b_delta));
+              const unsigned long long s2 = ta_pk(sf * 16777216.f, sf * 16777216.f), b2 = ta_pk(bf, bf);
+              const ulonglong2* const xs = reinterpret_cast<const ulonglong2*>(xsum + (d & 1u) * (kTaStages * NT));
+#pragma unroll
+              for (int h = 0; h < NT / 16; ++h) {
+                if (16u * h >= mrows) break;
+                uint32_t v[16];
+                tmem_ld16(tmem_base + lane_base + team * NT + 16u * h, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  const ulonglong2 x = xs[4 * h + i];
+                  unsigned long long* const to = sum + 8 * h + 2 * i;
+                  to[0] = ta_ffma2(b2, x.x, ta_ffma2(s2, ta_pk(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1])), to[0]));
+                  to[1] = ta_ffma2(b2, x.y, ta_ffma2(s2, ta_pk(__uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3])), to[1]));
+                }
+              }
+            }
+          }
+          __syncwarp();
+          if (lane == 0 && ((d & 1u) || c * kTaWChunk >= num_kb)) mbar_arrive(bar_sb_empty((int)sbs));
+        }
+        if (c * kTaWChunk >= num_kb) break;
+        if (c * kTaWChunk + team < num_kb) {
+          if (ok) ok = mbar_wait(bar_w_full((int)(c & 3u)), (c >> 2) & 1u, p.status, 7u, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (ok) {
+            const uint8_t* const wl = wrow_sm + (c & 3u) * L::kWBytes + (team >> 1) * (kTaRows * 128);
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+              uint32_t a[16];
+#pragma unroll
+              for (uint32_t j = 0; j < 2; ++j) {
+                const uint4 w = *reinterpret_cast<const uint4*>(wl + ((((team & 1u) * 4u + 2u * h + j) ^ (r_tile & 7)) << 4));
+                const uint32_t q[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { a[8 * j + 2 * i] = codes8_pair01(q[i]); a[8 * j + 2 * i + 1] = codes8_pair23(q[i]); }
+              }
+              tmem_st16(st_at + 16u * h, a);
+            }
+            // meanwhile: sums of the block's activations, two threads per token
+            ok = mbar_wait(bar_x((int)team), c & 1u, p.status, 3u, abort_flag);
+            static_assert(NT * 2 == kTaRows, "two threads of a team per token");
+            const uint32_t token = r_tile >> 1, part = r_tile & 1u;
+            const uint8_t* const xr = gen_base + team * L::kXBytes + token * 128u;
+            float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+              const uint4 w = *reinterpret_cast<const uint4*>(xr + (((part * 4u + j) ^ (token & 7u)) << 4));
+              x0 = ta_add2(x0, w.x); x1 = ta_add2(x1, w.y); x2 = ta_add2(x2, w.z); x3 = ta_add2(x3, w.w);
+            }
+            float x = (x0 + x1) + (x2 + x3);
+            x += __shfl_xor_sync(0xffffffffu, x, 1);
+            if (part == 0u) xsum[(c & 1u) * (kTaStages * NT) + token] = x;
+            tmem_st_wait();
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_full((int)team));
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_w_empty((int)(c & 3u)));
+      }
+      // The teams' sums meet in tensor memory, in team order, where the epilogue looks for them.
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+#pragma unroll
+        for (int h = 0; h < NT / 16; ++h) {
+          uint32_t v[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { v[2 * i] = (uint32_t)sum[8 * h + i]; v[2 * i + 1] = (uint32_t)(sum[8 * h + i] >> 32); }
+          tmem_st16(tmem_base + lane_base + team * NT + 16u * h, v);
+        }
+        tmem_st_wait();
+      }
+      tc_fence_before();
+      asm volatile("bar.sync 1, %0;" ::"n"(kTaDqWarps * 32) : "memory");
+      tc_fence_after();
+      if (ok && team * (NT / 4) < mrows) {
+        uint32_t v[16], u[16];
+        tmem_ld16(tmem_base + lane_base + team * (NT / 4), v);
+#pragma unroll
+        for (uint32_t t = 1; t < 4; ++t) {
+          tmem_ld16(tmem_base + lane_base + t * NT + team * (NT / 4), u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(u[i]));
+        }
+        tmem_st16(tmem_base + lane_base + team * (NT / 4), v);
+        tmem_st_wait();
+      }
+      tc_fence_before();
+      asm volatile("bar.sync 1, %0;" ::"n"(kTaDqWarps * 32) : "memory");
+    } else {
     uint32_t ws = 0, wph = 0, ss = 0, sph = 0;          // slot and phase of the packed ring and of the scales ring
     for (uint32_t c = 0; c * kTaWChunk < num_kb; ++c) {
       if (c * kTaWChunk + team < num_kb) {
         if (ok && (c & 1u) == 0u) ok = mbar_wait(bar_sb_full((int)ss), sph, p.status, 9u, abort_flag);
         if (ok) ok = mbar_wait(bar_w_full((int)ws), wph, p.status, 7u, abort_flag);
-        uint32_t a[BITS == 8 ? 1 : 32];
-        if (BITS == 4 && ok) {
+        uint32_t a[32];
+        if (ok) {
           const uint8_t* const wl = wrow_sm + ws * L::kWBytes;
           const uint4 w0 = *reinterpret_cast<const uint4*>(wl + w_at0), w1 = *reinterpret_cast<const uint4*>(wl + w_at1);
           const uint32_t k0 = ((c & 1u) * kTaWChunk + team) * (uint32_t)kGemmBK;
@@ -375,23 +484,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           ok = mbar_wait(bar_empty((int)team), (c & 1u) ^ 1u, p.status, 4u, abort_flag);
           tc_fence_after();
         }
-        if (BITS == 8 && ok) {
-          const uint8_t* const wl = wrow_sm + ws * L::kWBytes + (team >> 1) * (kTaRows * 128);
-          const uint32_t k0 = ((c & 1u) * kTaWChunk + team) * (uint32_t)kGemmBK;
-          const uint8_t* const sp = sb_row + ss * L::kSbBytes + (k0 >> 6) * 2u;
-          const float sf = __half2float(*reinterpret_cast<const __half*>(sp)) * row_unit, bf = __half2float(*reinterpret_cast<const __half*>(sp + b_delta)) * row_unit;
-#pragma unroll
-          for (uint32_t h = 0; h < 2; ++h) {                  // 32 codes at a time: 16 columns of each term
-            uint32_t hi[16], lo[16];
-#pragma unroll
-            for (uint32_t j = 0; j < 2; ++j)
-              ta_terms8(*reinterpret_cast<const uint4*>(wl + ((((team & 1u) * 4u + h * 2u + j) ^ (r_tile & 7)) << 4)), sf, bf, hi + 8 * j, lo + 8 * j);
-            tmem_st16(st_at + 16u * h, hi);
-            tmem_st16(st_at + 32u + 16u * h, lo);
-          }
-          tmem_st_wait();
-        }
-        if constexpr (BITS == 4) if (ok) {
+        if (ok) {
           // 64 weights of this row = 32 TMEM columns (two k-adjacent f16 per column) of this thread's lane
           tmem_st32(st_at, a);
           tmem_st_wait();
@@ -411,8 +504,9 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       if (++ws == (uint32_t)kTaWStages) { ws = 0; wph ^= 1u; }
       if (c & 1u) { if (++ss == (uint32_t)kTaSbStages) { ss = 0; sph ^= 1u; } }
     }
+    }
     // ---- epilogue: D[weight row][token] in TMEM -> y[token][weight row] ------------------------------------------
-    acc_ok = ok && mbar_wait(bar_accum, 0u, p.status, 5u, abort_flag);
+    acc_ok = ok && (BITS == 8 || mbar_wait(bar_accum, 0u, p.status, 5u, abort_flag));
     acc_ok = __all_sync(0xffffffffu, acc_ok);            // the loads from tensor memory below are the whole warp's
     tc_fence_after();
     asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be read by the previous kernel in the stream
@@ -433,10 +527,6 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           uint32_t v[32];
           tmem_ld32(tmem_base + lane_base + (uint32_t)(cb * 32), v);
           tmem_ld_wait();
-          if constexpr (BITS == 8) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * unscale);
-          }
           const uint32_t col = stage + (uint32_t)(cb * 32) * (kTaRows * 2u) + r_tile * 2u;
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -465,10 +555,6 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         uint32_t v[32];
         tmem_ld32(tmem_base + lane_base + (uint32_t)(cb * 32), v);
         tmem_ld_wait();
-        if constexpr (BITS == 8) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * unscale);
-        }
         const uint32_t m_first = m0 + cb * 32;
         if (n < p.N) {
           if (p.out_f32) {
@@ -535,7 +621,6 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 #pragma unroll
           for (uint32_t i = 0; i < 8; ++i) {
             if (b * 8u + i >= mrows) break;
-            if constexpr (BITS == 8) r[i] *= unscale;
             const size_t o = (size_t)(m0 + b * 8u + i) * p.N + n;
             if (p.out_f32) reinterpret_cast<float*>(p.Y)[o] = r[i];
             else reinterpret_cast<__half*>(p.Y)[o] = __float2half_rn(r[i]);
@@ -628,10 +713,9 @@ bool gemm_ta_supported(int bits, uint32_t group, uint32_t K) {
 
 template <int BITS>
 static uint32_t ta_at_once(uint32_t tm, uint32_t z, int sm_count) {
-  if (tm <= 64u) return ta_clusters<64, BITS>(z, sm_count);
-  if (tm <= 128u) return ta_clusters<128, BITS>(z, sm_count);
-  if (BITS == 8 || tm <= 256u) return ta_clusters<256, BITS>(z, sm_count);
-  return ta_clusters<352, 4>(z, sm_count);
+  if (BITS == 8 || tm <= 64u) return ta_clusters<64, BITS>(z, sm_count);
+  if (tm <= 128u) return ta_clusters<128, 4>(z, sm_count);
+  return tm <= 256u ? ta_clusters<256, 4>(z, sm_count) : ta_clusters<352, 4>(z, sm_count);
 }
 
 cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, const __half* X, void* Y, uint32_t M, uint32_t N, uint32_t K,
@@ -641,20 +725,19 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
   // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 8192 x 2048 .. 3072 x 8192:
   // a k block takes 340 + 1.4 per token (at least 390), a CTA 8500 to start, fill its rings and store, the exchange of
   // a cluster 5300 + 12 per token. Clusters run in as many waves as the device can place. The tokens are dealt evenly to
-  // the tiles. (Groups of 32 with biases do not fit beside the widest tile.) 8-bit, whose blocks are twice the MMAs and more than twice
-  // the dequantisation: 700 + 1 per token, at least 5.5 per token; the exchange more for every share beyond two; no shares of the
-  // 256-token tiles (2048 x 6144, 200 tokens, us: two tiles in four shares 26, one in four 46, one whole 52).
+  // the tiles. (Groups of 32 with biases do not fit beside the widest tile.) 8-bit: tiles of up to
+  // 64 tokens, a block 700 + 2 per token; the exchange more for every share beyond two.
   const uint32_t units = (K / kGemmBK + kTaSbChunk - 1) / kTaSbChunk, n_tiles = (N + kTaRows - 1) / kTaRows;
-  const uint32_t widest = bits == 8 || (B && group_shift == 5) ? 256u : 352u;
+  const uint32_t widest = bits == 8 ? 64u : B && group_shift == 5 ? 256u : 352u;
   uint32_t tile_m = 0, split = 1;
   uint64_t best = ~0ull;
   for (uint32_t t = 64; t <= widest; t += 32) {
     if (t > 64u && t - 32u >= M) break;
     const uint32_t m_tiles = (M + t - 1) / t, tm = ((M + m_tiles - 1) / m_tiles + 15u) & ~15u;
     const uint64_t tiles = (uint64_t)n_tiles * m_tiles;
-    const uint32_t live = M < tm ? M : tm, block = bits == 8 ? (live < 156u ? 700u + live : live * 55u / 10u) : live < 36u ? 390u : 340u + live * 14u / 10u;
+    const uint32_t live = M < tm ? M : tm, block = bits == 8 ? 700u + 2u * live : live < 36u ? 390u : 340u + live * 14u / 10u;
     for (uint32_t z = 1; z <= (uint32_t)kTaMaxSplit && z <= units; ++z) {
-      if (z > 1 && (tiles * z > (uint64_t)sm_count || (bits == 8 && tm > 128u))) break;
+      if (z > 1 && tiles * z > (uint64_t)sm_count) break;
       const uint32_t at_once = bits == 8 ? ta_at_once<8>(tm, z, sm_count) : ta_at_once<4>(tm, z, sm_count);
       const uint64_t waves = (tiles + at_once - 1) / at_once;
       const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + 8500u + (z > 1 ? 5300u + 12u * live + (bits == 8 && z > 2 ? 28u * live * (z - 2) : 0u) : 0u));
@@ -686,10 +769,7 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
   p.sb_pitch = group_shift == 5 ? 40u : 24u;
   p.tile_m = tile_m; p.box_rows = box_rows;
   p.status = status;
-  if (bits == 8) {
-    if (tile_m > 128u) return launch_ta_one<256, true, 8>(tx, tw, p, split, st);
-    return tile_m > 64u ? launch_ta_one<128, true, 8>(tx, tw, p, split, st) : launch_ta_one<64, true, 8>(tx, tw, p, split, st);
-  }
+  if (bits == 8) return launch_ta_one<64, true, 8>(tx, tw, p, split, st);
   const bool affine = B != nullptr;
   if (tile_m > 256u) return affine ? launch_ta_one<352, true, 4>(tx, tw, p, split, st) : launch_ta_one<352, false, 4>(tx, tw, p, split, st);
   if (tile_m > 128u) return affine ? launch_ta_one<256, true, 4>(tx, tw, p, split, st) : launch_ta_one<256, false, 4>(tx, tw, p, split, st);

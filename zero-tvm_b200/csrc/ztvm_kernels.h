@@ -101,7 +101,7 @@ bool batch_moe_supported(const GemvParams& g, int bits);
 uint32_t batch_moe_tile_rows(int bits, uint32_t experts, uint64_t pairs);
 cudaError_t launch_batch_moe(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, cudaStream_t st, bool reuse_plan);
 
-// 4-bit weights, and 8-bit ones as two f16 terms, M > 16: tcgen05 GEMM with the dequantised weights as the A operand in tensor memory and the activations
+// 4-bit weights, and 8-bit ones as codes, M > 16: tcgen05 GEMM with the dequantised weights as the A operand in tensor memory and the activations
 // as the only shared-memory operand (ztvm_gemm_ta.cu). status[0] receives a non-zero code if a pipeline wait inside the
 // kernel ran out.
 bool gemm_ta_supported(int bits, uint32_t group, uint32_t K);
