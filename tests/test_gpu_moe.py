@@ -374,7 +374,7 @@ def test_peer_store_expert_parallel_step_with_ranks_emulated_on_one_gpu(T, G, E,
 def test_dispatch_plan_on_the_device_matches_the_tensor_op_plan(backend, dev, T):
     """ztvm_moe_dispatch_plan against the plan recomputed on the host: same pairs per destination, a
     permutation of all pairs in destination order, the right local expert for every pair. The sizes sit on both
-    sides of the pair counts where the planner changes kernels (one block up to 32768 pairs, several above)."""
+    sides of the pair counts where the planner changes kernels (one block, a cluster of eight, several launches)."""
     import torch
     from zero_tvm_b200 import sharded
     K, E, world = 8, 64, 4
@@ -394,6 +394,53 @@ def test_dispatch_plan_on_the_device_matches_the_tensor_op_plan(backend, dev, T)
     dest = flat[order] // epr
     assert (np.diff(dest) >= 0).all()
     assert np.array_equal(local, (flat[order] % epr).astype(np.int32))
+
+
+@pytest.mark.parametrize("T,K", [(1, 1), (512, 1), (171, 3), (1024, 1), (205, 5), (1024, 4), (4097, 1), (2731, 3), (2304, 8), (32767, 1), (4096, 8), (32769, 1)])
+def test_dispatch_plan_of_every_length(backend, dev, T, K):
+    """Both sides of each pair count where the planner changes kernels or rounds: one expert of 1024 takes most pairs; ids outside the
+    experts, whatever their value, are counted and left out."""
+    import torch
+    from zero_tvm_b200 import sharded
+    E, world = 1024, 4
+    rng = np.random.default_rng(T + K)
+    ids = rng.integers(0, E, size=(T, K), dtype=np.uint32)
+    ids[rng.random((T, K)) < 0.4] = 700
+    flat = ids.reshape(-1)
+    outside = np.array([E, E + 77, 0x80000000, 0xFFFFFFFE, 0xFFFFFFFF], np.uint32)
+    at = rng.choice(T * K, min(T * K // 2, 3 * len(outside)), replace=False)
+    flat[at] = outside[np.arange(len(at)) % len(outside)]
+    order, local, send = sharded.CudaKernels(backend).dispatch_plan(dev.put(ids), E // world, world)
+    torch.cuda.synchronize()
+    assert backend.ctx.device_errors() == len(at)
+    good = np.flatnonzero(flat < E)
+    order, local = order.cpu().numpy()[:len(good)], local.cpu().numpy()[:len(good)]
+    assert np.array_equal(np.sort(order), good)
+    experts = flat[order].astype(np.int64)
+    assert (np.diff(experts) >= 0).all() and np.array_equal(local, experts % (E // world))
+    assert np.array_equal(send.cpu().numpy(), np.bincount(flat[good].astype(np.int64) // (E // world), minlength=world))
+
+
+@pytest.mark.parametrize("cap,counts", [(400, (400, 3, 0)), (1400, (1399, 0, 1400)), (3000, (17, 3000, 2999))])
+def test_receive_buffers_of_every_length(backend, dev, oracle_c, cap, counts):
+    """Rows past a region's count are no pairs, whatever id is left in them: in the plan of one block and in the cluster's."""
+    rng = np.random.default_rng(cap)
+    E, K, N, rows = 12, 256, 64, 3 * cap
+    _, W, s, b = z.synth.make_weights(rng, N, K, lead=(E,))
+    x, ids = z.synth.make_x(rng, rows, K), rng.integers(0, E, size=(rows, 1), dtype=np.uint32)
+    live = np.concatenate([np.arange(cap) < c for c in counts])
+    ids[~live] = rng.choice(np.array([0, E, 0xFFFFFFFE, 0xFFFFFFFF], np.uint32), size=(int((~live).sum()), 1))
+    y = dev.empty((rows, N), np.float16, fill=7.0)
+    layout = z.capi.MoeEpRows()
+    held = dev.put(np.array(counts, np.uint32))
+    layout.seg_counts, layout.seg_cap, layout.segments = held.data_ptr(), cap, 3
+    desc = z.MoeDesc(z.MmDesc(K, N, 1, 64, 4, 1, 0), E, 1, rows, 0, N, K, N, 1)
+    backend.ctx.int4_matmul_moe_ep(desc, layout, y, dev.put(x), dev.put(s), dev.put(W), dev.put(b), dev.put(ids))
+    assert backend.ctx.device_errors() == 0
+    got = dev.get(y)
+    assert (got[~live] == 7.0).all()
+    ref = oracle_c.moe_matmul_f64(x[live], W, s, b, ids[live], N, K, 64, 4, in_per_slot=False, w16=True)
+    assert zo.rel_err_scaled(got[live][:, None, :], ref, 1e-2) <= TOL
 
 
 def test_peer_barrier_alone_and_with_a_rank_that_never_arrives(backend, dev):

@@ -109,7 +109,29 @@ __device__ __forceinline__ uint32_t moe_agg_add(uint32_t* cnt, uint32_t key, boo
 // The whole plan in ONE block for pair lists up to a few thousand (kPlanClusterMin): histogram and cursors in shared memory,
 // same scans, same tables. Pairs are walked slot-major (a warp sees 32 tokens of one slot), so the pairs of a slot
 // that always carries the same expert (the shared expert) aggregate into one atomic per warp.
-constexpr uint32_t kPlanSmallMax = 32768;   // pairs the one-block plan takes: 32 per thread, kept in registers
+constexpr uint32_t kPlanClusterMin = 4096;  // pairs the one-block plan takes: four per thread, kept in registers
+constexpr uint32_t kPlanSmallMax = 32768;   // ... and the cluster: four per thread of eight CTAs
+constexpr int kPlanPer = 4;
+constexpr uint32_t kNoPair = 0xFFFFFFFFu;   // in place of an id: no pair, or one without an expert (counted)
+// Experts of the pairs first, first + step, .. of a list walked slot-major; returns how many ids lie outside [0, E).
+template <int PER>
+__device__ __forceinline__ uint32_t moe_plan_ids(const uint32_t* ids, uint32_t first, uint32_t step, uint32_t tokens, uint32_t slots,
+                                                 uint32_t ids_stride, uint32_t E, const MoeSegs& segs, uint32_t (&xs)[PER]) {
+  uint32_t pairs = 0, bad = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {                                    // (every load in flight before the first id is looked at)
+    const uint32_t j = first + step * k;                             // j = slot * tokens + token
+    xs[k] = kNoPair;
+    if (j < tokens * slots) {
+      const uint32_t s = j / tokens, t = j - s * tokens;
+      if (segs.live(t * slots + s)) { xs[k] = ids[(size_t)t * ids_stride + s]; pairs |= 1u << k; }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < PER; ++k)
+    if (xs[k] >= E) { bad += pairs >> k & 1u; xs[k] = kNoPair; }
+  return bad;
+}
 __global__ void __launch_bounds__(1024) moe_plan_small_kernel(const uint32_t* ids, uint32_t tokens, uint32_t slots,
                                                               uint32_t ids_stride, uint32_t E, uint32_t tile_rows,
                                                               MoeScratch sc, uint32_t* err, MoeSegs segs) {
@@ -119,23 +141,13 @@ __global__ void __launch_bounds__(1024) moe_plan_small_kernel(const uint32_t* id
   pdl_launch_dependents();
   pdl_wait();
   // every id of this thread is loaded up front (independent loads in flight together), then counted, then scattered
-  uint32_t xs[kPlanSmallMax / 1024];
-#pragma unroll
-  for (int k = 0; k < (int)(kPlanSmallMax / 1024); ++k) {
-    const uint32_t j = threadIdx.x + 1024u * k;                     // j = slot * tokens + token
-    xs[k] = 0xFFFFFFFFu;
-    if (j < P) {
-      const uint32_t s = j / tokens, t = j - s * tokens;
-      if (segs.live(t * slots + s)) xs[k] = ids[(size_t)t * ids_stride + s];
-      else xs[k] = 0xFFFFFFFEu;                                    // not a pair at all (past a region's live rows)
-    }
-  }
+  static_assert(kPlanClusterMin == 1024 * kPlanPer && kPlanSmallMax == 8 * kPlanClusterMin, "ids per thread");
+  uint32_t xs[kPlanPer];
+  const uint32_t bad = moe_plan_ids(ids, threadIdx.x, 1024u, tokens, slots, ids_stride, E, segs, xs);
   __syncthreads();
-  uint32_t bad = 0;
 #pragma unroll
-  for (int k = 0; k < (int)(kPlanSmallMax / 1024); ++k) {
+  for (int k = 0; k < kPlanPer; ++k) {
     if (1024u * k >= P) break;                                      // block-uniform
-    if (xs[k] >= E && xs[k] < 0xFFFFFFFEu) ++bad;
     moe_agg_add(cnt_sm, xs[k], xs[k] < E);
   }
   if (bad) atomicAdd(err, bad);
@@ -156,7 +168,7 @@ __global__ void __launch_bounds__(1024) moe_plan_small_kernel(const uint32_t* id
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < (int)(kPlanSmallMax / 1024); ++k) {
+  for (int k = 0; k < kPlanPer; ++k) {
     if (1024u * k >= P) break;
     const uint32_t j = threadIdx.x + 1024u * k;
     const bool ok = xs[k] < E;
@@ -406,32 +418,19 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeGemmPara
 // The same in a cluster of eight CTAs, each with an eighth of the pairs: one SM's shared-memory atomics and the loads of up to 32 ids a
 // thread bound the one-block plan (257 experts, us: 18432 pairs 21, 8.0 so; 9216 7.3, 4608 6.9 so, 2304 in one block 9.6 cold). Histograms
 // are exchanged through distributed shared memory; every CTA takes the scans for itself.
-constexpr uint32_t kPlanCtas = 8, kPlanClusterMin = 4096;
+constexpr uint32_t kPlanCtas = kPlanSmallMax / kPlanClusterMin;
 __global__ void __launch_bounds__(1024) moe_plan_cluster_kernel(const uint32_t* ids, uint32_t tokens, uint32_t slots, uint32_t ids_stride,
                                                                 uint32_t E, uint32_t tile_rows, MoeScratch sc, uint32_t* err, MoeSegs segs) {
   __shared__ uint32_t cnt_sm[1024], cur_sm[1024], warp_sums[32];
-  constexpr int kPer = (int)(kPlanSmallMax / (1024 * kPlanCtas));
-  const uint32_t e = threadIdx.x, P = tokens * slots, rank = blockIdx.x;      // (the grid is one cluster)
+  const uint32_t e = threadIdx.x, rank = blockIdx.x;      // (the grid is one cluster)
   cnt_sm[e] = 0u;
   pdl_launch_dependents();
   pdl_wait();
-  uint32_t xs[kPer];
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const uint32_t j = rank * 1024u + threadIdx.x + 1024u * kPlanCtas * k;    // j = slot * tokens + token
-    xs[k] = 0xFFFFFFFEu;                                                       // not a pair
-    if (j < P) {
-      const uint32_t s = j / tokens, t = j - s * tokens;
-      if (segs.live(t * slots + s)) xs[k] = ids[(size_t)t * ids_stride + s];
-    }
-  }
+  uint32_t xs[kPlanPer];
+  const uint32_t bad = moe_plan_ids(ids, rank * 1024u + threadIdx.x, 1024u * kPlanCtas, tokens, slots, ids_stride, E, segs, xs);
   __syncthreads();
-  uint32_t bad = 0;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    if (xs[k] >= E && xs[k] != 0xFFFFFFFEu) ++bad;
-    moe_agg_add(cnt_sm, xs[k], xs[k] < E);
-  }
+  for (int k = 0; k < kPlanPer; ++k) moe_agg_add(cnt_sm, xs[k], xs[k] < E);
   if (bad) atomicAdd(err, bad);
   cluster_sync_all();
   uint32_t cnt = 0, before = 0;                                                // of expert e: all pairs, those of the CTAs before this one
@@ -462,7 +461,7 @@ __global__ void __launch_bounds__(1024) moe_plan_cluster_kernel(const uint32_t* 
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
+  for (int k = 0; k < kPlanPer; ++k) {
     const uint32_t j = rank * 1024u + threadIdx.x + 1024u * kPlanCtas * k;
     const bool ok = xs[k] < E;
     const uint32_t pos = moe_agg_add(cur_sm, xs[k], ok);
