@@ -106,12 +106,11 @@ __device__ __forceinline__ uint32_t moe_agg_add(uint32_t* cnt, uint32_t key, boo
   return active ? atomicAdd(&cnt[key], 1u) : 0u;
 }
 
-// The whole plan in ONE block for pair lists up to a few thousand (kPlanClusterMin): histogram and cursors in shared memory,
+// The whole plan in ONE block for pair lists up to two thousand (kPlanSmallMax): histogram and cursors in shared memory,
 // same scans, same tables. Pairs are walked slot-major (a warp sees 32 tokens of one slot), so the pairs of a slot
 // that always carries the same expert (the shared expert) aggregate into one atomic per warp.
-constexpr uint32_t kPlanClusterMin = 4096;  // pairs the one-block plan takes: four per thread, kept in registers
-constexpr uint32_t kPlanSmallMax = 32768;   // ... and the cluster: four per thread of eight CTAs
-constexpr int kPlanPer = 4;
+constexpr uint32_t kPlanSmallMax = 2048;     // pairs the one-block plan takes: two per thread, kept in registers
+constexpr uint32_t kPlanClusterMax = 32768; // ... and the cluster: four per thread of eight CTAs
 constexpr uint32_t kNoPair = 0xFFFFFFFFu;   // in place of an id: no pair, or one without an expert (counted)
 // Experts of the pairs first, first + step, .. of a list walked slot-major; returns how many ids lie outside [0, E).
 template <int PER>
@@ -141,12 +140,12 @@ __global__ void __launch_bounds__(1024) moe_plan_small_kernel(const uint32_t* id
   pdl_launch_dependents();
   pdl_wait();
   // every id of this thread is loaded up front (independent loads in flight together), then counted, then scattered
-  static_assert(kPlanClusterMin == 1024 * kPlanPer && kPlanSmallMax == 8 * kPlanClusterMin, "ids per thread");
-  uint32_t xs[kPlanPer];
+  constexpr int kPer = (int)(kPlanSmallMax / 1024);
+  uint32_t xs[kPer];
   const uint32_t bad = moe_plan_ids(ids, threadIdx.x, 1024u, tokens, slots, ids_stride, E, segs, xs);
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kPlanPer; ++k) {
+  for (int k = 0; k < kPer; ++k) {
     if (1024u * k >= P) break;                                      // block-uniform
     moe_agg_add(cnt_sm, xs[k], xs[k] < E);
   }
@@ -168,7 +167,7 @@ __global__ void __launch_bounds__(1024) moe_plan_small_kernel(const uint32_t* id
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kPlanPer; ++k) {
+  for (int k = 0; k < kPer; ++k) {
     if (1024u * k >= P) break;
     const uint32_t j = threadIdx.x + 1024u * k;
     const bool ok = xs[k] < E;
@@ -415,22 +414,24 @@ moe_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeGemmPara
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
-// The same in a cluster of eight CTAs, each with an eighth of the pairs: one SM's shared-memory atomics and the loads of up to 32 ids a
-// thread bound the one-block plan (257 experts, us: 18432 pairs 21, 8.0 so; 9216 7.3, 4608 6.9 so, 2304 in one block 9.6 cold). Histograms
-// are exchanged through distributed shared memory; every CTA takes the scans for itself.
-constexpr uint32_t kPlanCtas = kPlanSmallMax / kPlanClusterMin;
+// The same in a cluster of eight CTAs, each with an eighth of the pairs: one SM's shared-memory atomics bound the one-block plan (257
+// experts, us beside a grouped matmul, one block and the cluster: 144 pairs 2.5, 4.3; 1026 3.3, 4.7; 2043 4.3, 5.1; 2304 5.2, 5.0; 4095 5.7, 5.1;
+// 9216 pairs 5.8 and 32760 8.0 in the cluster). Histograms are exchanged through distributed shared memory; every CTA takes the
+// scans for itself.
+constexpr uint32_t kPlanCtas = 8;
 __global__ void __launch_bounds__(1024) moe_plan_cluster_kernel(const uint32_t* ids, uint32_t tokens, uint32_t slots, uint32_t ids_stride,
                                                                 uint32_t E, uint32_t tile_rows, MoeScratch sc, uint32_t* err, MoeSegs segs) {
   __shared__ uint32_t cnt_sm[1024], cur_sm[1024], warp_sums[32];
+  constexpr int kPer = (int)(kPlanClusterMax / (1024 * kPlanCtas));
   const uint32_t e = threadIdx.x, rank = blockIdx.x;      // (the grid is one cluster)
   cnt_sm[e] = 0u;
   pdl_launch_dependents();
   pdl_wait();
-  uint32_t xs[kPlanPer];
+  uint32_t xs[kPer];
   const uint32_t bad = moe_plan_ids(ids, rank * 1024u + threadIdx.x, 1024u * kPlanCtas, tokens, slots, ids_stride, E, segs, xs);
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kPlanPer; ++k) moe_agg_add(cnt_sm, xs[k], xs[k] < E);
+  for (int k = 0; k < kPer; ++k) moe_agg_add(cnt_sm, xs[k], xs[k] < E);
   if (bad) atomicAdd(err, bad);
   cluster_sync_all();
   uint32_t cnt = 0, before = 0;                                                // of expert e: all pairs, those of the CTAs before this one
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(1024) moe_plan_cluster_kernel(const uint32_t* 
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kPlanPer; ++k) {
+  for (int k = 0; k < kPer; ++k) {
     const uint32_t j = rank * 1024u + threadIdx.x + 1024u * kPlanCtas * k;
     const bool ok = xs[k] < E;
     const uint32_t pos = moe_agg_add(cur_sm, xs[k], ok);
@@ -478,7 +479,7 @@ cudaError_t launch_moe_plan(const GemvParams& g, uint32_t tokens, uint32_t slots
                             cudaStream_t st) {
   const uint32_t P = tokens * slots, E = g.experts;
   const MoeSegs segs{g.seg_counts, g.seg_cap ? g.seg_cap : 1u};
-  if (P > kPlanClusterMin && P <= kPlanSmallMax) {
+  if (P > kPlanSmallMax && P <= kPlanClusterMax) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kPlanCtas);
     cfg.blockDim = dim3(1024);
