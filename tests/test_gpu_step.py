@@ -139,6 +139,38 @@ def test_more_calls_than_one_launch_takes_and_formats_in_turn(backend, dev):
     st.check(replays=2)
 
 
+def test_a_wait_that_runs_out(dev, monkeypatch):
+    """The limit of a step's waits is set so short that they expire: the step ends all the same and says so, every time, and calls that wait
+    for nothing are right."""
+    import time
+    import torch
+    monkeypatch.setenv("ZTVM_STEP_WAIT_CYCLES", "1")
+    be = z.backend.CudaMatmulBackend(0)
+    st = Step(be, dev, np.random.default_rng(4), 4, False)
+    for i in range(5):
+        st.buf(f"v{i}", 2048, values=z.synth.make_x(st.rng, 1, 2048))
+    for i in range(4):
+        st.matmul(f"v{i + 1}", f"v{i}", 2048, 2048)
+    step = st.rec.capture()
+    with pytest.raises(z.ZtvmError, match="code 11"):
+        be.ctx.device_errors()
+    t0 = time.perf_counter()
+    for run in [step.replay] * 20 + [st.rec.run_eager] * 20:
+        run()
+        torch.cuda.synchronize()
+        with pytest.raises(z.ZtvmError, match="code 11"):
+            be.ctx.device_errors()
+    assert time.perf_counter() - t0 < 2.0
+    be.ctx.step_begin(1)
+    fn, args, _ = st.rec._calls[0]
+    fn(*args, stream=1)
+    be.ctx.step_end()
+    torch.cuda.synchronize()
+    assert be.ctx.device_errors() == 0
+    st.against_oracle({k: v.clone() for k, v in st.bufs.items()}, "v1")
+    be.close()
+
+
 def test_two_captured_steps_replay_side_by_side(backend, dev):
     """Each captured step counts arrivals in words of its own."""
     import torch

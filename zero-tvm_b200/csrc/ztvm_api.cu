@@ -40,6 +40,7 @@ struct ztvm_ctx {
   ztvm::StepBuilder* step;
   int step_on;
   cudaStream_t step_stream;
+  uint64_t step_wait;  // cycles, about a second; env ZTVM_STEP_WAIT_CYCLES
   int moe_tiles_sm; // env ZTVM_MOE_TILES=sm: the grouped MoE tiles with both operands in shared memory (a measurement knob)
 };
 
@@ -99,7 +100,7 @@ ztvm_status step_flush(ztvm_ctx* ctx) {
     }
     if (e == cudaSuccess) counters = static_cast<uint32_t*>(buf->p);
   }
-  if (e == cudaSuccess) e = ctx->step->launch(counters, ctx->err_counter + 1, ctx->sm_count, ctx->step_stream);
+  if (e == cudaSuccess) e = ctx->step->launch(counters, ctx->err_counter + 1, ctx->step_wait, ctx->sm_count, ctx->step_stream);
   ctx->step->clear();
   return e == cudaSuccess ? ZTVM_OK : cuda_fail(e, "launch of the matmuls held back");
 }
@@ -260,6 +261,8 @@ ztvm_status ztvm_init(int32_t device_ordinal, ztvm_ctx** out_ctx) {
   c->moe_grouped = !mg ? -1 : (mg[0] == '1' ? 1 : mg[0] == '2' ? 2 : 0);
   const char* gp = getenv("ZTVM_GEMV_PATH");
   c->gemv_path = !gp ? 0 : !strcmp(gp, "fma") ? 1 : !strcmp(gp, "mma") ? 2 : !strcmp(gp, "tc_m2") ? 3 : 0;
+  const char* sw = getenv("ZTVM_STEP_WAIT_CYCLES");
+  c->step_wait = sw && strtoull(sw, nullptr, 10) ? strtoull(sw, nullptr, 10) : 2000000000ull;
   c->magic = kMagic;
   *out_ctx = c;
   return ZTVM_OK;
@@ -353,7 +356,7 @@ static ztvm_status matmul_now(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, con
     const bool want_tc = ctx->gemv_path == 0 || (ctx->gemv_path == 3 && dd.M > 1);
     if (d->M == 1 && ctx->gemv_path == 0 && ztvm::step_alone_faster((int)d->bits, d->affine != 0, d->N, d->K, ctx->sm_count) &&
         ctx->step->add(p, (int)d->bits, ctx->sm_count)) {      // (nothing is held back here)
-      const cudaError_t e = ctx->step->launch(nullptr, ctx->err_counter + 1, ctx->sm_count, st);
+      const cudaError_t e = ctx->step->launch(nullptr, ctx->err_counter + 1, ctx->step_wait, ctx->sm_count, st);
       ctx->step->clear();
       if (e != cudaSuccess) return cuda_fail(e, "one-row matmul");
     } else if (want_tc && ztvm::gemv_tc_supported(p, (int)d->bits, ctx->sm_count)) ZTVM_CUDA(ztvm::launch_gemv_tc(p, (int)d->bits, ctx->sm_count, st, &half));

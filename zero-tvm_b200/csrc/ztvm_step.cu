@@ -166,13 +166,14 @@ bool StepBuilder::add_silu(const void* gate_up, void* h, uint32_t rows, uint32_t
   return true;
 }
 
-cudaError_t StepBuilder::launch(uint32_t* counters, uint32_t* status, int sm_count, cudaStream_t st) {
+cudaError_t StepBuilder::launch(uint32_t* counters, uint32_t* status, uint64_t wait_cycles, int sm_count, cudaStream_t st) {
   StepProgram& p = prog_;
   if (p.n == 0) return cudaSuccess;
   if (!layout()) return cudaErrorInvalidValue;
   const bool together = waits();
   p.counters = together ? counters : nullptr;
   p.status = status;
+  p.wait_cycles = wait_cycles;
   const bool al = all_aligned(p, format_);
   switch (format_) {
     case 3: return launch_step_w3(p, al, smem_, sm_count, together, st);

@@ -291,7 +291,7 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
         const uint32_t* const cnt = p.counters + (o.wait - 1u);
         const long long t0 = clock64();
         while (step_ld_acquire(cnt) < gridDim.x) {
-          if ((unsigned long long)(clock64() - t0) > kWaitCycles) { dead = true; atomicExch(p.status, 11u); break; }
+          if ((unsigned long long)(clock64() - t0) > p.wait_cycles) { dead = true; atomicExch(p.status, 11u); break; }
         }
       }
       __syncthreads();
@@ -601,7 +601,7 @@ cudaError_t launch_step_format(const StepProgram& p, bool al, size_t smem, int g
     StepProgramT<1> q;
     q.op[0] = p.op[0];
     q.n = 1; q.x_bytes = p.x_bytes; q.off_part = p.off_part; q.off_x = p.off_x; q.off_xsum = p.off_xsum;
-    q.counters = nullptr; q.status = p.status;
+    q.counters = nullptr; q.status = p.status; q.wait_cycles = p.wait_cycles;
     return al ? launch_step_one<BITS, G32, AFFINE, true>(q, smem, grid, false, st) : launch_step_one<BITS, G32, AFFINE, false>(q, smem, grid, false, st);
   }
   return al ? launch_step_one<BITS, G32, AFFINE, true>(p, smem, grid, together, st) : launch_step_one<BITS, G32, AFFINE, false>(p, smem, grid, together, st);

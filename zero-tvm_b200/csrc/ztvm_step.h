@@ -34,7 +34,9 @@ struct alignas(16) StepOp {
   uint32_t signal;           // a later one waits for this one
 };
 
-// A launch's parameter. One matmul by itself has a type of its own: 6 KB of parameters would be copied for nothing.
+static_assert(sizeof(StepOp) == 112, "kStepMaxOps of them travel as kernel parameters");
+
+// A launch's parameter. One matmul by itself has a type of its own: 7 KB of parameters would be copied for nothing.
 template <int MAX>
 struct StepProgramT {
   StepOp op[MAX];
@@ -43,6 +45,7 @@ struct StepProgramT {
   uint32_t x_bytes;          // of the longest activation row (a row in two parts takes two)
   uint32_t* counters;        // n + 1 words, zero between launches; nullptr where no matmul waits
   uint32_t* status;
+  uint64_t wait_cycles;      // limit of a wait
 };
 using StepProgram = StepProgramT<kStepMaxOps>;
 
@@ -55,7 +58,7 @@ class StepBuilder {
   int size() const { return (int)prog_.n; }
   bool waits() const;
   void clear() { prog_.n = 0; }
-  cudaError_t launch(uint32_t* counters, uint32_t* status, int sm_count, cudaStream_t st);
+  cudaError_t launch(uint32_t* counters, uint32_t* status, uint64_t wait_cycles, int sm_count, cudaStream_t st);
 
  private:
   struct Span { uintptr_t lo, hi; };
