@@ -21,7 +21,7 @@
  *    A caller whose other work runs on the legacy default stream passes cudaStreamLegacy (handle 1),
  *    not NULL, to have the call ordered with that work.
  *  - Work buffers: the calls that need device memory of their own (the grouped MoE matmul for its plan, the two-launch fused
- *    FFN) take it from the context. Calls on different streams use different buffers. A captured call uses one that belongs
+ *    FFN, a step whose matmuls wait for one another for its counters) take it from the context. Calls on different streams use different buffers. A captured call uses one that belongs
  *    to its graph, which no other call touches; beyond the first 64 MB of those the context gets one back when the graph and
  *    its executables are gone. A buffer is allocated when a stream or a capture first needs it, or needs more (a stream synchronises for that;
  *    a capture is not disturbed).
@@ -335,6 +335,9 @@ ZTVM_API ztvm_status ztvm_fused_ffn(ztvm_ctx* ctx, const ztvm_mm_desc* desc, voi
  * first, so the order is that of the calls, and results are theirs up to the order of f32 sums (a matmul's is the same in every
  * step, whatever it is joined with); an error of the launch is reported by the call that made it. Events recorded and work
  * submitted on `stream` by other means between begin and end would not find it in order: end the step before.
+ * A launch whose matmuls wait for one another needs all SMs at once: it starts when no kernel of another stream holds any (a single
+ * matmul's launch shares them), so a long kernel beside it delays the whole step, and a kernel beside it that waits for something later in
+ * `stream` (a peer barrier) keeps it from starting until that wait runs out. Call the matmuls outside a step where that can happen.
  * (The reference submits a token's dispatches as one command buffer, src/zero-tvm/engine-core.ts:2194-2202.) */
 ZTVM_API ztvm_status ztvm_step_begin(ztvm_ctx* ctx, void* stream);
 ZTVM_API ztvm_status ztvm_step_end(ztvm_ctx* ctx);

@@ -147,10 +147,11 @@ def test_a_wait_that_runs_out(dev, monkeypatch):
     monkeypatch.setenv("ZTVM_STEP_WAIT_CYCLES", "1")
     be = z.backend.CudaMatmulBackend(0)
     st = Step(be, dev, np.random.default_rng(4), 4, False)
-    for i in range(5):
-        st.buf(f"v{i}", 2048, values=z.synth.make_x(st.rng, 1, 2048))
-    for i in range(4):
-        st.matmul(f"v{i + 1}", f"v{i}", 2048, 2048)
+    sizes = (8256, 64, 8256, 64)                           # (of 64 rows most CTAs have none: they wait while the others multiply)
+    for i, n in enumerate(sizes):
+        st.buf(f"v{i}", n, values=z.synth.make_x(st.rng, 1, n))
+    for i in range(3):
+        st.matmul(f"v{i + 1}", f"v{i}", sizes[i + 1], sizes[i])
     step = st.rec.capture()
     with pytest.raises(z.ZtvmError, match="code 11"):
         be.ctx.device_errors()
@@ -169,6 +170,31 @@ def test_a_wait_that_runs_out(dev, monkeypatch):
     assert be.ctx.device_errors() == 0
     st.against_oracle({k: v.clone() for k, v in st.bufs.items()}, "v1")
     be.close()
+
+
+@pytest.mark.parametrize("bits,symmetric", FORMATS)
+def test_a_launch_per_call(bits, symmetric, backend, dev):
+    """joined=False: what the same calls give one by one, bit for bit, replayed and eager."""
+    import torch
+    st = Step(backend, dev, np.random.default_rng(bits), bits, symmetric)
+    for name, d in (("a", 1024), ("b", 1024), ("c", 320), ("d", 1024)):
+        st.buf(name, d, values=z.synth.make_x(st.rng, 1, d))
+    st.matmul("b", "a", 1024, 1024)
+    st.matmul("c", "b", 320, 1024)
+    st.matmul("d", "c", 1024, 320)
+    for fn, args, _ in st.rec._calls:
+        fn(*args, stream=1)
+    torch.cuda.synchronize()
+    want = {k: v.clone() for k, v in st.bufs.items()}
+    step = st.rec.capture(joined=False)
+    for run in (step.replay, step.run_eager):
+        for name in ("b", "c", "d"):
+            st.bufs[name].fill_(float("nan"))
+        torch.cuda.synchronize()
+        run()
+        torch.cuda.synchronize()
+        assert all(torch.equal(v, want[k]) for k, v in st.bufs.items())
+    assert backend.ctx.device_errors() == 0
 
 
 def test_two_captured_steps_replay_side_by_side(backend, dev):

@@ -94,6 +94,26 @@ def test_calls_that_use_the_plan_are_captured_in_sequence(plan, want):
     assert log == want
 
 
+@pytest.mark.parametrize("joined,want", [(True, ["begin", "runs", "runs", "end"]), (False, ["runs", "runs"])])
+def test_steps_are_joined_unless_asked_otherwise(joined, want):
+    log = []
+
+    class Backend:
+        class ctx:
+            step_begin, step_end = staticmethod(lambda stream: log.append("begin")), staticmethod(lambda: log.append("end"))
+
+        def dispatch(self, entry, bindings, grid, stream=None):
+            log.append("runs")
+
+        def uses_moe_plan(self, entry, bindings, grid):
+            return True
+
+    rec = recorded_token(Backend())
+    rec._joined = joined
+    rec._run_captured(FakeStream("main", log), FakeStream("side", log))
+    assert log == want
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("knob,tokens,want", [(None, 1, False), (None, 16, True), ("0", 64, False), ("1", 1, True), ("2", 1, True)])
 def test_the_library_says_which_calls_use_the_plan(knob, tokens, want, dev, monkeypatch):

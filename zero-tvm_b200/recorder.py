@@ -56,6 +56,7 @@ class DecodeRecorder:
         self._calls: List[Tuple[Callable, tuple, dict]] = []
         self._graph = None
         self._stream = None
+        self._joined = True
 
     # -- recording: the same surface as CudaMatmulBackend, minus the stream (the recorder owns it) --------------------
     def dispatch(self, entry, bindings, grid=(1, 1, 1)):
@@ -107,8 +108,8 @@ class DecodeRecorder:
             i = end
 
     def _run_joined(self, stream, first, last):
-        """Calls first..last - 1 as one step: consecutive one-row matmuls become one launch."""
-        step_begin = getattr(getattr(self.be, "ctx", None), "step_begin", None)
+        """Calls first..last - 1 as one step: consecutive one-row matmuls become one launch (unless captured with joined=False)."""
+        step_begin = getattr(getattr(self.be, "ctx", None), "step_begin", None) if self._joined else None
         if step_begin is None:
             for fn, args, kw in self._calls[first:last]:
                 fn(*args, stream=stream, **kw)
@@ -126,13 +127,17 @@ class DecodeRecorder:
         s = stream if stream is not None else torch.cuda.current_stream()
         self._run_joined(s.cuda_stream if s.cuda_stream else 1, 0, len(self._calls))
 
-    def capture(self, plan_reuse: bool = True):
+    def capture(self, plan_reuse: bool = True, joined: bool = True):
         """One eager pass (loads the kernels and sets their attributes; what it rejects is rejected before a
         capture), then the capture. plan_reuse: the MoE matmuls of the step share one expert-sorted plan per id list
-        (valid because, inside the recorded sequence, only the recorded router writes the id list)."""
+        (valid because, inside the recorded sequence, only the recorded router writes the id list). joined: consecutive one-row
+        matmuls become one launch, which starts when every SM is free of other work; False keeps a launch per call, for a step that
+        must get on beside long kernels of other streams, or beside one that waits for something this step's stream does later.
+        Results then are those of the same calls dispatched one by one, bit for bit."""
         import torch
         if not self._calls:
             raise ValueError("nothing recorded")
+        self._joined = joined
         self._stream = torch.cuda.Stream()
         self._stream.wait_stream(torch.cuda.current_stream())
         self.be.ctx.moe_plan_reuse(plan_reuse)
