@@ -24,6 +24,7 @@ def f16_bound(ref, magnitudes, K):
 @pytest.mark.parametrize("M,N,K,f32", [
     # on 148 SMs: the tile whose busiest SM has the least to do
     (9, 257, 64, True), (32, 64, 192, False), (33, 65, 2112, False), (40, 19001, 128, False),    # 64 x 32 tiles, K split four ways
+    (31, 65, 2112, False), (33, 65, 2112, True), (256, 9472, 256, True), (256, 9472, 192, False),  # (f16 results of more rows and work are the prefill GEMM's)
     (64, 18944, 320, True), (61, 18943, 320, False), (35, 18817, 64, True),     # 128 x 64 tiles: one wave of 148, 64 x 32 would be four
     (250, 9409, 192, True), (256, 9472, 256, False),                            # 128 x 128 tiles
 ])
