@@ -96,3 +96,29 @@ def test_single_rows_round_the_f32_result(symmetric, N, K, backend, dev):
     backend.ctx.int4_matmul(z.MmDesc(K, N, 1, group, 4, int(not symmetric), 1), y32, *args)
     backend.ctx.sync()
     assert (dev.get(y16) == dev.get(y32).astype(np.float16)).all()
+
+
+@pytest.mark.parametrize("bits,symmetric,K,M", [(4, True, 320, 1), (4, False, 320, 1), (3, False, 320, 1), (8, False, 1600, 40)])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 65504.0])
+def test_activations_that_are_not_finite(bits, symmetric, K, M, value, backend, dev):
+    """One such activation (or f16's largest) makes of a result what it makes of the f32 one: other kernels, the same folds."""
+    group, N = 32 if symmetric else 64, 400
+    rng = np.random.default_rng(K)
+    _, W, s, b = z.synth.make_weights(rng, N, K, bits=bits, group=group, affine=not symmetric, sigma_s=0.01 * 15 / (2**bits - 1))
+    x = z.synth.make_x(rng, M, K)
+    x[M // 2, 77] = value
+    args = [dev.put(x), dev.put(s), dev.put(W), None if symmetric else dev.put(b)]
+    y32, ys = dev.empty((M, N), np.float32, fill=9.0), [dev.empty((M, N), np.float16, fill=9.0) for _ in range(2)]
+    backend.ctx.int4_matmul(z.MmDesc(K, N, M, group, bits, int(not symmetric), 1), y32, *args)
+    backend.ctx.step_begin()
+    for y in ys:
+        backend.ctx.int4_matmul(z.MmDesc(K, N, M, group, bits, int(not symmetric), 0), y, *args)
+    backend.ctx.step_end()
+    backend.ctx.sync()
+    want = dev.get(y32).astype(np.float64)
+    for y in ys:
+        got = dev.get(y).astype(np.float64)
+        for kind in (np.isnan, np.isposinf, np.isneginf):
+            assert np.array_equal(kind(got), kind(want)), kind
+        ok = np.isfinite(want)
+        assert np.allclose(got[ok], want[ok], rtol=2.0**-10, atol=2.0**-10 * np.abs(want[ok]).max(initial=0) / 16)

@@ -17,7 +17,8 @@
 //     different row tiles (see step_split).
 //   * activations lie in shared memory with the sums of their scale groups; a warp turns its slice into MMA B fragments once per
 //     K tile.
-//   * codes masked where they sit are f16 subnormals (codes4_inplace, codes3_inplace, codes8_pair01): exact products; every scale
+//   * codes masked where they sit are f16 subnormals (codes4_inplace, codes3_inplace, codes8_pair01): exact products (3-bit codes put powers
+//     of two on their activations, which in one part rounds those below 2^-9, by 2^-20 at most; kTwo's lose nothing); every scale
 //     group is summed inside the matrix unit and folded into f32 accumulators, acc += s*(ratio*lo + hi) + b*sum(x). With one
 //     token the MMA's columns are the scale groups of the slice: a lane's codes belong to one group, and its activations stand in that
 //     group's column.
