@@ -1,4 +1,4 @@
-// Prefill GEMM, M > 16, 4-bit weights: y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS (8-bit ones: codes) AS THE
+// Prefill GEMM, M > 16, 4-bit weights (8-bit ones: below): y[M, N] = x[M, K] * W16[N, K]^T on tcgen05 with the DEQUANTISED WEIGHTS AS THE
 // A OPERAND IN TENSOR MEMORY (replaces the matrix-unit GEMMs of int4_matmul.gen.ts:1058-1456; contract of
 // ztvm_int4_matmul for M > 16). W16 = f16_rne(fl32(s * q + b)) (or s * (q - 7)), the value the reference's numpy
 // dequantiser produces (scripts/make-dsv2-layer-ref.py:108-116); f32 accumulation in tensor memory.
@@ -35,6 +35,7 @@
 // share; at the end every CTA sends its f32 partial sums of token slice j to CTA j through distributed shared memory, and
 // each reduces and stores its own slice, in CTA order.
 #include "ztvm_kernels.h"
+#include "ztvm_stream_mma.cuh"
 #include "ztvm_tc.cuh"
 
 namespace ztvm {
@@ -88,18 +89,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                : "r"(taddr) : "memory");
 }
-// two f32 at a time (fma.rn.f32x2)
-__device__ __forceinline__ unsigned long long ta_pk(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long ta_ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // acc + the two halves of h
 __device__ __forceinline__ float ta_add2(float acc, uint32_t h) {
   asm("{\n\t.reg .f16 a, b, one;\n\tmov.b16 one, 0x3C00;\n\tmov.b32 {a, b}, %1;\n\t"
@@ -364,7 +353,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             if (ok) {
               const uint8_t* const sp = sb_row + sbs * L::kSbBytes + ((d & 1u) * kTaWChunk + team) * 2u;
               const float sf = __half2float(*reinterpret_cast<const __half*>(sp)), bf = __half2float(*reinterpret_cast<const __half*>(sp + b_delta));
-              const unsigned long long s2 = ta_pk(sf * 16777216.f, sf * 16777216.f), b2 = ta_pk(bf, bf);
+              const unsigned long long s2 = tc_pk(sf * 16777216.f, sf * 16777216.f), b2 = tc_pk(bf, bf);
               const ulonglong2* const xs = reinterpret_cast<const ulonglong2*>(xsum + (d & 1u) * (kTaStages * NT));
 #pragma unroll
               for (int h = 0; h < NT / 16; ++h) {
@@ -376,8 +365,8 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 for (int i = 0; i < 4; ++i) {
                   const ulonglong2 x = xs[4 * h + i];
                   unsigned long long* const to = sum + 8 * h + 2 * i;
-                  to[0] = ta_ffma2(b2, x.x, ta_ffma2(s2, ta_pk(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1])), to[0]));
-                  to[1] = ta_ffma2(b2, x.y, ta_ffma2(s2, ta_pk(__uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3])), to[1]));
+                  to[0] = tc_ffma2(b2, x.x, tc_ffma2(s2, tc_pk(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1])), to[0]));
+                  to[1] = tc_ffma2(b2, x.y, tc_ffma2(s2, tc_pk(__uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3])), to[1]));
                 }
               }
             }
