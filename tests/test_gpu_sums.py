@@ -84,6 +84,31 @@ def test_small_activations_of_3_bit_rows(K, size, backend, dev, oracle_c):
         assert np.linalg.norm(got - ref) <= 2.0**-11 * np.linalg.norm(ref) + 2.0**-25 * np.sqrt(N)
 
 
+@pytest.mark.parametrize("K", [256, 1536, 4352])
+@pytest.mark.parametrize("size", [1.0, 2.0**-10, 2.0**-14])
+def test_small_activations_of_whole_3_bit_slices(K, size, backend, dev, oracle_c):
+    """K % 256 == 0: an activation under a code's power of two (1/32 at most) is f16 again, off by 2^-25 * 32 = 2^-20 where it falls among
+    the subnormals; beside that, f32 sums that the matrix unit truncates, and the rounding to f16."""
+    rng = np.random.default_rng(K)
+    N = 333
+    _, W, s, b = z.synth.make_weights(rng, N, K, bits=3, sigma_s=0.02)
+    x = (z.synth.make_x(rng, 1, K) * np.float32(size)).astype(np.float16)
+    ref = oracle_c.matmul_f64(x, W, s, b, 64, 3, True)
+    mags = oracle_c.matmul_f64(np.abs(x), W, s, np.abs(b), 64, 3, True)
+    codes = oracle_c.matmul_f64(np.ones_like(x), W, s, np.zeros_like(b), 64, 3, True)
+    args = [dev.put(x), dev.put(s), dev.put(W), dev.put(b)]
+    ys = [dev.empty((1, N), np.float16, fill=9.0) for _ in range(3)]
+    backend.ctx.int4_matmul(z.MmDesc(K, N, 1, 64, 3, 1, 0), ys[0], *args)
+    backend.ctx.step_begin()
+    for y in ys[1:]:
+        backend.ctx.int4_matmul(z.MmDesc(K, N, 1, 64, 3, 1, 0), y, *args)
+    backend.ctx.step_end()
+    backend.ctx.sync()
+    for y in ys:
+        got = dev.get(y).astype(np.float64)
+        assert (np.abs(got - ref) <= 2.0**-11 * np.abs(ref) + 2.0**-25 + 1.001 * (2.0**-20 * codes + (K / 16 + 3 * K / 64 + 20) * 2.0**-23 * mags)).all()
+
+
 @pytest.mark.parametrize("symmetric,N,K", [(False, 60000, 320), (False, 9000, 2112), (False, 1200, 9024), (True, 60000, 320), (True, 4096, 8192), (True, 1200, 9024)])
 def test_single_rows_round_the_f32_result(symmetric, N, K, backend, dev):
     """4-bit rows of K % 256 != 0 or groups of 32 by themselves: one kernel whatever the result's type, so f16 results are the f32 ones rounded."""
