@@ -459,14 +459,11 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           const uint8_t* const sp = sb_row + ss * L::kSbBytes + (k0 >> p.group_shift) * 2u;
           const DqGroup dq = dq_group<AFFINE>(*reinterpret_cast<const unsigned short*>(sp),
                                               AFFINE ? *reinterpret_cast<const unsigned short*>(sp + b_delta) : (unsigned short)0);
-          dequant_words_w16<AFFINE>(w0, dq, a);
-          if (p.group_shift == 5) {                     // the second half of the block is the next group
-            const DqGroup dq2 = dq_group<AFFINE>(*reinterpret_cast<const unsigned short*>(sp + 2),
-                                                 AFFINE ? *reinterpret_cast<const unsigned short*>(sp + b_delta + 2) : (unsigned short)0);
-            dequant_words_w16<AFFINE>(w1, dq2, a + 16);
-          } else {
-            dequant_words_w16<AFFINE>(w1, dq, a + 16);
-          }
+          DqGroup dq2 = dq;
+          if (p.group_shift == 5)                       // the second half of the block is the next group
+            dq2 = dq_group<AFFINE>(*reinterpret_cast<const unsigned short*>(sp + 2),
+                                   AFFINE ? *reinterpret_cast<const unsigned short*>(sp + b_delta + 2) : (unsigned short)0);
+          dequant_block_w16<AFFINE>(w0, w1, dq, dq2, a);
         }
         // the TMEM slice of this stage was last read by the MMAs of the block one slot back
         if (ok && c > 0) {
