@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libztvm_b200.so")
 SOURCES = ["ztvm_api.cu", "ztvm_gemv.cu", "ztvm_gemv_mma.cu", "ztvm_gemv_tc.cu", "ztvm_gemv_tc_w4.cu", "ztvm_gemv_tc_w4sym.cu", "ztvm_gemv_tc_w4g32.cu", "ztvm_gemv_tc_w8.cu", "ztvm_gemv_tc3.cu", "ztvm_step.cu", "ztvm_step_w4.cu", "ztvm_step_w4g32.cu", "ztvm_step_w8.cu", "ztvm_step_w3.cu", "ztvm_batch_mma.cu", "ztvm_gemm_ta.cu", "ztvm_moe_gemm.cu", "ztvm_moe_ta.cu", "ztvm_moe_ep.cu", "ztvm_moe_tc.cu", "ztvm_glue.cu"]
-HEADERS = ["ztvm_device.cuh", "ztvm_tc.cuh", "ztvm_stream_mma.cuh", "ztvm_frag.cuh", "ztvm_gemv_tc.cuh", "ztvm_step.cuh", "ztvm_step.h", "ztvm_moe_plan.cuh", "ztvm_kernels.h", "ztvm_workbuf.h", os.path.join("..", "..", "include", "ztvm_b200.h")]
+HEADERS = ["ztvm_device.cuh", "ztvm_tc.cuh", "ztvm_stream_mma.cuh", "ztvm_frag.cuh", "ztvm_gemv_tc.cuh", "ztvm_step.cuh", "ztvm_step.h", "ztvm_moe_plan.cuh", "ztvm_moe_tile.cuh", "ztvm_kernels.h", "ztvm_workbuf.h", os.path.join("..", "..", "include", "ztvm_b200.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

@@ -642,13 +642,21 @@ static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::Ge
   const int tiles = ctx->moe_tiles_sm ? (sm_ok ? 3 : ta_ok ? 1 : 0) : (ta_ok ? 1 : sm_ok ? 3 : 0);
   const bool stream_ok = ztvm::moe_tc_supported(p, (int)d->bits) && !p.dst_index;
   // The tiles cost the same whatever the pair count (every expert's weights are dequantised once), the streaming kernel grows
-  // with the 8-pair chunks it walks. 257 experts, plan kept, us: gate / up, 512 x 2048: tiles 69, streaming 49 / 54 / 68 / 80 / 91
-  // at 4 / 6 / 8 / 10 / 12 pairs per expert; down, 2048 x 512: tiles 68, streaming 58 / 69 / 80 / 98 / 115 at 2 / 4 / 6 / 8 / 10.
-  // (64 experts: 21 against 18 / 19 / 21 / 25 at 4 / 6 / 8 / 10, 22 against 22 / 24 / 28 / 35.) So they meet at eight and four
-  // pairs per expert. The line is at ten for all three projections of a block: below it they keep exact codes and f32 weights,
+  // with the 8-pair chunks it walks. 257 experts, plan kept, us: gate / up, 512 x 2048: tiles 70, streaming 43 / 48 / 58 / 68
+  // at 4 / 6 / 8 / 10 pairs per expert; down, 2048 x 512: tiles 68, streaming 43 / 50 / 54 / 66 / 76 at 2 / 4 / 6 / 8 / 10. So they meet at ten
+  // and at eight pairs per expert. The line is at ten for all three projections of a block: below it they keep exact codes and f32 weights,
   // which the tiles round to f16, and one kernel, whose plan they share.
   const bool few_per_expert = pairs < 10ull * md->experts;
-  if (d->bits == 3) return ztvm::batch_moe_supported(p, 3) ? 4 : 0;    // exact codes at every pair count
+  // 3-bit codes stay exact at every pair count: streamed where that leaves at most a quarter of the sixteen warps without a slice, else on the
+  // batched kernel, whose tiles unpack a code for 16 pairs and more. us, streamed against it, 257 experts: 512 x 2048 30 : 40, 44 : 57, 59 : 65
+  // and 70 : 69 at 1 / 4 / 8 / 10 pairs per expert, 2048 x 512 30 : 42, 49 : 67, 65 : 73, 79 : 76; 40 experts of 2048 x 2304, nine slices, 27 : 26, 37 : 42, 51 : 45.
+  // The K of a block's other projections is this one's N: all of them stream or none, as they share a plan (54 experts, 1408 and 256 wide, 40
+  // pairs, a plan for the down projection alone: 31 us a block became 36).
+  auto fills = [](uint32_t k) { return k % 256u == 0 && k / 256u <= 16u && 16u / (k / 256u) * (k / 256u) >= 12u; };
+  if (d->bits == 3) {
+    const bool streams = stream_ok && (forced == 2 || (forced != 1 && pairs < 9ull * md->experts && fills(d->K) && fills(d->N)));
+    return streams ? 2 : ztvm::batch_moe_supported(p, 3) ? 4 : 0;
+  }
   // A K that the streaming kernel does not take: the batched kernel, exact codes as well, holds its place (257 experts of 512 x
   // 2240, us: 55 / 63 / 67 at 4 / 8 / 10 pairs per expert against 80 on the tiles).
   if (forced < 0 && !stream_ok && few_per_expert && !p.dst_index && !p.seg_counts && ztvm::batch_moe_supported(p, 4)) return 4;
@@ -753,7 +761,7 @@ ztvm_status ztvm_int4_matmul_moe(ztvm_ctx* ctx, const ztvm_moe_desc* md, void* y
     const bool reuse = ctx->plan_reuse && pick != 3 && buf->plan == key;
     buf->plan.ids = nullptr;
     if (pick == 4) ZTVM_CUDA(ztvm::launch_batch_moe(p, (int)d->bits, md->tokens, md->slots, ws, st, reuse));
-    else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
+    else if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, (int)d->bits, md->tokens, md->slots, ws, ctx->sm_count, st, reuse));
     else if (pick == 1) ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, md->slots, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
     else ZTVM_CUDA(ztvm::launch_moe_grouped(p, md->tokens, md->slots, ws, ctx->err_counter + 1, st));
     if (pick != 3) buf->plan = key;
@@ -929,7 +937,8 @@ ztvm_status ztvm_int4_matmul_moe_ep(ztvm_ctx* ctx, const ztvm_moe_desc* md, cons
   p.seg_counts = rows->seg_counts; p.seg_cap = rows->seg_cap; p.dst_index = rows->dst_index;
   for (uint32_t i = 0; i < rows->segments; ++i) p.y_seg[i] = rows->y_seg[i];
   const int pick = moe_pick(ctx, md, p, y_check);
-  if (pick != 1 && pick != 2)
+  // (moe_pick also takes 3-bit codes and any N: this entry point's contract does not)
+  if ((pick != 1 && pick != 2) || d->bits != 4 || d->N % 8)
     return fail(ZTVM_ERR_UNSUPPORTED, "the expert-parallel form runs the grouped kernels only: bits=4, group=64, K %% 64 == 0 "
                 "(got bits=%u group=%u K=%u N=%u)", d->bits, d->group, d->K, d->N);
   ztvm::WorkBuf* buf = nullptr;
@@ -939,7 +948,7 @@ ztvm_status ztvm_int4_matmul_moe_ep(ztvm_ctx* ctx, const ztvm_moe_desc* md, cons
   const bool reuse = rows->reuse_plan && buf->plan == key;
   buf->plan.ids = nullptr;
   uint32_t* ws = static_cast<uint32_t*>(buf->p);
-  if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, md->tokens, 1, ws, ctx->sm_count, st, reuse));
+  if (pick == 2) ZTVM_CUDA(ztvm::launch_moe_tc(p, 4, md->tokens, 1, ws, ctx->sm_count, st, reuse));
   else ZTVM_CUDA(ztvm::launch_moe_ta(p, md->tokens, 1, ws, ctx->err_counter + 1, ctx->sm_count, st, reuse));
   buf->plan = key;
   return ZTVM_OK;

@@ -161,15 +161,15 @@ __device__ __forceinline__ void codes3_inplace(const uint32_t (&w)[6], int k, ui
   r1 = v & (k < 15 ? kM1 : (kM1 & 0xFFFFu));
 }
 
-// Sixteen consecutive codes (48 bits: f0 = the first 32, the low half of f1 = the rest) as eight registers of code pairs
+// Sixteen consecutive codes (48 bits of the two words w0, w1, from bit 0 or, `odd`, bit 16 on) as eight registers of code pairs
 // (i | i + 8): r[i / 2] for even i holds fields at bits 0..2 of each half (q * 2^-24), r[4 + i / 2] holds codes
 // (i + 1 | i + 9) at bits 3..5 (q * 2^-21). Both halves of a register carry the same power of two, so the activations
 // go in unscaled. Bits of a neighbouring half that a shift drags along land above bit 5 and are masked off.
-__device__ __forceinline__ void codes3_inplace16(uint32_t f0, uint32_t f1, uint32_t (&r)[8]) {
-  const uint32_t fh = __funnelshift_r(f0, f1, 24);            // codes 8..15 from bit 0
-  const uint32_t p0 = __byte_perm(f0, fh, 0x5410);            // bits 0..15 of both runs of eight codes
-  const uint32_t p1 = __byte_perm(f0, fh, 0x6521);            // bits 8..23
-  const uint32_t v[4] = {p0, p0 >> 6, p1 >> 4, p1 >> 10};     // codes 0,1 | 2,3 | 4,5 | 6,7 (and + 8) at bits 0, 3
+// Eight codes are three bytes, so two byte permutations find the views wherever the 48 bits start (13 instructions for 16 codes).
+__device__ __forceinline__ void codes3_inplace16(uint32_t w0, uint32_t w1, bool odd, uint32_t (&r)[8]) {
+  const uint32_t p0 = __byte_perm(w0, w1, odd ? 0x6532u : 0x4310u);   // bits 0..15 of both runs of eight codes
+  const uint32_t p1 = __byte_perm(w0, w1, odd ? 0x7643u : 0x5421u);   // bits 8..23
+  const uint32_t v[4] = {p0, p0 >> 6, p1 >> 4, p1 >> 10};             // codes 0,1 | 2,3 | 4,5 | 6,7 (and + 8) at bits 0, 3
 #pragma unroll
   for (int i = 0; i < 4; ++i) { r[i] = v[i] & 0x00070007u; r[4 + i] = v[i] & 0x00380038u; }
 }

@@ -65,14 +65,13 @@ struct Frag<3> {
   static constexpr int kRunBytes = 24;
   static constexpr bool kTwoClasses = true;
   static constexpr float kUnit = 2097152.f, kRatio = 8.f;
-  struct Raw { uint32_t f0, f1; };   // the lane's 48 bits (f1: 16 valid bits, rubbish above)
+  struct Raw { uint32_t w0, w1; bool odd; };   // the words around the lane's 48 bits, which start in the middle of the first in odd lanes
   // byte 6c of the run: words 0,1 | 1,2 | 3,4 | 4,5; odd lanes start in the middle of their first word
   __host__ __device__ static constexpr uint32_t lane_byte(int c) { return (6u * (uint32_t)c) & ~3u; }
   __device__ __forceinline__ static Raw load(const uint8_t* p, int c) {
-    const uint32_t w0 = *reinterpret_cast<const uint32_t*>(p), w1 = *reinterpret_cast<const uint32_t*>(p + 4), sh = ((uint32_t)c & 1u) << 4;
-    return Raw{__funnelshift_r(w0, w1, sh), w1 >> sh};
+    return Raw{*reinterpret_cast<const uint32_t*>(p), *reinterpret_cast<const uint32_t*>(p + 4), (c & 1) != 0};
   }
-  __device__ __forceinline__ static void a(const Raw& v, uint32_t (&r)[8]) { codes3_inplace16(v.f0, v.f1, r); }
+  __device__ __forceinline__ static void a(const Raw& v, uint32_t (&r)[8]) { codes3_inplace16(v.w0, v.w1, v.odd, r); }
   __device__ __forceinline__ static void b(const uint4& x0, const uint4& x1, uint32_t (&r)[8]) {
     r[0] = __byte_perm(x0.x, x1.x, 0x5410); r[1] = __byte_perm(x0.y, x1.y, 0x5410);   // codes (0 | 8), (2 | 10)
     r[2] = __byte_perm(x0.z, x1.z, 0x5410); r[3] = __byte_perm(x0.w, x1.w, 0x5410);   // codes (4 | 12), (6 | 14)

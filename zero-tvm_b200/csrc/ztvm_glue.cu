@@ -132,7 +132,7 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
       for (int q = 0; q < 4; ++q) {
         const int j = 3 * q / 2, sh = (q & 1) * 16;
         uint32_t r[8];
-        codes3_inplace16(__funnelshift_r(w[j], w[j + 1], sh), w[j + 1] >> sh, r);
+        codes3_inplace16(w[j], w[j + 1], sh != 0u, r);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll

@@ -123,7 +123,7 @@ constexpr uint32_t kMoeTaTileRows = 128, kMoeTcTileRows = 8;   // pairs per tile
 // Streaming form of the grouped MoE matmul (ztvm_moe_tc.cu) for launches where an expert sees only a few pairs: bound
 // by reading each active expert's weights once. Same scratch as launch_moe_grouped.
 bool moe_tc_supported(const GemvParams& g, int bits);
-cudaError_t launch_moe_tc(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t* scratch, int sm_count,
+cudaError_t launch_moe_tc(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, int sm_count,
                           cudaStream_t st, bool reuse_plan = false);
 // Dispatch plan of the expert-parallel form: pairs in owner-rank order, their local expert index, pairs per rank.
 cudaError_t launch_moe_dispatch_plan(const GemvParams& g, uint32_t tokens, uint32_t slots, uint32_t epr, uint32_t world,

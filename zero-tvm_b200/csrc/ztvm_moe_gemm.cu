@@ -664,7 +664,7 @@ cudaError_t launch_moe_tc_static(const GemvParams& g, uint32_t tokens, uint32_t 
   uint32_t* scratch = nullptr;
   const cudaError_t e = moe_static_scratch_ptr(&scratch);
   if (e != cudaSuccess) return e;
-  return launch_moe_tc(g, tokens, slots, scratch, sm_count, st);   // its plan launch clears what must start at zero
+  return launch_moe_tc(g, 4, tokens, slots, scratch, sm_count, st);   // its plan launch clears what must start at zero
 }
 
 cudaError_t launch_batch_moe_static(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, cudaStream_t st) {
