@@ -33,7 +33,9 @@
 //
 // Few tiles (short prompts, small N): the K range is split over a cluster of CTAs. Each CTA keeps the k blocks of its
 // share; at the end every CTA sends its f32 partial sums of token slice j to CTA j through distributed shared memory, and
-// each reduces and stores its own slice, in CTA order.
+// each reduces and stores its own slice, in CTA order. The sums travel as whole 512-byte rows of a warp, into a place of their own where there is
+// room: a CTA then waits for the others to have started, not to have finished (stores 32 bytes apart into the idle rings, behind a barrier of the
+// whole cluster: 4096 x 4096, 128 rows 15.7 us, now 12.9; 200 rows 19.4, 15.1; 3072 x 8192, 128 rows 17.6, 14.7).
 #include "ztvm_kernels.h"
 #include "ztvm_stream_mma.cuh"
 #include "ztvm_tc.cuh"
@@ -73,7 +75,12 @@ struct GemmTaSmem {
   static constexpr int kOffSb = kOffW + kWStages * kWBytes;
   static constexpr int kOffBar = kOffSb + kTaSbStages * kSbBytes;
   static constexpr int kOffXsum = kOffBar + 256;              // 8-bit: sums of a block's activations per token, two rounds of the stages
-  static constexpr int kTotal = kOffXsum + (BITS == 8 ? 2 * kTaStages * NT * 4 : 0);
+  // Partial sums that the other CTAs of a cluster send: a place of their own where there is room, else the idle rings.
+  static constexpr bool kApart = NT <= 128 && BITS == 4;
+  static constexpr int kPartBytes = (NT + 56) * kTaRows * 4;
+  static constexpr int kOffPart = kApart ? (kOffXsum + 127) / 128 * 128 : 0;
+  static constexpr int kTotal = kApart ? kOffPart + kPartBytes : kOffXsum + (BITS == 8 ? 2 * kTaStages * NT * 4 : 0);
+  static_assert(kTotal + 1024 <= 227 * 1024 && (kApart || kPartBytes <= kTaStages * kXBytes + kWStages * kWBytes), "shared memory of a CTA");
   static constexpr int kAccs = BITS == 8 ? kTaStages : 1;     // accumulators: 8-bit blocks have one each
 };
 
@@ -206,6 +213,8 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // (that this CTA runs, so that the others of its cluster may write to its shared memory)
+  if (L::kApart && split > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -560,12 +569,12 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     }
   }
   if (split > 1) {
-    // ---- K shares meet: token blocks of eight, dealt to the CTAs in runs of `per`; partial sums as [sender][block][row][8
-    // tokens] in the receiver's idle rings. Every thread of the cluster takes both barriers, whatever became of its waits.
+    // ---- K shares meet: token blocks of eight, dealt to the CTAs in runs of `per`; partial sums as [sender][block][half][row][4
+    // tokens], so that a warp's stores and loads are contiguous. Every thread of the cluster takes both barriers, whatever became of its waits.
     const uint32_t nb = (mrows + 7u) / 8u, per = (nb + split - 1) / split;
-    static_assert((NT + 56) * kTaRows * 4 <= kTaStages * L::kXBytes + L::kWStages * L::kWBytes, "partial sums of the other CTAs fit the rings");
     __syncwarp();
-    cluster_sync_all();                                  // every CTA's MMAs have read its rings for the last time
+    if constexpr (L::kApart) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else cluster_sync_all();                             // every CTA's MMAs have read its rings for the last time
     if (is_dq && acc_ok) {
       for (uint32_t b = wpart; b < nb; b += 4u) {
         const uint32_t to = b / per;
@@ -575,10 +584,10 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         tmem_ld_wait();
         const uint32_t slot = kz < to ? kz : kz - 1u;     // the receiver's own sums stay in its tensor memory
         uint32_t dst;
-        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(base + (((slot * per + b - to * per) * kTaRows + r_tile) * 32u)), "r"(to));
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(base + L::kOffPart + (((slot * per + b - to * per) * 2u * kTaRows + r_tile) * 16u)), "r"(to));
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-          asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16u * i), "r"(v[4 * i]), "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3]) : "memory");
+          asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(kTaRows * 16) * i), "r"(v[4 * i]), "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3]) : "memory");
       }
     }
     __syncwarp();
@@ -598,8 +607,8 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 #pragma unroll
               for (int i = 0; i < 8; ++i) r[i] += __uint_as_float(v[i]);
             } else {
-              const float4* const got = reinterpret_cast<const float4*>(gen_base) + (((z < kz ? z : z - 1u) * per + b - kz * per) * kTaRows + r_tile) * 2u;
-              const float4 g0 = got[0], g1 = got[1];
+              const float4* const got = reinterpret_cast<const float4*>(gen_base + L::kOffPart) + ((z < kz ? z : z - 1u) * per + b - kz * per) * 2u * kTaRows + r_tile;
+              const float4 g0 = got[0], g1 = got[kTaRows];
               r[0] += g0.x; r[1] += g0.y; r[2] += g0.z; r[3] += g0.w;
               r[4] += g1.x; r[5] += g1.y; r[6] += g1.z; r[7] += g1.w;
             }
@@ -708,11 +717,12 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
                            int bits, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count, cudaStream_t st) {
   TaEncodeFn enc = ta_encode_fn();
   if (!enc) return cudaErrorNotSupported;
-  // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 8192 x 2048 .. 3072 x 8192:
-  // a k block takes 340 + 1.4 per token (at least 390), a CTA 8500 to start, fill its rings and store, the exchange of
-  // a cluster 5300 + 12 per token. Clusters run in as many waves as the device can place. The tokens are dealt evenly to
-  // the tiles. (Groups of 32 with biases do not fit beside the widest tile.) 8-bit: tiles of up to
-  // 64 tokens, a block 700 + 2 per token; the exchange more for every share beyond two.
+  // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 2048 x 1024 .. 4096 x 12288, 24 to 512 rows:
+  // a k block takes 340 + 1.4 per token, with biases at least 500, without 415; a CTA 6500 to start, fill its rings and store; the exchange of a
+  // cluster 1500 + 34 per token, 8 per tile and 1200 for every share beyond two. (4096 x 4096, 128 rows, us: one share 19.7, two 15.0, three 14.1, four 12.9;
+  // 9216 x 3072, 200 rows, whole-K tiles of 100 tokens 14.3, two shares of 200 15.2; 2048 x 1024, 24 rows 7.0 : 6.1.) Clusters run in as many
+  // waves as the device can place. The tokens are dealt evenly to the tiles. (Groups of 32 with biases do not fit beside the widest tile.)
+  // 8-bit: tiles of up to 64 tokens, a block 700 + 2 per token, 8500 and 5300 + 12 per token; the exchange more for every share beyond two.
   const uint32_t units = (K / kGemmBK + kTaSbChunk - 1) / kTaSbChunk, n_tiles = (N + kTaRows - 1) / kTaRows;
   const uint32_t widest = bits == 8 ? 64u : B && group_shift == 5 ? 256u : 352u;
   uint32_t tile_m = 0, split = 1;
@@ -721,12 +731,14 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
     if (t > 64u && t - 32u >= M) break;
     const uint32_t m_tiles = (M + t - 1) / t, tm = ((M + m_tiles - 1) / m_tiles + 15u) & ~15u;
     const uint64_t tiles = (uint64_t)n_tiles * m_tiles;
-    const uint32_t live = M < tm ? M : tm, block = bits == 8 ? 700u + 2u * live : live < 36u ? 390u : 340u + live * 14u / 10u;
+    const uint32_t live = M < tm ? M : tm, least = B ? 500u : 415u;
+    const uint32_t block = bits == 8 ? 700u + 2u * live : 340u + live * 14u / 10u < least ? least : 340u + live * 14u / 10u;
     for (uint32_t z = 1; z <= (uint32_t)kTaMaxSplit && z <= units; ++z) {
       if (z > 1 && tiles * z > (uint64_t)sm_count) break;
       const uint32_t at_once = bits == 8 ? ta_at_once<8>(tm, z, sm_count) : ta_at_once<4>(tm, z, sm_count);
       const uint64_t waves = (tiles + at_once - 1) / at_once;
-      const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + 8500u + (z > 1 ? 5300u + 12u * live + (bits == 8 && z > 2 ? 28u * live * (z - 2) : 0u) : 0u));
+      const uint32_t more = z > 2 ? z - 2u : 0u, exchange = z == 1 ? 0u : bits == 8 ? 5300u + (12u + 28u * more) * live : 1500u + 34u * live + 8u * (uint32_t)tiles + 1200u * more;
+      const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + (bits == 8 ? 8500u : 6500u) + exchange);
       if (cost < best) { best = cost; tile_m = tm; split = z; }
     }
   }
