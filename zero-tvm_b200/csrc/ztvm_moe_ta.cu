@@ -31,7 +31,7 @@ namespace ztvm {
 
 constexpr int kMtaStages = 4;        // weight slices in tensor memory (64 k elements x two row halves each)
 constexpr int kMtaXStages = 4;       // activation tiles in shared memory (64 k elements each), a ring of their own
-constexpr int kMtaWStages = 4;       // packed-weight ring; a slot holds four k blocks of both row halves
+constexpr int kMtaWStages = 2;       // packed-weight ring; a slot holds four k blocks of both row halves, 2.4 us of work
 constexpr int kMtaWChunk = 4;        // k blocks per packed-weight slot
 constexpr int kMtaNP = 128;          // pairs per tile = widest MMA N used
 constexpr int kMtaRows = 128;        // weight rows per half = TMEM lanes
@@ -67,10 +67,11 @@ struct MtaSmem {
   static constexpr int kOffW = kMtaXStages * kXBytes;
   static constexpr int kOffBar = kOffW + kMtaWStages * kWBytes;
   static constexpr int kOffUnits = kOffBar + 256;                // this CTA's first kMtaUnitTable units: expert, r0, rows, n0
-  static constexpr int kStagePitch = kMtaUnitRows * 2;           // epilogue stage: 32 pairs x 256 weight rows, f16
+  static constexpr int kStagePitch = kMtaUnitRows * 2;           // epilogue stage: a unit's pairs x 256 weight rows, f16
   static constexpr int kOffStage = kOffUnits + kMtaUnitTable * 16;
-  static constexpr int kOffDst = kOffStage + 32 * kStagePitch;   // output row address of each pair of a unit, two units
+  static constexpr int kOffDst = kOffStage + kMtaNP * kStagePitch;   // output row address of each pair of a unit, two units
   static constexpr int kTotal = kOffDst + 2 * kMtaNP * 8;
+  static_assert(kTotal + 1024 <= 227 * 1024, "shared memory of a CTA");
 };
 
 // Named barrier 1: the epilogue warps among themselves (barrier 0 is __syncthreads).
@@ -393,7 +394,9 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
   } else {
     // ================= epilogue: D[weight row][pair] in TMEM -> y rows of the pairs =================
     // A thread holds one weight row of 32 pairs, an output row wants 256 weight rows of one pair side by side: the tile
-    // turns round in shared memory, 32 pairs at a time. Phase 1: every thread stores its 32 values as f16 into
+    // turns round in shared memory, all of its pairs at once, so that the accumulators are free before the first row is out (32 pairs at a
+    // time the next unit's MMAs waited for 3800 cycles of some 11000 at K = 512: 72 pairs each, 257 experts of 2048 x 512 85.5 us, now 76.3, of
+    // 512 x 2048 77.0, 70.5). Phase 1: every thread stores its values as f16 into
     // stage[pair][weight row] (a warp's 32 lanes fill 64 consecutive bytes). Phase 2: a warp reads one pair's 512 bytes
     // (16 per lane) and stores them to the pair's output row in one instruction. The accumulators are free again as
     // soon as the last 32 pairs have been read, before their rows have left.
@@ -430,36 +433,34 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
       if (!ep_bar_and(got)) break;
       tc_fence_after();
       const bool two = n0 + kMtaRows < p.N;
-      const uint32_t ncb = (rows + 31u) / 32u;
-      for (uint32_t cb = 0; cb < ncb; ++cb) {
-        const uint32_t lim = min(32u, rows - cb * 32u);
+      // (the stage is free: the rows of the unit before were out when the last of the four warps came to the barrier above)
+      for (uint32_t cb = 0; cb * 32u < rows; ++cb) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (h == 1 && !two) break;                                   // warp-uniform
           uint32_t v[32];
           tmem_ld32(tmem_base + lane_base + (uint32_t)h * kMtaNP + cb * 32u, v);
           tmem_ld_wait();
-          const uint32_t col = stage + ((uint32_t)h * kMtaRows + r_half) * 2u;
+          const uint32_t col = stage + cb * (32u * (uint32_t)L::kStagePitch) + ((uint32_t)h * kMtaRows + r_half) * 2u;
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             const unsigned short hv = __half_as_ushort(__float2half_rn(__uint_as_float(v[i])));
             asm volatile("st.shared.u16 [%0], %1;" ::"r"(col + (uint32_t)i * (uint32_t)L::kStagePitch), "h"(hv) : "memory");
           }
         }
-        if (cb + 1 == ncb) {       // the accumulators have been read: the next unit's MMAs may start
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_acc_empty);
-        }
-        ep_bar();
+      }
+      // the accumulators have been read: the next unit's MMAs may start
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_acc_empty);
+      ep_bar();
+      {
         // rows out: warp q takes pairs q, q + 4, ...; lane l the eight weight rows n0 + 8 l .. of the pair
         const uint32_t n = n0 + 8u * (uint32_t)lane;
         const bool mine = n < p.N && (two || lane < 16);               // N % 8 == 0: eight rows are in or out together
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint32_t i = (uint32_t)quarter + 4u * (uint32_t)j;
-          if (i >= lim) break;
-          __half* const d = reinterpret_cast<__half*>(dst_tab[cb * 32u + i]) + n;
+#pragma unroll 4
+        for (uint32_t i = (uint32_t)quarter; i < rows; i += 4u) {
+          __half* const d = reinterpret_cast<__half*>(dst_tab[i]) + n;
           if (mine) {
             const uint4 q = stage_g[i * (L::kStagePitch / 16) + lane];
             if (vec_out) {
@@ -474,7 +475,6 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
             }
           }
         }
-        ep_bar();                  // the stage is free for the next 32 pairs
       }
     }
   }
