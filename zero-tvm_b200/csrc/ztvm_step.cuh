@@ -299,9 +299,15 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
     }
     // 16-byte pieces; past K, up to whole slices: zeros
     const uint32_t pieces = (o.slices * (uint32_t)C::kSlice + 255u) / 256u * 32u, have = o.K / 8u;
-    for (uint32_t i = tid; i < pieces; i += kStepWarps * 32u) {
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (i < have) v = __ldcg(reinterpret_cast<const uint4*>(o.X) + i);      // (other SMs may just have written it)
+    // (a thread's pieces are asked for three at a time: a long row, one after the other, took a trip to L2 for each)
+    auto piece = [&](uint32_t i) {
+      return i < have ? __ldcg(reinterpret_cast<const uint4*>(o.X) + i) : make_uint4(0u, 0u, 0u, 0u);      // (other SMs may just have written it)
+    };
+    constexpr uint32_t kAll = kStepWarps * 32u;
+    uint4 v1 = piece(tid), v2 = piece(tid + kAll), v3 = piece(tid + 2u * kAll);
+    for (uint32_t i = tid; i < pieces; i += kAll) {
+      const uint4 v = v1;
+      v1 = v2; v2 = v3; v3 = piece(i + 3u * kAll);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
       float2 x[4];
 #pragma unroll
