@@ -52,11 +52,15 @@ __device__ __forceinline__ void tc_cp4_zfill(uint32_t dst, const void* src, uint
 // other groups), so the per-group fold after the MMAs is spread over the lanes of a quad instead of being repeated
 // by each of them: lane (g, c) owns columns 2c and 2c + 1.
 // AL: K is whole slices and the tables allow a slice's scales to be copied in one piece.
+// ONCE: a CTA's tiles are one block of rounds, and its sums stay in registers over all of K and meet once, so that the warps need not wait for one
+// another at every K tile. us, 8-bit (K tiles of 2048): 4096 x 12288, 4 rows 17.3 -> 15.5, 2048 x 6144 7.9 -> 7.3, 1024 x 8000 10.4 -> 9.5; 4-bit,
+// groups of 64 (of 4096): 4096 x 12288, 2 rows 12.2 -> 11.7, 8 rows 12.4 -> 11.8, but 4 rows 2048 x 7936 7.1 -> 7.2; groups of 32 lose by it (3072 x
+// 8192 9.1 -> 9.5). An instance of its own: as a choice at run time the longer-lived sums cost every other shape 4 %.
 // W = warps per CTA: 16 (one CTA per SM, the whole shared memory as its ring) for projections that keep an SM busy for
 // tens of microseconds; 8 (registers and shared memory halve) for small ones, so that a CTA of the NEXT launch in the stream
 // -- already started under programmatic dependent launch -- can sit beside this launch's and stream its first weights while it
 // finishes, instead of waiting for the SM to empty. Two CTAs of ONE launch must not: each has a fixed share of the rows.
-template <int BITS, bool G32, int NT, bool AFFINE, bool AL, int W>
+template <int BITS, bool G32, int NT, bool AFFINE, bool AL, int W, bool ONCE>
 __global__ void __launch_bounds__(W * 32, 16 / W)
 gemv_tc_kernel(const GemvParams p) {
   extern __shared__ __align__(128) uint8_t tc_smem[];
@@ -343,6 +347,7 @@ gemv_tc_kernel(const GemvParams p) {
         }
         __syncwarp();   // every lane is done with the stage before the next issue refills it
       }
+      if (ONCE && kt + 1 < num_kt) continue;
       // ---- meeting: K-slice partials of the block's rows -> shared, then one fixed-order sum per output --------
       float* mine = partial + ((size_t)((meet & 1u) * W + (uint32_t)warp) * kBlkRows) * NT;
 #pragma unroll
@@ -350,7 +355,7 @@ gemv_tc_kernel(const GemvParams p) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float2 av = tc_unpk(acc[q][h]);
-          float v0 = slice_ok ? av.x : 0.f, v1 = slice_ok ? av.y : 0.f;
+          float v0 = slice_ok || ONCE ? av.x : 0.f, v1 = slice_ok || ONCE ? av.y : 0.f;
           acc[q][h] = 0ull;
           float* dst = mine + (q * 16 + g + 8 * h) * NT;
           if constexpr (NT == 1) {          // the quad's columns are groups of token 0
@@ -381,7 +386,7 @@ gemv_tc_kernel(const GemvParams p) {
         if (row >= nrows || r16 >= tile_live(row & ~15u)) continue;
         float v = 0.f;
         for (uint32_t k2 = 0; k2 < KS; ++k2) v += buf[((size_t)(rgi * KS + k2) * kBlkRows + q * 16 + r16) * NT + tok];
-        if (num_kt > 1) {
+        if (num_kt > 1 && !ONCE) {
           float* a = acc_sm + (size_t)row * p.M + tok;
           if (kt) v += *a;
           if (kt + 1 < num_kt) { *a = v; continue; }
@@ -394,7 +399,7 @@ gemv_tc_kernel(const GemvParams p) {
           const uint32_t tg = tb - 1u, qg = tg / RG, rgg = tg - qg * RG;
           float gsum = 0.f;
           for (uint32_t k2 = 0; k2 < KS; ++k2) gsum += buf[((size_t)(rgg * KS + k2) * kBlkRows + qg * 16 + r16) * NT + tok];
-          if (num_kt > 1 && kt) gsum += acc_sm[(size_t)(row - 16u) * p.M + tok];
+          if (num_kt > 1 && !ONCE && kt) gsum += acc_sm[(size_t)(row - 16u) * p.M + tok];
           const float silu = gsum * (1.0f / (1.0f + expf(-gsum)));
           reinterpret_cast<__half*>(p.Y)[(size_t)tok * p.y_row_stride + r0 + (tile >> 1) * 16u + r16] = __float2half_rn(v * silu);
           continue;
@@ -456,9 +461,9 @@ inline bool tc_fits(const GemvParams& p, int sm_count) {
   return tc_smem<BITS, G32>(p, sm_count, w) <= tc_smem_limit(w);
 }
 
-template <int BITS, bool G32, int NT, bool AFFINE, bool AL, int W>
+template <int BITS, bool G32, int NT, bool AFFINE, bool AL, int W, bool ONCE = false>
 cudaError_t launch_tc_one(const GemvParams& p, unsigned grid, size_t smem, int sm_count, cudaStream_t st, HalfSm* half) {
-  auto kern = gemv_tc_kernel<BITS, G32, NT, AFFINE, AL, W>;
+  auto kern = gemv_tc_kernel<BITS, G32, NT, AFFINE, AL, W, ONCE>;
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -490,6 +495,17 @@ template <int BITS, bool G32, bool AFFINE, bool AL, int W>
 cudaError_t launch_tc_w(const GemvParams& p, int sm_count, cudaStream_t st, HalfSm* half) {
   const unsigned grid = tc_grid_for(p, sm_count);
   const size_t smem = tc_smem<BITS, G32>(p, sm_count, W);
+  if constexpr (W == 16 && !G32) {
+    const uint64_t rows = ((uint64_t)(p.pair_rows ? p.pair_rows : p.N) + grid - 1) / grid, tiles = p.pair_rows ? 2 * ((rows + 15) / 16) : (rows + 15) / 16;
+    if (tc_slices<BITS>(p) > (uint32_t)W && tiles <= (uint64_t)tc_rounds(tc_tokens(p))) {
+      switch (tc_tokens(p)) {
+        case 1: if constexpr (BITS == 8) return launch_tc_one<BITS, G32, 1, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half); break;
+        case 2: return launch_tc_one<BITS, G32, 2, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half);
+        case 4: if constexpr (BITS == 8) return launch_tc_one<BITS, G32, 4, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half); break;
+        default: return launch_tc_one<BITS, G32, 8, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half);
+      }
+    }
+  }
   switch (tc_tokens(p)) {
     case 1: return launch_tc_one<BITS, G32, 1, AFFINE, AL, W>(p, grid, smem, sm_count, st, half);
     case 2: return launch_tc_one<BITS, G32, 2, AFFINE, AL, W>(p, grid, smem, sm_count, st, half);
