@@ -33,7 +33,7 @@ def test_sums_that_meet_once(bits, N, K, M, backend, dev, oracle_c):
 
 
 def test_paired_form_meets_once(backend, dev):
-    D, F, M = 8192, 148 * 16, 2                                   # gate and up: two tiles a CTA
+    D, F, M = 8192, 148 * 16, 8                                   # gate and up: two tiles a CTA
     p = z.synth.projection(2 * F, D, M=M, bits=4, seed=5, sigma_s=0.01)
     h, gu = dev.empty((M, F), np.float16, fill=0.0), dev.empty((M, 2 * F), np.float16, fill=0.0)
     args = [dev.put(p[k]) for k in ("x", "scales", "W", "biases")]

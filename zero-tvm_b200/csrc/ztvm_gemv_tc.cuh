@@ -53,9 +53,11 @@ __device__ __forceinline__ void tc_cp4_zfill(uint32_t dst, const void* src, uint
 // by each of them: lane (g, c) owns columns 2c and 2c + 1.
 // AL: K is whole slices and the tables allow a slice's scales to be copied in one piece.
 // ONCE: a CTA's tiles are one block of rounds, and its sums stay in registers over all of K and meet once, so that the warps need not wait for one
-// another at every K tile. us, 8-bit (K tiles of 2048): 4096 x 12288, 4 rows 17.3 -> 15.5, 2048 x 6144 7.9 -> 7.3, 1024 x 8000 10.4 -> 9.5; 4-bit,
-// groups of 64 (of 4096): 4096 x 12288, 2 rows 12.2 -> 11.7, 8 rows 12.4 -> 11.8, but 4 rows 2048 x 7936 7.1 -> 7.2; groups of 32 lose by it (3072 x
-// 8192 9.1 -> 9.5). An instance of its own: as a choice at run time the longer-lived sums cost every other shape 4 %.
+// another at every K tile. us, 8-bit (K tiles of 2048), 2 to 8 rows: 4096 x 12288, 4 rows 17.1 -> 15.7, 2048 x 6144 7.9 -> 7.4, 1024 x 8000 10.4 -> 9.6;
+// 4-bit, groups of 64 (of 4096), 5 to 8 rows: 4096 x 12288 12.4 -> 11.8, 1536 x 9024 10.0 -> 9.8, but 4 rows 2048 x 7936 7.1 -> 7.2, 2 rows 2752 x 7040
+// 9.6 -> 9.9; groups of 32 lose by it (3072 x 8192 9.1 -> 9.5). An instance of its own: as a choice at run time the longer-lived sums cost every other
+// shape 4 %. A K tile's sums are added up before they join the rest: one running sum over all of K had up to 1.2 times the error (8 rows of 8-bit
+// 4096 x 12288, against 64 bits: 1.29e-7, so 1.13e-7, and 1.12e-7 where they meet at every K tile).
 // W = warps per CTA: 16 (one CTA per SM, the whole shared memory as its ring) for projections that keep an SM busy for
 // tens of microseconds; 8 (registers and shared memory halve) for small ones, so that a CTA of the NEXT launch in the stream
 // -- already started under programmatic dependent launch -- can sit beside this launch's and stream its first weights while it
@@ -255,6 +257,11 @@ gemv_tc_kernel(const GemvParams p) {
   unsigned long long acc[kTcRounds][2];   // per round and row half: the two columns of this lane, packed
 #pragma unroll
   for (int q = 0; q < kTcRounds; ++q) acc[q][0] = acc[q][1] = 0ull;
+  unsigned long long tot[ONCE ? kTcRounds : 1][2];   // ONCE: over the K tiles before
+  if constexpr (ONCE) {
+#pragma unroll
+    for (int q = 0; q < kTcRounds; ++q) tot[q][0] = tot[q][1] = 0ull;
+  }
   const unsigned long long kR = tc_pk(F::kTwoClasses ? F::kRatio : 1.f, F::kTwoClasses ? F::kRatio : 1.f);
   const float kZero[4] = {0.f, 0.f, 0.f, 0.f};
   const uint32_t swz = BITS == 8 ? (uint32_t)g & 1u : (uint32_t)g & 3u;
@@ -347,14 +354,23 @@ gemv_tc_kernel(const GemvParams p) {
         }
         __syncwarp();   // every lane is done with the stage before the next issue refills it
       }
-      if (ONCE && kt + 1 < num_kt) continue;
+      if constexpr (ONCE) {
+#pragma unroll
+        for (int q = 0; q < kTcRounds; ++q)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(tot[q][h]) : "l"(acc[q][h]));
+            acc[q][h] = 0ull;
+          }
+        if (kt + 1 < num_kt) continue;
+      }
       // ---- meeting: K-slice partials of the block's rows -> shared, then one fixed-order sum per output --------
       float* mine = partial + ((size_t)((meet & 1u) * W + (uint32_t)warp) * kBlkRows) * NT;
 #pragma unroll
       for (int q = 0; q < kTcRounds; ++q)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const float2 av = tc_unpk(acc[q][h]);
+          const float2 av = tc_unpk(ONCE ? tot[ONCE ? q : 0][h] : acc[q][h]);
           float v0 = slice_ok || ONCE ? av.x : 0.f, v1 = slice_ok || ONCE ? av.y : 0.f;
           acc[q][h] = 0ull;
           float* dst = mine + (q * 16 + g + 8 * h) * NT;
@@ -499,8 +515,8 @@ cudaError_t launch_tc_w(const GemvParams& p, int sm_count, cudaStream_t st, Half
     const uint64_t rows = ((uint64_t)(p.pair_rows ? p.pair_rows : p.N) + grid - 1) / grid, tiles = p.pair_rows ? 2 * ((rows + 15) / 16) : (rows + 15) / 16;
     if (tc_slices<BITS>(p) > (uint32_t)W && tiles <= (uint64_t)tc_rounds(tc_tokens(p))) {
       switch (tc_tokens(p)) {
-        case 1: if constexpr (BITS == 8) return launch_tc_one<BITS, G32, 1, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half); break;
-        case 2: return launch_tc_one<BITS, G32, 2, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half);
+        case 1: break;
+        case 2: if constexpr (BITS == 8) return launch_tc_one<BITS, G32, 2, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half); break;
         case 4: if constexpr (BITS == 8) return launch_tc_one<BITS, G32, 4, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half); break;
         default: return launch_tc_one<BITS, G32, 8, AFFINE, AL, W, true>(p, grid, smem, sm_count, st, half);
       }
