@@ -30,8 +30,8 @@ struct ztvm_ctx {
   uint32_t next_lane;
   void* d_y; size_t d_y_bytes;
   ztvm::WorkBufs* work;   // plans of the grouped MoE matmul, f32 gate/up rows of ztvm_fused_ffn's two-launch form
-  // env ZTVM_MOE_GROUPED (a measurement knob): 0 forces the per-pair GEMV, 1 the tensor-core tiles, 2 the streaming
-  // grouped kernel; unset = by size (few pairs per-pair; then the exact-code kernels while an expert sees few of them)
+  // env ZTVM_MOE_GROUPED (a measurement knob): 0 forces the per-pair GEMV, 1 the tensor-core tiles (3-bit codes: the
+  // batched exact-code kernel), 2 the streaming grouped kernel; unset = by size (few pairs per-pair; then the exact-code kernels while an expert sees few of them)
   int moe_grouped;
   int plan_reuse;   // ztvm_moe_plan_reuse: consecutive ztvm_int4_matmul_moe calls over one id list share its plan
   // The last call's last launch, for HalfSm: its weight bytes if it was a half-SM one, and its stream. `call`: the call being made.
@@ -631,7 +631,7 @@ ztvm_status ztvm_host_wait(ztvm_ctx* ctx) {
 
 // Which grouped kernel serves a MoE launch: 0 none (per-pair GEMV), 1 tensor-core tiles with the weights in tensor
 // memory, 2 streaming kernel, 3 tensor-core tiles with both operands in shared memory (ZTVM_MOE_TILES=sm, or shapes
-// only it takes), 4 the exact-code batched kernel (3-bit experts; 4-bit ones of few pairs over a K that 2 does not take). `forced` is the context's ZTVM_MOE_GROUPED knob (-1 = by size).
+// only it takes), 4 the exact-code batched kernel (what 2 leaves of 3-bit experts; 4-bit ones of few pairs over a K that 2 does not take). `forced` is the context's ZTVM_MOE_GROUPED knob (-1 = by size).
 static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::GemvParams& p, const void* y) {
   const int forced = ctx->moe_grouped;
   const ztvm_mm_desc* d = &md->mm;

@@ -2,7 +2,7 @@
 // activation rows, dense or grouped by expert, where the weights may not be rounded to f16 first:
 //   * router logits (moe_router_logits.wgsl: f32 sums over exact codes feed a softmax and a top-k),
 //   * 8-bit projections of 9 to 32 rows, and of any more with f32 results (int8_affine_batched.wgsl),
-//   * 3-bit expert matmuls (int4_matmul.gen.ts:229-254, :409-448), and 4-bit ones of few pairs per expert over a ragged K.
+//   * 3-bit expert matmuls that the streaming kernel leaves (int4_matmul.gen.ts:229-254, :409-448), and 4-bit ones of few pairs per expert over a ragged K.
 // Those used to run as slabs of eight rows (or, for experts, one GEMV per pair) on the CUDA cores.
 //
 // Codes enter the MMA as f16 subnormals masked in place (ztvm_frag.cuh): no dequantisation, exact products, one f32
