@@ -304,10 +304,12 @@ step_kernel(const __grid_constant__ StepProgramT<MAX> p) {
       return i < have ? __ldcg(reinterpret_cast<const uint4*>(o.X) + i) : make_uint4(0u, 0u, 0u, 0u);      // (other SMs may just have written it)
     };
     constexpr uint32_t kAll = kStepWarps * 32u;
-    uint4 v1 = piece(tid), v2 = piece(tid + kAll), v3 = piece(tid + 2u * kAll);
+    uint4 v1 = piece(tid), v2 = make_uint4(0u, 0u, 0u, 0u), v3 = v2;
+    if (pieces > kAll) { v2 = piece(tid + kAll); v3 = piece(tid + 2u * kAll); }
     for (uint32_t i = tid; i < pieces; i += kAll) {
       const uint4 v = v1;
-      v1 = v2; v2 = v3; v3 = piece(i + 3u * kAll);
+      v1 = v2; v2 = v3;
+      if (pieces > 3u * kAll) v3 = piece(i + 3u * kAll);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
       float2 x[4];
 #pragma unroll
