@@ -717,9 +717,10 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
                            int bits, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count, cudaStream_t st) {
   TaEncodeFn enc = ta_encode_fn();
   if (!enc) return cudaErrorNotSupported;
-  // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 2048 x 1024 .. 4096 x 12288, 24 to 512 rows:
+  // Tokens per tile and K shares, by the time of the busiest SM in cycles, from measurements on 1088 x 1088 .. 4096 x 12288, 20 to 512 rows:
   // a k block takes 340 + 1.4 per token, with biases at least 500, without 415; a CTA 6500 to start, fill its rings and store; the exchange of a
-  // cluster 1500 + 34 per token, 8 per tile and 1200 for every share beyond two. (4096 x 4096, 128 rows, us: one share 19.7, two 15.0, three 14.1, four 12.9;
+  // cluster 1500 + 34 per token, 8 per tile and 450 for every share beyond two. (4096 x 4096, 128 rows, us: one share 19.7, two 15.0, three 14.1, four 12.9;
+  // 1088 x 2944, 20 rows: three shares 7.7, six 6.8;
   // 9216 x 3072, 200 rows, whole-K tiles of 100 tokens 14.3, two shares of 200 15.2; 2048 x 1024, 24 rows 7.0 : 6.1.) Clusters run in as many
   // waves as the device can place. The tokens are dealt evenly to the tiles. (Groups of 32 with biases do not fit beside the widest tile.)
   // 8-bit: tiles of up to 64 tokens, a block 700 + 2 per token, 8500 and 5300 + 12 per token; the exchange more for every share beyond two.
@@ -737,7 +738,7 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
       if (z > 1 && tiles * z > (uint64_t)sm_count) break;
       const uint32_t at_once = bits == 8 ? ta_at_once<8>(tm, z, sm_count) : ta_at_once<4>(tm, z, sm_count);
       const uint64_t waves = (tiles + at_once - 1) / at_once;
-      const uint32_t more = z > 2 ? z - 2u : 0u, exchange = z == 1 ? 0u : bits == 8 ? 5300u + (12u + 28u * more) * live : 1500u + 34u * live + 8u * (uint32_t)tiles + 1200u * more;
+      const uint32_t more = z > 2 ? z - 2u : 0u, exchange = z == 1 ? 0u : bits == 8 ? 5300u + (12u + 28u * more) * live : 1500u + 34u * live + 8u * (uint32_t)tiles + 450u * more;
       const uint64_t cost = waves * ((z == 1 ? K / kGemmBK : (units + z - 1) / z * kTaSbChunk) * block + (bits == 8 ? 8500u : 6500u) + exchange);
       if (cost < best) { best = cost; tile_m = tm; split = z; }
     }
