@@ -256,3 +256,27 @@ def test_other_calls_inside_a_step(bits, symmetric, backend, dev, oracle_c):
     assert zo.rel_err_scaled(dev.get(mid).astype(np.float64), oracle_c.matmul_f64(x0, W2, s2, b2, group, bits, not symmetric), 1e-3) < 2e-3
     gate, up = want[2][:, :N // 2], want[2][:, N // 2:]
     assert zo.rel_err_scaled(dev.get(h).astype(np.float64), up * gate / (1 + np.exp(-gate)), 1e-2) < 4e-3
+
+
+@pytest.mark.parametrize("bits,K", [(4, 4096), (4, 4352), (4, 8448), (4, 12288), (4, 12544), (4, 16640), (3, 12544), (8, 12544), (8, 16640)])
+def test_rows_of_several_pieces_a_thread(bits, K, backend, dev, oracle_c):
+    """A thread takes up eight activations at a time, 4096 a round, three rounds ahead: either side of one round and of three, and one more. Bound as in
+    test_small_activations_of_whole_3_bit_slices: f32 sums that the matrix unit truncates, and the rounding to f16."""
+    rng = np.random.default_rng(K + bits)
+    N = 200
+    _, W, s, b = z.synth.make_weights(rng, N, K, bits=bits, sigma_s=0.01 * 15 / (2**bits - 1))
+    x = z.synth.make_x(rng, 1, K)
+    ref = oracle_c.matmul_f64(x, W, s, b, 64, bits, True)
+    mags = oracle_c.matmul_f64(np.abs(x), W, s, np.abs(b), 64, bits, True)
+    codes = oracle_c.matmul_f64(np.ones_like(x), W, s, np.zeros_like(b), 64, bits, True)
+    args = [dev.put(x), dev.put(s), dev.put(W), dev.put(b)]
+    ys = [dev.empty((1, N), np.float16, fill=9.0) for _ in range(3)]
+    backend.ctx.step_begin()
+    for y in ys:
+        backend.ctx.int4_matmul(z.MmDesc(K, N, 1, 64, bits, 1, 0), y, *args)
+    backend.ctx.step_end()
+    backend.ctx.sync()
+    for y in ys:
+        got = dev.get(y).astype(np.float64)
+        tiny = 2.0**-20 * codes if bits == 3 else 0.0          # 3-bit: an activation under a code's power of two
+        assert (np.abs(got - ref) <= 2.0**-11 * np.abs(ref) + 2.0**-25 + tiny + 1.001 * (K / 16 + 3 * K / 64 + 20) * 2.0**-23 * mags).all()
