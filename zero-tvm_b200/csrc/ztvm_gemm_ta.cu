@@ -572,7 +572,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       }
     }
   }
-  if (shares()) {
+  if constexpr (SHARES) if (shares()) {
     // ---- K shares meet: token blocks of eight, dealt to the CTAs in runs of `per`; partial sums as [sender][block][half][row][4
     // tokens], so that a warp's stores and loads are contiguous. Every thread of the cluster takes both barriers, whatever became of its waits.
     const uint32_t nb = (mrows + 7u) / 8u, per = (nb + split - 1) / split;
