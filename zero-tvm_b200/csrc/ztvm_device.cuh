@@ -173,6 +173,14 @@ __device__ __forceinline__ void codes3_inplace16(uint32_t w0, uint32_t w1, bool 
 #pragma unroll
   for (int i = 0; i < 4; ++i) { r[i] = v[i] & 0x00070007u; r[4 + i] = v[i] & 0x00380038u; }
 }
+// ... and by shifting them to bit 0 first: 15 instructions, but one shift to keep in a register instead of two permutations.
+__device__ __forceinline__ void codes3_inplace16_shifted(uint32_t w0, uint32_t w1, bool odd, uint32_t (&r)[8]) {
+  const uint32_t sh = (uint32_t)odd << 4, f0 = __funnelshift_r(w0, w1, sh), fh = __funnelshift_r(f0, w1 >> sh, 24);   // codes 0.., 8.. from bit 0
+  const uint32_t p0 = __byte_perm(f0, fh, 0x5410), p1 = __byte_perm(f0, fh, 0x6521);
+  const uint32_t v[4] = {p0, p0 >> 6, p1 >> 4, p1 >> 10};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { r[i] = v[i] & 0x00070007u; r[4 + i] = v[i] & 0x00380038u; }
+}
 
 // ---- canonical dequantisers ----------------------------------------------------------------
 // W32 = fl32(s*q + b) (affine) or fl32(s*(q-7)) (symmetric). s*q is exact in f32 (11-bit

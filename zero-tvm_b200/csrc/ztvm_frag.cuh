@@ -72,6 +72,7 @@ struct Frag<3> {
     return Raw{*reinterpret_cast<const uint32_t*>(p), *reinterpret_cast<const uint32_t*>(p + 4), (c & 1) != 0};
   }
   __device__ __forceinline__ static void a(const Raw& v, uint32_t (&r)[8]) { codes3_inplace16(v.w0, v.w1, v.odd, r); }
+  __device__ __forceinline__ static void a_shifted(const Raw& v, uint32_t (&r)[8]) { codes3_inplace16_shifted(v.w0, v.w1, v.odd, r); }
   __device__ __forceinline__ static void b(const uint4& x0, const uint4& x1, uint32_t (&r)[8]) {
     r[0] = __byte_perm(x0.x, x1.x, 0x5410); r[1] = __byte_perm(x0.y, x1.y, 0x5410);   // codes (0 | 8), (2 | 10)
     r[2] = __byte_perm(x0.z, x1.z, 0x5410); r[3] = __byte_perm(x0.w, x1.w, 0x5410);   // codes (4 | 12), (6 | 14)

@@ -82,7 +82,7 @@ __global__ void dequant_kernel(const uint32_t* W, const __half* S, const __half*
   }
 }
 
-// The codes as the streaming kernels see them: in-place masks that are f16 subnormals (codes4_inplace / codes3_inplace / codes3_inplace16,
+// The codes as the streaming kernels see them: in-place masks that are f16 subnormals (codes4_inplace / codes3_inplace / codes3_inplace16 and its _shifted form,
 // the functions those kernels call), scaled back to integers. 4-bit: one thread per word. 3-bit: one thread per
 // (row, scale group of 64 codes = six words), the run a quad of the 3-bit kernels owns.
 __device__ __forceinline__ uint32_t sub_to_code(uint32_t halfbits, float scale) {
@@ -114,7 +114,7 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
 #pragma unroll
       for (int j = 0; j < 6; ++j) w[j] = W[(size_t)n * KP + g * 6 + j];
       uint8_t* dst = codes + (size_t)n * K + (size_t)g * 64;
-      // Both in-place views of the stream: the single-row GEMV's 17 windows, and the quad fragments of the batched kernel
+      // Both in-place views of the stream: the single-row GEMV's 17 windows, and the quad fragments of the batched and streamed kernels
       // (lane q: codes 16 q .. 16 q + 15, the 48 bits from byte 6 q). A code they disagree on comes out as 255.
 #pragma unroll
       for (int k = 0; k < kCodes3Views; ++k) {
@@ -130,9 +130,10 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int j = 3 * q / 2, sh = (q & 1) * 16;
-        uint32_t r[8];
-        codes3_inplace16(w[j], w[j + 1], sh != 0u, r);
+        const int j = 3 * q / 2;
+        uint32_t r[8], shifted[8];
+        codes3_inplace16(w[j], w[j + 1], (q & 1) != 0, r);
+        codes3_inplace16_shifted(w[j], w[j + 1], (q & 1) != 0, shifted);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -140,8 +141,8 @@ __global__ void unpack_codes_streamed_kernel(const uint32_t* W, uint8_t* codes, 
             const int c0 = 16 * q + 2 * i + 8 * h;
             const uint32_t even = sub_to_code(h ? r[i] >> 16 : r[i] & 0xFFFFu, 16777216.f);          // offset 0: q * 2^-24
             const uint32_t odd = sub_to_code(h ? r[4 + i] >> 16 : r[4 + i] & 0xFFFFu, 2097152.f);    // offset 3: q * 2^-21
-            if (dst[c0] != even) dst[c0] = 255;
-            if (dst[c0 + 1] != odd) dst[c0 + 1] = 255;
+            if (dst[c0] != even || r[i] != shifted[i]) dst[c0] = 255;
+            if (dst[c0 + 1] != odd || r[4 + i] != shifted[4 + i]) dst[c0 + 1] = 255;
           }
       }
     }
