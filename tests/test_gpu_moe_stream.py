@@ -44,3 +44,34 @@ def test_streamed_experts(bits, K, N, E, T, slots, pad, dev, oracle_c, monkeypat
     mags = oracle_c.moe_matmul_f64(np.abs(x), W, s, np.abs(b), ids, N, K, 64, bits, in_per_slot=False)
     assert (np.abs(got - ref) <= f16_bound(ref, mags, K)).all()
     be.close()
+
+
+@pytest.mark.parametrize("reuse", [False, True])
+@pytest.mark.parametrize("d,ffn,E,T,slots", [
+    (512, 256, 5, 11, 4), (512, 256, 5, 15, 3),          # one pair below nine per expert, and nine
+    (2048, 256, 6, 9, 4), (256, 2048, 6, 9, 4),          # long and short K first: by itself the short one is batched, with a shared plan both go one way
+    (1792, 512, 7, 12, 4), (2304, 512, 7, 12, 4),        # seven slices fill the warps, nine do not
+    (1280, 640, 7, 12, 4), (320, 256, 7, 12, 4),         # one projection over whole slices, the other not: plans of two tile heights
+    (512, 512, 3, 40, 2),                                # many pairs per expert: batched
+])
+def test_three_bit_experts_by_size(d, ffn, E, T, slots, reuse, dev, oracle_c):
+    """The choice for 3-bit experts left to the library: both projections of a block over one id list, with a plan each and with one
+    that they may share."""
+    be = z.backend.CudaMatmulBackend(0)
+    be.ctx.moe_plan_reuse(reuse)
+    rng = np.random.default_rng(d + ffn + T)
+    ids = rng.integers(0, E, size=(T, slots), dtype=np.uint32)
+    ids_dev = dev.put(ids)
+    for N, K, per_slot in ((ffn, d, False), (d, ffn, True)):
+        _, W, s, b = z.synth.make_weights(rng, N, K, bits=3, sigma_s=0.02, lead=(E,))
+        x = z.synth.make_x(rng, T * slots if per_slot else T, K)
+        y = dev.empty((T, slots, N), np.float16, fill=float("nan"))
+        desc = z.MoeDesc(z.MmDesc(K, N, 1, 64, 3, 1, 0), E, slots, T, K if per_slot else 0, N, slots * K if per_slot else K, slots * N, slots)
+        be.ctx.int4_matmul_moe(desc, y, dev.put(x), dev.put(s), dev.put(W), dev.put(b), ids_dev)
+        got = dev.get(y)
+        assert be.ctx.device_errors() == 0 and np.isfinite(got).all()
+        ref = oracle_c.moe_matmul_f64(x, W, s, b, ids, N, K, 64, 3, in_per_slot=per_slot)
+        record_parity(zo.rel_err_scaled(got, ref, 1e-3), zo.rel_err(got, ref))
+        mags = oracle_c.moe_matmul_f64(np.abs(x), W, s, np.abs(b), ids, N, K, 64, 3, in_per_slot=per_slot)
+        assert (np.abs(got - ref) <= f16_bound(ref, mags, K)).all()
+    be.close()

@@ -1,5 +1,6 @@
 // C ABI of libztvm_b200.so: context, argument validation, kernel selection. Every entry point
 // validates before it launches and reports through a status code plus a thread-local message.
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -629,6 +630,28 @@ ztvm_status ztvm_host_wait(ztvm_ctx* ctx) {
   return ZTVM_OK;
 }
 
+// What a 3-bit expert matmul takes on the streaming kernel less what it takes on the batched one, plan kept, in us. Fitted to 3584 pairs of launches on 148
+// SMs (16 to 256 experts, 256 to 2816 rows, K of 256 to 2048, 32 pairs to 9 per expert) for the choice: it is 0.3 % from the faster of the two on
+// average. `n8`, `n16`: tiles of that many pairs that tokens routed evenly make. Streamed: the start, rounds of a row group of warps, chunks that a CTA walks.
+// Batched: the start and the K slices of a CTA, those of every CTA beyond two on an SM, the second half of tiles with more than eight pairs. So short K whose CTAs fit at
+// once is the batched kernel's, nearly all else the streaming kernel's: us, streamed against batched, 16 experts of 2048 x 256 at 4 pairs each 6.5 : 4.6, 32 of
+// 1024 x 1024 10.8 : 9.4, 16 of 512 x 2048 7.4 : 11.2, 256 of 1024 x 1024 44.8 : 57.2.
+static float moe3_streamed_less_batched(const ztvm_ctx* ctx, const ztvm_moe_desc* md, uint32_t N, uint32_t K) {
+  const float q = fminf((float)md->slots / (float)md->experts, 0.99f), T = (float)md->tokens;
+  float n8 = 0.f, n16 = 0.f, p = powf(1.f - q, T);             // p: an expert has j pairs
+  for (uint32_t j = 0; j <= 40u && j <= md->tokens; ++j) {
+    n8 += p * (float)((j + 7u) / 8u);
+    n16 += p * (float)((j + 15u) / 16u);
+    p *= (T - (float)j) / (float)(j + 1u) * q / (1.f - q);
+  }
+  n8 = fmaxf(ceilf(n8 * (float)md->experts), 1.f); n16 = fmaxf(ceilf(n16 * (float)md->experts), 1.f);
+  const float sms = (float)ctx->sm_count, slices = (float)(K / 256u);
+  const float chunks = n8 / sms, rounds = chunks * (float)((N + 15u) / 16u) / (float)(16u / (K / 256u));
+  const float ctas = ceilf(n16 * (float)((N + 127u) / 128u) / sms);
+  const float batched = 1.85f + 1.9f * slices + fmaxf(ctas - 2.f, 0.f) * (0.78f + 0.69f * slices) + 0.77f * slices * (n8 - n16) / n16;
+  return 6.f + rounds + 1.15f * chunks - batched;
+}
+
 // Which grouped kernel serves a MoE launch: 0 none (per-pair GEMV), 1 tensor-core tiles with the weights in tensor
 // memory, 2 streaming kernel, 3 tensor-core tiles with both operands in shared memory (ZTVM_MOE_TILES=sm, or shapes
 // only it takes), 4 the exact-code batched kernel (what 2 leaves of 3-bit experts; 4-bit ones of few pairs over a K that 2 does not take). `forced` is the context's ZTVM_MOE_GROUPED knob (-1 = by size).
@@ -647,14 +670,20 @@ static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::Ge
   // and at eight pairs per expert. The line is at ten for all three projections of a block: below it they keep exact codes and f32 weights,
   // which the tiles round to f16, and one kernel, whose plan they share.
   const bool few_per_expert = pairs < 10ull * md->experts;
-  // 3-bit codes stay exact at every pair count: streamed where that leaves at most a quarter of the sixteen warps without a slice, else on the
-  // batched kernel, whose tiles unpack a code for 16 pairs and more. us, streamed against it, 257 experts: 512 x 2048 30 : 40, 44 : 57, 59 : 65
-  // and 70 : 69 at 1 / 4 / 8 / 10 pairs per expert, 2048 x 512 30 : 42, 49 : 67, 65 : 73, 79 : 76; 40 experts of 2048 x 2304, nine slices, 27 : 26, 37 : 42, 51 : 45.
-  // The K of a block's other projections is this one's N: all of them stream or none, as they share a plan (54 experts, 1408 and 256 wide, 40
-  // pairs, a plan for the down projection alone: 31 us a block became 36).
-  auto fills = [](uint32_t k) { return k % 256u == 0 && k / 256u <= 16u && 16u / (k / 256u) * (k / 256u) >= 12u; };
+  // 3-bit codes stay exact at every pair count: streamed where that leaves at most a quarter of the sixteen warps without a slice and is the shorter way
+  // (moe3_streamed_less_batched), else on the batched kernel, whose tiles unpack a code for 16 pairs and more (70 : 69 us, streamed against it, for 257
+  // experts of 512 x 2048 at 10 pairs each; 51 : 45 for 40 of 2048 x 2304, nine slices). The projections of a block that share a plan all stream or none (54
+  // experts, 1408 and 256 wide, 40 pairs, a plan for the down projection alone: 31 us a block became 36): the K of the others is taken to be this one's N.
   if (d->bits == 3) {
-    const bool streams = stream_ok && (forced == 2 || (forced != 1 && pairs < 9ull * md->experts && fills(d->K) && fills(d->N)));
+    auto fills = [](uint32_t k) { return k % 256u == 0 && k / 256u <= 16u && 16u / (k / 256u) * (k / 256u) >= 12u; };
+    auto shorter = [&]() {
+      if (pairs >= 9ull * md->experts || !fills(d->K)) return false;
+      const float mine = moe3_streamed_less_batched(ctx, md, d->N, d->K);
+      if (!ctx->plan_reuse) return mine < 0.f;
+      // (a block has one of its two shapes twice, which one is not known here: 1.2 us of 20 to 500 in the streaming kernel's favour fit 290 blocks best)
+      return fills(d->N) && mine + moe3_streamed_less_batched(ctx, md, d->K, d->N) < (d->K == d->N ? 0.f : 1.2f);
+    };
+    const bool streams = stream_ok && (forced == 2 || (forced != 1 && shorter()));
     return streams ? 2 : ztvm::batch_moe_supported(p, 3) ? 4 : 0;
   }
   // A K that the streaming kernel does not take: the batched kernel, exact codes as well, holds its place (257 experts of 512 x
