@@ -103,10 +103,7 @@ __device__ __forceinline__ float ta_add2(float acc, uint32_t h) {
   return acc;
 }
 
-// SHARES: the instance for clusters (4-bit; the 8-bit one serves both). A launch of one share is an instance without the exchange, which its code
-// otherwise paid for, 1600 to 9216 x 1088 without biases, 24 to 330 rows, 1 to 2 % (1600 x 1088, 77 rows 6.69 us with it in the same code, 6.59 so).
-// 8-bit codes lose by the same cut (7696 x 10112, 89 rows 69.6 us in one, 73.7 in two instances).
-template <int NT, bool AFFINE, int BITS, bool SHARES>
+template <int NT, bool AFFINE, int BITS>
 __global__ void __launch_bounds__(kTaThreads, 1)
 gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                   const GemmTaParams p) {
@@ -136,8 +133,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   const uint32_t m0 = blockIdx.y * p.tile_m;
   const uint32_t mrows = p.M - m0 < p.tile_m ? p.M - m0 : p.tile_m;     // tokens of this tile
   // k blocks of this CTA: whole scale stages, so that every share starts on a multiple of eight
-  const uint32_t split = SHARES ? gridDim.z : 1u, kz = SHARES ? blockIdx.z : 0u;
-  auto shares = [&]() { return BITS == 8 ? split > 1u : SHARES; };
+  const uint32_t split = gridDim.z, kz = blockIdx.z;
   const uint32_t all_kb = p.K / kGemmBK, units = (all_kb + kTaSbChunk - 1) / kTaSbChunk;
   const uint32_t kb_first = kz * units / split * kTaSbChunk;
   const uint32_t kb_last = kz + 1 == split ? all_kb : (kz + 1) * units / split * kTaSbChunk;
@@ -218,7 +214,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   __syncthreads();
   tc_fence_after();
   // (that this CTA runs, so that the others of its cluster may write to its shared memory)
-  if (L::kApart && shares()) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (L::kApart && split > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -516,7 +512,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     static_assert(NT * kTaRows * 2 <= kTaStages * L::kXBytes, "the output stage lives in the activation ring");
     const bool staged = !p.out_f32 && (p.N % 8u) == 0;
     const int ncb = (int)((mrows + 31u) / 32u);
-    if (shares()) {
+    if (split > 1) {
       // below, with the whole cluster
     } else if (staged) {
       const uint32_t stage = x_ring;
@@ -572,7 +568,7 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       }
     }
   }
-  if constexpr (SHARES) if (shares()) {
+  if (split > 1) {
     // ---- K shares meet: token blocks of eight, dealt to the CTAs in runs of `per`; partial sums as [sender][block][half][row][4
     // tokens], so that a warp's stores and loads are contiguous. Every thread of the cluster takes both barriers, whatever became of its waits.
     const uint32_t nb = (mrows + 7u) / 8u, per = (nb + split - 1) / split;
@@ -650,13 +646,13 @@ static TaEncodeFn ta_encode_fn() {
   return fn;
 }
 
-template <int NT, bool AFFINE, int BITS, bool SHARES>
+template <int NT, bool AFFINE, int BITS>
 static cudaError_t ta_kernel_ready() {
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 16 && attr_set[dev]) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_ta_kernel<NT, AFFINE, BITS, SHARES>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmTaSmem<NT, BITS>::kTotal + 1024);
+  const cudaError_t e = cudaFuncSetAttribute(gemm_ta_kernel<NT, AFFINE, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmTaSmem<NT, BITS>::kTotal + 1024);
   if (e == cudaSuccess && dev < 16) attr_set[dev] = true;
   return e;
 }
@@ -678,18 +674,12 @@ struct TaLaunch {
     cfg.numAttrs = grid.z > 1 ? 2 : 1;
   }
 };
-template <int NT, bool AFFINE, int BITS, bool SHARES>
-static cudaError_t launch_ta_inst(const CUtensorMap& tx, const CUtensorMap& tw, const GemmTaParams& p, uint32_t split, cudaStream_t st) {
-  const cudaError_t e = ta_kernel_ready<NT, AFFINE, BITS, SHARES>();
-  if (e != cudaSuccess) return e;
-  TaLaunch l(dim3((p.N + kTaRows - 1) / kTaRows, (p.M + p.tile_m - 1) / p.tile_m, split), GemmTaSmem<NT, BITS>::kTotal + 1024, st);
-  return cudaLaunchKernelEx(&l.cfg, gemm_ta_kernel<NT, AFFINE, BITS, SHARES>, tx, tw, p);
-}
 template <int NT, bool AFFINE, int BITS>
 static cudaError_t launch_ta_one(const CUtensorMap& tx, const CUtensorMap& tw, const GemmTaParams& p, uint32_t split, cudaStream_t st) {
-  if constexpr (BITS == 4)
-    if (split == 1) return launch_ta_inst<NT, AFFINE, BITS, false>(tx, tw, p, split, st);
-  return launch_ta_inst<NT, AFFINE, BITS, true>(tx, tw, p, split, st);
+  const cudaError_t e = ta_kernel_ready<NT, AFFINE, BITS>();
+  if (e != cudaSuccess) return e;
+  TaLaunch l(dim3((p.N + kTaRows - 1) / kTaRows, (p.M + p.tile_m - 1) / p.tile_m, split), GemmTaSmem<NT, BITS>::kTotal + 1024, st);
+  return cudaLaunchKernelEx(&l.cfg, gemm_ta_kernel<NT, AFFINE, BITS>, tx, tw, p);
 }
 // Clusters of `split` CTAs that the device holds at once (a cluster sits inside one GPC, so this is less than SMs / split).
 template <int NT, int BITS>
@@ -702,7 +692,7 @@ static uint32_t ta_clusters(uint32_t split, int sm_count) {
   int n = known[dev][split];
   if (n == 0) {
     TaLaunch l(dim3(1, 1, split), GemmTaSmem<NT, BITS>::kTotal + 1024, nullptr);
-    if (ta_kernel_ready<NT, true, BITS, true>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_ta_kernel<NT, true, BITS, true>, &l.cfg) != cudaSuccess || n < 1) {
+    if (ta_kernel_ready<NT, true, BITS>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_ta_kernel<NT, true, BITS>, &l.cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       n = 1;
     }
