@@ -213,8 +213,9 @@ gemm_ta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // (that this CTA runs, so that the others of its cluster may write to its shared memory)
-  if (L::kApart && split > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  // That this CTA runs, so that the others of its cluster may write to the place of their sums: nothing was written that they read, so
+  // the arrival is relaxed. (As a release it waited for the loads in flight: 4096 x 4096, 128 rows without biases 11.5 us, now 10.9; 2624 x 2624 10.1, 9.7.)
+  if (L::kApart && split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
