@@ -718,14 +718,15 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
                            int bits, uint32_t group_shift, bool out_f32, uint32_t* status, int sm_count, cudaStream_t st) {
   TaEncodeFn enc = ta_encode_fn();
   if (!enc) return cudaErrorNotSupported;
-  // Tokens per tile and K shares, by the time of the busiest SM in cycles. 4-bit, fitted to 1120 shapes (512 to 16384 rows, K of 512 to 12288, 17 to 600
-  // tokens) of which every tile and number of shares was timed, 0.3 % from the best of them on average: a k block takes 400 with biases and 340 without, + 1.3 per
-  // token, at least 547 and 440; a CTA of a launch without shares 6150 + 28 per token to start, fill its rings and store, one of a cluster 8850 + 34.5 per
-  // token, 12 per tile, 8 per CTA, 280 for every share beyond two and 950 where the sums have no place of their own. (4096 x 4096, 128 rows, us: one share 19.7, two 15.0, three 14.1, four 12.9; 9216 x 1472,
-  // 24 rows 7.9 : 8.4 with two; 9384 x 1024, 38 rows 7.2 : 8.1; 9216 x 3072, 200 rows, whole-K tiles of 100 tokens 14.3, two shares of 200 15.2.) The longest
-  // share counts: all are whole scale stages but the last. Clusters run in as many waves as the device can place. The tokens are dealt evenly to the tiles. (Groups
-  // of 32 with biases do not fit beside the widest tile.) 8-bit: tiles of up to 64 tokens, a block 700 + 2 per token, 8500 and 5300 + 12 per token; the exchange
-  // more for every share beyond two.
+  // Tokens per tile and K shares, by the time of the busiest SM in cycles. 4-bit, fitted to 1980 shapes (512 to 16384 rows, K of 512 to 12288, 17 to 1100
+  // tokens) of which every tile and number of shares was timed, 0.2 % from the best of them on average: a k block takes 340 + 1.4 per token, with biases at least
+  // 620; a CTA of a launch without shares 7000 to start, fill its rings and store, and the last ones 12 per token; one of a cluster 7500 + 35 per token, 4 per
+  // tile, 2.8 per CTA and 320 for every share beyond two, and 100 + 13 per token with tiles of more than 128 tokens, whose sums have no place of their own. More
+  // CTAs than half the SMs: 8 % more with biases, 3 % without. The longest share counts: all are whole scale stages but the last. Clusters run in as many waves as
+  // the device can place. The tokens are dealt evenly to the tiles. (us: 4096 x 4096, 128 rows with biases, one share 20.7, two 14.4, three 13.5, four 12.5; 9216
+  // x 1472, 24 rows with biases, one 9.4, two 10.0; 9216 x 3072, 200 rows without, whole-K tiles of 100 tokens 14.3, two shares of 200 15.0.) (Groups of 32 with
+  // biases do not fit beside the widest tile.) 8-bit: tiles of up to 64 tokens, a block 700 + 2 per token, 8500 and 5300 + 12 per token; the exchange more for
+  // every share beyond two.
   const uint32_t units = (K / kGemmBK + kTaSbChunk - 1) / kTaSbChunk, n_tiles = (N + kTaRows - 1) / kTaRows;
   const uint32_t widest = bits == 8 ? 64u : B && group_shift == 5 ? 256u : 352u;
   uint32_t tile_m = 0, split = 1;
@@ -734,23 +735,22 @@ cudaError_t launch_gemm_ta(const uint32_t* W, const __half* S, const __half* B, 
     if (t > 64u && t - 32u >= M) break;
     const uint32_t m_tiles = (M + t - 1) / t, tm = ((M + m_tiles - 1) / m_tiles + 15u) & ~15u;
     const uint64_t tiles = (uint64_t)n_tiles * m_tiles;
-    const uint32_t live = M < tm ? M : tm, least = B ? 547u : 440u, by_tokens = (B ? 400u : 340u) + live * 13u / 10u;
-    const uint32_t block = bits == 8 ? 700u + 2u * live : by_tokens < least ? least : by_tokens;
+    const uint32_t live = M < tm ? M : tm, by_tokens = 340u + live * 14u / 10u;
+    const uint32_t block = bits == 8 ? 700u + 2u * live : B && by_tokens < 620u ? 620u : by_tokens;
     for (uint32_t z = 1; z <= (uint32_t)kTaMaxSplit && z <= units; ++z) {
       if (z > 1 && tiles * z > (uint64_t)sm_count) break;
       const uint32_t at_once = bits == 8 ? ta_at_once<8>(tm, z, sm_count) : ta_at_once<4>(tm, z, sm_count);
       const uint64_t waves = (tiles + at_once - 1) / at_once;
       const uint32_t more = z > 2 ? z - 2u : 0u, all = K / kGemmBK;
-      uint32_t blocks, rest;
+      uint64_t cost;
       if (bits == 8) {
-        blocks = z == 1 ? all : (units + z - 1) / z * kTaSbChunk;
-        rest = 8500u + (z == 1 ? 0u : 5300u + (12u + 28u * more) * live);
+        cost = waves * ((z == 1 ? all : (units + z - 1) / z * kTaSbChunk) * block + 8500u + (z == 1 ? 0u : 5300u + (12u + 28u * more) * live));
       } else {
         const uint32_t last = all - (z - 1u) * units / z * kTaSbChunk, others = (units / z + (units % z > 1u ? 1u : 0u)) * kTaSbChunk;
-        blocks = z == 1 || last > others ? last : others;
-        rest = z == 1 ? 6150u + 28u * live : 8850u + 69u * live / 2u + (12u + 8u * z) * (uint32_t)tiles + 280u * more + (tm > 128u ? 950u : 0u);
+        const uint32_t blocks = z == 1 || last > others ? last : others, per_tile = 40u + 28u * z;
+        const uint32_t rest = z == 1 ? 7000u : 7500u + 35u * live + per_tile * (uint32_t)tiles / 10u + 320u * more + (tm > 128u ? 100u + 13u * live : 0u);
+        cost = waves * (blocks * block + rest) * (2u * tiles * z <= (uint64_t)sm_count ? 100u : B ? 108u : 103u) / 100u + (z == 1 ? 12u * live : 0u);
       }
-      const uint64_t cost = waves * (blocks * block + rest);
       if (cost < best) { best = cost; tile_m = tm; split = z; }
     }
   }
