@@ -42,7 +42,7 @@ struct MoeTcParams {
 
 template <int BITS>
 struct MtCfg {
-  using T = MtTile<BITS, true>;
+  using T = MtTile<BITS>;
   static constexpr int kOffPartial = kTcWarps * kTcDepth * T::kBytes;   // float [2][warps][kMtRounds][8 pairs][kMtPitch]
   static constexpr int kOffRows = kOffPartial + 2 * kTcWarps * kMtRounds * kMtUnitFloats * 4;   // uint64 [chunks][in, out][8 pairs]
   static constexpr int kOffExpert = kOffRows + kMtChunks * 16 * 8;                              // uint32 [chunks][expert, pairs]
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kTcWarps * 32, 1)
 moe_tc_kernel(const MoeTcParams p) {
   extern __shared__ __align__(128) uint8_t mt_smem[];
   using C = MtCfg<BITS>;
-  using T = MtTile<BITS, true>;
+  using T = MtTile<BITS>;
   pdl_launch_dependents();
   pdl_wait();                                            // the plan may come from the kernel before
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -144,7 +144,7 @@ moe_tc_kernel(const MoeTcParams p) {
   float xs[4][2];                 // per run: sums of x for the pairs of columns 2c, 2c + 1
   auto load_chunk = [&](uint32_t ec) {
     const bool on = (uint32_t)g < chunk_pairs(ec);
-    mt_fragments<BITS, false>(p.X + (on ? chunk_row(ec, (uint32_t)g, false) : 0ull) + (size_t)ks * kTcSlice + 16 * c, on, 4u, c, xf, xs);
+    mt_fragments<BITS>(p.X + (on ? chunk_row(ec, (uint32_t)g, false) : 0ull) + (size_t)ks * kTcSlice + 16 * c, on, c, xf, xs);
   };
 
   float acc[kMtRounds][2][2];
@@ -164,7 +164,7 @@ moe_tc_kernel(const MoeTcParams p) {
       }
       asm volatile("cp.async.wait_group %0;" ::"n"(kTcDepth - 1) : "memory");
       __syncwarp();
-      if (live) mt_multiply<BITS, true>(st, 4u, 0u, g, c, xf, xs, acc[q]);
+      if (live) mt_multiply<BITS>(st, g, c, xf, xs, acc[q]);
       __syncwarp();
       st = st + T::kBytes == ring_end ? ring : st + T::kBytes;
       c_u += RG; c_tile += RG;

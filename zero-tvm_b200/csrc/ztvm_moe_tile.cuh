@@ -1,4 +1,4 @@
-// One step of the kernels that stream expert weights (ztvm_moe_tc.cu, ztvm_moe_block.cu): a tile of 16 weight rows x up to 256 codes
+// One step of the kernel that streams expert weights (ztvm_moe_tc.cu): a tile of 16 weight rows x 256 codes
 // times up to eight activation rows, one per column of mma.sync.m16n8k16. Codes enter as f16 subnormals masked where they sit
 // (ztvm_frag.cuh), a run of 64 is folded with its scale and bias by f32 FMAs.
 #pragma once
@@ -7,29 +7,28 @@
 
 namespace ztvm {
 
-// AL: scales come as aligned 8-byte words, four of a row (then its four biases); else as the 4-byte words around them.
-template <int BITS, bool AL>
+// The codes of the sixteen rows, then per row its four scales and its four biases.
+template <int BITS>
 struct MtTile {
   static constexpr int kRowBytes = 32 * BITS;                       // 256 codes
-  static constexpr int kSbSlot = AL ? 8 : 12;
-  static constexpr int kCodes = 16 * kRowBytes, kBytes = kCodes + 32 * kSbSlot;
+  static constexpr int kCodes = 16 * kRowBytes, kBytes = kCodes + 16 * 16;
   // Place of 16-byte piece j of row `row`. 4-bit: a row's runs are permuted by the row so that fragment loads touch all banks.
   __device__ __forceinline__ static uint32_t piece(uint32_t row, uint32_t j) {
     return row * kRowBytes + (BITS == 4 ? (((j >> 1) ^ (row & 3u)) << 5) + ((j & 1u) << 4) : j * 16u);
   }
 };
 
-// B fragments of a slice of `runs` runs: lane (g, c) has row g's 16 activations of each run from xr on (`on`: there is a row g). xs: sums
-// per run of the rows of columns 2c, 2c + 1. CG: the row may have been written by this very launch.
-template <int BITS, bool CG>
-__device__ __forceinline__ void mt_fragments(const __half* xr, bool on, uint32_t runs, int c, uint32_t (&xf)[4][8], float (&xs)[4][2]) {
+// B fragments of a slice of four runs: lane (g, c) has row g's 16 activations of each run from xr on (`on`: there is a row g). xs: sums
+// per run of the rows of columns 2c, 2c + 1.
+template <int BITS>
+__device__ __forceinline__ void mt_fragments(const __half* xr, bool on, int c, uint32_t (&xf)[4][8], float (&xs)[4][2]) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
-    if (on && (uint32_t)r < runs) {
+    if (on) {
       const uint4* const q = reinterpret_cast<const uint4*>(xr + 64 * r);
-      x0 = CG ? __ldcg(q) : q[0];
-      x1 = CG ? __ldcg(q + 1) : q[1];
+      x0 = q[0];
+      x1 = q[1];
     }
     Frag<BITS>::b(x0, x1, xf[r]);
     float sum = 0.f;
@@ -46,20 +45,16 @@ __device__ __forceinline__ void mt_fragments(const __half* xr, bool on, uint32_t
   }
 }
 
-// acc[h][v] += rows g + 8 h of the tile at `st` times the activations of column 2c + v. `runs`: those that exist (AL: four).
-// `odd` (AL false): 1 where the rows' scales start on the second half of their first word.
-template <int BITS, bool AL>
-__device__ __forceinline__ void mt_multiply(uint32_t st, uint32_t runs, uint32_t odd, int g, int c, const uint32_t (&xf)[4][8], const float (&xs)[4][2],
-                                            float (&acc)[2][2]) {
-  using T = MtTile<BITS, AL>;
+// acc[h][v] += rows g + 8 h of the tile at `st` times the activations of column 2c + v.
+template <int BITS>
+__device__ __forceinline__ void mt_multiply(uint32_t st, int g, int c, const uint32_t (&xf)[4][8], const float (&xs)[4][2], float (&acc)[2][2]) {
+  using T = MtTile<BITS>;
   using F = Frag<BITS>;
   const float kZero[4] = {0.f, 0.f, 0.f, 0.f};
-  const uint32_t sb_at = st + T::kCodes + (uint32_t)g * (2 * T::kSbSlot);
-  uint4 sg, sh;                            // rows g, g + 8: four scales, four biases
-  if constexpr (AL) { sg = tc_lds128(sb_at); sh = tc_lds128(sb_at + 16u * T::kSbSlot); }
+  const uint32_t sb_at = st + T::kCodes + (uint32_t)g * 16u;
+  const uint4 sg = tc_lds128(sb_at), sh = tc_lds128(sb_at + 128u);   // rows g, g + 8: four scales, four biases
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    if (!AL && (uint32_t)r >= runs) break;
     uint32_t ag[8], ah[8];                 // rows g and g + 8
     if constexpr (BITS == 4) {
       const uint32_t at = st + (uint32_t)g * 128u + (((uint32_t)r ^ ((uint32_t)g & 3u)) << 5) + ((uint32_t)c << 3);
@@ -77,17 +72,9 @@ __device__ __forceinline__ void mt_multiply(uint32_t st, uint32_t runs, uint32_t
     tc_mma(d1, ag[6], ah[6], ag[7], ah[7], xf[r][6], xf[r][7], d1);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      float s, b;
-      if constexpr (AL) {
-        const uint4 w = h ? sh : sg;
-        const float2 s2 = __half22float2(u32_as_h2(r & 2 ? w.y : w.x)), b2 = __half22float2(u32_as_h2(r & 2 ? w.w : w.z));
-        s = r & 1 ? s2.y : s2.x; b = r & 1 ? b2.y : b2.x;
-      } else {
-        const uint32_t at = sb_at + (uint32_t)h * (16 * T::kSbSlot) + (odd + (uint32_t)r) * 2u;
-        s = __half2float(__ushort_as_half((unsigned short)tc_lds16(at)));
-        b = __half2float(__ushort_as_half((unsigned short)tc_lds16(at + T::kSbSlot)));
-      }
-      s *= F::kUnit;
+      const uint4 w = h ? sh : sg;
+      const float2 s2 = __half22float2(u32_as_h2(r & 2 ? w.y : w.x)), b2 = __half22float2(u32_as_h2(r & 2 ? w.w : w.z));
+      const float s = (r & 1 ? s2.y : s2.x) * F::kUnit, b = r & 1 ? b2.y : b2.x;
       // (two-wide FMAs would want the scale and the bias twice each, side by side: more moves than they save)
 #pragma unroll
       for (int v = 0; v < 2; ++v)

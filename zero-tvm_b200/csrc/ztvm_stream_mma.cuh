@@ -9,8 +9,6 @@ constexpr int kTcWarps = 16;
 constexpr int kTcDepth = 4;
 constexpr int kTcSlice = 256;                        // codes per warp slice = 128 B per row = 4 scale groups
 constexpr int kTcTileW = 16 * 128;                   // packed codes of one (tile, slice)
-constexpr int kTcTileBytes = kTcTileW + 16 * 16;     // + per row 4 scales, 4 biases (f16)
-constexpr int kTcRingBytes = kTcWarps * kTcDepth * kTcTileBytes;
 
 __device__ __forceinline__ void tc_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                        uint32_t b1, const float (&c)[4]) {
