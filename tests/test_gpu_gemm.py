@@ -1,7 +1,8 @@
 """GPU parity of the prefill GEMM (M > 8): tcgen05 MMA over weights dequantised to f16 on the fly.
 Reference for the outputs: an fp64 dot product over W16 = f16(fl32(s*q+b)), the value the reference's own numpy
 dequantiser produces and its matrix-unit GEMMs multiply with; W16 itself is checked bit for bit through the
-dequant hook, which calls the same device function the GEMM inlines."""
+dequant hook, which calls the word's form of the device functions that the GEMM inlines a row of a k block at a time; the
+GEMM's own weights are read back bit for bit in test_gpu_weight_builder.py."""
 import numpy as np
 import pytest
 

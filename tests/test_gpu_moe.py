@@ -13,11 +13,12 @@ TOL = 2e-3   # with the scale-tied floor of oracle.rel_err_scaled (1e-3 of the o
 
 
 def moe_kernel_kind(pairs, experts, K, N, bits):
-    """Which kernel ztvm_int4_matmul_moe picks (mirrors moe_pick in ztvm_api.cu): 'pair', 'stream' or 'tiles'."""
+    """What anchors the kernel that ztvm_int4_matmul_moe picks for 4-bit experts of a kept plan (as moe_pick in ztvm_api.cu): 'tiles' round the
+    weights to f16, 'stream' and 'pair' (which stands for every other exact-code kernel, too) do not."""
     if bits != 4 or pairs < 128 or experts > 1024:
         return "pair"
     tiles_ok = K % 64 == 0 and N % 8 == 0
-    stream_ok = K % 256 == 0 and K <= 4096 and N % 16 == 0
+    stream_ok = K % 256 == 0 and K <= 4096
     if stream_ok and (pairs < 10 * experts or not tiles_ok):
         return "stream"
     return "tiles" if tiles_ok else "pair"

@@ -54,7 +54,7 @@ __global__ void dequant_kernel(const uint32_t* W, const __half* S, const __half*
     const uint32_t n = (uint32_t)(i / nblk), blk = (uint32_t)(i - (size_t)n * nblk);
     const uint32_t g = (blk << 3) >> group_shift;
     if constexpr (AS_F16 && BITS == 4) {
-      // the tensor-core GEMMs (dense and grouped) build their f16 operand with dequant_word_w16: so does the hook
+      // a word at a time: the dense GEMM and the tiles in tensor memory build their f16 operand by the same three word functions, four or eight words at once
       const unsigned short s16 = reinterpret_cast<const unsigned short*>(S)[(size_t)n * SPR + g];
       const unsigned short b16 = AFFINE ? reinterpret_cast<const unsigned short*>(B)[(size_t)n * SPR + g] : (unsigned short)0;
       const uint4 v = dequant_word_w16<AFFINE>(W[(size_t)n * KP + blk], dq_group<AFFINE>(s16, b16));
