@@ -322,11 +322,11 @@ static ztvm_status matmul_now(ztvm_ctx* ctx, const ztvm_mm_desc* d, void* y, con
                               const void* biases, cudaStream_t st) {
   // Up to 16 rows the GEMV in slabs of eight: exact codes and f32 weights, the reference's choice for short chunks (runtime-M
   // matvec; its GEMMs start at 64 rows). From 17 on a third slab costs more than the GEMM at every width. Weight sets from HBM,
-  // GEMM against slabs, us: 8192 x 2048 9.8 : 11.1 at 16 rows, 10.1 : 15.8 at 17; 24576 x 4096 40.7 : 34.2 and 40.8 : 48.0;
-  // 4096 x 12288 18.6 : 24.2 and 19.0 : 35.6. (The GEMM is ahead at 9..16 rows too where K is long, but rounds the weights to f16.)
+  // GEMM against slabs, us: 8192 x 2048 9.8 : 10.3 at 16 rows, 9.9 : 14.9 at 17; 24576 x 4096 39.7 : 34.2 and 39.7 : 48.0;
+  // 4096 x 12288 18.5 : 23.2 and 18.5 : 32.8. (The GEMM is ahead at 9..16 rows too where K is long, but rounds the weights to f16.)
   // 8-bit weights go as exact codes, with f32 folds, like in the batched kernel below. f32 results (router logits) stay with that one, and so
   // do up to 32 rows, one token tile of it, and small matmuls over a short K, its serial part, us, GEMM against it: 12288 x 2048 17.5 : 25.8 at
-  // 33 rows, 33.6 : 31.5 at 77, 51.7 : 80.6 at 200; 2048 x 6144 14.1 : 30.1 at 33; 2048 x 2048 9.2 : 11.0 at 33; 1536 x 1088 11.1 : 10.0 at 256,
+  // 33 rows, 33.6 : 31.5 at 77, 51.7 : 80.6 at 200; 2048 x 6144 13.4 : 30.1 at 33; 2048 x 2048 8.6 : 11.0 at 33; 1536 x 1088 11.1 : 10.0 at 256,
   // 12.3 : 16.3 at 500.
   const bool codes8 = d->bits == 8 && d->M > 32 && (d->K >= 1536 || (uint64_t)d->M * d->N * d->K > 600000000ull) && d->affine && !d->out_f32 && aligned(y, 16);
   if (d->M > 16 && (d->bits == 4 || codes8) && ztvm::gemm_ta_supported((int)d->bits, d->group, d->K) && !ctx->no_gemm) {
@@ -665,14 +665,15 @@ static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::Ge
   const int tiles = ctx->moe_tiles_sm ? (sm_ok ? 3 : ta_ok ? 1 : 0) : (ta_ok ? 1 : sm_ok ? 3 : 0);
   const bool stream_ok = ztvm::moe_tc_supported(p, (int)d->bits) && !p.dst_index;
   // The tiles cost the same whatever the pair count (every expert's weights are dequantised once), the streaming kernel grows
-  // with the 8-pair chunks it walks. 257 experts, plan kept, us: gate / up, 512 x 2048: tiles 70, streaming 43 / 48 / 58 / 68
-  // at 4 / 6 / 8 / 10 pairs per expert; down, 2048 x 512: tiles 68, streaming 43 / 50 / 54 / 66 / 76 at 2 / 4 / 6 / 8 / 10. So they meet at ten
-  // and at eight pairs per expert. The line is at ten for all three projections of a block: below it they keep exact codes and f32 weights,
+  // with the 8-pair chunks it walks. 257 experts, plan kept, us: gate / up, 512 x 2048: tiles 65, streaming 44 / 49 / 58 / 68
+  // at 4 / 6 / 8 / 10 pairs per expert; down, 2048 x 512: tiles 65, streaming 44 / 50 / 55 / 65 / 76 at 2 / 4 / 6 / 8 / 10. So they meet at nearly ten
+  // and at eight pairs per expert (K of nine to eleven slices, whose warps idle: 40 experts of 2048 x 2304 41 : 60 at 4, 55 : 61 at 8, 60 : 60 at 10, of 2048 x 2816
+  // 56 : 73 at 8, 66 : 73 at 10). The line is at ten for all three projections of a block: below it they keep exact codes and f32 weights,
   // which the tiles round to f16, and one kernel, whose plan they share.
   const bool few_per_expert = pairs < 10ull * md->experts;
   // 3-bit codes stay exact at every pair count: streamed where that leaves at most a quarter of the sixteen warps without a slice and is the shorter way
-  // (moe3_streamed_less_batched), else on the batched kernel, whose tiles unpack a code for 16 pairs and more (70 : 69 us, streamed against it, for 257
-  // experts of 512 x 2048 at 10 pairs each; 51 : 45 for 40 of 2048 x 2304, nine slices). The projections of a block that share a plan all stream or none (54
+  // (moe3_streamed_less_batched), else on the batched kernel, whose tiles unpack a code for 16 pairs and more (70 : 68 us, streamed against it, for 257
+  // experts of 512 x 2048 at 10 pairs each; 53 : 44 for 40 of 2048 x 2304, nine slices, at eight). The projections of a block that share a plan all stream or none (54
   // experts, 1408 and 256 wide, 40 pairs, a plan for the down projection alone: 31 us a block became 36): the K of the others is taken to be this one's N.
   if (d->bits == 3) {
     auto fills = [](uint32_t k) { return k % 256u == 0 && k / 256u <= 16u && 16u / (k / 256u) * (k / 256u) >= 12u; };
@@ -687,7 +688,7 @@ static int moe_pick(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::Ge
     return streams ? 2 : ztvm::batch_moe_supported(p, 3) ? 4 : 0;
   }
   // A K that the streaming kernel does not take: the batched kernel, exact codes as well, holds its place (257 experts of 512 x
-  // 2240, us: 55 / 63 / 67 at 4 / 8 / 10 pairs per expert against 80 on the tiles).
+  // 2240, us: 56 / 64 at 4 / 8 pairs per expert against 77 on the tiles).
   if (forced < 0 && !stream_ok && few_per_expert && !p.dst_index && !p.seg_counts && ztvm::batch_moe_supported(p, 4)) return 4;
   if (forced == 1) return tiles ? tiles : stream_ok ? 2 : 0;
   if (forced == 2) return stream_ok ? 2 : tiles;
@@ -709,8 +710,8 @@ static ztvm::GemvParams moe_params(ztvm_ctx* ctx, const ztvm_moe_desc* md, void*
 }
 
 // The kernel ztvm_int4_matmul_moe runs a call on: one of moe_pick's grouped kernels, which read an expert-sorted plan, or 0
-// for the per-pair GEMV. Many pairs are sorted by expert: while an expert sees only a few of them the job is bound by
-// streaming each active expert's weights once, with many it is a real contraction.
+// for the per-pair GEMV. Many pairs are sorted by expert: while an expert sees only a few of them each active expert's weights are
+// unpacked once per eight (or sixteen) of them, with many it is a real contraction.
 // (3-bit codes, whose per-pair kernel is slow, from 32 pairs on; the exact-code grouped kernels of 4-bit ones from 64 on,
 // the tiles with f16 weights from 128 on.)
 static int moe_route(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::GemvParams& p, const void* y) {
@@ -719,12 +720,12 @@ static int moe_route(const ztvm_ctx* ctx, const ztvm_moe_desc* md, const ztvm::G
   if (ctx->moe_grouped >= 0) return ctx->moe_grouped ? moe_pick(ctx, md, p, y) : 0;
   const ztvm_mm_desc* d = &md->mm;
   if (pairs < (d->bits == 3 ? 32u : 64u)) return 0;
-  // A plan that no other call shares (5 to 8 us of its own, for one projection instead of a block's three) pays where the pairs
-  // are more, where they share experts, or where K is shorter than N, which the per-pair kernels are slow at. Per-pair against
-  // grouped with its plan, us: 4-bit, 257 experts of 512 x 2048: 12.5 : 18.9 at 64 pairs, 21.7 : 26.0 at 126, 29.8 : 28.6 at 160
-  // (64 experts 15.4 : 18.5 at 80, 21.8 : 20.4 at 126; 16 experts 12.2 : 11.5 at 64), of 2048 x 512: 24.7 : 23.4 at 64. 3-bit,
-  // 257 experts of 512 x 2048: 15.4 : 21.0 at 44, 24.2 : 21.4 at 80 (16 experts 15.5 : 15.4 at 44), of 1408 x 704: 14.8 : 17.3
-  // at 32, 19.4 : 19.7 at 44, of 2048 x 512: 19.8 : 14.6 at 32.
+  // A plan that no other call shares (5 to 8 us of its own, for one projection instead of a block's three) pays where the pairs are more, where they share
+  // experts, or where K is shorter than N. Per-pair against grouped with its plan, us: 4-bit, 257 experts of 512 x 2048: 12.7 : 16.0 at 64 pairs, 18.0 : 19.7 at
+  // 100, 22.1 : 20.9 at 126, 27.0 : 23.8 at 160 (64 experts 14.4 : 14.2 at 80, 21.1 : 16.1 at 126; 16 experts 11.8 : 9.5 at 64), of 2048 x 512 13.8 : 15.8 at
+  // 64. 3-bit, 257 experts of 512 x 2048: 12.4 : 12.7 at 32, 15.6 : 14.1 at 44, 20.1 : 15.5 at 64, 24.2 : 17.5 at 80 (16 experts 12.1 : 9.6 at 32, 14.6 : 9.6
+  // at 44), of 1408 x 704 14.4 : 14.8 at 32, 19.0 : 17.4 at 44, of 2048 x 512 19.6 : 13.1 at 32. (Drawn for slower grouped kernels and a slower 4-bit per-pair
+  // one over short K: today they meet at some 110 pairs, with 3-bit codes at 36, and with 4-bit ones over short K above 64.)
   if (!ctx->plan_reuse) {
     if (d->bits == 3) {
       if (pairs < (3ull * d->K <= d->N ? 32u : d->K < d->N ? 40u : 72u) && 2 * pairs < 5ull * md->experts) return 0;

@@ -34,8 +34,10 @@
 // Few tiles (short prompts, small N): the K range is split over a cluster of CTAs. Each CTA keeps the k blocks of its
 // share; at the end every CTA sends its f32 partial sums of token slice j to CTA j through distributed shared memory, and
 // each reduces and stores its own slice, in CTA order. The sums travel as whole 512-byte rows of a warp, into a place of their own where there is
-// room: a CTA then waits for the others to have started, not to have finished (stores 32 bytes apart into the idle rings, behind a barrier of the
-// whole cluster: 4096 x 4096, 128 rows 15.7 us, now 12.9; 200 rows 19.4, 15.1; 3072 x 8192, 128 rows 17.6, 14.7).
+// room: a CTA then waits for the others to have started, not to have finished (with biases, stores 32 bytes apart into the idle rings, behind a barrier of
+// the whole cluster: 4096 x 4096, 128 rows 15.7 us, now 12.5; 200 rows 19.3, 15.1; 3072 x 8192, 128 rows 19.3, 16.0). The exchange stays in the same instance as
+// launches without shares, which are up to 1 % slower for its code where K is some 1100: with instances of their own a pass that alternates fetches code anew
+// (41 rows of a layer 1280 wide 57.9 -> 61.1 us).
 #include "ztvm_kernels.h"
 #include "ztvm_stream_mma.cuh"
 #include "ztvm_tc.cuh"

@@ -111,7 +111,7 @@ gemv_tc_kernel(const GemvParams p) {
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(tc_smem) + (uint32_t)warp * (kTcDepth * kTile);
   float* partial = reinterpret_cast<float*>(tc_smem + (W * kTcDepth * kTile));            // [2][warps][kBlkRows][NT]
-  float* acc_sm = partial + 2 * W * kBlkRows * NT;                       // [nrows][M], only if num_kt > 1
+  float* acc_sm = partial + 2 * W * kBlkRows * NT;                       // [nrows][M], only if num_kt > 1 (ONCE: there, and unused)
 
   // ---- producer side: one (tile, slice) per step, issued kTcDepth - 1 steps ahead ----------------------------
   const uint32_t cp_row = (uint32_t)lane >> 3, cp_chunk = (uint32_t)lane & 7;   // codes: 4 rows x 8 chunks per pass

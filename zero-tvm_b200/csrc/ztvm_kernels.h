@@ -121,7 +121,7 @@ cudaError_t launch_moe_ta(const GemvParams& g, uint32_t tokens, uint32_t slots, 
                           int sm_count, cudaStream_t st, bool reuse_plan = false);
 constexpr uint32_t kMoeTaTileRows = 128, kMoeTcTileRows = 8;   // pairs per tile each kernel asks the plan for
 // Streaming form of the grouped MoE matmul (ztvm_moe_tc.cu) for launches where an expert sees only a few pairs: bound
-// by reading each active expert's weights once. Same scratch as launch_moe_grouped.
+// by issue slots, each active expert's weights unpacked once per eight of them. Same scratch as launch_moe_grouped.
 bool moe_tc_supported(const GemvParams& g, int bits);
 cudaError_t launch_moe_tc(const GemvParams& g, int bits, uint32_t tokens, uint32_t slots, uint32_t* scratch, int sm_count,
                           cudaStream_t st, bool reuse_plan = false);

@@ -399,7 +399,7 @@ moe_ta_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeTaParams p) {
     // 512 x 2048 77.0, 70.5). Phase 1: every thread stores its values as f16 into
     // stage[pair][weight row] (a warp's 32 lanes fill 64 consecutive bytes). Phase 2: a warp reads one pair's 512 bytes
     // (16 per lane) and stores them to the pair's output row in one instruction. The accumulators are free again as
-    // soon as the last 32 pairs have been read, before their rows have left.
+    // soon as all pairs have been read, before their rows have left.
     const int quarter = warp & 3;
     const uint32_t r_half = (uint32_t)(quarter * 32 + lane);
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;

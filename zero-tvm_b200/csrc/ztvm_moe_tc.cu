@@ -1,8 +1,8 @@
 // Grouped MoE expert matmul, streaming form, 4-bit and 3-bit codes: the contract of the ids-indirect GEMV
 //   y[token, slot, :] = x[token, slot, :] * W[ids[token, slot]]^T        (int4_matmul.gen.ts:229-254)
-// for token counts where an expert sees a handful of pairs (a few hundred tokens over 256 experts). There the job
-// is bound by reading every active expert's weights once, not by the multiplies, so it is built like the
-// persistent decode GEMV (ztvm_gemv_tc.cuh) rather than like the tensor-core tiles of ztvm_moe_gemm.cu:
+// for token counts where an expert sees a handful of pairs (a few hundred tokens over 256 experts). There every active
+// expert's weights are read and unpacked for a few products each, so it is built like the persistent decode GEMV
+// (ztvm_gemv_tc.cuh) rather than like the tensor-core tiles of ztvm_moe_gemm.cu:
 //   * the plan (ztvm_moe_plan.cuh) sorts the pairs by expert and cuts each expert's list into chunks of <= 8 pairs:
 //     a chunk is the 8 columns of an mma.sync.m16n8k16;
 //   * work unit = (chunk, 16 weight rows). The units, in chunk-major order, are split evenly over one CTA per SM;
@@ -14,7 +14,7 @@
 //     themselves (a barrier of their own), every third round;
 //   * which expert a chunk belongs to and where its pairs' rows lie is looked up once, at the start: with the chains of loads from the plan at
 //     every chunk and every meeting 257 experts of 2048 x 512 took 97.5 us at 8 pairs each, now 66; 512 x 2048 68, now 58.
-// What bounds it now are issue slots (58 % used): about 400 instructions per 4096 3-bit codes, half of them the unpacking.
+// What bounds it are issue slots (58 % used, DRAM at 25 to 38 %): about 400 instructions per 4096 3-bit codes, half of them the unpacking.
 // An expert with more than 8 pairs is streamed once per chunk (the repeats hit L2): the host side sends launches
 // with many pairs per expert to the tensor-core tiles instead.
 #include "ztvm_moe_plan.cuh"

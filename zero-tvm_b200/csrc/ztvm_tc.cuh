@@ -182,7 +182,7 @@ __host__ __device__ constexpr uint32_t idesc_f16(int n) {
 // both paths give the canonical bits, always; the fast one needs no f16 <-> f32 conversion at all (those run on the
 // quarter-rate conversion unit and used to bound every kernel that dequantises on the fly).
 struct DqGroup {
-  __half2 s2, b2;        // scale (small groups: 2^20 times it) and bias of the group in both halves
+  __half2 s2, b2;        // scale and bias of the group in both halves (2^20 times the scale, for small groups: dq_s20)
   float bf;              // the bias, widened (slow path)
   unsigned short s16;
   bool fast, small;
