@@ -203,8 +203,8 @@ batch_mma_kernel(const BatchParams p) {
 
   // 3-bit codes by permuted bytes (codes3_inplace16) or shifted to bit 0 first. Permuted, tiles of 16 pairs take 2 to 5 % less time on 85 of 102 shapes and up to
   // 9 % more on the others, all of 1.3 to 2.5 waves of CTAs (257 experts of 512 x 2048, 4 pairs each, 56.8 us shifted, 55.0; 33 of 1472 x 2816, 10 pairs, 37.1,
-  // 40.2); tiles of 64 over rows of whole 16-byte pieces 1.4 % less. With tiles of 32, and of 64 over other rows, it gained nothing on average and cost up to 10 %.
-  constexpr bool kShifted = BITS == 3 && (C::kTok == 32 || (C::kTok == 64 && !W16));
+  // 40.2); tiles of 64 take 1 % less. With tiles of 32 it gained nothing on average and cost up to 10 % (33 of 1472 x 2816, 14 pairs, 50.1, 55.1).
+  constexpr bool kShifted = BITS == 3 && C::kTok == 32;
   constexpr int RPW = RUNS / WK;
   static_assert(RPW >= 1 && RPW * WK == RUNS, "runs per warp");
   float acc[2][NBW][4];
