@@ -253,8 +253,10 @@ def run_reference_arm(args, rank, world):
         return
     shapes = workload_shapes(args.workload)
     cb = cpu_reference(shapes, max(1, args.steps), max(0, min(args.warmup, 2)))
-    if cb is None:      # oracle/_ref/ missing: the oracle's C restatement of the reference word order
-        cb = cpu_port(shapes, limit_s=20.0)
+    if cb is None:      # nothing of the reference's own code to time: a restatement of it is not the reference
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's code is not on this machine (oracle/_ref, made from a checkout of it), or it has "
+                                                             "no CPU code for this workload"}))
+        return
     v, unit = rate_of(cb, shapes)
     extra = {k: cb[k] for k in ("dequant_s", "matmul_s", "host_cores") if k in cb}
     print(json.dumps({

@@ -3,6 +3,7 @@ loads and exports every symbol the header declares (no compute without a GPU).""
 import ctypes
 import os
 import re
+import sys
 
 import numpy as np
 import pytest
@@ -288,3 +289,17 @@ def test_public_header_is_plain_c():
         r = subprocess.run(["gcc", "-std=c99", "-Wall", "-Wextra", "-pedantic", "-Werror", "-fsyntax-only",
                             "-I", os.path.join(root, "include"), src], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+def test_reference_arm_without_the_reference(monkeypatch, capsys):
+    """Without the reference's own code the reference arm of the benchmark says so; it times no restatement in its place."""
+    import importlib.util
+    import json
+    spec = importlib.util.spec_from_file_location("bench_under_test", os.path.join(ROOT, "bench.py"))
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    monkeypatch.setattr(bench, "cpu_reference", lambda *a: None)
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--steps", "1"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out.strip())
+    assert line["impl"] == "reference" and set(line) == {"impl", "unavailable"}
