@@ -19,6 +19,8 @@ pytestmark = pytest.mark.gpu
     (65, 1001, 2176, False), (77, 2176, 3072, False), (128, 392, 8192, True),                           # 128
     (129, 250, 4224, False), (200, 5000, 1152, False), (257, 9600, 640, False), (300, 2048, 4096, False),  # 256, one to many shares
     (273, 12200, 1088, False), (700, 6200, 2176, True), (1000, 5900, 320, False), (352, 130, 4160, False),  # up to 352
+    (65, 1696, 1152, False), (69, 1216, 1664, False), (390, 2338, 2112, False), (139, 1693, 2560, True), (130, 954, 4096, False),   # 128 in three and four
+    (266, 2088, 5312, False), (259, 1692, 7232, False), (258, 2140, 4992, True),    # shares, 256 in two, five and eight, up to 352 in five, six and eight
     (1000, 6100, 1088, False), (300, 1003, 4096, True), (350, 20011, 128, False), (50, 20000, 1664, False), (260, 19900, 640, False),  # whole waves and a rest
 ])
 def test_tiles_and_shares(group, affine, M, N, K, f32, backend, dev, oracle_c):
